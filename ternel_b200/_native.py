@@ -8,11 +8,12 @@ PyTorch path.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 from pathlib import Path
 from ctypes import c_char_p, c_int, c_int64, c_size_t, c_void_p, POINTER
 
-from .build import LIB_PATH
+from .build import BINDING_PATH, LIB_PATH
 
 TQ1_OK = 0
 TQ1_ERR_INVALID = -1
@@ -115,6 +116,25 @@ def lib() -> ctypes.CDLL:
             handle.tq1_debug_bounds.argtypes = [POINTER(ctypes.c_uint64)]
         _lib = handle
     return _lib
+
+
+_binding = None
+
+
+def binding():
+    """The eager call path (``_ternel_torch``, built from csrc/torch_binding.cpp), bound to the loaded library."""
+    global _binding
+    if _binding is None:
+        if not BINDING_PATH.exists():
+            raise NativeLibraryMissing(f"{BINDING_PATH} is missing: build it with `python -m ternel_b200.build`")
+        handle = lib()
+        spec = importlib.util.spec_from_file_location("_ternel_torch", BINDING_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.bind(*(ctypes.cast(getattr(handle, name), c_void_p).value for name in (
+            "tq1_linear_workspace_bytes", "tq1_linear_f16", "tq1_linear_swiglu_f16", "tq1_embedding_f16")))
+        _binding = module
+    return _binding
 
 
 def bounds_record() -> "tuple[int, int, int, int] | None":

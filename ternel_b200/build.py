@@ -1,10 +1,12 @@
-"""Compile the CUDA sources into the in-tree C-ABI shared library (sm_100a only)."""
+"""Compile the CUDA sources into the in-tree C-ABI shared library (sm_100a only), and the small C++ module through
+which eager PyTorch calls reach it."""
 
 from __future__ import annotations
 
 import os
 import shutil
 import subprocess
+import sysconfig
 from pathlib import Path
 
 PACKAGE_DIR = Path(__file__).resolve().parent
@@ -18,6 +20,9 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "-shared",
 ]
 
+
+BINDING_SOURCE = CSRC_DIR / "torch_binding.cpp"
+BINDING_PATH = LIB_DIR / "_ternel_torch.so"
 
 CHECKED_LIB_PATH = LIB_DIR / "libternel_b200_checked.so"
 # The checked build: every global store tests its index first and records a violation instead of writing
@@ -67,5 +72,31 @@ def build(force: bool = False, verbose: bool = False, target: Path = LIB_PATH, e
     return target
 
 
+def build_binding(force: bool = False) -> Path:
+    """Build ``_lib/_ternel_torch.so``, the eager call path, against the installed PyTorch (host code only)."""
+    header = PACKAGE_DIR.parent / "include" / "ternel_b200.h"
+    if not force and BINDING_PATH.exists() and all(
+            p.stat().st_mtime <= BINDING_PATH.stat().st_mtime for p in (BINDING_SOURCE, header)):
+        return BINDING_PATH
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    LIB_DIR.mkdir(exist_ok=True)
+    tmp = LIB_DIR / f".{BINDING_PATH.stem}.{os.getpid()}.so"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           "-isystem", str(root / "include"), "-isystem", str(root / "include/torch/csrc/api/include"),
+           "-isystem", str(cuda / "include"), "-isystem", sysconfig.get_paths()["include"],
+           str(BINDING_SOURCE), "-o", str(tmp), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu",
+           "-ltorch_cuda", "-lc10", "-lc10_cuda", f"-Wl,-rpath,{root / 'lib'}"]
+    done = subprocess.run(cmd, capture_output=True, text=True)
+    if done.returncode != 0:
+        tmp.unlink(missing_ok=True)
+        raise RuntimeError(f"g++ failed:\n{done.stdout}\n{done.stderr}")
+    os.replace(tmp, BINDING_PATH)
+    return BINDING_PATH
+
+
 if __name__ == "__main__":
     print(build(force=True, verbose=True))
+    print(build_binding(force=True))

@@ -22,7 +22,7 @@ from torch import nn
 
 from .format import BLOCK_BYTES, FormatError, validate_blocks
 from .layout import CODES_SUFFIX, SCALES_SUFFIX, PackedTensorLayout, unpack_blocks, validate_packed_codes
-from .ops import tq1_get_rows, tq1_matmul, validate_device_blocks
+from .ops import eager_embedding, eager_linear, tq1_get_rows, tq1_matmul, validate_device_blocks
 
 
 def packed_matmul(blocks: torch.Tensor, x: torch.Tensor, *, layout: PackedTensorLayout,
@@ -31,6 +31,10 @@ def packed_matmul(blocks: torch.Tensor, x: torch.Tensor, *, layout: PackedTensor
     if x.shape[-1] != layout.columns:
         raise FormatError(
             f"activation has {x.shape[-1]} columns, weight expects {layout.columns}")
+    if blocks.shape[0] == layout.rows:
+        out = eager_linear(blocks, x, out_dtype, False, False)
+        if out is not None:
+            return out
     flat = x.reshape(-1, layout.columns)
     out = tq1_matmul(blocks, flat, out_dtype=out_dtype)
     return out.reshape(*x.shape[:-1], layout.rows)
@@ -146,6 +150,9 @@ class PackedEmbedding(_PackedBase):
 
     def forward(self, indices: torch.Tensor) -> torch.Tensor:
         """Gather rows for ``indices`` of any shape and integer dtype, as ``nn.Embedding`` does."""
+        out = eager_embedding(self.blocks, indices, self.dtype, False)
+        if out is not None:
+            return out
         flat = indices.reshape(-1)
         rows = tq1_get_rows(self.blocks, flat, dtype=self.dtype)
         return rows.reshape(*indices.shape, self.layout.columns)

@@ -7,6 +7,10 @@ work happens in ``libternel_b200.so``. The ops are registered for the CUDA
 dispatch key alone, so a CPU tensor is refused by the dispatcher instead of
 being served by some other path.
 
+Eager calls do not pass through the dispatcher: the wrappers first offer the call to
+the C function of csrc/torch_binding.cpp, which takes the plain case in one step and
+declines everything else (wrong arguments, gradients, tensor subclasses, tracing).
+
 The Python wrappers below (`tq1_matmul`, `tq1_gemm`, `tq1_get_rows`) keep the
 names and the pre-launch checks of the reference's kernel wrappers
 (src/ternel_mlx/kernels.py:1191-1284,1360-1398).
@@ -45,6 +49,7 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor | None:
     if buf is None or buf.numel() < nbytes:
         buf = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)   # slots start at zero
         _workspaces[index] = buf
+        _native.binding().set_workspace(index, buf.data_ptr(), buf.numel())
     return buf
 
 
@@ -159,6 +164,36 @@ def _(blocks):
     return blocks.new_empty(2, dtype=torch.int64)
 
 
+def eager_linear(blocks, x, out_dtype, swiglu: bool, flat: bool):
+    """The product through the eager call path, or None where that path does not apply. ``flat``: ``x`` must be
+    two-dimensional; otherwise its leading dimensions carry over to the result."""
+    if torch.compiler.is_compiling():
+        return None
+    return (_fast or _load_fast()).linear(blocks, x, out_dtype, swiglu, flat)
+
+
+def eager_embedding(blocks, ids, dtype, flat: bool):
+    """The row gather through the eager call path, or None where that path does not apply."""
+    if torch.compiler.is_compiling():
+        return None
+    return (_fast or _load_fast()).embedding(blocks, ids, dtype, flat)
+
+
+_fast = None
+
+
+class _NoFastPath:
+    """Stands in where there is no GPU: every call is left to the ordinary path, which says so."""
+
+    linear = embedding = staticmethod(lambda *args: None)
+
+
+def _load_fast():
+    global _fast
+    _fast = _native.binding() if torch.cuda.is_available() else _NoFastPath
+    return _fast
+
+
 def _require_cuda(tensor: torch.Tensor, name: str) -> None:
     if not tensor.is_cuda:
         raise RuntimeError(
@@ -196,6 +231,9 @@ def tq1_matmul(blocks: torch.Tensor, x: torch.Tensor, *, out_dtype: torch.dtype 
     The kernel (streaming GEMV, small-batch split-K, or tiled GEMM) is chosen
     inside the library from the batch size.
     """
+    out = eager_linear(blocks, x, out_dtype, False, True)
+    if out is not None:
+        return out
     _, groups = _check_blocks(blocks)
     _check_activations(x, groups)
     out_dtype = out_dtype or x.dtype
@@ -212,6 +250,9 @@ def tq1_swiglu(blocks: torch.Tensor, x: torch.Tensor, *, out_dtype: torch.dtype 
     """``silu(x @ Wg.T) * (x @ Wu.T)`` in one call, for ``blocks`` holding the gate and up rows interleaved
     (row ``2i`` = gate row ``i``, row ``2i + 1`` = up row ``i``; see ``interleave_gate_up``). Dot products and
     the activation are FP32, with one narrowing at the store. Result ``(batch, rows / 2)``."""
+    out = eager_linear(blocks, x, out_dtype, True, True)
+    if out is not None:
+        return out
     rows, groups = _check_blocks(blocks)
     if rows % 2:
         raise FormatError(f"{rows} rows cannot be (gate, up) pairs")
@@ -242,6 +283,9 @@ tq1_gemm = tq1_matmul
 
 def tq1_get_rows(blocks: torch.Tensor, indices: torch.Tensor, *, dtype: torch.dtype = torch.float16) -> torch.Tensor:
     """Decode the rows named by 1-D ``indices``; an id outside ``[0, rows)`` gives a zero row."""
+    out = eager_embedding(blocks, indices, dtype, True)
+    if out is not None:
+        return out
     _check_blocks(blocks)
     if dtype not in OUTPUT_DTYPES:
         raise FormatError(f"output dtype must be one of {OUTPUT_DTYPES}, got {dtype}")

@@ -1,0 +1,63 @@
+"""The eager call path (csrc/torch_binding.cpp) against the dispatcher's: same bytes out, and everything that is
+not the plain case declined. Needs a B200."""
+
+import numpy as np
+import pytest
+import torch
+
+from tests.gpu_util import random_blocks
+
+pytestmark = pytest.mark.gpu
+
+
+def _setup(rows=48, columns=640, batch=3):
+    packed, rng = random_blocks(rows, columns, rows + columns)
+    blocks = torch.from_numpy(packed).cuda()
+    return blocks, torch.from_numpy(rng.standard_normal((batch, columns)).astype(np.float16)).cuda()
+
+
+@pytest.mark.parametrize("rows,columns", [(1, 512), (48, 640), (1000, 1536)])
+@pytest.mark.parametrize("lead", [(), (1,), (3,), (2, 17)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_same_bytes_as_the_dispatcher(rows, columns, lead, dtype):
+    from ternel_b200.layout import PackedTensorLayout
+    from ternel_b200.modules import packed_matmul
+    from ternel_b200.ops import eager_embedding, eager_linear, tq1_get_rows
+    blocks, _ = _setup(rows, columns)
+    x = torch.randn((*lead, columns), device="cuda").half()
+    got = packed_matmul(blocks, x, layout=PackedTensorLayout.for_tensor(rows, columns), out_dtype=dtype)
+    want = torch.ops.ternel.tq1_linear(blocks, x.reshape(-1, columns), dtype == torch.float32)
+    assert got.shape == (*lead, rows) and got.dtype == dtype
+    assert torch.equal(got.reshape(-1, rows), want)
+    assert torch.equal(eager_linear(blocks, x, dtype, False, False), got)         # the workspace has grown: taken here
+    if rows % 2 == 0 and columns % 512 == 0:
+        want = torch.ops.ternel.tq1_linear_swiglu(blocks, x.reshape(-1, columns), dtype == torch.float32)
+        assert torch.equal(eager_linear(blocks, x, dtype, True, False).reshape(-1, rows // 2), want)
+    ids = torch.randint(-1, rows + 1, (*lead, 5), device="cuda")
+    assert torch.equal(eager_embedding(blocks, ids, dtype, False).reshape(-1, columns),
+                       torch.ops.ternel.tq1_embedding(blocks, ids.reshape(-1), dtype == torch.float32))
+    assert tq1_get_rows(blocks, ids.reshape(-1).int(), dtype=dtype).shape == (ids.numel(), columns)
+
+
+def test_declines_what_is_not_the_plain_case():
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from ternel_b200.ops import eager_embedding, eager_linear, tq1_matmul
+    blocks, x = _setup()
+    tq1_matmul(blocks, x)
+    ids = torch.zeros(3, dtype=torch.int64, device="cuda")
+    assert eager_linear(blocks, x, None, False, False) is not None
+    for b, v, dtype, swiglu, flat in (
+            (blocks, x.float(), None, False, False), (blocks, x.cpu(), None, False, False),
+            (blocks.cpu(), x, None, False, False), (blocks[:, :, :27], x, None, False, False),
+            (blocks[:, 1:], x, None, False, False), (blocks, x[:, 128:], None, False, False),
+            (blocks, x[:, ::2], None, False, False), (blocks, x[0], None, False, True), (blocks, x[:0], None, False, False),
+            (blocks, x, torch.bfloat16, False, False), (blocks, x, "f16", False, False), (None, x, None, False, False),
+            (blocks, x.clone().requires_grad_(), None, False, False), (blocks[:47].contiguous(), x, None, True, False)):
+        assert eager_linear(b, v, dtype, swiglu, flat) is None
+    for i, flat in ((ids.int(), True), (ids.cpu(), True), (ids[:0], True), (ids[None], True), (ids.float(), True)):
+        assert eager_embedding(blocks, i, torch.float16, flat) is None
+    assert eager_embedding(blocks, ids, torch.bfloat16, True) is None
+    with FakeTensorMode() as mode:
+        fake = mode.from_tensor(x)
+        assert eager_linear(mode.from_tensor(blocks), fake, None, False, False) is None
+        assert tq1_matmul(mode.from_tensor(blocks), fake).shape == (3, 48)
