@@ -24,8 +24,12 @@
 // fixed point (23 bits below the group's maximum, as exact as FP32 accumulation) split into
 // four signed byte planes; s32 accumulators give 81 * (group sum) modulo 2^32, a multiplication
 // by 81^-1 (mod 2^32) recovers the integer, then acc = fma(scale_g, 2^(E-21) * sum, acc) in
-// FP32 as in src/bonsai_tq1/reference.py:33-38. Groups holding NaN/Inf activations take an
-// FP32 path that multiplies every weight, so non-finite values propagate as in the reference.
+// FP32 as in src/bonsai_tq1/reference.py:33-38. In a group holding NaN/Inf activations the reference
+// multiplies every weight, so 0 * Inf, Inf - Inf and NaN give NaN, and the sum is +-Inf only if all of the
+// group's n infinite products have one sign. Such a group's fixed-point activations are the signs of its
+// infinities (0 elsewhere): the same integer dot product then is +n, -n, or anything else for NaN. (A separate
+// FP32 pass over the group's weights, the earlier form, made a launch five times slower once a value overflowed:
+// eight decoder layers 1305 us against 260 us.)
 //
 // Work decomposition per link: a unit is 16 rows x 4 groups (1792 bytes, one TMA box); units
 // are numbered chunk-major (a chunk = 512 columns) and dealt out in contiguous ranges to the
@@ -75,7 +79,8 @@ constexpr int kRegsPerSub = 18;                                // A/B registers 
 static_assert(kWarps >= kPrepWarps, "one warp per activation group of the CTA's chunks");
 
 // Per activation group, written by the warp that prepared it: 121 * (sum of the fifth-trit activations),
-// 2^(E-21) for the group's exponent E, and whether the group holds NaN/Inf.
+// 2^(E-21) for the group's exponent E, and how many of its activations are Inf (kGroupNan: one is NaN).
+constexpr int kGroupNan = 1 << 30;
 struct alignas(16) GroupConst {
     int sum;
     float pow;
@@ -339,31 +344,6 @@ __device__ __forceinline__ float word_value(unsigned long long w, bool f32) {
 // A sum of partial sums becomes the activation the next link reads by one rounding to FP16.
 __device__ __forceinline__ float round_to_half(float v) { return __half2float(__float2half_rn(v)); }
 
-// Activation `idx` of a link, whichever form it arrives in (the hand-off words have been waited for).
-__device__ float link_x(const ChainLinkDev &L, size_t idx) {
-    if (L.x) return __half2float(L.x[idx]);
-    const bool f32 = (L.flags & kFlagSrcF32) != 0;
-    const int parts = max(1, (int)((L.flags >> kFlagSrcPartsShift) & 15u));
-    float sum = 0.0f;
-    for (int r = 0; r < parts; ++r) sum += word_value(word_read(L.xin + (size_t)r * L.src_stride + idx), f32);
-    return f32 ? round_to_half(sum) : sum;
-}
-// FP32 fallback for one block (row-major canonical bytes in shared memory): multiplies every
-// weight so that NaN and Inf propagate exactly as in the reference.
-__device__ float block_dot_fp32(const uint8_t *blk, const ChainLinkDev &L, size_t x0) {
-    float sum = 0.0f;
-    for (int j = 0; j < kCodeBytes; ++j) {
-        uint32_t v = blk[2 + j];
-        const int n = j == 25 ? 3 : 5;
-        for (int i = 0; i < n; ++i) {
-            const float w = (float)((int)(v % 3u) - 1);
-            v /= 3u;
-            sum = fmaf(w, link_x(L, x0 + 5 * j + i), sum);
-        }
-    }
-    return sum;
-}
-
 // Units of a link that one warp of one CTA processes (units are numbered chunk-major).
 struct WarpRange {
     int u_begin, n_units, c_first, t_first;
@@ -407,7 +387,6 @@ template <bool ALL_PANELS>
 __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __grid_constant__ ChainParams P) {
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t window = (uint32_t)__cvta_generic_to_shared(smem);
-    unsigned char *ring = smem;
     unsigned char *high = smem + (kWindowEnd - window);
     uint32_t *btab_all = reinterpret_cast<uint32_t *>(high);
     uint64_t *mbars = reinterpret_cast<uint64_t *>(high + kBtabBytes);
@@ -639,7 +618,18 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
                 mbits = max(mbits, bad[k] ? 0u : __float_as_uint(a));
             }
             mbits = __reduce_max_sync(0xffffffffu, mbits);
-            const int group_bad = __any_sync(0xffffffffu, anybad);
+            int group_bad = __any_sync(0xffffffffu, anybad);           // infinite activations, or kGroupNan
+            if (group_bad) {
+                int infs = 0;
+                bool nan = false;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    infs += bad[k] ? 1 : 0;
+                    nan = nan || xv[k] != xv[k];
+                }
+                infs = __reduce_add_sync(0xffffffffu, infs);
+                group_bad = __any_sync(0xffffffffu, nan) ? kGroupNan : infs;
+            }
             // 2^E <= m < 2^(E+1); fixed point xi = round(v * 2^(21-E)), |xi| <= 2^22
             const int e_biased = mbits != 0u ? (int)(mbits >> 23) : 127;
             const float up = __uint_as_float((uint32_t)(275 - e_biased) << 23);                // 2^(21-E)
@@ -647,7 +637,7 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
             uint32_t ent[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                xi[k] = bad[k] ? 0 : __float2int_rn(xv[k] * up);
+                xi[k] = group_bad ? (bad[k] ? (xv[k] < 0.0f ? -1 : 1) : 0) : __float2int_rn(xv[k] * up);
                 xchg[lane + 32 * k] = xi[k];                       // a code byte's first four trits need its fifth
                 ent[k] = preptab[lane + 32 * k];
                 s5 += (ent[k] >> 24) == 0u ? 121 * xi[k] : 0;      // 121 * sum of the fifth-trit activations
@@ -753,8 +743,8 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
             }
             const int seg = min(left, tiles - t);       // units of this chunk
             left -= seg;
-            // One unit. BAD: some group of the chunk holds NaN/Inf activations and takes the FP32 path (rare; kept out
-            // of the common loop so that it costs the common loop neither branches nor registers).
+            // One unit. BAD: some group of the chunk holds NaN/Inf activations (rare; kept out of the common loop so that
+            // it costs the common loop neither branches nor registers).
             auto unit = [&](auto bad_tag) {
                 constexpr bool BAD = decltype(bad_tag)::value;
                 const uint32_t bar = bar0 + 8u * cstage;
@@ -803,12 +793,10 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
                     float dot1 = (float)s1 * gpow[sub];
                     float dot2 = (float)s2 * gpow[sub];
                     if (BAD) {
-                        if (h == 0 && gbad[sub]) {
-                            const int group = sub + 2 * cls;
-                            const unsigned char *tile = ring + (warp * kStages + cstage) * kUnitBytes;
-                            const size_t x0 = ((size_t)c * kChunkGroups + group) * kGroup;
-                            dot1 = block_dot_fp32(tile + (g * kChunkGroups + group) * kBlockBytes, L, x0);
-                            dot2 = block_dot_fp32(tile + ((g + 8) * kChunkGroups + group) * kBlockBytes, L, x0);
+                        if (gbad[sub]) {
+                            const float inf = __int_as_float(0x7f800000), nan = __int_as_float(0x7fffffff);
+                            dot1 = s1 == gbad[sub] ? inf : s1 == -gbad[sub] ? -inf : nan;
+                            dot2 = s2 == gbad[sub] ? inf : s2 == -gbad[sub] ? -inf : nan;
                         }
                     }
                     const float sc1 = __half2float(__ushort_as_half((unsigned short)(w1a & 0xffffu)));

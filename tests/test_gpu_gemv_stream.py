@@ -162,3 +162,27 @@ def test_very_tall_matrix_runs_as_row_ranges():
     got = run_linear(blocks, x)
     assert got.shape == (1, rows)
     assert o.normalised_error(got, want) < 1e-5
+
+
+@pytest.mark.parametrize("batch", (1, 2))
+@pytest.mark.parametrize("infinite", (1, 2, 3, 128))
+def test_infinite_products_of_a_group(infinite, batch):
+    """A group's sum is +-Inf when all its infinite products have one sign, NaN otherwise (0 * Inf, Inf - Inf or a
+    NaN activation): every count and sign of infinities, in one group and in two, against the reference order."""
+    rows, columns = 200, 1024
+    blocks, rng = random_blocks(rows, columns, seed=41 + infinite, dist="tests")
+    for groups in ((0,), (5,), (2, 7)):
+        for with_nan in (False, True):
+            x = rng.standard_normal((batch, columns)).astype(np.float16)
+            for m in range(batch):
+                for grp in groups:
+                    at = 128 * grp + rng.permutation(128)[:infinite]
+                    x[m, at] = np.where(rng.integers(0, 2, infinite) > 0, np.inf, -np.inf) if infinite < 128 else np.inf
+                if with_nan:
+                    x[m, 128 * groups[0] + 127] = np.nan
+            with np.errstate(invalid="ignore"):
+                want = o.reference_matmul(blocks, x.astype(np.float32), rows=rows, columns=columns)
+            got = run_linear(blocks, x)
+            assert np.array_equal(o.nonfinite_classes(got), o.nonfinite_classes(want))
+            if infinite == 1 and not with_nan and len(groups) == 1:
+                assert np.isinf(got).any() and np.isnan(got).any()
