@@ -88,6 +88,15 @@ int tq1_untile_blocks(const uint8_t *codes, const uint16_t *scales, uint8_t *blo
 int tq1_validate_blocks_device(const uint8_t *blocks_dev, int64_t groups,
                                int64_t *counts_dev, void *stream);
 
+/* The tiled pair on the device (codes [rows/tile][gpr][26][tile], scales [rows/tile][gpr][tile], tile divides rows):
+ * a count of the code bytes above their limits (counts_dev: int64[2], full and tail slots), and the conversion to
+ * canonical blocks. Together they are validate_packed_codes + unpack_blocks (src/ternel_mlx/packing.py:29-82) for
+ * arrays that have been uploaded as they are. */
+int tq1_validate_codes_device(const uint8_t *codes_dev, int64_t rows, int64_t gpr, int64_t tile, int64_t *counts_dev,
+                              void *stream);
+int tq1_untile_blocks_device(const uint8_t *codes_dev, const uint16_t *scales_dev, uint8_t *blocks_dev, int64_t rows,
+                             int64_t gpr, int64_t tile, void *stream);
+
 /* Scratch the linear entry point needs for this shape (0 when none). The
  * caller owns the buffer, as the caller of launch_tq1_lut23_smem_streamk owns
  * its workspace (cuda/tq1_lut23_streamk.cu:320-367, lut23_workspace_bytes). */

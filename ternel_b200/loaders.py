@@ -413,9 +413,8 @@ def write_safetensors(path, arrays: dict[str, np.ndarray], metadata: dict | None
             handle.write(data)
 
 
-def load_packed_pair(file: SafetensorsFile, module_path: str, layout: PackedTensorLayout) -> np.ndarray:
-    """Canonical blocks from the ``<module_path>.codes`` / ``.scales`` pair of a converted checkpoint,
-    with the shape checks and the byte scan of the reference loader (src/ternel_mlx/packing.py:29-82)."""
+def _read_packed_pair(file: SafetensorsFile, module_path: str, layout: PackedTensorLayout) -> tuple[np.ndarray, np.ndarray]:
+    """The ``<module_path>.codes`` / ``.scales`` arrays of a converted checkpoint, of the layout's shapes."""
     codes = file.read(f"{module_path}.codes")
     scales = file.read(f"{module_path}.scales")
     if codes.dtype != np.uint8 or tuple(codes.shape) != layout.codes_shape:
@@ -423,8 +422,15 @@ def load_packed_pair(file: SafetensorsFile, module_path: str, layout: PackedTens
     if scales.dtype.itemsize != 2 or tuple(scales.shape) != layout.scales_shape:
         raise FormatError(
             f"{module_path}.scales: expected uint16 {layout.scales_shape}, got {scales.dtype} {scales.shape}")
+    return codes, scales.view("<u2")
+
+
+def load_packed_pair(file: SafetensorsFile, module_path: str, layout: PackedTensorLayout) -> np.ndarray:
+    """Canonical blocks from the ``<module_path>.codes`` / ``.scales`` pair of a converted checkpoint,
+    with the shape checks and the byte scan of the reference loader (src/ternel_mlx/packing.py:29-82)."""
+    codes, scales = _read_packed_pair(file, module_path, layout)
     validate_packed_codes(codes)
-    return unpack_blocks(codes, scales.view("<u2"), layout=layout)
+    return unpack_blocks(codes, scales, layout=layout)
 
 
 def load_packed_model(model, file: SafetensorsFile, *, strict: bool = True) -> dict[str, int]:
@@ -442,7 +448,6 @@ def load_packed_model(model, file: SafetensorsFile, *, strict: bool = True) -> d
                 raise FormatError(f"checkpoint has no codes/scales pair for {path}")
             missing += 1
             continue
-        module.load_blocks(load_packed_pair(file, path, module.layout), validate=False)
-        module._validated = True
+        module.load_tiled(*_read_packed_pair(file, path, module.layout))
         loaded += 1
     return {"loaded": loaded, "missing": missing}

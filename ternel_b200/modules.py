@@ -22,7 +22,7 @@ from torch import nn
 
 from .format import BLOCK_BYTES, FormatError, validate_blocks
 from .layout import CODES_SUFFIX, SCALES_SUFFIX, PackedTensorLayout, unpack_blocks, validate_packed_codes
-from .ops import eager_embedding, eager_linear, tq1_get_rows, tq1_matmul, validate_device_blocks
+from .ops import eager_embedding, eager_linear, load_tiled_device, tq1_get_rows, tq1_matmul, validate_device_blocks
 
 
 def packed_matmul(blocks: torch.Tensor, x: torch.Tensor, *, layout: PackedTensorLayout,
@@ -38,6 +38,16 @@ def packed_matmul(blocks: torch.Tensor, x: torch.Tensor, *, layout: PackedTensor
     flat = x.reshape(-1, layout.columns)
     out = tq1_matmul(blocks, flat, out_dtype=out_dtype)
     return out.reshape(*x.shape[:-1], layout.rows)
+
+
+def _tensor_of(array) -> "torch.Tensor | None":
+    """A tensor over ``array``'s memory, or None where PyTorch cannot stand over it (byte order, read-only memory)."""
+    if isinstance(array, torch.Tensor):
+        return array
+    array = np.asarray(array)
+    if not array.dtype.isnative or not array.flags.writeable or array.dtype not in (np.uint8, np.uint16, np.int16):
+        return None
+    return torch.from_numpy(np.ascontiguousarray(array))
 
 
 class _PackedBase(nn.Module):
@@ -74,7 +84,17 @@ class _PackedBase(nn.Module):
         self._validated = validate
 
     def load_tiled(self, codes, scales) -> None:
-        """Install the reference's tiled ``codes`` / ``scales`` pair."""
+        """Install the reference's tiled ``codes`` / ``scales`` pair. A module on the GPU takes well-formed arrays as
+        they are and scans and converts them there; anything else goes through the host converter and its checks."""
+        if self.blocks.is_cuda and self.blocks.is_contiguous():
+            device_codes, device_scales = _tensor_of(codes), _tensor_of(scales)
+            if (device_codes is not None and device_codes.dtype == torch.uint8
+                    and device_codes.shape == self.layout.codes_shape
+                    and device_scales is not None and device_scales.dtype in (torch.int16, torch.uint16)
+                    and device_scales.shape == self.layout.scales_shape):
+                load_tiled_device(self.blocks, device_codes, device_scales, self.layout.tile)
+                self._validated = True
+                return
         code_array = codes.cpu().numpy() if isinstance(codes, torch.Tensor) else np.asarray(codes)
         scale_array = scales.cpu().numpy() if isinstance(scales, torch.Tensor) else np.asarray(scales)
         if scale_array.dtype == np.int16:      # torch has no first-class uint16 storage

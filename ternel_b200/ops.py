@@ -24,6 +24,7 @@ import torch
 
 from . import _native
 from .format import BLOCK_BYTES, BLOCK_SIZE, FormatError, check
+from .layout import out_of_range_message
 
 ACTIVATION_DTYPES = (torch.float16,)
 OUTPUT_DTYPES = (torch.float16, torch.float32)
@@ -208,6 +209,24 @@ def validate_device_blocks(blocks: torch.Tensor) -> None:
     bad_full, bad_tail = (int(v) for v in _tq1_validate_op(blocks).tolist())
     if bad_full or bad_tail:
         raise FormatError(f"invalid base-3 bytes: regular={bad_full}, tail={bad_tail}")
+
+
+def load_tiled_device(blocks: torch.Tensor, codes: torch.Tensor, scales: torch.Tensor, tile: int) -> None:
+    """Fill canonical ``blocks`` on the GPU from the tiled pair (``uint8[tiles, groups, 26, tile]`` and 16-bit
+    ``[tiles, groups, tile]``, on the host or the GPU): the arrays are uploaded as they are, scanned there, and
+    converted only if every byte is legal (fail closed, as ``validate_packed_codes``)."""
+    rows, groups = _check_blocks(blocks)
+    codes = codes.to(blocks.device).contiguous()
+    scales = scales.to(blocks.device).contiguous()
+    counts = torch.empty(2, dtype=torch.int64, device=blocks.device)
+    lib, stream = _native.lib(), _stream_ptr(blocks.device)
+    with torch.cuda.device(blocks.device):
+        check(lib.tq1_validate_codes_device(codes.data_ptr(), rows, groups, tile, counts.data_ptr(), stream))
+        bad_full, bad_tail = counts.tolist()
+        if bad_full or bad_tail:
+            raise FormatError(out_of_range_message(bad_full, bad_tail))
+        check(lib.tq1_untile_blocks_device(codes.data_ptr(), scales.data_ptr(), blocks.data_ptr(), rows, groups, tile,
+                                           stream))
 
 
 def _check_activations(x: torch.Tensor, groups_per_row: int) -> int:

@@ -13,6 +13,7 @@ import torch
 from oracle import tq1_oracle as o
 from ternel_b200 import loaders
 from tests.conftest import GOLDEN
+from tests.gpu_util import random_blocks
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +45,24 @@ def test_lut23_sidecar_tensors_run_on_the_gpu():
     _, manifest = loaders.read_lut23_sidecar(GOLDEN / "sidecar_small.lut23")
     for name in NAMES:
         _run(loaders.load_lut23_tensor(GOLDEN / "sidecar_small.lut23", manifest, name), name)
+
+
+@pytest.mark.parametrize("rows,columns", [(1, 128), (48, 5120), (100, 640), (256, 128), (768, 1408)])
+def test_tiled_pair_is_converted_on_the_gpu(rows, columns):
+    """One tile or several, rows that fill no thread block: the same blocks as the host converter's; an illegal byte
+    in any slot is counted and leaves the module as it was."""
+    from ternel_b200.format import FormatError
+    from ternel_b200.layout import PackedTensorLayout, pack_blocks
+    from ternel_b200.modules import PackedLinear
+    layout = PackedTensorLayout.for_tensor(rows, columns)
+    blocks, _ = random_blocks(rows, columns, seed=rows)
+    codes, scales = pack_blocks(blocks, layout=layout)
+    module = PackedLinear(layout, device="cuda")
+    module.load_tiled(codes, scales)
+    assert np.array_equal(module.blocks.cpu().numpy(), blocks)
+    module.load_tiled(torch.from_numpy(codes), torch.from_numpy(scales.view(np.int16)).cuda())
+    assert np.array_equal(module.blocks.cpu().numpy(), blocks)
+    codes[0, 0, 0, 0], codes[-1, -1, 24, -1], codes[-1, -1, 25, 0] = 243, 255, 27
+    with pytest.raises(FormatError, match=r"regular=2 \(max 242\), tail=1 \(max 26\)"):
+        module.load_tiled(codes, np.zeros_like(scales))
+    assert np.array_equal(module.blocks.cpu().numpy(), blocks)

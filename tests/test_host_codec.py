@@ -217,3 +217,27 @@ def test_dequantize_blocks_is_the_decoded_trits_times_the_scale():
     want = (trits.astype(np.float32) - 1.0) * scales.astype(np.float32)[:, None]
     assert got.dtype == np.float32 and got.shape == (groups, 128)
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+def test_parts_of_several_threads_agree_with_one():
+    """Sizes around the codec's part size (8192 groups a thread): every group of every part, and bad codes in the
+    first and last of them."""
+    rng = np.random.default_rng(5)
+    for count in (8191, 16384, 40961):
+        codes = rng.integers(0, 3, (count, 128), dtype=np.uint8)
+        scales = rng.integers(0, 256, (count, 2), dtype=np.uint8)
+        packed = tb.encode_tq1_blocks(scales, codes)
+        digits = codes[:, :125].reshape(count, 25, 5).astype(np.int64) @ (3 ** np.arange(5))
+        tail = codes[:, 125:].astype(np.int64) @ (3 ** np.arange(3))
+        assert np.array_equal(packed[:, :2], scales)
+        assert np.array_equal(packed[:, 2:27], digits) and np.array_equal(packed[:, 27], tail)
+        got_scales, got_codes = tb.decode_tq1_blocks(packed)
+        assert np.array_equal(got_scales, scales) and np.array_equal(got_codes, codes)
+        for value in (3, 4, 128, 255):
+            broken = codes.copy()
+            broken[0, 0] = broken[-1, 127] = value
+            with pytest.raises(tb.FormatError, match=r"2 non-ternary"):
+                tb.encode_tq1_blocks(scales, broken)
+        packed[0, 2], packed[-1, 27] = 243, 27
+        with pytest.raises(tb.FormatError, match="regular=1, tail=1"):
+            tb.decode_tq1_blocks(packed)
