@@ -11,7 +11,8 @@ extern "C" {
 size_t tq1_linear_workspace_bytes(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0 || K % kGroup) return 0;
     if (M == 1 && gemv_chain_shape_ok(N, K)) return gemv_chain_workspace_bytes(N, K);
-    if (gemm_tc_shape_ok(M, N, K)) return gemm_tc_workspace_bytes(M, N, K);
+    // blocks that turn out not to be 16-byte aligned may take the kernel for fewer shapes, never for more
+    if (gemm_tc_preferred(true, M, N, K)) return gemm_tc_workspace_bytes(M, N, K);
     return 0;
 }
 
@@ -36,7 +37,7 @@ int tq1_linear_f16(const uint8_t *blocks, const void *x, void *y, int y_is_f32,
                                   kWsSlotRegionBytes, s);
     if (gemv_looped_fits(blocks, M, N, K) && need >= kWsScratchOffset)
         return launch_gemv_looped(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, false, workspace, s);
-    if (gemm_tc_supported(blocks, static_cast<const __half *>(x), M, N, K))
+    if (gemm_tc_preferred((reinterpret_cast<uintptr_t>(blocks) & 15) == 0, M, N, K))
         return launch_gemm_tc(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, workspace, s);
     return launch_gemv_rows(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, s);
 }
@@ -52,7 +53,7 @@ int tq1_linear_swiglu_f16(const uint8_t *blocks, const void *x, void *y, int y_i
         return fail(TQ1_ERR_INVALID, "tq1_linear_swiglu_f16: x must be 16-byte aligned");
     const __half *xh = static_cast<const __half *>(x);
     const bool gemv = M == 1 && gemv_chain_fits(blocks, rows, K);
-    if (!gemv && !gemm_tc_supported(blocks, xh, M, rows, K))
+    if (!gemv && (M < 2 || K % 512 || (reinterpret_cast<uintptr_t>(blocks) & 15)))
         return fail(TQ1_ERR_INVALID,
                     "tq1_linear_swiglu_f16: needs K %% 512 == 0 and 16-byte aligned blocks (got %dx%d)", rows, K);
     const size_t need = tq1_linear_workspace_bytes(M, rows, K);
@@ -69,9 +70,9 @@ int tq1_linear_plan(int M, int N, int K, int aligned, int *kernel, int *token_ti
     if (!kernel || !token_tile || !ctas || !parts) return fail(TQ1_ERR_INVALID, "tq1_linear_plan: null pointer");
     if (M <= 0 || N <= 0 || K <= 0 || K % kGroup) return fail(TQ1_ERR_INVALID, "tq1_linear_plan: bad shape");
     *token_tile = *ctas = *parts = 0;
-    if (M <= (gemv_loop_tokens() > 1 ? gemv_loop_tokens() : 1) && aligned && gemv_chain_shape_ok(N, K)) {
+    if ((M == 1 || gemv_loop_preferred(M, N, K)) && aligned && gemv_chain_shape_ok(N, K)) {
         *kernel = TQ1_KERNEL_STREAM_GEMV;       // M > 1: one launch of M passes of the batch-1 kernel
-    } else if (aligned && gemm_tc_shape_ok(M, N, K)) {
+    } else if (gemm_tc_preferred(aligned != 0, M, N, K)) {
         *kernel = TQ1_KERNEL_TENSOR_CORE;
         gemm_tc_plan(M, N, K, token_tile, ctas, parts);
     } else {

@@ -17,13 +17,15 @@ constexpr int kMaxFull = 242;
 constexpr int kMaxTail = 26;
 
 // Workspace layout shared by every linear kernel: [control words, 256 B][partial-sum slots of the
-// batch-1 kernel, 16 MiB][scratch of the batched kernel, or the hand-off words of a chain]. Slots
-// carry sequence tags, so nothing in the slot region ever has to be cleared; no other kernel writes
-// there, so calls of any shape and kind can share one workspace. The workspace must be zero-filled
-// once before its first use.
+// batch-1 kernel][counters of the batched kernel, 4 KiB; 16 MiB with the slots][scratch of the batched
+// kernel, or the hand-off words of a chain]. Slots carry sequence tags, so nothing in the slot region ever
+// has to be cleared, and the counters are zero between calls; no other kernel writes to either, so calls of
+// any shape and kind can share one workspace. The workspace must be zero-filled once before its first use.
 constexpr size_t kWsStatusBytes = 256;
-constexpr size_t kWsSlotRegionBytes = (size_t)16 << 20;
-constexpr size_t kWsScratchOffset = kWsStatusBytes + kWsSlotRegionBytes;
+constexpr size_t kWsCounterBytes = 4096;
+constexpr size_t kWsSlotRegionBytes = ((size_t)16 << 20) - kWsCounterBytes;
+constexpr size_t kWsCounterOffset = kWsStatusBytes + kWsSlotRegionBytes;
+constexpr size_t kWsScratchOffset = kWsCounterOffset + kWsCounterBytes;
 
 // Checked build (-DTQ1_BOUNDS_CHECK -rdc=true): every global store of a kernel (and the reads of scratch that
 // other CTAs write) first tests its index against the extent the launcher knows. A violation is counted in
@@ -85,11 +87,11 @@ bool gemv_chain_shape_ok(int N, int K);
 bool gemv_chain_supported(const uint8_t *blocks, int N, int K);
 bool gemv_chain_fits(const uint8_t *blocks, int N, int K);      // also checks the current device's SM count
 size_t gemv_chain_workspace_bytes(int N, int K);
-// M = 2 .. gemv_loop_tokens() activation rows as M links of one launch over the same weights
+// a few activation rows as M links of one launch over the same weights, where that is the better choice
 bool gemv_looped_fits(const uint8_t *blocks, int M, int N, int K);
 int launch_gemv_looped(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, bool swiglu,
                        void *workspace, cudaStream_t stream);
-int gemv_loop_tokens();
+bool gemv_loop_preferred(int M, int N, int K);
 int gemv_set_loop_tokens(int tokens);       // sweep recording only; process-global
 // slot_bytes: room for partial-sum slots behind the workspace's control words
 int launch_gemv_single(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int N, int K, bool swiglu,
@@ -101,9 +103,10 @@ int launch_epoch_advance(unsigned *epoch_base, unsigned delta, cudaStream_t stre
 int gemv_noalloc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int N, int K, cudaStream_t stream);
 int gemv_noalloc_status(unsigned *out_host, cudaStream_t stream);
 
-// Batched linear (M >= 2) on tcgen05 tensor cores; needs K % 512 == 0 and 16-byte aligned pointers.
+// Batched linear (M >= 2) on tcgen05 tensor cores; needs 16-byte aligned activations.
 bool gemm_tc_shape_ok(int M, int N, int K);
-bool gemm_tc_supported(const uint8_t *blocks, const __half *x, int M, int N, int K);
+// whether the kernel is the better choice for the shape (aligned: blocks on a 16-byte boundary)
+bool gemm_tc_preferred(bool aligned, int M, int N, int K);
 size_t gemm_tc_workspace_bytes(int M, int N, int K);
 int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K,
                    void *workspace, cudaStream_t stream, bool swiglu = false);

@@ -1,0 +1,1035 @@
+// Batched linear (M >= 2 activation rows) for TQ1_G128 on sm_100a: trits are decoded into FP16 weights in tensor
+// memory, activations come to shared memory by TMA, and tcgen05.mma multiplies them into FP32 accumulators in
+// tensor memory.
+//
+// Stands in for the reference's prefill GEMM and small-batch kernels behind packed_matmul
+// (src/ternel_mlx/kernels.py:409-858,1287-1357; src/ternel_mlx/modules.py:425-457). As in the reference's GEMM,
+// the group scale is folded into the FP16 weight, which is exact: (c-1)*s is -s, 0 or +s
+// (src/ternel_mlx/kernels.py:435-440).
+//
+// An output tile is 128 weight rows x NT activation rows per CTA (with CG = 2 a CTA pair takes 256 weight rows x NT):
+//   D[n][m] = sum_k W[n][k] * x[m][k]      (A = W, in tensor memory; B = x tile, K-major FP16, 128-byte swizzle)
+// The unit of work is a chunk of a tile: 4 K blocks of 128 columns = 112 packed bytes per row. A segment is a run of
+// consecutive chunks of one tile; a CTA (pair) walks the segments it was dealt.
+//   decode warps (G groups of four)  A group takes every G-th chunk of a segment. Its warp q fetches the packed bytes
+//        of rows 32q..32q+31 of the chunk into a buffer of its own (TMA, or 4-byte cp.async where rows are not
+//        16-byte aligned), so decoding needs no barrier between warps before the operand is complete. Thread = weight
+//        row: code byte -> 8-byte table entry of PRMT selectors -> pairs of FP16 weights picked out of
+//        [0, s_lo, s_hi, s_hi ^ 0x80] -> 32 registers = 64 K columns, stored to the row's lane of tensor memory.
+//        All groups also read out finished accumulators and store the results.
+//   one warp   issues tcgen05.mma for the halves (64 K columns) in a fixed order: chunk wave, K block, group, half
+//   one warp   fetches the activation tiles in the same order
+// Shared memory traffic of the table bounds the decode (two 128-byte wavefronts per 32 code bytes), so decode warps are
+// many and keep no state between chunks. Weights are decoded in natural column order (a byte's five trits straddle
+// register pairs differently in even and odd bytes, which the wide table holds as two entries), so activations are used
+// as they are: an earlier version permuted them in a launch of its own, a tenth of a prefill call.
+//
+// Segments that cover only a part of a tile's K range leave an FP32 partial tile in the workspace; the CTA that finishes
+// the tile's last part (a counter per tile) adds the parts in ascending K order, so results never depend on timing, and no
+// CTA waits for another. A separate launch for these sums cost 3 to 14 us.
+#include <cuda.h>
+#include <math.h>
+
+#include "tq1_common.cuh"
+
+namespace tq1 {
+
+namespace {
+
+constexpr int kTileW = 128;                                         // weight rows per CTA and tile
+constexpr int kChunkGroups = 4;
+constexpr int kChunkBytes = kChunkGroups * kBlockBytes;             // 112 packed bytes per row
+constexpr int kPackBytes = 32 * kChunkBytes;                        // a warp's rows of a chunk: 3584
+constexpr int kStageCols = 64;                                      // tensor-memory columns of a K block of FP16 weights
+constexpr uint32_t kSpinLimit = 1u << 20;
+
+// Variants:
+//   S  up to 32 tokens: two CTAs per SM with two decode groups each hide each other's latencies; the narrow table
+//      (one 8-byte entry per byte and lane pair, 32 KB) leaves room for that
+//   L  33..128 tokens: one CTA per SM, four groups, wide table (even and odd entries, 64 KB)
+//   P  larger: CTA pairs (cta_group::2), each CTA holds half of the activation tile, which halves the activation
+//      traffic out of L2 and through shared memory
+template <int CG_, int G_, bool WIDE_, int PACK_STAGES_, int RING_, int MAX_COLS_>
+struct Variant {
+    static constexpr int CG = CG_, G = G_, PACK_STAGES = PACK_STAGES_;
+    static constexpr bool WIDE = WIDE_;
+    static constexpr int RING = RING_;                              // K blocks of decoded weights in tensor memory
+    static constexpr int MAX_COLS = MAX_COLS_;                      // accumulator columns
+    static constexpr int kDecodeWarps = 4 * G;
+    static constexpr int kThreads = 32 * (kDecodeWarps + 2);
+    static constexpr int kGroupCols = MAX_COLS / G < 16 ? 16 : MAX_COLS / G;      // columns a group reads out
+    static constexpr int kABase = MAX_COLS < 32 ? 32 : MAX_COLS;
+    static constexpr int kTmemCols = G == 2 ? 256 : 512;
+    static_assert(kABase + RING * kStageCols <= kTmemCols, "tensor memory budget");
+    static constexpr int kMinCtas = G == 2 ? 2 : 1;
+    static constexpr uint32_t kTableBytes = WIDE ? 65536 : 32768;
+    // shared-memory window addresses; the wide table sits at a 64 KiB multiple so that one PRMT builds an entry address
+    static constexpr uint32_t kBase = 1024;
+    static constexpr uint32_t kPackAddr = kBase;
+    static constexpr uint32_t kPackOne = kDecodeWarps * kPackBytes;
+    static constexpr uint32_t kTableAddr = WIDE ? 65536 : kPackAddr + PACK_STAGES * kPackOne;
+    static constexpr uint32_t kBarAddr = WIDE ? kPackAddr + kPackOne : kTableAddr + kTableBytes;
+    static constexpr uint32_t kPack2Addr = kTableAddr + kTableBytes;              // wide: second packed stage
+    static constexpr uint32_t kBarBytes = 1024;
+    static constexpr uint32_t kBAddr = WIDE ? kPack2Addr + (PACK_STAGES - 1) * kPackOne : kBarAddr + kBarBytes;
+    static_assert(!WIDE || kBarAddr + kBarBytes <= kTableAddr, "barriers must end below the table");
+    static_assert(kBAddr % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
+    static constexpr uint32_t kWindowEnd = G == 2 ? 1024 + 115712 : 233472;
+    static constexpr uint32_t kBRoom = kWindowEnd - kBAddr;
+    static constexpr uint32_t kSmemBytes = kWindowEnd - kBase;
+    __device__ static __forceinline__ uint32_t pack_addr(int warp, int stage) {
+        if (WIDE) return (stage == 0 ? kPackAddr : kPack2Addr) + warp * kPackBytes;
+        return kPackAddr + stage * kPackOne + warp * kPackBytes;
+    }
+};
+using VariantS = Variant<1, 2, false, 2, 3, 32>;
+using VariantL = Variant<1, 4, true, 1, 6, 128>;
+using VariantP = Variant<2, 4, true, 1, 4, 256>;
+
+// Table entries. An 8-bit selector picks the two bytes of one FP16 weight out of the pool [0x00, s_lo, s_hi, s_hi ^ 0x80]:
+// code 0 -> -s = (1,3), code 1 -> 0 = (0,0), code 2 -> +s = (1,2). A 16-bit selector of two trits is a PRMT control word.
+//   even byte (its first trit in the lower half of a register): word0 = (t0,t1) | t4 << 16, word1 = (t2,t3)
+//   odd byte: word0 = (t1,t2) | t0 << 16, word1 = (t3,t4)
+// The narrow table holds the even form only; an odd byte's pairs then cost two more byte permutes.
+// Sixteen copies of an entry (lanes l and l + 16 share one: a 64-bit shared load serves half a warp at a time) make every
+// lookup free of bank conflicts. 256 entries (the 13 past 242 decode to zero weights): a byte that escaped the load-time
+// scan still reads inside the table.
+struct WideTable { uint32_t w[256 * 64]; };
+struct NarrowTable { uint32_t w[256 * 32]; };
+constexpr uint32_t sel8(uint32_t c) { return c == 0 ? 0x31u : c == 1 ? 0x00u : 0x21u; }
+constexpr void digits(int v, uint32_t (&c)[5]) {
+    for (int d = 0; d < 5; ++d) { c[d] = sel8((uint32_t)(v % 3)); v /= 3; }
+}
+constexpr WideTable make_wide() {
+    WideTable t{};
+    for (int v = 0; v < 243; ++v) {
+        uint32_t c[5] = {};
+        digits(v, c);
+        for (int l = 0; l < 16; ++l) {
+            t.w[v * 64 + 2 * l] = c[0] | (c[1] << 8) | (c[4] << 16);
+            t.w[v * 64 + 2 * l + 1] = c[2] | (c[3] << 8);
+            t.w[v * 64 + 32 + 2 * l] = c[1] | (c[2] << 8) | (c[0] << 16);
+            t.w[v * 64 + 32 + 2 * l + 1] = c[3] | (c[4] << 8);
+        }
+    }
+    return t;
+}
+constexpr NarrowTable make_narrow() {
+    NarrowTable t{};
+    for (int v = 0; v < 243; ++v) {
+        uint32_t c[5] = {};
+        digits(v, c);
+        for (int l = 0; l < 16; ++l) {
+            t.w[v * 32 + 2 * l] = c[0] | (c[1] << 8) | (c[4] << 16);
+            t.w[v * 32 + 2 * l + 1] = c[2] | (c[3] << 8);
+        }
+    }
+    return t;
+}
+__device__ __align__(128) const WideTable g_wide = make_wide();
+__device__ __align__(128) const NarrowTable g_narrow = make_narrow();
+
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+    return d;
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Address, in the cluster's shared window, of `addr` in the leading CTA of the pair.
+__device__ __forceinline__ uint32_t leader_addr(uint32_t addr) {
+    uint32_t d;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(d) : "r"(addr));
+    return d;
+}
+template <int CG>
+__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {       // bar: from leader_addr() with CG = 2
+    // CTA-scope release: what the leader's MMA reads lies in tensor memory and is ordered by tcgen05.wait::st and the
+    // tcgen05 fences; a cluster-scope release waits for every global store of the thread (2000 clocks a time)
+    if (CG == 2) asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+    else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Bounded wait: after the limit *status is set and `dead` stops every further wait of the thread, so that the
+// kernel ends (with results that the status marks as bad) instead of hanging. The loop is a few instructions: up to
+// twenty warps of an SM wait at a time, and what they issue while they do is taken from the decoding ones.
+__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, unsigned *status, bool &dead) {
+    if (dead) return;
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\t"
+                 "mov.u32 n, %3;\n"
+                 "TRY:\n\t"
+                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 4000;\n\t"
+                 "@p bra DONE;\n\t"
+                 "sub.u32 n, n, 1;\n\t"
+                 "setp.ne.u32 q, n, 0;\n\t"
+                 "@q bra TRY;\n"
+                 "DONE:\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity), "n"(kSpinLimit) : "memory");
+    if (!ok) {
+        atomicExch(status, 3u);
+        dead = true;
+    }
+}
+// One lane of a converged warp. Branching on it (and not on the lane number) tells the compiler that a single thread
+// runs the branch, so the operands of tcgen05.mma stay in uniform registers: 25 clocks per MMA issued instead of 134
+// (a loop over the lanes that might hold different operands), which had paced every token tile below 256.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+// Activation tile half: {64 columns, box rows} at (x, y). With a CTA pair the bytes count on the leader's barrier.
+template <int CG>
+__device__ __forceinline__ void tma_load_x(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
+    if (CG == 2)
+        asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+                     "[%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes "
+                     "[%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+// Called by all 32 lanes: one elected lane arms the warp's barrier and requests its 32 rows x 112 bytes.
+__device__ __forceinline__ void elected_load_packed(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "elect.sync _|p, 0xffffffff;\n\t"
+                 "@p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%4], %5;\n\t"
+                 "@p cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar), "n"(kPackBytes) : "memory");
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row groups 1024 B apart.
+__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
+    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
+           (2ull << 61);
+}
+// A operand in tensor memory (lane = weight row, 8 columns per K = 16 step), B in shared memory.
+template <int CG>
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+                                            uint32_t accumulate) {
+    if (CG == 2)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                     ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                     ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+// Arrives on `bar` (of both CTAs of a pair) when every MMA issued so far has finished.
+template <int CG>
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+    if (CG == 2)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                     ::"r"(bar), "h"((uint16_t)3) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tmem_store32(uint32_t taddr, const uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+        "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
+          "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
+          "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_load16(uint32_t taddr, float *v) {
+    uint32_t u[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]),
+          "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
+        : "r"(taddr) : "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(u[i]);
+}
+
+// n / d for 0 <= n < 2^31 by one multiplication: mul = ceil(2^64 / d), so the error n * (mul * d - 2^64) stays below 2^64.
+struct Divisor {
+    unsigned long long mul;
+    int d;
+    __host__ __device__ __forceinline__ void set(int divisor) {
+        d = divisor;
+        mul = divisor > 1 ? ~0ull / (unsigned)divisor + 1 : 0ull;
+    }
+    __host__ __device__ __forceinline__ int div(int n) const {
+        if (d == 1) return n;
+#ifdef __CUDA_ARCH__
+        return (int)__umul64hi((unsigned long long)(unsigned)n, mul);
+#else
+        return n / d;
+#endif
+    }
+};
+
+// How the chunks of all tiles, numbered tile-major, are dealt out. A slot is a CTA (a CTA pair with CG = 2).
+//   splits > 0: every tile in `splits` equal parts, one part per slot (fewer tiles than slots).
+//   splits == 0: every slot first computes whole_rounds whole tiles (slot * whole_rounds + k); the tiles from whole_tiles
+//     on are cut into equal contiguous ranges of chunks, one per slot (stream-K), so that all slots do the same number.
+struct WorkSplit {
+    int total_iters, slots, chunks, splits;
+    int quot, rem;                              // total_iters = slots * quot + rem: the first `rem` ranges get one more
+    int whole_rounds, whole_tiles;
+    int tiles_total;                            // output tiles of the call (a slot's last whole tiles may lie beyond)
+    Divisor by_splits, by_chunks;
+    __host__ __device__ __forceinline__ int first_iter(int slot) const {
+        if (slot >= slots) return total_iters;
+        if (splits == 0) return slot * quot + (slot < rem ? slot : rem);
+        const int tile = by_splits.div(slot), part = slot - tile * splits;
+        return tile * chunks + by_splits.div(chunks * part);
+    }
+};
+
+// A slot's segments in order: its whole tiles, then the pieces of its range of the shared tiles.
+struct SegmentWalk {
+    const Divisor &by_chunks;
+    int chunks, whole_rounds, whole_tiles, tiles_total, slot, round, it, end, pieces;
+    __device__ __forceinline__ SegmentWalk(const WorkSplit &work, int slot_)
+        : by_chunks(work.by_chunks), chunks(work.chunks), whole_rounds(work.whole_rounds), whole_tiles(work.whole_tiles),
+          tiles_total(work.tiles_total), slot(slot_), round(0), it(work.first_iter(slot_)),
+          end(work.first_iter(slot_ + 1)), pieces(0) {}
+    // part: which of the slot's two partial-tile areas a partial segment is stored to
+    __device__ __forceinline__ bool next(int &tile, int &c0, int &len, int &part) {
+        if (round < whole_rounds && slot * whole_rounds + round < tiles_total) {
+            tile = slot * whole_rounds + round++;
+            c0 = 0;
+            len = chunks;
+            part = 0;
+            return true;
+        }
+        if (it >= end) return false;
+        const int t = by_chunks.div(it);
+        c0 = it - t * chunks;
+        len = min(chunks - c0, end - it);
+        tile = whole_tiles + t;
+        part = pieces++ == 0 ? 0 : 1;
+        it += len;
+        return true;
+    }
+};
+
+struct GemmParams {
+    const uint8_t *blocks;
+    void *y;                  // [M][N] (FP16/FP32), with swiglu [M][N / 2]
+    float *partials;          // [2 * CTAs][nt][128] FP32
+    unsigned *counters;       // per shared tile (and CTA of a pair): parts stored so far; zero between calls
+    unsigned *status;
+    int M, N, groups;         // groups: K / 128
+    int tiles_m;              // token tiles; output tile t covers weight tile t / tiles_m, token tile t % tiles_m
+    Divisor by_tiles_m;
+    int nt;                   // tokens per tile, a multiple of 16 * CG; the last token tile takes what is left
+    int b_stages, b_rows;     // activation ring: stages and rows per CTA of one stage
+    WorkSplit work;
+    int y_f32, swiglu;
+};
+
+template <class V, bool TMA_W>
+__global__ void __launch_bounds__(V::kThreads, V::kMinCtas)
+tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
+                const __grid_constant__ GemmParams prm) {
+    constexpr int CG = V::CG, G = V::G, RING = V::RING, kDecode = V::kDecodeWarps;
+    constexpr int kMmaWarp = kDecode, kXWarp = kDecode + 1;
+    extern __shared__ __align__(1024) unsigned char smem[];
+    // In a cluster launch the upper byte of a shared-memory address names the CTA; the offsets below it are fixed.
+    const uint32_t window = (uint32_t)__cvta_generic_to_shared(smem);
+    const uint32_t wbase = CG == 2 ? window & 0xff000000u : 0u;
+    if (window != wbase + V::kBase) {                                // the fixed window addresses do not hold
+        if (threadIdx.x == 0) atomicExch(prm.status, 2u);
+        return;
+    }
+    constexpr int TAB = 0, PACK = 1, FULL_A = PACK + kDecode * V::PACK_STAGES, FULL_B = FULL_A + RING,
+                  EMPTY = FULL_B + RING, ACC_FULL = EMPTY + RING, ACC_FREE = ACC_FULL + 1, NUM_BARS = ACC_FREE + 1;
+    static_assert(NUM_BARS * 8 <= 1000, "barrier area");
+    auto bar = [wbase](int i) { return wbase + V::kBarAddr + 8u * (uint32_t)i; };
+    volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(smem + (V::kBarAddr - V::kBase) + 1008);
+    volatile uint32_t *last_flag = tmem_slot + 1;
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int slot = CG == 2 ? blockIdx.x >> 1 : blockIdx.x, rank = CG == 2 ? blockIdx.x & 1 : 0;
+    const int chunks = prm.work.chunks;
+
+    // ---- set-up that depends on no earlier kernel: barriers, decode table, tensor memory ---------------------
+    if (tid == 0) {
+        mbar_init(bar(TAB), 1);
+        for (int i = 0; i < kDecode * V::PACK_STAGES; ++i) mbar_init(bar(PACK + i), 1);
+        for (int i = 0; i < RING; ++i) {
+            mbar_init(bar(FULL_A + i), 4 * CG);
+            mbar_init(bar(FULL_B + i), 1);
+            mbar_init(bar(EMPTY + i), 1);
+        }
+        mbar_init(bar(ACC_FULL), 1);
+        mbar_init(bar(ACC_FREE), kDecode * CG);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_expect_tx(bar(TAB), V::kTableBytes);
+        if (V::WIDE) bulk_load(wbase + V::kTableAddr, &g_wide, V::kTableBytes, bar(TAB));
+        else bulk_load(wbase + V::kTableAddr, &g_narrow, V::kTableBytes, bar(TAB));
+    }
+    if (warp == kMmaWarp) {
+        const uint32_t where = wbase + V::kBarAddr + 1008;
+        if (CG == 2) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(where), "r"((uint32_t)V::kTmemCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(where), "r"((uint32_t)V::kTmemCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (CG == 2) {
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    } else {
+        __syncthreads();
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *tmem_slot;
+    // The next kernel in the stream may start its own set-up; everything below touches memory that earlier kernels
+    // may have written or may still read.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    bool dead = false;
+    SegmentWalk walk(prm.work, slot);
+    int tile, c0, len, part;
+
+    auto weight_tile = [&](int t) { return prm.by_tiles_m.div(t); };
+    auto token_tile0 = [&](int t) { return (t - prm.by_tiles_m.div(t) * prm.tiles_m) * prm.nt; };     // first token
+    // tokens of a token tile, as the MMA's N (whole steps of 16 per CTA)
+    auto tile_tokens = [&](int m0) {
+        const int left = min(prm.nt, prm.M - m0);
+        return (left + 16 * CG - 1) / (16 * CG) * (16 * CG);
+    };
+
+    // K blocks are numbered in the order the MMA warp takes them, over all segments: block i of a CTA uses stage i % RING of
+    // the decoded weights and stage i % b_stages (<= RING) of the activations. EMPTY[i % RING] completes when its MMAs have
+    // read both, one commit for decoders and activations alike.
+    // A wave is the G chunks (fewer at a segment's end) that the groups decode side by side; its blocks are ordered by K
+    // block first. Only a matrix row's last chunk can have fewer than four.
+    if (warp == kXWarp) {
+        // ------------------------------------------------------------------ activation tiles
+        if (elect_one()) {
+            uint32_t stage = 0, freed = 0, phase = 0, filled = 0;      // freed: stage of the block that used this buffer before
+            const uint32_t bytes = (uint32_t)prm.b_rows * 256u;
+            while (walk.next(tile, c0, len, part)) {
+                const int m0 = token_tile0(tile);
+                const int row = m0 + (CG == 2 ? rank * (tile_tokens(m0) / 2) : 0);
+                for (int u0 = 0; u0 < len; u0 += G) {
+                    const int width = min(G, len - u0), k0 = (c0 + u0) * kChunkGroups;
+                    for (int kb = 0; kb < kChunkGroups; ++kb) {
+                        for (int g = 0; g < width; ++g) {
+                            const int k = k0 + g * kChunkGroups + kb;
+                            if (k >= prm.groups) continue;
+                            if (filled < (uint32_t)prm.b_stages) {
+                                ++filled;
+                            } else {
+                                mbar_wait(bar(EMPTY + freed), phase, prm.status, dead);
+                                if (++freed == RING) { freed = 0; phase ^= 1u; }
+                            }
+                            if (dead) break;
+                            const uint32_t full = CG == 2 ? leader_addr(bar(FULL_B + stage)) : bar(FULL_B + stage);
+                            if (rank == 0) mbar_expect_tx(bar(FULL_B + stage), CG * bytes);
+                            const uint32_t dst = wbase + V::kBAddr + stage * bytes;
+                            tma_load_x<CG>(dst, &xmap, k * kGroup, row, full);
+                            tma_load_x<CG>(dst + bytes / 2, &xmap, k * kGroup + 64, row, full);
+                            if (++stage == (uint32_t)prm.b_stages) stage = 0;
+                        }
+                    }
+                }
+            }
+        }
+    } else if (warp == kMmaWarp) {
+        // ------------------------------------------------------------------ MMA issue (leading CTA of a pair)
+        if (rank == 0 && elect_one()) {
+            uint32_t bstage = 0, bphase = 0, astage = 0, aphase = 0, seg = 0;
+            const uint32_t b_bytes = (uint32_t)prm.b_rows * 256u;
+            while (walk.next(tile, c0, len, part)) {
+                const int n_tok = tile_tokens(token_tile0(tile));
+                // FP32 accumulate, FP16 A and B, both K-major, M = 128 per CTA, N = tokens
+                const uint32_t idesc = (1u << 4) | ((uint32_t)(n_tok >> 3) << 17) | ((uint32_t)(kTileW * CG >> 4) << 24);
+                const int blocks = min(len * kChunkGroups, prm.groups - c0 * kChunkGroups);
+                if (seg > 0) mbar_wait(bar(ACC_FREE), (seg - 1) & 1u, prm.status, dead);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int i = 0; i < blocks; ++i) {
+                    mbar_wait(bar(FULL_B + bstage), bphase, prm.status, dead);
+                    mbar_wait(bar(FULL_A + astage), aphase, prm.status, dead);
+                    if (dead) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t a_tmem = tmem_base + (uint32_t)V::kABase + astage * kStageCols;
+                    const uint32_t b_addr = wbase + V::kBAddr + bstage * b_bytes;
+                    const uint64_t b_lo = umma_desc(b_addr), b_hi = umma_desc(b_addr + b_bytes / 2);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)                    // K = 16 steps: four of each 64-wide swizzle atom
+                        umma_f16_ts<CG>(tmem_base, a_tmem + 8u * j, (j < 4 ? b_lo : b_hi) + 2u * (j & 3), idesc,
+                                        (i > 0 || j > 0) ? 1u : 0u);
+                    umma_commit<CG>(bar(EMPTY + astage));
+                    if (++astage == RING) { astage = 0; aphase ^= 1u; }
+                    if (++bstage == (uint32_t)prm.b_stages) { bstage = 0; bphase ^= 1u; }
+                }
+                if (!dead) umma_commit<CG>(bar(ACC_FULL));
+                ++seg;
+            }
+        }
+    } else {
+        // ------------------------------------------------------------------ decode and results
+        const int group = warp >> 2, quad = warp & 3;
+        const int row_in_tile = quad * 32 + lane;                       // = tensor-memory lane
+        const uint32_t tmem_lane = tmem_base + ((uint32_t)(quad * 32) << 16);
+        const uint32_t lane_entry = wbase + V::kTableAddr + (uint32_t)(lane & 15) * 8u;
+        const size_t row_bytes = (size_t)prm.groups * kBlockBytes;
+
+        // cursor of the packed bytes this warp requests ahead of its decoding
+        SegmentWalk pwalk(prm.work, slot);
+        int p_tile = 0, p_c0 = 0, p_len = 0, p_part, p_unit = group;
+        uint32_t requested = 0, consumed = 0;
+        auto request = [&]() {
+            bool more = true;
+            while (p_unit >= p_len) {
+                if (!pwalk.next(p_tile, p_c0, p_len, p_part)) { p_len = 0; more = false; break; }
+                p_unit = group;
+            }
+            const uint32_t s = requested % V::PACK_STAGES;
+            const int chunk = p_c0 + p_unit, n0 = (weight_tile(p_tile) * CG + rank) * kTileW + quad * 32;
+            const uint32_t dst = wbase + V::pack_addr(warp, (int)s);
+            if (more) {
+                if (TMA_W) {
+                    elected_load_packed(dst, &wmap, chunk * kChunkBytes, n0, bar(PACK + warp * V::PACK_STAGES + (int)s));
+                } else if (lane < kChunkBytes / 4) {
+                    // rows whose byte length is no multiple of 16 cannot be a tensor map's: one row per instruction
+                    const bool in_row = chunk * kChunkBytes + lane * 4 < (int)row_bytes;
+                    const uint8_t *src = prm.blocks + (in_row ? (size_t)chunk * kChunkBytes + lane * 4 : 0);
+#pragma unroll 8
+                    for (int r = 0; r < 32; ++r) {
+                        const bool live = in_row && n0 + r < prm.N;
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;"
+                                     ::"r"(dst + (uint32_t)(r * kChunkBytes + lane * 4)),
+                                       "l"(src + (live ? (size_t)(n0 + r) * row_bytes : 0)), "r"(live ? 4 : 0) : "memory");
+                    }
+                }
+                ++requested;
+                p_unit += G;
+            }
+            if (!TMA_W) asm volatile("cp.async.commit_group;" ::: "memory");       // one group per call, empty at the end
+        };
+#pragma unroll
+        for (int s = 0; s < V::PACK_STAGES; ++s) request();
+
+        int block0 = 0;                                                 // number of the wave's first K block
+        uint32_t seg = 0;
+        mbar_wait(bar(TAB), 0, prm.status, dead);
+
+        while (walk.next(tile, c0, len, part)) {
+            for (int u0 = 0; u0 < len; u0 += G) {
+                const int width = min(G, len - u0), unit = u0 + group;
+                // the wave's last chunk may be short; blocks past its end are missing from the numbering
+                const int last_blocks = min(kChunkGroups, prm.groups - (c0 + u0 + width - 1) * kChunkGroups);
+                const int wave0 = block0;
+                block0 += (width - 1) * kChunkGroups + last_blocks;
+                if (unit >= len) continue;
+                const int blocks_here = group == width - 1 ? last_blocks : kChunkGroups;
+                const uint32_t s = consumed % V::PACK_STAGES;
+                if (TMA_W) {
+                    mbar_wait(bar(PACK + warp * V::PACK_STAGES + (int)s), (consumed / V::PACK_STAGES) & 1u, prm.status, dead);
+                } else {
+                    asm volatile("cp.async.wait_group %0;" ::"n"(V::PACK_STAGES - 1) : "memory");
+                    __syncwarp();
+                }
+                // This row's 112 bytes come into registers in two steps (all at once spills); after the second the
+                // buffer is free for the next request.
+                uint32_t words[4 * 7];
+                const uint32_t src = wbase + V::pack_addr(warp, (int)s) + (uint32_t)lane * kChunkBytes;
+                auto fetch = [&](int i) {
+                    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(words[4 * i]), "=r"(words[4 * i + 1]), "=r"(words[4 * i + 2]), "=r"(words[4 * i + 3])
+                                 : "r"(src + 16u * i) : "memory");
+                };
+#pragma unroll
+                for (int i = 0; i < 4; ++i) fetch(i);
+                ++consumed;
+#pragma unroll
+                for (int b = 0; b < kChunkGroups; ++b) {
+                    if (b == 2) {
+#pragma unroll
+                        for (int i = 4; i < 7; ++i) fetch(i);
+                        __syncwarp();
+                        request();
+                    }
+                    if (b >= blocks_here) continue;
+                    const uint32_t *w = words + 7 * b;
+                    const uint32_t pool = (w[0] << 16 >> 8) | (((w[0] & 0xff00u) ^ 0x8000u) << 16);
+                    // table entry of code byte j
+                    auto lookup = [&](int j, uint32_t &e0, uint32_t &e1) {
+                        const uint32_t word = w[(2 + j) >> 2];
+                        const int k = (2 + j) & 3;
+                        uint32_t addr;
+                        if (V::WIDE) addr = prmt(word, lane_entry | (j & 1 ? 128u : 0u), 0x7604u | (uint32_t)(k << 4));
+                        else addr = prmt(word, 0u, 0x4440u | (uint32_t)k) * 128u + lane_entry;
+                        asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(e0), "=r"(e1) : "r"(addr));
+                    };
+                    auto pick = [&](uint32_t sel) { return prmt(pool, 0u, sel); };
+                    auto even = [&](uint32_t e0, uint32_t e1, uint32_t &a, uint32_t &c) { a = pick(e0); c = pick(e1); };
+                    auto odd = [&](uint32_t e0, uint32_t e1, uint32_t &a, uint32_t &c) {
+                        a = pick(V::WIDE ? e0 : prmt(e0, e1, 0x0041));
+                        c = pick(V::WIDE ? e1 : prmt(e0, e1, 0x0025));
+                    };
+                    // trit 4 of an even byte beside trit 0 of the odd byte after it
+                    auto straddle = [&](uint32_t p0, uint32_t q0) { return pick(prmt(p0, q0, V::WIDE ? 0x0062 : 0x0042)); };
+                    const uint32_t number = (uint32_t)(wave0 + b * width - max(b - last_blocks, 0) + group);
+                    const uint32_t stage = number % RING, use = number / RING;
+                    const uint32_t a_addr = tmem_lane + (uint32_t)V::kABase + stage * kStageCols;
+                    uint32_t m0w, m1w;                                  // byte 12 belongs to both halves
+                    {
+                        uint32_t v[32];
+#pragma unroll
+                        for (int a = 0; a < 6; ++a) {
+                            uint32_t e0, e1, f0, f1;
+                            lookup(2 * a, e0, e1);
+                            lookup(2 * a + 1, f0, f1);
+                            even(e0, e1, v[5 * a], v[5 * a + 1]);
+                            v[5 * a + 2] = straddle(e0, f0);
+                            odd(f0, f1, v[5 * a + 3], v[5 * a + 4]);
+                        }
+                        lookup(12, m0w, m1w);
+                        even(m0w, m1w, v[30], v[31]);
+                        mbar_wait(bar(EMPTY + (int)stage), (use & 1u) ^ 1u, prm.status, dead);
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        tmem_store32(a_addr, v);
+                    }
+                    {
+                        uint32_t v[32], f0, f1;
+                        lookup(13, f0, f1);
+                        v[0] = straddle(m0w, f0);
+                        odd(f0, f1, v[1], v[2]);
+#pragma unroll
+                        for (int a = 7; a < 12; ++a) {
+                            uint32_t e0, e1, g0, g1;
+                            lookup(2 * a, e0, e1);
+                            lookup(2 * a + 1, g0, g1);
+                            even(e0, e1, v[5 * a - 32], v[5 * a - 31]);
+                            v[5 * a - 30] = straddle(e0, g0);
+                            odd(g0, g1, v[5 * a - 29], v[5 * a - 28]);
+                        }
+                        uint32_t e0, e1, t0, t1, none;
+                        lookup(24, e0, e1);
+                        lookup(25, t0, t1);                             // the tail byte's three trits
+                        even(e0, e1, v[28], v[29]);
+                        v[30] = straddle(e0, t0);
+                        odd(t0, t1, v[31], none);
+                        tmem_store32(a_addr + 32u, v);
+                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncwarp();
+                        const uint32_t full = bar(FULL_A + (int)stage);
+                        if (lane == 0) mbar_arrive_leader<CG>(CG == 2 ? leader_addr(full) : full);
+                    }
+                }
+            }
+
+            // ---- the segment's accumulator -------------------------------------------------------------------
+            const int m0 = token_tile0(tile), n_tok = tile_tokens(m0);
+            const int n = (weight_tile(tile) * CG + rank) * kTileW + row_in_tile;
+            const int per_group = (n_tok / 16 + G - 1) / G * 16;
+            const int c_begin = group * per_group, cols = min(per_group, n_tok - c_begin);     // cols <= 0: none
+            // the slots that share this tile, worked out while the last products are still being added
+            const int shared_tile = tile - prm.work.whole_tiles, it0 = shared_tile * chunks;
+            int lo = slot, hi = slot;
+            if (len != chunks) {
+                if (prm.work.splits > 0) {
+                    lo = shared_tile * prm.work.splits;
+                    hi = lo + prm.work.splits - 1;
+                } else {
+                    while (prm.work.first_iter(lo) > it0) --lo;
+                    while (prm.work.first_iter(hi + 1) < it0 + chunks) ++hi;
+                }
+            }
+            mbar_wait(bar(ACC_FULL), seg & 1u, prm.status, dead);
+            ++seg;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            constexpr int kStep = V::kGroupCols < 32 ? V::kGroupCols : 32;                     // columns in registers at a time
+            const bool whole = len == chunks;
+            const size_t area = (size_t)prm.nt * kTileW;
+            float *slot_part = prm.partials + ((size_t)2 * blockIdx.x + part) * area + row_in_tile;
+#pragma unroll
+            for (int s0 = 0; s0 < V::kGroupCols; s0 += kStep) {
+                float v[kStep];
+#pragma unroll
+                for (int c = 0; c < kStep; c += 16)
+                    if (s0 + c < cols) tmem_load16(tmem_lane + (uint32_t)(c_begin + s0 + c), v + c);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int c = 0; c < kStep; ++c) asm volatile("" : "+f"(v[c]));                 // no use before the wait
+                if (s0 + kStep >= V::kGroupCols) {
+                    // the columns are in registers: the next segment may overwrite them while the results are stored
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_leader<CG>(CG == 2 ? leader_addr(bar(ACC_FREE)) : bar(ACC_FREE));
+                }
+                const int col0 = c_begin + s0, tokens = min(cols - s0, prm.M - (m0 + col0));   // of this step's columns
+                if (!whole) {
+                    // a part of the tile's K range: kept as FP32
+#pragma unroll
+                    for (int c = 0; c < kStep; ++c)
+                        if (c < tokens && TQ1_IN_BOUNDS((size_t)(col0 + c) * kTileW + row_in_tile, area, 41u))
+                            __stcg(slot_part + (size_t)(col0 + c) * kTileW, v[c]);
+                } else if (prm.swiglu) {                // (gate, up) row pairs: the even row stores silu(gate) * up
+                    const int out_n = prm.N >> 1;
+#pragma unroll
+                    for (int c = 0; c < kStep; ++c) {
+                        const float up = __shfl_down_sync(0xffffffffu, v[c], 1);
+                        if (c < tokens && (lane & 1) == 0 && n + 1 < prm.N) {
+                            const float out = swiglu_f32(v[c], up);
+                            const size_t o = (size_t)(m0 + col0 + c) * out_n + (n >> 1);
+                            if (!TQ1_IN_BOUNDS(o, (size_t)prm.M * out_n, 40u)) continue;
+                            if (prm.y_f32) static_cast<float *>(prm.y)[o] = out;
+                            else static_cast<__half *>(prm.y)[o] = __float2half_rn(out);
+                        }
+                    }
+                } else if (n < prm.N) {
+                    const size_t o = (size_t)(m0 + col0) * prm.N + n;
+#pragma unroll
+                    for (int c = 0; c < kStep; ++c) {
+                        if (c < tokens && TQ1_IN_BOUNDS(o + (size_t)c * prm.N, (size_t)prm.M * prm.N, 40u)) {
+                            if (prm.y_f32) static_cast<float *>(prm.y)[o + (size_t)c * prm.N] = v[c];
+                            else static_cast<__half *>(prm.y)[o + (size_t)c * prm.N] = __float2half_rn(v[c]);
+                        }
+                    }
+                }
+            }
+            if (whole) continue;
+            // The slot that completes the tile's count adds the parts.
+            asm volatile("bar.sync 1, %0;" ::"n"(kDecode * 32) : "memory");
+            if (tid == 0) {
+                // the barrier orders the other warps' stores before this thread's release, and its acquire before their reads
+                unsigned *counter = prm.counters + shared_tile * CG + rank, before;
+                asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
+                const bool last = before == (unsigned)(hi - lo);
+                if (last) *counter = 0u;                // zero for the next call
+                *last_flag = last ? 1u : 0u;
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(kDecode * 32) : "memory");
+            if (*last_flag == 0u) continue;
+            const int all = min(n_tok, prm.M - m0), quads = all * (kTileW / 4);      // four rows of a column each
+            constexpr int kThreadsR = kDecode * 32, kFlight = 4;
+            const int tile_n0 = (weight_tile(tile) * CG + rank) * kTileW;
+            for (int i0 = tid; i0 < quads; i0 += kThreadsR * kFlight) {
+                float4 total[kFlight];
+#pragma unroll
+                for (int f = 0; f < kFlight; ++f) total[f] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 2
+                for (int sl = lo; sl <= hi; ++sl) {
+                    // the tile is that slot's first segment of shared tiles if its range starts inside the tile
+                    const int which = prm.work.splits > 0 || prm.work.first_iter(sl) >= it0 ? 0 : 1;
+                    const float4 *src = reinterpret_cast<const float4 *>(
+                        prm.partials + ((size_t)2 * (sl * CG + rank) + which) * area);
+#pragma unroll
+                    for (int f = 0; f < kFlight; ++f) {
+                        const int i = i0 + f * kThreadsR;
+                        const float4 p = i < quads ? __ldcg(src + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        total[f].x += p.x; total[f].y += p.y; total[f].z += p.z; total[f].w += p.w;
+                    }
+                }
+#pragma unroll
+                for (int f = 0; f < kFlight; ++f) {
+                    const int i = i0 + f * kThreadsR, m = m0 + (i >> 5), nq = tile_n0 + (i & 31) * 4;
+                    if (i >= quads) break;
+                    float r[4] = {total[f].x, total[f].y, total[f].z, total[f].w};
+                    int count = min(4, prm.N - nq);
+                    size_t o = (size_t)m * prm.N + nq;
+                    size_t limit = (size_t)prm.M * prm.N;
+                    if (prm.swiglu) {
+                        r[0] = swiglu_f32(r[0], r[1]);
+                        r[1] = swiglu_f32(r[2], r[3]);
+                        count >>= 1;
+                        o = (size_t)m * (prm.N >> 1) + (nq >> 1);
+                        limit >>= 1;
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        if (e < count && TQ1_IN_BOUNDS(o + e, limit, 40u)) {
+                            if (prm.y_f32) static_cast<float *>(prm.y)[o + e] = r[e];
+                            else static_cast<__half *>(prm.y)[o + e] = __float2half_rn(r[e]);
+                        }
+                    }
+                }
+            }
+        }
+        if (!TMA_W) asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+
+    // ---- leave: nothing of this CTA (or of its pair) is in flight any more ---------------------------------------
+    __syncwarp();
+    if (dead)                                           // a wait ran out: give the copies still in flight time to land
+        for (int i = 0; i < 64; ++i) __nanosleep(20000);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (CG == 2) {
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    } else {
+        __syncthreads();
+    }
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (CG == 2)
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)V::kTmemCols) : "memory");
+        else
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)V::kTmemCols) : "memory");
+    }
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn gemm_encode_fn() {
+    static EncodeTiledFn fn = nullptr;
+    static bool tried = false;
+    if (!tried) {
+        tried = true;
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult qres;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) == cudaSuccess &&
+            qres == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<EncodeTiledFn>(p);
+    }
+    return fn;
+}
+
+// Launch state is per DEVICE: the SM count differs between devices and the shared-memory opt-in is an
+// attribute of a function on one device, so a process that drives several GPUs needs one record each.
+constexpr int kMaxDevices = 64;
+int current_device_slot() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+    return dev;
+}
+int sm_count_cached() {
+    static int sm_count[kMaxDevices] = {};
+    const int dev = current_device_slot();
+    if (!sm_count[dev]) {
+        if (cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count[dev] <= 0)
+            sm_count[dev] = 148;
+    }
+    return sm_count[dev];
+}
+
+// The token tile names the variant: 16 and 32 run as S, 64 and 128 as L, 256 as P.
+int tile_cg(int tile) { return tile > 128 ? 2 : 1; }
+
+struct Tiling {
+    int tile, tiles_m, nt;
+    WorkSplit work;
+    int ctas() const { return work.slots * tile_cg(tile); }
+};
+
+// How the chunks of a shape are dealt out for a given token tile.
+Tiling make_tiling(int tile, int M, int N, int K) {
+    Tiling t;
+    const int cg = tile_cg(tile);
+    t.tile = tile;
+    t.tiles_m = (M + tile - 1) / tile;
+    // equal token tiles: a prompt of 777 tokens is three tiles of 224 and one of 105 rather than three of 256 and one of 9
+    const int even = (M + t.tiles_m - 1) / t.tiles_m;
+    t.nt = (even + 16 * cg - 1) / (16 * cg) * (16 * cg);
+    t.tiles_m = (M + t.nt - 1) / t.nt;
+    const long long tiles = (long long)((N + kTileW * cg - 1) / (kTileW * cg)) * t.tiles_m;
+    const long long slots = (long long)sm_count_cached() * (tile <= 32 ? 2 : 1) / cg;
+    WorkSplit &w = t.work;
+    w.chunks = (K / kGroup + kChunkGroups - 1) / kChunkGroups;
+    w.total_iters = (int)(tiles * w.chunks);
+    w.whole_rounds = w.whole_tiles = 0;
+    w.tiles_total = (int)tiles;
+    // With more than half as many tiles as slots, cutting every tile in two would need a second wave and one
+    // part per tile leaves up to half of the SMs idle: those shapes are shared stream-K fashion as well.
+    if (tiles >= slots || (tile > 16 && 2 * tiles > slots)) {
+        w.splits = 0;
+        w.slots = (int)slots;
+        // whole tiles first; what is left over is shared. A share of fewer than two chunks per slot
+        // would cost more in partial stores than it balances, so then one round of whole tiles is shared too.
+        long long rounds = tiles / slots;
+        long long shared = tiles - rounds * slots;
+        if (rounds > 0 && shared > 0 && shared * w.chunks < 2 * slots) {
+            --rounds;
+            shared += slots;
+        }
+        w.whole_rounds = (int)rounds;
+        w.whole_tiles = (int)(rounds * slots);
+        w.total_iters = (int)(shared * w.chunks);
+        if (shared == 0) w.slots = (int)(tiles < rounds * slots ? (tiles + rounds - 1) / rounds : slots);
+    } else {
+        int splits = (int)(slots / tiles);
+        const int max_splits = w.chunks / 2 > 0 ? w.chunks / 2 : 1;
+        if (splits > max_splits) splits = max_splits;
+        if (splits > 32) splits = 32;
+        w.splits = splits;
+        w.slots = (int)tiles * splits;
+    }
+    w.by_splits.set(w.splits > 0 ? w.splits : 1);
+    w.by_chunks.set(w.chunks);
+    w.quot = w.total_iters / w.slots;
+    w.rem = w.total_iters % w.slots;
+    return t;
+}
+
+// Activation rows per tile. Up to 16 rows always take the 16-row tile. Beyond that the tile with the smallest modelled
+// time wins: launch and pipeline fill, chunks a slot works through (decode, plus products per token), segments it stores,
+// and the sums of shared tiles. The constants (us) are fitted to the recorded sweep in
+// ternel_b200/dispatch_sweep_b200.json; tests replay the file (the choice is within 10% of the best recorded tile for every
+// case). g_forced_tile overrides the rule while a sweep is being recorded.
+int g_forced_tile = 0;
+struct TileCost { int tile; float fixed, chunk, chunk_token, segment, shared_token; };
+int token_tile(int M, int N, int K) {
+    if (g_forced_tile) return g_forced_tile;
+    if (M <= 16) return 16;
+    static const TileCost costs[5] = {{16, 2.076f, 0.0f, 0.1592f, 0.0f, 0.1997f},
+                                      {32, 4.394f, 2.3991f, 0.0f, 0.9688f, 0.0369f},
+                                      {64, 2.7955f, 1.2087f, 0.0007f, 2.716f, 0.0684f},
+                                      {128, 4.3587f, 0.8426f, 0.0065f, 2.4854f, 0.0441f},
+                                      {256, 5.532f, 0.207f, 0.0102f, 3.4731f, 0.0424f}};
+    int best = 128;
+    float best_cost = 0.0f;
+    for (int i = 0; i < 5; ++i) {
+        const TileCost &c = costs[i];
+        if (c.tile > 16 && c.tile >= 4 * M) continue;           // a tile mostly of padding
+        const Tiling t = make_tiling(c.tile, M, N, K);
+        const WorkSplit &w = t.work;
+        const float shared = (float)w.total_iters / w.slots;    // chunks of shared tiles per slot
+        const float chunks = w.splits ? (float)((w.chunks + w.splits - 1) / w.splits)
+                                      : (float)w.whole_rounds * w.chunks + ceilf(shared);
+        const float segments = w.splits ? 1.0f : (float)w.whole_rounds + (w.total_iters ? shared / w.chunks + 1.0f : 0.0f);
+        const bool sums = w.splits ? w.splits > 1 : w.total_iters > 0;
+        const float cost = c.fixed + chunks * (c.chunk + c.chunk_token * t.nt) + segments * c.segment +
+                           (sums ? c.shared_token * t.nt : 0.0f);
+        if (i == 0 || cost < best_cost) { best = c.tile; best_cost = cost; }
+    }
+    return best;
+}
+Tiling pick_tiling(int M, int N, int K) { return make_tiling(token_tile(M, N, K), M, N, K); }
+
+size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
+
+template <class V, bool TMA_W>
+int launch_variant(const CUtensorMap &wmap, const CUtensorMap &xmap, const GemmParams &prm, int ctas, cudaStream_t stream) {
+    auto kern = tq1_gemm_kernel<V, TMA_W>;
+    static bool attr_set[kMaxDevices] = {};
+    const int dev = current_device_slot();
+    if (!attr_set[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)V::kSmemBytes);
+        if (e != cudaSuccess) return cuda_fail(e, "tq1_linear_f16: shared memory opt-in (GEMM)");
+        attr_set[dev] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(V::kThreads);
+    cfg.dynamicSmemBytes = V::kSmemBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = V::CG;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = V::CG > 1 ? 2 : 1;
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, kern, wmap, xmap, prm);
+    return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: GEMM launch");
+}
+
+template <class V>
+int launch_aligned(bool tma, const CUtensorMap &wmap, const CUtensorMap &xmap, GemmParams &prm, int ctas, cudaStream_t stream) {
+    const int stages = (int)(V::kBRoom / ((uint32_t)prm.b_rows * 256u));
+    prm.b_stages = stages < V::RING ? stages : V::RING;
+    return tma ? launch_variant<V, true>(wmap, xmap, prm, ctas, stream) : launch_variant<V, false>(wmap, xmap, prm, ctas, stream);
+}
+
+}  // namespace
+
+int gemm_tc_force_tile(int nt) {
+    if (nt != 0 && nt != 16 && nt != 32 && nt != 64 && nt != 128 && nt != 256) return TQ1_ERR_INVALID;
+    g_forced_tile = nt;
+    return TQ1_OK;
+}
+
+void gemm_tc_plan(int M, int N, int K, int *tile, int *ctas, int *parts) {
+    const Tiling t = pick_tiling(M, N, K);
+    *tile = t.tile;
+    *ctas = t.ctas();
+    *parts = t.work.splits;
+}
+
+// Any M >= 2 and K a multiple of the group. Widths that are no multiple of a chunk take the kernel only where the
+// product is large enough to pay for its set-up (see gemm_tc_preferred).
+bool gemm_tc_shape_ok(int M, int N, int K) { return M >= 2 && N >= 1 && K % kGroup == 0; }
+
+// The row kernel keeps small products of widths that are no multiple of 512 (and of blocks that are not 16-byte aligned).
+bool gemm_tc_preferred(bool aligned, int M, int N, int K) {
+    return gemm_tc_shape_ok(M, N, K) && ((aligned && K % (kChunkGroups * kGroup) == 0) || (long long)M * N * K >= (1 << 20));
+}
+
+size_t gemm_tc_workspace_bytes(int M, int N, int K) {
+    const Tiling t = pick_tiling(M, N, K);
+    return kWsScratchOffset + align256((size_t)2 * t.ctas() * t.nt * kTileW * sizeof(float));
+}
+
+int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K,
+                   void *workspace, cudaStream_t stream, bool swiglu) {
+    EncodeTiledFn encode = gemm_encode_fn();
+    if (!encode) return fail(TQ1_ERR_CUDA, "tq1_linear_f16: cuTensorMapEncodeTiled is unavailable");
+    unsigned char *ws = static_cast<unsigned char *>(workspace);
+    const Tiling t = pick_tiling(M, N, K);
+    const int cg = tile_cg(t.tile);
+    GemmParams prm;
+    prm.blocks = blocks;
+    prm.y = y;
+    prm.partials = reinterpret_cast<float *>(ws + kWsScratchOffset);
+    prm.counters = reinterpret_cast<unsigned *>(ws + kWsCounterOffset);
+    prm.status = reinterpret_cast<unsigned *>(ws);
+    prm.M = M;
+    prm.N = N;
+    prm.groups = K / kGroup;
+    prm.tiles_m = t.tiles_m;
+    prm.by_tiles_m.set(t.tiles_m);
+    prm.nt = t.nt;
+    prm.b_rows = t.nt / cg;
+    prm.work = t.work;
+    prm.y_f32 = y_f32 ? 1 : 0;
+    prm.swiglu = swiglu ? 1 : 0;
+
+    // rows of packed bytes as a tensor map: the row length must be a multiple of 16 bytes, the base aligned to 16
+    const bool tma = K % (kChunkGroups * kGroup) == 0 && (reinterpret_cast<uintptr_t>(blocks) & 15) == 0;
+    CUtensorMap wmap = {}, xmap;
+    const cuuint32_t estr[2] = {1, 1};
+    if (tma) {
+        const cuuint64_t row_bytes = (cuuint64_t)(K / kGroup) * kBlockBytes;
+        const cuuint64_t dims[2] = {row_bytes, (cuuint64_t)N};
+        const cuuint64_t strides[1] = {row_bytes};
+        const cuuint32_t box[2] = {kChunkBytes, 32};
+        CUresult res = encode(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(blocks), dims, strides,
+                              box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (res != CUDA_SUCCESS) return fail(TQ1_ERR_CUDA, "tq1_linear_f16: weight tensor map failed (%d)", (int)res);
+    }
+    {
+        const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
+        const cuuint64_t strides[1] = {(cuuint64_t)K * sizeof(__half)};
+        const cuuint32_t box[2] = {64, (cuuint32_t)prm.b_rows};
+        CUresult res = encode(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(x), dims, strides, box, estr,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (res != CUDA_SUCCESS)
+            return fail(TQ1_ERR_CUDA, "tq1_linear_f16: activation tensor map failed (%d)", (int)res);
+    }
+    return t.tile <= 32    ? launch_aligned<VariantS>(tma, wmap, xmap, prm, t.ctas(), stream)
+           : t.tile <= 128 ? launch_aligned<VariantL>(tma, wmap, xmap, prm, t.ctas(), stream)
+                           : launch_aligned<VariantP>(tma, wmap, xmap, prm, t.ctas(), stream);
+}
+
+}  // namespace tq1

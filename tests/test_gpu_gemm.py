@@ -168,3 +168,27 @@ def test_every_token_tile_gives_the_right_answer(rows, columns, batch):
         assert lib.tq1_debug_force_token_tile(48) == _native.TQ1_ERR_INVALID
     finally:
         assert lib.tq1_debug_force_token_tile(0) == 0
+
+
+@pytest.mark.parametrize("batch", (2, 16, 17, 32, 33, 64, 65, 128, 129, 255, 257, 520))
+@pytest.mark.parametrize(("rows", "columns"), ((129, 8064), (4099, 2176), (383, 4224), (1000, 1408)))
+def test_widths_of_whole_groups(rows, columns, batch):
+    """Widths that are no multiple of 512 (a short last chunk of 1, 2 or 3 groups, rows off the 16-byte grid) and rows that
+    fill no tile, in every token tile's range and around its edges: FP32 sums of FP16 products, in any order, stay within
+    columns * 2^-24 of the largest output (F32_TOL is ten times that); a second run gives the same bits. The same holds for
+    blocks that start off the 16-byte grid."""
+    if batch * rows * columns < 1 << 20:
+        pytest.skip("below the tensor-core kernel's range")
+    from ternel_b200.ops import check_status, tq1_matmul
+    blocks, rng = random_blocks(rows, columns, seed=rows + batch, dist="tests")
+    x = rng.standard_normal((batch, columns)).astype(np.float16)
+    want = o.float64_matmul(blocks, x, rows=rows, columns=columns)
+    got = run_linear(blocks, x)
+    assert o.normalised_error(got, want) < F32_TOL
+    assert np.array_equal(run_linear(blocks, x), got)
+    backing = torch.zeros(blocks.size + 16, dtype=torch.uint8, device="cuda")
+    shifted = backing[4:4 + blocks.size].view(blocks.shape)
+    shifted.copy_(torch.from_numpy(blocks))
+    again = tq1_matmul(shifted, torch.from_numpy(x).cuda(), out_dtype=torch.float32)
+    assert np.array_equal(again.cpu().numpy(), got)
+    check_status()

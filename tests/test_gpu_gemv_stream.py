@@ -186,3 +186,20 @@ def test_infinite_products_of_a_group(infinite, batch):
             assert np.array_equal(o.nonfinite_classes(got), o.nonfinite_classes(want))
             if infinite == 1 and not with_nan and len(groups) == 1:
                 assert np.isinf(got).any() and np.isnan(got).any()
+
+
+@pytest.mark.parametrize("rows,columns", [(17408, 5120), (3088, 16384)])
+def test_two_rows_of_a_large_matrix_equal_two_batch_1_calls(rows, columns):
+    """From 48 Mi weights on two activation rows are two passes of the batch-1 kernel in one launch: the bits of two calls."""
+    import torch
+    from ternel_b200.dispatch import plan
+    from ternel_b200.ops import tq1_matmul
+    from ternel_b200.stack import random_blocks_device
+    assert plan(2, rows, columns).kernel == "stream_gemv"
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(rows)
+    blocks = random_blocks_device(rows, columns, gen, "cuda")
+    x = torch.randn((2, columns), generator=gen, device="cuda").half()
+    both = tq1_matmul(blocks, x, out_dtype=torch.float32)
+    for m in range(2):
+        assert torch.equal(both[m:m + 1], tq1_matmul(blocks, x[m:m + 1], out_dtype=torch.float32))
