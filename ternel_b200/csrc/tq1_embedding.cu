@@ -7,9 +7,14 @@
 // Sixteen threads decode one 28-byte block into 128 outputs, eight consecutive outputs (one 16-byte
 // FP16 store, or two for FP32) per thread; a warp therefore writes 512 contiguous bytes. A thread's
 // eight trits start somewhere inside a code byte and span at most three: the bytes are looked up in a
-// 243-entry table of five 2-bit trits (global memory, L1-resident), concatenated and shifted. Every
-// output is one of three values per block, -1*s, 0*s, +1*s, computed once by multiplication (so that
-// 0*Inf and 0*NaN give NaN and zeros keep the sign NumPy gives them) and then selected by the trit.
+// table of five nibbles (twice the trit), joined and shifted, so that one multiply-add turns
+// every second nibble into a byte-permute selector. Every output is one of three values per block, -1*s, 0*s, +1*s,
+// computed once by multiplication (so that 0*Inf and 0*NaN give NaN and zeros keep the sign NumPy gives them) and
+// then selected by the trit.
+//
+// What bounds it: up to a wave or two of CTAs the chain id -> code bytes -> table entries -> store, beyond that the stores
+// (8192 tokens of 5120 columns: 21.4 us = 4.35 TB/s in FP16, 38.8 us = 5.3 TB/s in FP32). 2-bit trits unpacked one by one
+// took 123 instructions per eight outputs: 6.5 us for 2048 tokens against 6.06 now, 23.1 for 8192.
 #include "tq1_common.cuh"
 
 namespace tq1 {
@@ -17,17 +22,16 @@ namespace tq1 {
 namespace {
 
 struct TritTable {
-    uint16_t e[256];
+    uint32_t e[256];
 };
 constexpr TritTable make_trit_table() {
     TritTable t{};
     for (int v = 0; v < 243; ++v) {
-        int x = v, e = 0;
+        int x = v;
         for (int i = 0; i < 5; ++i) {
-            e |= (x % 3) << (2 * i);
+            t.e[v] |= (uint32_t)(2 * (x % 3)) << (4 * i);
             x /= 3;
         }
-        t.e[v] = (uint16_t)e;
     }
     return t;
 }
@@ -39,13 +43,17 @@ constexpr int kTokensPerThread = 4;
 
 }  // namespace
 
-template <bool OUT_F32>
+// SHARED: a CTA first copies the table to shared memory, which the few CTAs of a short call gain from; in a long one the
+// barrier behind the copy costs more than lookups through L1 (launch_embedding has the line and the figures).
+template <bool OUT_F32, bool SHARED>
 __global__ void __launch_bounds__(kThreadsPerBlockRow * kBlocksPerCta)
 embedding_kernel(const uint8_t *__restrict__ blocks, const int64_t *__restrict__ ids, void *__restrict__ out,
                  int64_t T, int64_t V, int gpr) {
     const int j = threadIdx.x & (kThreadsPerBlockRow - 1);      // which eight outputs of the block
     const int g = blockIdx.x * kBlocksPerCta + (threadIdx.x >> 4);
-    if (g >= gpr) return;
+    const bool in_row = g < gpr;                                // threads past the row only help to fill the table
+    __shared__ uint32_t shared_trits[SHARED ? 256 : 1];
+    const uint32_t *trits = SHARED ? shared_trits : g_trits.e;
     const int k0 = 8 * j;
     const int a = (k0 * 205) >> 10, off = k0 - 5 * a;            // k0 / 5 for k0 <= 120; first trit inside byte a
     const int64_t t0 = (int64_t)blockIdx.y * kTokensPerThread;
@@ -56,62 +64,73 @@ embedding_kernel(const uint8_t *__restrict__ blocks, const int64_t *__restrict__
     int64_t id[kTokensPerThread];
     bool live[kTokensPerThread];
 #pragma unroll
-    for (int q = 0; q < kTokensPerThread; ++q) id[q] = t0 + q < T ? ids[t0 + q] : -1;
+    for (int q = 0; q < kTokensPerThread; ++q) id[q] = in_row && t0 + q < T ? ids[t0 + q] : -1;
+    if (SHARED) {
+#pragma unroll
+        for (int i = 0; i < 256; i += kThreadsPerBlockRow * kBlocksPerCta)
+            shared_trits[i + threadIdx.x] = g_trits.e[i + threadIdx.x];
+    }
     const uint8_t *blk[kTokensPerThread];
     uint32_t sbits[kTokensPerThread], b0[kTokensPerThread], b1[kTokensPerThread], b2[kTokensPerThread];
 #pragma unroll
     for (int q = 0; q < kTokensPerThread; ++q) {
         live[q] = id[q] >= 0 && id[q] < V;
-        blk[q] = blocks + (size_t)((unsigned)(live[q] ? id[q] : 0) * (unsigned)gpr + (unsigned)g) * kBlockBytes;
+        blk[q] = blocks + (size_t)((unsigned)(live[q] ? id[q] : 0) * (unsigned)gpr + (unsigned)(in_row ? g : 0)) * kBlockBytes;
         sbits[q] = *reinterpret_cast<const unsigned short *>(blk[q]);
         b0[q] = __ldg(blk[q] + 2 + a);
         b1[q] = __ldg(blk[q] + 3 + a);
         b2[q] = off >= 3 ? __ldg(blk[q] + 4 + a) : 0u;          // the third byte exists whenever it is needed
     }
-    uint32_t sel[kTokensPerThread];                             // eight 2-bit trits, output i at bits 2i..2i+1
+    if (SHARED) __syncthreads();
+    if (!in_row) return;
+    uint32_t sel[kTokensPerThread];                             // eight nibbles, output i at bits 4i..4i+3
 #pragma unroll
     for (int q = 0; q < kTokensPerThread; ++q) {
-        const uint32_t stream = (uint32_t)g_trits.e[b0[q]] | ((uint32_t)g_trits.e[b1[q]] << 10) |
-                                ((uint32_t)g_trits.e[b2[q]] << 20);
-        sel[q] = (stream >> (2 * off)) & 0xffffu;
+        const uint32_t n0 = trits[b0[q]], n1 = trits[b1[q]], n2 = trits[b2[q]];
+        sel[q] = __funnelshift_r(n0 | (n1 << 20), (n1 >> 12) | (n2 << 8), 4 * off);
     }
 #pragma unroll
     for (int q = 0; q < kTokensPerThread; ++q) {
         if (t0 + q >= T) break;
-        const float scale = __half2float(__ushort_as_half((unsigned short)sbits[q]));
-        // a row outside the table is all zeros, not 0 * scale
-        const float c0 = live[q] ? -1.0f * scale : 0.0f, c1 = live[q] ? 0.0f * scale : 0.0f,
-                    c2 = live[q] ? 1.0f * scale : 0.0f;
+        const __half scale = __ushort_as_half((unsigned short)sbits[q]);
         const size_t base = ((size_t)(t0 + q) * gpr + g) * kGroup + 8 * j;
         if (!TQ1_IN_BOUNDS(base + 7, (size_t)T * gpr * kGroup, 30u)) continue;
         if (OUT_F32) {
+            // a row outside the table is all zeros, not 0 * scale
+            const float sf = __half2float(scale);
+            const float c0 = live[q] ? -1.0f * sf : 0.0f, c1 = live[q] ? 0.0f * sf : 0.0f, c2 = live[q] ? 1.0f * sf : 0.0f;
             float v[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const uint32_t trit = (sel[q] >> (2 * i)) & 3u;
-                v[i] = trit == 0 ? c0 : trit == 1 ? c1 : c2;
+                const uint32_t trit2 = sel[q] >> (4 * i) & 15u;
+                v[i] = trit2 == 0 ? c0 : trit2 == 2 ? c1 : c2;
             }
             float4 *dst = reinterpret_cast<float4 *>(static_cast<float *>(out) + base);
             dst[0] = make_float4(v[0], v[1], v[2], v[3]);
             dst[1] = make_float4(v[4], v[5], v[6], v[7]);
         } else {
-            // The three candidate halves sit in an 8-byte pool; one byte permute per output pair picks two
-            // of them. A trit t selects pool bytes 2t and 2t+1: selector nibbles (2t, 2t+1) = 0x10 + 0x22 * t.
-            const uint32_t h0 = __half_as_ushort(__float2half_rn(c0));
-            const uint32_t h1 = __half_as_ushort(__float2half_rn(c1));
-            const uint32_t h2 = __half_as_ushort(__float2half_rn(c2));
-            const uint32_t pool_lo = h0 | (h1 << 16), pool_hi = h2;
+            // The three candidate halves sit in an 8-byte pool. A trit t selects pool bytes 2t and 2t+1, selector nibbles
+            // (2t, 2t+1): a nibble n in a byte of its own becomes 0x11 * n + 0x10.
+            const __half2 c01 = __hmul2(__half2half2(scale), __floats2half2_rn(-1.0f, 0.0f));
+            const __half c2 = __hmul(scale, __float2half_rn(1.0f));
+            // a row outside the table is all zeros, not 0 * scale
+            const uint32_t pool_lo = live[q] ? reinterpret_cast<const uint32_t &>(c01) : 0u;
+            const uint32_t pool_hi = live[q] ? (uint32_t)__half_as_ushort(c2) : 0u;
+            const uint32_t even = (sel[q] & 0x0f0f0f0fu) * 0x11u + 0x10101010u;
+            const uint32_t odd = (sel[q] >> 4 & 0x0f0f0f0fu) * 0x11u + 0x10101010u;
             uint32_t w[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const uint32_t ta = (sel[q] >> (4 * i)) & 3u, tb = (sel[q] >> (4 * i + 2)) & 3u;
-                const uint32_t selector = 0x1010u + ta * 0x22u + tb * 0x2200u;
-                asm("prmt.b32 %0, %1, %2, %3;" : "=r"(w[i]) : "r"(pool_lo), "r"(pool_hi), "r"(selector));
-            }
+            for (int i = 0; i < 4; ++i)
+                w[i] = __byte_perm(pool_lo, pool_hi, __byte_perm(even, odd, 0x40u + 0x11u * i));
             *reinterpret_cast<uint4 *>(static_cast<__half *>(out) + base) = make_uint4(w[0], w[1], w[2], w[3]);
         }
     }
 }
+
+// Up to this many CTAs (two waves of sixteen per SM) the table goes through shared memory: 512 / 2048 / 8192 tokens of 5120
+// columns, FP16, take 3.03 / 6.06 / 22.7 us with it and 3.21 / 6.12 / 21.4 without; FP32 5.06 / 12.9 / 43.3 and
+// 5.23 / 13.7 / 38.8.
+constexpr long long kSharedTableCtas = 2 * 16 * 148;
 
 int launch_embedding(const uint8_t *blocks, const int64_t *ids, void *out, bool out_f32,
                      int64_t T, int64_t V, int K, cudaStream_t stream) {
@@ -120,14 +139,12 @@ int launch_embedding(const uint8_t *blocks, const int64_t *ids, void *out, bool 
     for (int64_t t0 = 0; t0 < T; t0 += per_launch) {
         const int64_t n = T - t0 < per_launch ? T - t0 : per_launch;
         dim3 grid((gpr + kBlocksPerCta - 1) / kBlocksPerCta, (unsigned)((n + kTokensPerThread - 1) / kTokensPerThread));
-        const int64_t *id_ptr = ids + t0;
-        if (out_f32) {
-            embedding_kernel<true><<<grid, kThreadsPerBlockRow * kBlocksPerCta, 0, stream>>>(
-                blocks, id_ptr, static_cast<float *>(out) + t0 * K, n, V, gpr);
-        } else {
-            embedding_kernel<false><<<grid, kThreadsPerBlockRow * kBlocksPerCta, 0, stream>>>(
-                blocks, id_ptr, static_cast<__half *>(out) + t0 * K, n, V, gpr);
-        }
+        const bool shared = (long long)grid.x * grid.y <= kSharedTableCtas;
+        void *first = out_f32 ? static_cast<void *>(static_cast<float *>(out) + t0 * K)
+                              : static_cast<void *>(static_cast<__half *>(out) + t0 * K);
+        auto kernel = out_f32 ? (shared ? embedding_kernel<true, true> : embedding_kernel<true, false>)
+                              : (shared ? embedding_kernel<false, true> : embedding_kernel<false, false>);
+        kernel<<<grid, kThreadsPerBlockRow * kBlocksPerCta, 0, stream>>>(blocks, ids + t0, first, n, V, gpr);
         cudaError_t err = cudaGetLastError();
         if (err != cudaSuccess) return cuda_fail(err, "tq1_embedding_f16: launch");
     }

@@ -56,6 +56,18 @@ def test_every_byte_value_and_every_scale_pattern():
     assert np.array_equal(got[finite].view(np.uint16), want[finite].view(np.uint16))
 
 
+@pytest.mark.parametrize("tokens", (18944, 18945))      # 4736 CTAs of four tokens, and one more: both homes of the table
+@pytest.mark.parametrize("dtype", (torch.float16, torch.float32))
+def test_both_sides_of_the_table_line(tokens, dtype):
+    blocks, rng = random_blocks(500, 128, seed=tokens)
+    ids = rng.integers(-1, 501, size=tokens)
+    npdt = np.float16 if dtype == torch.float16 else np.float32
+    inside = (ids >= 0) & (ids < 500)
+    want = o.get_rows(blocks, np.where(inside, ids, 0), rows=500, columns=128, dtype=npdt)
+    want[~inside] = 0
+    assert np.array_equal(gather(blocks, ids, dtype), want)
+
+
 def test_out_of_range_ids_give_zero_rows():
     blocks, rng = random_blocks(64, 256, seed=2)
     ids = np.array([0, 63, 64, -1, 1 << 40, -(1 << 40), 5], dtype=np.int64)
