@@ -29,9 +29,13 @@ int tq1_linear_f16(const uint8_t *blocks, const void *x, void *y, int y_is_f32,
     if (reinterpret_cast<uintptr_t>(x) & 15)
         return fail(TQ1_ERR_INVALID, "tq1_linear_f16: x must be 16-byte aligned");
     const size_t need = tq1_linear_workspace_bytes(M, N, K);
-    if (need && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255)))
-        return fail(TQ1_ERR_WORKSPACE, "tq1_linear_f16: workspace of %zu bytes (256-byte aligned) required", need);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (need && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255))) {
+        // the row kernel takes widths that are no multiple of 512 without a workspace (five tokens of 4099x2176: 45.8 us
+        // against the batched kernel's 12.1)
+        if (K % 512) return launch_gemv_rows(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, s);
+        return fail(TQ1_ERR_WORKSPACE, "tq1_linear_f16: workspace of %zu bytes (256-byte aligned) required", need);
+    }
     if (M == 1 && gemv_chain_fits(blocks, N, K))
         return launch_gemv_single(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, N, K, false, workspace,
                                   kWsSlotRegionBytes, s);

@@ -192,3 +192,20 @@ def test_widths_of_whole_groups(rows, columns, batch):
     again = tq1_matmul(shifted, torch.from_numpy(x).cuda(), out_dtype=torch.float32)
     assert np.array_equal(again.cpu().numpy(), got)
     check_status()
+
+
+@pytest.mark.parametrize(("rows", "columns", "batch"), ((256, 640, 8), (4099, 128, 2)))
+def test_other_widths_need_no_workspace(rows, columns, batch):
+    """Widths that are no multiple of 512: without a workspace the row kernel computes what the batched kernel does with
+    one. FP32 sums of at most 640 products in two orders: relative difference below 640 * 2^-24 = 4e-5."""
+    from ternel_b200 import _native
+    lib = _native.lib()
+    blocks, rng = random_blocks(rows, columns, seed=rows)
+    x = rng.standard_normal((batch, columns)).astype(np.float16)
+    bd, xd = torch.from_numpy(blocks).cuda(), torch.from_numpy(x).cuda()
+    assert lib.tq1_linear_workspace_bytes(batch, rows, columns) > 0
+    y = torch.empty((batch, rows), dtype=torch.float32, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    assert lib.tq1_linear_f16(bd.data_ptr(), xd.data_ptr(), y.data_ptr(), 1, batch, rows, columns, None, 0, stream) == 0
+    want = run_linear(blocks, x)
+    assert np.abs(y.cpu().numpy() - want).max() <= 4e-5 * np.abs(want).max()
