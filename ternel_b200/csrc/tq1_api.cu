@@ -74,7 +74,7 @@ int tq1_linear_plan(int M, int N, int K, int aligned, int *kernel, int *token_ti
     if (!kernel || !token_tile || !ctas || !parts) return fail(TQ1_ERR_INVALID, "tq1_linear_plan: null pointer");
     if (M <= 0 || N <= 0 || K <= 0 || K % kGroup) return fail(TQ1_ERR_INVALID, "tq1_linear_plan: bad shape");
     *token_tile = *ctas = *parts = 0;
-    if ((M == 1 || gemv_loop_preferred(M, N, K)) && aligned && gemv_chain_shape_ok(N, K)) {
+    if ((M == 1 || gemv_loop_preferred(M)) && aligned && gemv_chain_shape_ok(N, K)) {
         *kernel = TQ1_KERNEL_STREAM_GEMV;       // M > 1: one launch of M passes of the batch-1 kernel
     } else if (gemm_tc_preferred(aligned != 0, M, N, K)) {
         *kernel = TQ1_KERNEL_TENSOR_CORE;

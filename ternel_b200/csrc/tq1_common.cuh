@@ -87,11 +87,11 @@ bool gemv_chain_shape_ok(int N, int K);
 bool gemv_chain_supported(const uint8_t *blocks, int N, int K);
 bool gemv_chain_fits(const uint8_t *blocks, int N, int K);      // also checks the current device's SM count
 size_t gemv_chain_workspace_bytes(int N, int K);
-// a few activation rows as M links of one launch over the same weights, where that is the better choice
+// a few activation rows as M links of one launch over the same weights
 bool gemv_looped_fits(const uint8_t *blocks, int M, int N, int K);
 int launch_gemv_looped(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, bool swiglu,
                        void *workspace, cudaStream_t stream);
-bool gemv_loop_preferred(int M, int N, int K);
+bool gemv_loop_preferred(int M);
 int gemv_set_loop_tokens(int tokens);       // sweep recording only; process-global
 // slot_bytes: room for partial-sum slots behind the workspace's control words
 int launch_gemv_single(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int N, int K, bool swiglu,

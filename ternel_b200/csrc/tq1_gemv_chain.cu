@@ -1279,20 +1279,20 @@ int launch_gemv_looped(const uint8_t *blocks, const __half *x, void *y, bool y_f
                              kRegionSlotsTwo, 2, stream);
 }
 
-// Largest M that tq1_linear_f16 sends through launch_gemv_looped (0 or 1: none), and the smallest matrix (weights) it does
-// so for: below it the batched kernel's shorter reduction wins (two tokens on 5120x5120: 11.0 us against 12.3).
+// Largest M that tq1_linear_f16 sends through launch_gemv_looped (0 or 1: none). Every matrix that the batch-1 kernel takes
+// goes this way, because its sums are exact integers per group: two tokens of 5120x5120 are 7e-8 from the FP64 result
+// (2-norm) against 1.2e-6 of the batched kernel's FP32 accumulators. Two tokens, weights out of HBM, this path and the
+// batched kernel: 1024x5120 8.9 and 9.7 us, 5120x5120 11.6 and 10.8, 17408x5120 19.0 and 17.9.
 static int g_loop_tokens = 2;
-static long long g_loop_weights = 48ll << 20;
-bool gemv_loop_preferred(int M, int N, int K) { return M >= 2 && M <= g_loop_tokens && (long long)N * K >= g_loop_weights; }
+bool gemv_loop_preferred(int M) { return M >= 2 && M <= g_loop_tokens; }
 int gemv_set_loop_tokens(int tokens) {
     if (tokens < 0 || tokens > kInlineLinks) return TQ1_ERR_INVALID;
     g_loop_tokens = tokens;
-    g_loop_weights = 0;                         // a sweep times every size
     return TQ1_OK;
 }
 // The looped path takes the shape when one link holds the whole matrix in one slot region of the two.
 bool gemv_looped_fits(const uint8_t *blocks, int M, int N, int K) {
-    if (!gemv_loop_preferred(M, N, K) || !gemv_chain_supported(blocks, N, K)) return false;
+    if (!gemv_loop_preferred(M) || !gemv_chain_supported(blocks, N, K)) return false;
     int grid = 0;
     if (gemv_chain_grid(&grid) != TQ1_OK) return false;
     if (rows_per_link(N, K, kRegionSlotsTwo) != N) return false;

@@ -71,9 +71,10 @@ def load_sweep(path: Path = SWEEP_PATH) -> dict:
     return json.loads(Path(path).read_text())
 
 
-def record_sweep(batches=SWEEP_BATCHES, shapes=SWEEP_SHAPES, tiles=TOKEN_TILES, ring: int = 6, replays: int = 3) -> dict:
-    """Time every (batch, shape, token tile) on the current GPU: CUDA-graph replays over a ring of
-    distinct weight buffers, CUDA events. Returns the JSON-ready record."""
+def record_sweep(batches=SWEEP_BATCHES, shapes=SWEEP_SHAPES, tiles=TOKEN_TILES, replays: int = 3) -> dict:
+    """Time every (batch, shape, token tile) on the current GPU: CUDA-graph replays over a ring of distinct weight
+    buffers of more than twice the L2 cache, so that every call reads its weights from HBM, CUDA events. Returns the
+    JSON-ready record."""
     import torch
     from .stack import random_blocks_device
 
@@ -117,7 +118,9 @@ def record_sweep(batches=SWEEP_BATCHES, shapes=SWEEP_SHAPES, tiles=TOKEN_TILES, 
 
     try:
         for rows, columns in shapes:
-            weights = [random_blocks_device(rows, columns, gen, device) for _ in range(ring)]
+            packed = random_blocks_device(rows, columns, gen, device)
+            ring = 2 * torch.cuda.get_device_properties(device).L2_cache_size // packed.numel() + 1
+            weights = [packed.clone() for _ in range(ring)]
             for batch in batches:
                 x = torch.randn((batch, columns), generator=gen, device=device).to(torch.float16)
                 y = torch.empty((batch, rows), dtype=torch.float16, device=device)
@@ -138,8 +141,7 @@ def record_sweep(batches=SWEEP_BATCHES, shapes=SWEEP_SHAPES, tiles=TOKEN_TILES, 
     finally:
         check(lib.tq1_debug_force_token_tile(0))
         check(lib.tq1_debug_set_loop_tokens(default_loop))
-    return {"device": torch.cuda.get_device_name(device), "ring_buffers": ring,
-            "unit": "microseconds per call, CUDA-graph replays, distinct weight buffers", "cases": cases}
+    return {"device": torch.cuda.get_device_name(device), "unit": "microseconds per call, CUDA-graph replays, distinct weight buffers of more than twice L2", "cases": cases}
 
 
 def main() -> None:

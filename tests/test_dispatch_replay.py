@@ -35,3 +35,22 @@ def test_plan_boundaries():
     assert plan(192, 17408, 5120).token_tile == 256            # one 256-row tile beats two 128-row tiles
     with pytest.raises(ValueError):
         plan(0, 128, 512)
+
+
+def test_two_rows_of_any_matrix_take_the_exact_kernel():
+    """Two activation rows of every matrix that the batch-1 kernel takes are two passes of it (exact integer group
+    sums), and recording a sweep leaves that rule as it found it."""
+    import ctypes
+    from ternel_b200 import _native
+    from ternel_b200.dispatch import looped_tokens
+    shapes = [(16, 512), (1024, 5120), (5120, 5120), (4096, 4096), (17408, 5120)]
+    assert looped_tokens() == 2
+    for rows, columns in shapes:
+        assert plan(2, rows, columns).kernel == "stream_gemv"
+        assert plan(3, rows, columns).kernel == "tensor_core"
+    setter = _native.lib().tq1_debug_set_loop_tokens           # what record_sweep does around its timings
+    setter.argtypes, before = [ctypes.c_int], looped_tokens()
+    assert setter(0) == 0 and plan(2, 17408, 5120).kernel == "tensor_core"
+    assert setter(before) == 0
+    for rows, columns in shapes:
+        assert plan(2, rows, columns).kernel == "stream_gemv"

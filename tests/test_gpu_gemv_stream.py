@@ -188,12 +188,13 @@ def test_infinite_products_of_a_group(infinite, batch):
                 assert np.isinf(got).any() and np.isnan(got).any()
 
 
-@pytest.mark.parametrize("rows,columns", [(17408, 5120), (3088, 16384)])
+@pytest.mark.parametrize("rows,columns", [(48, 512), (1024, 5120), (5120, 5120), (17408, 5120), (3088, 16384)])
 def test_two_rows_of_a_large_matrix_equal_two_batch_1_calls(rows, columns):
-    """From 48 Mi weights on two activation rows are two passes of the batch-1 kernel in one launch: the bits of two calls."""
+    """Two activation rows are two passes of the batch-1 kernel in one launch: the bits of two calls, and within 1e-6 of
+    the FP64 product (exact integer group sums, one FP32 rounding per group; one FP32 sum over the columns is not)."""
     import torch
     from ternel_b200.dispatch import plan
-    from ternel_b200.ops import tq1_matmul
+    from ternel_b200.ops import tq1_get_rows, tq1_matmul
     from ternel_b200.stack import random_blocks_device
     assert plan(2, rows, columns).kernel == "stream_gemv"
     gen = torch.Generator(device="cuda")
@@ -203,3 +204,6 @@ def test_two_rows_of_a_large_matrix_equal_two_batch_1_calls(rows, columns):
     both = tq1_matmul(blocks, x, out_dtype=torch.float32)
     for m in range(2):
         assert torch.equal(both[m:m + 1], tq1_matmul(blocks, x[m:m + 1], out_dtype=torch.float32))
+    dense = tq1_get_rows(blocks, torch.arange(rows, device="cuda"), dtype=torch.float32).double()
+    want = x.double() @ dense.T
+    assert float((both.double() - want).norm() / want.norm()) < 1e-6
