@@ -241,3 +241,28 @@ def test_parts_of_several_threads_agree_with_one():
         packed[0, 2], packed[-1, 27] = 243, 27
         with pytest.raises(tb.FormatError, match="regular=1, tail=1"):
             tb.decode_tq1_blocks(packed)
+
+
+@pytest.mark.parametrize("groups,at", [(4, 300), (40961, 0), (40961, 40961 * 128 - 1)])
+def test_refused_calls_write_nothing(groups, at):
+    """One illegal trit, in any part of any thread: the error, its count, and an output buffer that was not touched."""
+    import ctypes
+    from ternel_b200 import _native
+    lib = _native.lib()
+    rng = np.random.default_rng(9)
+    trits = rng.integers(0, 3, groups * 128, dtype=np.uint8)
+    trits[at] = 7
+    scales = rng.integers(0, 256, (groups, 2), dtype=np.uint8)
+    blocks = np.full((groups, 28), 170, dtype=np.uint8)
+    bad = ctypes.c_int64(-1)
+    assert lib.tq1_pack_blocks(scales.ctypes.data, trits.ctypes.data, blocks.ctypes.data, groups,
+                               ctypes.byref(bad)) == _native.TQ1_ERR_FORMAT
+    assert bad.value == 1 and (blocks == 170).all()
+    trits[at] = 2
+    assert lib.tq1_pack_blocks(scales.ctypes.data, trits.ctypes.data, blocks.ctypes.data, groups, ctypes.byref(bad)) == 0
+    blocks[groups // 2, 27] = 27
+    out_scales, out_trits = np.full((groups, 2), 170, np.uint8), np.full((groups, 128), 170, np.uint8)
+    full, tail = ctypes.c_int64(), ctypes.c_int64()
+    assert lib.tq1_unpack_blocks(blocks.ctypes.data, out_scales.ctypes.data, out_trits.ctypes.data, groups, 1,
+                                 ctypes.byref(full), ctypes.byref(tail)) == _native.TQ1_ERR_FORMAT
+    assert (full.value, tail.value) == (0, 1) and (out_scales == 170).all() and (out_trits == 170).all()
