@@ -112,10 +112,11 @@ embedding_kernel(const uint8_t *__restrict__ blocks, const int64_t *__restrict__
             // The three candidate halves sit in an 8-byte pool. A trit t selects pool bytes 2t and 2t+1, selector nibbles
             // (2t, 2t+1): a nibble n in a byte of its own becomes 0x11 * n + 0x10.
             const __half2 c01 = __hmul2(__half2half2(scale), __floats2half2_rn(-1.0f, 0.0f));
-            const __half c2 = __hmul(scale, __float2half_rn(1.0f));
+            // 1 * s, which the compiler takes for s itself: a NaN scale gives the NaN 0x7fff that a multiplication gives
+            const uint32_t c2 = __hisnan(scale) ? 0x7fffu : sbits[q];
             // a row outside the table is all zeros, not 0 * scale
             const uint32_t pool_lo = live[q] ? reinterpret_cast<const uint32_t &>(c01) : 0u;
-            const uint32_t pool_hi = live[q] ? (uint32_t)__half_as_ushort(c2) : 0u;
+            const uint32_t pool_hi = live[q] ? c2 : 0u;
             const uint32_t even = (sel[q] & 0x0f0f0f0fu) * 0x11u + 0x10101010u;
             const uint32_t odd = (sel[q] >> 4 & 0x0f0f0f0fu) * 0x11u + 0x10101010u;
             uint32_t w[4];

@@ -110,3 +110,20 @@ def test_full_vocabulary_table_round_trip():
     want = o.get_rows(blocks, ids[:-1], rows=rows, columns=columns, dtype=np.float16)
     assert np.array_equal(got[:-1].view(np.uint16), want.view(np.uint16))
     assert not got[-1].any()
+
+
+@pytest.mark.parametrize("rows_named", (2000, 65536))           # table in shared memory, table in L1
+def test_every_scale_pattern_gives_the_bits_of_a_multiplication(rows_named):
+    """-1 * s, 0 * s and 1 * s for all 65536 FP16 scales, FP16 out, bit for bit: signed zeros, subnormals, infinities
+    (0 * Inf is NaN), and the one NaN 0x7fff whatever the payload and sign of a NaN scale."""
+    rng = np.random.default_rng(3)
+    trits = rng.integers(0, 3, size=(65536, 128)).astype(np.uint8)
+    bits = np.arange(65536, dtype=np.uint16)
+    blocks = o.encode_blocks(bits.view(np.uint8).reshape(-1, 2), trits).reshape(65536, 1, 28)
+    ids = np.arange(65536) if rows_named == 65536 else np.concatenate([np.arange(0x7bf0, 0x7bf0 + 1000),
+                                                                       np.arange(0xfbf0, 0xfbf0 + 1000)])
+    with np.errstate(invalid="ignore"):
+        want = ((trits[ids].astype(np.float32) - 1) * bits.view(np.float16)[ids].astype(np.float32)[:, None]).astype(np.float16)
+    want = np.where(np.isnan(want), np.uint16(0x7fff), want.view(np.uint16))
+    got = gather(blocks, ids, torch.float16)
+    assert np.array_equal(got.view(np.uint16), want)
