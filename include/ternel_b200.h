@@ -150,6 +150,7 @@ int tq1_linear_swiglu_f16(const uint8_t *blocks, const void *x, void *y, int y_i
 #define TQ1_KERNEL_ROWS 0
 #define TQ1_KERNEL_STREAM_GEMV 1
 #define TQ1_KERNEL_TENSOR_CORE 2
+#define TQ1_KERNEL_GROUP_SUMS 3
 int tq1_linear_plan(int M, int N, int K, int aligned, int *kernel, int *token_tile, int *ctas, int *parts);
 
 /* ---- row-sharded linear over several GPUs -------------------------------- */

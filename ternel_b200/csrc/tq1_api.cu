@@ -11,9 +11,9 @@ extern "C" {
 size_t tq1_linear_workspace_bytes(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0 || K % kGroup) return 0;
     if (M == 1 && gemv_chain_shape_ok(N, K)) return gemv_chain_workspace_bytes(N, K);
-    // blocks that turn out not to be 16-byte aligned may take the kernel for fewer shapes, never for more
-    if (gemm_tc_preferred(true, M, N, K)) return gemm_tc_workspace_bytes(M, N, K);
-    return 0;
+    if (gemm_tc_shape_ok(M, N, K)) return gemm_tc_workspace_bytes(M, N, K);
+    // the kernel for the other widths runs without a workspace; a caller that has one finds its status word in place
+    return gemm_groups_preferred(M, N, K) ? kWsStatusBytes : 0;
 }
 
 int tq1_linear_f16(const uint8_t *blocks, const void *x, void *y, int y_is_f32,
@@ -30,19 +30,17 @@ int tq1_linear_f16(const uint8_t *blocks, const void *x, void *y, int y_is_f32,
         return fail(TQ1_ERR_INVALID, "tq1_linear_f16: x must be 16-byte aligned");
     const size_t need = tq1_linear_workspace_bytes(M, N, K);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (need && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255))) {
-        // the row kernel takes widths that are no multiple of 512 without a workspace (five tokens of 4099x2176: 45.8 us
-        // against the batched kernel's 12.1)
-        if (K % 512) return launch_gemv_rows(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, s);
+    if (need && K % 512 == 0 && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255)))
         return fail(TQ1_ERR_WORKSPACE, "tq1_linear_f16: workspace of %zu bytes (256-byte aligned) required", need);
-    }
     if (M == 1 && gemv_chain_fits(blocks, N, K))
         return launch_gemv_single(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, N, K, false, workspace,
                                   kWsSlotRegionBytes, s);
     if (gemv_looped_fits(blocks, M, N, K) && need >= kWsScratchOffset)
         return launch_gemv_looped(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, false, workspace, s);
-    if (gemm_tc_preferred((reinterpret_cast<uintptr_t>(blocks) & 15) == 0, M, N, K))
+    if ((reinterpret_cast<uintptr_t>(blocks) & 15) == 0 && gemm_tc_shape_ok(M, N, K))
         return launch_gemm_tc(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, workspace, s);
+    if (gemm_groups_preferred(M, N, K))
+        return launch_gemm_groups(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, s);
     return launch_gemv_rows(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, s);
 }
 
@@ -76,9 +74,11 @@ int tq1_linear_plan(int M, int N, int K, int aligned, int *kernel, int *token_ti
     *token_tile = *ctas = *parts = 0;
     if ((M == 1 || gemv_loop_preferred(M)) && aligned && gemv_chain_shape_ok(N, K)) {
         *kernel = TQ1_KERNEL_STREAM_GEMV;       // M > 1: one launch of M passes of the batch-1 kernel
-    } else if (gemm_tc_preferred(aligned != 0, M, N, K)) {
+    } else if (aligned && gemm_tc_shape_ok(M, N, K)) {
         *kernel = TQ1_KERNEL_TENSOR_CORE;
         gemm_tc_plan(M, N, K, token_tile, ctas, parts);
+    } else if (gemm_groups_preferred(M, N, K)) {
+        *kernel = TQ1_KERNEL_GROUP_SUMS;
     } else {
         *kernel = TQ1_KERNEL_ROWS;
     }

@@ -103,10 +103,8 @@ int launch_epoch_advance(unsigned *epoch_base, unsigned delta, cudaStream_t stre
 int gemv_noalloc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int N, int K, cudaStream_t stream);
 int gemv_noalloc_status(unsigned *out_host, cudaStream_t stream);
 
-// Batched linear (M >= 2) on tcgen05 tensor cores; needs 16-byte aligned activations.
+// Batched linear (M >= 2) on tcgen05 tensor cores; needs K % 512 == 0 and 16-byte aligned pointers.
 bool gemm_tc_shape_ok(int M, int N, int K);
-// whether the kernel is the better choice for the shape (aligned: blocks on a 16-byte boundary)
-bool gemm_tc_preferred(bool aligned, int M, int N, int K);
 size_t gemm_tc_workspace_bytes(int M, int N, int K);
 int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K,
                    void *workspace, cudaStream_t stream, bool swiglu = false);
@@ -115,6 +113,11 @@ int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, 
 __host__ __device__ inline float swiglu_f32(float gate, float up) { return gate / (1.0f + expf(-gate)) * up; }
 void gemm_tc_plan(int M, int N, int K, int *tile, int *ctas, int *parts);
 int gemm_tc_force_tile(int nt);
+
+// Batched linear (M >= 2) with an FP32 sum per group, for every other width and alignment.
+bool gemm_groups_preferred(int M, int N, int K);
+int launch_gemm_groups(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K,
+                       cudaStream_t stream);
 
 // Five base-3 digits of a byte packed two bits each (digit i at bits 2i..2i+1).
 __host__ __device__ inline uint32_t trits_2bit(uint32_t byte) {

@@ -12,12 +12,13 @@
 // The unit of work is a chunk of a tile: 4 K blocks of 128 columns = 112 packed bytes per row. A segment is a run of
 // consecutive chunks of one tile; a CTA (pair) walks the segments it was dealt.
 //   decode warps (G groups of four)  A group takes every G-th chunk of a segment. Its warp q fetches the packed bytes
-//        of rows 32q..32q+31 of the chunk into a buffer of its own (TMA, or 4-byte cp.async where rows are not
-//        16-byte aligned), so decoding needs no barrier between warps before the operand is complete. Thread = weight
-//        row: code byte -> 8-byte table entry of PRMT selectors -> pairs of FP16 weights picked out of
-//        [0, s_lo, s_hi, s_hi ^ 0x80] -> 32 registers = 64 K columns, stored to the row's lane of tensor memory.
+//        of rows 32q..32q+31 of the chunk into a buffer of its own by TMA, so decoding needs no barrier between warps
+//        before the operand is complete. Thread = weight row: code byte -> 8-byte table entry of PRMT selectors ->
+//        pairs of FP16 weights picked out of [0, s_lo, s_hi, s_hi ^ 0x80] -> 32 registers = 64 K columns, stored to the
+//        row's lane of tensor memory.
 //        All groups also read out finished accumulators and store the results.
-//   one warp   issues tcgen05.mma for the halves (64 K columns) in a fixed order: chunk wave, K block, group, half
+//   one warp   issues tcgen05.mma for the halves (64 K columns) in a fixed order: chunk wave, K block, group, half; up to 128
+//        tokens the K blocks take turns on two accumulators, which are added when the segment is read out
 //   one warp   fetches the activation tiles in the same order
 // Shared memory traffic of the table bounds the decode (two 128-byte wavefronts per 32 code bytes), so decode warps are
 // many and keep no state between chunks. Weights are decoded in natural column order (a byte's five trits straddle
@@ -27,6 +28,10 @@
 // Segments that cover only a part of a tile's K range leave an FP32 partial tile in the workspace; the CTA that finishes
 // the tile's last part (a counter per tile) adds the parts in ascending K order, so results never depend on timing, and no
 // CTA waits for another. A separate launch for these sums cost 3 to 14 us.
+//
+// Precision: the tensor core adds to an accumulator by truncation, so the error grows with the columns that one accumulator
+// covers: 6.3e-7 of the result (2-norm) for 512, 1.2e-6 for 1024, 3.0e-6 for 2560. Two accumulators halve it. Shares of
+// tiles are spread evenly (WorkSplit::first_iter), so that few tiles stay in one piece.
 #include <cuda.h>
 #include <math.h>
 
@@ -46,7 +51,8 @@ constexpr uint32_t kSpinLimit = 1u << 20;
 // Variants:
 //   S  up to 32 tokens: two CTAs per SM with two decode groups each hide each other's latencies; the narrow table
 //      (one 8-byte entry per byte and lane pair, 32 KB) leaves room for that
-//   L  33..128 tokens: one CTA per SM, four groups, wide table (even and odd entries, 64 KB)
+//   M  33..64, L  65..128 tokens: one CTA per SM, four groups, wide table (even and odd entries, 64 KB); they differ in
+//      how tensor memory is shared between accumulators and decoded weights
 //   P  larger: CTA pairs (cta_group::2), each CTA holds half of the activation tile, which halves the activation
 //      traffic out of L2 and through shared memory
 template <int CG_, int G_, bool WIDE_, int PACK_STAGES_, int RING_, int MAX_COLS_>
@@ -54,11 +60,12 @@ struct Variant {
     static constexpr int CG = CG_, G = G_, PACK_STAGES = PACK_STAGES_;
     static constexpr bool WIDE = WIDE_;
     static constexpr int RING = RING_;                              // K blocks of decoded weights in tensor memory
-    static constexpr int MAX_COLS = MAX_COLS_;                      // accumulator columns
+    static constexpr int MAX_COLS = MAX_COLS_;                      // columns of an accumulator
+    static constexpr int ACCS = CG == 1 ? 2 : 1;                    // accumulators that the K blocks take turns on
     static constexpr int kDecodeWarps = 4 * G;
     static constexpr int kThreads = 32 * (kDecodeWarps + 2);
     static constexpr int kGroupCols = MAX_COLS / G < 16 ? 16 : MAX_COLS / G;      // columns a group reads out
-    static constexpr int kABase = MAX_COLS < 32 ? 32 : MAX_COLS;
+    static constexpr int kABase = ACCS * MAX_COLS;
     static constexpr int kTmemCols = G == 2 ? 256 : 512;
     static_assert(kABase + RING * kStageCols <= kTmemCols, "tensor memory budget");
     static constexpr int kMinCtas = G == 2 ? 2 : 1;
@@ -83,7 +90,8 @@ struct Variant {
     }
 };
 using VariantS = Variant<1, 2, false, 2, 3, 32>;
-using VariantL = Variant<1, 4, true, 1, 6, 128>;
+using VariantM = Variant<1, 4, true, 1, 6, 64>;
+using VariantL = Variant<1, 4, true, 1, 4, 128>;
 using VariantP = Variant<2, 4, true, 1, 4, 256>;
 
 // Table entries. An 8-bit selector picks the two bytes of one FP16 weight out of the pool [0x00, s_lo, s_hi, s_hi ^ 0x80]:
@@ -277,13 +285,13 @@ struct Divisor {
 //     on are cut into equal contiguous ranges of chunks, one per slot (stream-K), so that all slots do the same number.
 struct WorkSplit {
     int total_iters, slots, chunks, splits;
-    int quot, rem;                              // total_iters = slots * quot + rem: the first `rem` ranges get one more
     int whole_rounds, whole_tiles;
     int tiles_total;                            // output tiles of the call (a slot's last whole tiles may lie beyond)
-    Divisor by_splits, by_chunks;
+    Divisor by_splits, by_chunks, by_slots;
     __host__ __device__ __forceinline__ int first_iter(int slot) const {
         if (slot >= slots) return total_iters;
-        if (splits == 0) return slot * quot + (slot < rem ? slot : rem);
+        // the shares of one chunk more lie between the others: side by side they would end where tiles end
+        if (splits == 0) return by_slots.div(slot * total_iters);
         const int tile = by_splits.div(slot), part = slot - tile * splits;
         return tile * chunks + by_splits.div(chunks * part);
     }
@@ -318,7 +326,6 @@ struct SegmentWalk {
 };
 
 struct GemmParams {
-    const uint8_t *blocks;
     void *y;                  // [M][N] (FP16/FP32), with swiglu [M][N / 2]
     float *partials;          // [2 * CTAs][nt][128] FP32
     unsigned *counters;       // per shared tile (and CTA of a pair): parts stored so far; zero between calls
@@ -332,7 +339,7 @@ struct GemmParams {
     int y_f32, swiglu;
 };
 
-template <class V, bool TMA_W>
+template <class V>
 __global__ void __launch_bounds__(V::kThreads, V::kMinCtas)
 tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
                 const __grid_constant__ GemmParams prm) {
@@ -414,7 +421,7 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
     // the decoded weights and stage i % b_stages (<= RING) of the activations. EMPTY[i % RING] completes when its MMAs have
     // read both, one commit for decoders and activations alike.
     // A wave is the G chunks (fewer at a segment's end) that the groups decode side by side; its blocks are ordered by K
-    // block first. Only a matrix row's last chunk can have fewer than four.
+    // block first.
     if (warp == kXWarp) {
         // ------------------------------------------------------------------ activation tiles
         if (elect_one()) {
@@ -428,7 +435,6 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                     for (int kb = 0; kb < kChunkGroups; ++kb) {
                         for (int g = 0; g < width; ++g) {
                             const int k = k0 + g * kChunkGroups + kb;
-                            if (k >= prm.groups) continue;
                             if (filled < (uint32_t)prm.b_stages) {
                                 ++filled;
                             } else {
@@ -456,7 +462,7 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                 const int n_tok = tile_tokens(token_tile0(tile));
                 // FP32 accumulate, FP16 A and B, both K-major, M = 128 per CTA, N = tokens
                 const uint32_t idesc = (1u << 4) | ((uint32_t)(n_tok >> 3) << 17) | ((uint32_t)(kTileW * CG >> 4) << 24);
-                const int blocks = min(len * kChunkGroups, prm.groups - c0 * kChunkGroups);
+                const int blocks = len * kChunkGroups;
                 if (seg > 0) mbar_wait(bar(ACC_FREE), (seg - 1) & 1u, prm.status, dead);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (int i = 0; i < blocks; ++i) {
@@ -467,10 +473,11 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                     const uint32_t a_tmem = tmem_base + (uint32_t)V::kABase + astage * kStageCols;
                     const uint32_t b_addr = wbase + V::kBAddr + bstage * b_bytes;
                     const uint64_t b_lo = umma_desc(b_addr), b_hi = umma_desc(b_addr + b_bytes / 2);
+                    const uint32_t acc = tmem_base + (V::ACCS == 2 && (i & 1) ? (uint32_t)V::MAX_COLS : 0u);
 #pragma unroll
                     for (int j = 0; j < 8; ++j)                    // K = 16 steps: four of each 64-wide swizzle atom
-                        umma_f16_ts<CG>(tmem_base, a_tmem + 8u * j, (j < 4 ? b_lo : b_hi) + 2u * (j & 3), idesc,
-                                        (i > 0 || j > 0) ? 1u : 0u);
+                        umma_f16_ts<CG>(acc, a_tmem + 8u * j, (j < 4 ? b_lo : b_hi) + 2u * (j & 3), idesc,
+                                        (i >= V::ACCS || j > 0) ? 1u : 0u);
                     umma_commit<CG>(bar(EMPTY + astage));
                     if (++astage == RING) { astage = 0; aphase ^= 1u; }
                     if (++bstage == (uint32_t)prm.b_stages) { bstage = 0; bphase ^= 1u; }
@@ -485,40 +492,22 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         const int row_in_tile = quad * 32 + lane;                       // = tensor-memory lane
         const uint32_t tmem_lane = tmem_base + ((uint32_t)(quad * 32) << 16);
         const uint32_t lane_entry = wbase + V::kTableAddr + (uint32_t)(lane & 15) * 8u;
-        const size_t row_bytes = (size_t)prm.groups * kBlockBytes;
 
         // cursor of the packed bytes this warp requests ahead of its decoding
         SegmentWalk pwalk(prm.work, slot);
         int p_tile = 0, p_c0 = 0, p_len = 0, p_part, p_unit = group;
         uint32_t requested = 0, consumed = 0;
         auto request = [&]() {
-            bool more = true;
             while (p_unit >= p_len) {
-                if (!pwalk.next(p_tile, p_c0, p_len, p_part)) { p_len = 0; more = false; break; }
+                if (!pwalk.next(p_tile, p_c0, p_len, p_part)) { p_len = 0; return; }
                 p_unit = group;
             }
             const uint32_t s = requested % V::PACK_STAGES;
-            const int chunk = p_c0 + p_unit, n0 = (weight_tile(p_tile) * CG + rank) * kTileW + quad * 32;
-            const uint32_t dst = wbase + V::pack_addr(warp, (int)s);
-            if (more) {
-                if (TMA_W) {
-                    elected_load_packed(dst, &wmap, chunk * kChunkBytes, n0, bar(PACK + warp * V::PACK_STAGES + (int)s));
-                } else if (lane < kChunkBytes / 4) {
-                    // rows whose byte length is no multiple of 16 cannot be a tensor map's: one row per instruction
-                    const bool in_row = chunk * kChunkBytes + lane * 4 < (int)row_bytes;
-                    const uint8_t *src = prm.blocks + (in_row ? (size_t)chunk * kChunkBytes + lane * 4 : 0);
-#pragma unroll 8
-                    for (int r = 0; r < 32; ++r) {
-                        const bool live = in_row && n0 + r < prm.N;
-                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;"
-                                     ::"r"(dst + (uint32_t)(r * kChunkBytes + lane * 4)),
-                                       "l"(src + (live ? (size_t)(n0 + r) * row_bytes : 0)), "r"(live ? 4 : 0) : "memory");
-                    }
-                }
-                ++requested;
-                p_unit += G;
-            }
-            if (!TMA_W) asm volatile("cp.async.commit_group;" ::: "memory");       // one group per call, empty at the end
+            const int n0 = (weight_tile(p_tile) * CG + rank) * kTileW + quad * 32;
+            elected_load_packed(wbase + V::pack_addr(warp, (int)s), &wmap, (p_c0 + p_unit) * kChunkBytes, n0,
+                                bar(PACK + warp * V::PACK_STAGES + (int)s));
+            ++requested;
+            p_unit += G;
         };
 #pragma unroll
         for (int s = 0; s < V::PACK_STAGES; ++s) request();
@@ -530,19 +519,11 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         while (walk.next(tile, c0, len, part)) {
             for (int u0 = 0; u0 < len; u0 += G) {
                 const int width = min(G, len - u0), unit = u0 + group;
-                // the wave's last chunk may be short; blocks past its end are missing from the numbering
-                const int last_blocks = min(kChunkGroups, prm.groups - (c0 + u0 + width - 1) * kChunkGroups);
                 const int wave0 = block0;
-                block0 += (width - 1) * kChunkGroups + last_blocks;
+                block0 += width * kChunkGroups;
                 if (unit >= len) continue;
-                const int blocks_here = group == width - 1 ? last_blocks : kChunkGroups;
                 const uint32_t s = consumed % V::PACK_STAGES;
-                if (TMA_W) {
-                    mbar_wait(bar(PACK + warp * V::PACK_STAGES + (int)s), (consumed / V::PACK_STAGES) & 1u, prm.status, dead);
-                } else {
-                    asm volatile("cp.async.wait_group %0;" ::"n"(V::PACK_STAGES - 1) : "memory");
-                    __syncwarp();
-                }
+                mbar_wait(bar(PACK + warp * V::PACK_STAGES + (int)s), (consumed / V::PACK_STAGES) & 1u, prm.status, dead);
                 // This row's 112 bytes come into registers in two steps (all at once spills); after the second the
                 // buffer is free for the next request.
                 uint32_t words[4 * 7];
@@ -563,7 +544,6 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                         __syncwarp();
                         request();
                     }
-                    if (b >= blocks_here) continue;
                     const uint32_t *w = words + 7 * b;
                     const uint32_t pool = (w[0] << 16 >> 8) | (((w[0] & 0xff00u) ^ 0x8000u) << 16);
                     // table entry of code byte j
@@ -583,7 +563,7 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                     };
                     // trit 4 of an even byte beside trit 0 of the odd byte after it
                     auto straddle = [&](uint32_t p0, uint32_t q0) { return pick(prmt(p0, q0, V::WIDE ? 0x0062 : 0x0042)); };
-                    const uint32_t number = (uint32_t)(wave0 + b * width - max(b - last_blocks, 0) + group);
+                    const uint32_t number = (uint32_t)(wave0 + b * width + group);
                     const uint32_t stage = number % RING, use = number / RING;
                     const uint32_t a_addr = tmem_lane + (uint32_t)V::kABase + stage * kStageCols;
                     uint32_t m0w, m1w;                                  // byte 12 belongs to both halves
@@ -654,19 +634,29 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
             mbar_wait(bar(ACC_FULL), seg & 1u, prm.status, dead);
             ++seg;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            constexpr int kStep = V::kGroupCols < 32 ? V::kGroupCols : 32;                     // columns in registers at a time
+            constexpr int kStep = V::ACCS == 2 ? 16 : 32;                                      // columns in registers at a time
+            static_assert(V::kGroupCols % kStep == 0, "whole steps");
             const bool whole = len == chunks;
             const size_t area = (size_t)prm.nt * kTileW;
             float *slot_part = prm.partials + ((size_t)2 * blockIdx.x + part) * area + row_in_tile;
 #pragma unroll
             for (int s0 = 0; s0 < V::kGroupCols; s0 += kStep) {
-                float v[kStep];
+                float v[kStep], second[V::ACCS == 2 ? kStep : 1];
 #pragma unroll
                 for (int c = 0; c < kStep; c += 16)
-                    if (s0 + c < cols) tmem_load16(tmem_lane + (uint32_t)(c_begin + s0 + c), v + c);
+                    if (s0 + c < cols) {
+                        tmem_load16(tmem_lane + (uint32_t)(c_begin + s0 + c), v + c);
+                        if (V::ACCS == 2) tmem_load16(tmem_lane + (uint32_t)(V::MAX_COLS + c_begin + s0 + c), second + c);
+                    }
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int c = 0; c < kStep; ++c) asm volatile("" : "+f"(v[c]));                 // no use before the wait
+                for (int c = 0; c < kStep; ++c) {
+                    asm volatile("" : "+f"(v[c]));                                             // no use before the wait
+                    if (V::ACCS == 2) {
+                        asm volatile("" : "+f"(second[c]));
+                        v[c] += second[c];
+                    }
+                }
                 if (s0 + kStep >= V::kGroupCols) {
                     // the columns are in registers: the next segment may overwrite them while the results are stored
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -762,7 +752,6 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                 }
             }
         }
-        if (!TMA_W) asm volatile("cp.async.wait_all;" ::: "memory");
     }
 
     // ---- leave: nothing of this CTA (or of its pair) is in flight any more ---------------------------------------
@@ -821,7 +810,7 @@ int sm_count_cached() {
     return sm_count[dev];
 }
 
-// The token tile names the variant: 16 and 32 run as S, 64 and 128 as L, 256 as P.
+// The token tile names the variant: 16 and 32 run as S, 64 as M, 128 as L, 256 as P.
 int tile_cg(int tile) { return tile > 128 ? 2 : 1; }
 
 struct Tiling {
@@ -864,6 +853,8 @@ Tiling make_tiling(int tile, int M, int N, int K) {
         w.whole_tiles = (int)(rounds * slots);
         w.total_iters = (int)(shared * w.chunks);
         if (shared == 0) w.slots = (int)(tiles < rounds * slots ? (tiles + rounds - 1) / rounds : slots);
+        // a slot without a share must not lie between two that share a tile: their sum counts the slots from first to last
+        if (rounds == 0 && w.total_iters < w.slots) w.slots = w.total_iters;
     } else {
         int splits = (int)(slots / tiles);
         const int max_splits = w.chunks / 2 > 0 ? w.chunks / 2 : 1;
@@ -874,8 +865,7 @@ Tiling make_tiling(int tile, int M, int N, int K) {
     }
     w.by_splits.set(w.splits > 0 ? w.splits : 1);
     w.by_chunks.set(w.chunks);
-    w.quot = w.total_iters / w.slots;
-    w.rem = w.total_iters % w.slots;
+    w.by_slots.set(w.slots);
     return t;
 }
 
@@ -916,9 +906,11 @@ Tiling pick_tiling(int M, int N, int K) { return make_tiling(token_tile(M, N, K)
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
-template <class V, bool TMA_W>
-int launch_variant(const CUtensorMap &wmap, const CUtensorMap &xmap, const GemmParams &prm, int ctas, cudaStream_t stream) {
-    auto kern = tq1_gemm_kernel<V, TMA_W>;
+template <class V>
+int launch_variant(const CUtensorMap &wmap, const CUtensorMap &xmap, GemmParams &prm, int ctas, cudaStream_t stream) {
+    const int stages = (int)(V::kBRoom / ((uint32_t)prm.b_rows * 256u));
+    prm.b_stages = stages < V::RING ? stages : V::RING;
+    auto kern = tq1_gemm_kernel<V>;
     static bool attr_set[kMaxDevices] = {};
     const int dev = current_device_slot();
     if (!attr_set[dev]) {
@@ -943,13 +935,6 @@ int launch_variant(const CUtensorMap &wmap, const CUtensorMap &xmap, const GemmP
     return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: GEMM launch");
 }
 
-template <class V>
-int launch_aligned(bool tma, const CUtensorMap &wmap, const CUtensorMap &xmap, GemmParams &prm, int ctas, cudaStream_t stream) {
-    const int stages = (int)(V::kBRoom / ((uint32_t)prm.b_rows * 256u));
-    prm.b_stages = stages < V::RING ? stages : V::RING;
-    return tma ? launch_variant<V, true>(wmap, xmap, prm, ctas, stream) : launch_variant<V, false>(wmap, xmap, prm, ctas, stream);
-}
-
 }  // namespace
 
 int gemm_tc_force_tile(int nt) {
@@ -965,14 +950,7 @@ void gemm_tc_plan(int M, int N, int K, int *tile, int *ctas, int *parts) {
     *parts = t.work.splits;
 }
 
-// Any M >= 2 and K a multiple of the group. Widths that are no multiple of a chunk take the kernel only where the
-// product is large enough to pay for its set-up (see gemm_tc_preferred).
-bool gemm_tc_shape_ok(int M, int N, int K) { return M >= 2 && N >= 1 && K % kGroup == 0; }
-
-// The row kernel keeps small products of widths that are no multiple of 512 (and of blocks that are not 16-byte aligned).
-bool gemm_tc_preferred(bool aligned, int M, int N, int K) {
-    return gemm_tc_shape_ok(M, N, K) && ((aligned && K % (kChunkGroups * kGroup) == 0) || (long long)M * N * K >= (1 << 20));
-}
+bool gemm_tc_shape_ok(int M, int N, int K) { return M >= 2 && N >= 1 && K % (kChunkGroups * kGroup) == 0; }
 
 size_t gemm_tc_workspace_bytes(int M, int N, int K) {
     const Tiling t = pick_tiling(M, N, K);
@@ -987,7 +965,6 @@ int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, 
     const Tiling t = pick_tiling(M, N, K);
     const int cg = tile_cg(t.tile);
     GemmParams prm;
-    prm.blocks = blocks;
     prm.y = y;
     prm.partials = reinterpret_cast<float *>(ws + kWsScratchOffset);
     prm.counters = reinterpret_cast<unsigned *>(ws + kWsCounterOffset);
@@ -1003,11 +980,9 @@ int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, 
     prm.y_f32 = y_f32 ? 1 : 0;
     prm.swiglu = swiglu ? 1 : 0;
 
-    // rows of packed bytes as a tensor map: the row length must be a multiple of 16 bytes, the base aligned to 16
-    const bool tma = K % (kChunkGroups * kGroup) == 0 && (reinterpret_cast<uintptr_t>(blocks) & 15) == 0;
-    CUtensorMap wmap = {}, xmap;
+    CUtensorMap wmap, xmap;
     const cuuint32_t estr[2] = {1, 1};
-    if (tma) {
+    {
         const cuuint64_t row_bytes = (cuuint64_t)(K / kGroup) * kBlockBytes;
         const cuuint64_t dims[2] = {row_bytes, (cuuint64_t)N};
         const cuuint64_t strides[1] = {row_bytes};
@@ -1031,9 +1006,10 @@ int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, 
         if (res != CUDA_SUCCESS)
             return fail(TQ1_ERR_CUDA, "tq1_linear_f16: activation tensor map failed (%d)", (int)res);
     }
-    return t.tile <= 32    ? launch_aligned<VariantS>(tma, wmap, xmap, prm, t.ctas(), stream)
-           : t.tile <= 128 ? launch_aligned<VariantL>(tma, wmap, xmap, prm, t.ctas(), stream)
-                           : launch_aligned<VariantP>(tma, wmap, xmap, prm, t.ctas(), stream);
+    return t.tile <= 32    ? launch_variant<VariantS>(wmap, xmap, prm, t.ctas(), stream)
+           : t.tile <= 64  ? launch_variant<VariantM>(wmap, xmap, prm, t.ctas(), stream)
+           : t.tile <= 128 ? launch_variant<VariantL>(wmap, xmap, prm, t.ctas(), stream)
+                           : launch_variant<VariantP>(wmap, xmap, prm, t.ctas(), stream);
 }
 
 }  // namespace tq1

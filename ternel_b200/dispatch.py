@@ -25,7 +25,7 @@ from . import _native
 from .format import check
 
 SWEEP_PATH = Path(__file__).resolve().parent / "dispatch_sweep_b200.json"
-KERNELS = {0: "rows", 1: "stream_gemv", 2: "tensor_core"}
+KERNELS = {0: "rows", 1: "stream_gemv", 2: "tensor_core", 3: "group_sums"}
 TOKEN_TILES = (16, 32, 64, 128, 256)
 LOOPED_MAX = 4          # largest batch also timed as passes of the batch-1 kernel
 SWEEP_BATCHES = (2, 3, 4, 8, 16, 17, 24, 32, 33, 48, 64, 65, 96, 128, 192, 256, 512, 1023, 1024, 2048)
@@ -34,7 +34,7 @@ SWEEP_SHAPES = ((5120, 5120), (1024, 5120), (17408, 5120), (5120, 17408))
 
 @dataclass(frozen=True)
 class LinearPlan:
-    kernel: str          # "rows", "stream_gemv" or "tensor_core"
+    kernel: str          # "rows", "stream_gemv", "tensor_core" or "group_sums"
     token_tile: int      # activation rows per tile (tensor-core kernel), else 0
     ctas: int
     parts: int           # equal K parts per tile, 0 = stream-K ranges

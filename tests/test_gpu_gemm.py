@@ -173,12 +173,11 @@ def test_every_token_tile_gives_the_right_answer(rows, columns, batch):
 @pytest.mark.parametrize("batch", (2, 16, 17, 32, 33, 64, 65, 128, 129, 255, 257, 520))
 @pytest.mark.parametrize(("rows", "columns"), ((129, 8064), (4099, 2176), (383, 4224), (1000, 1408)))
 def test_widths_of_whole_groups(rows, columns, batch):
-    """Widths that are no multiple of 512 (a short last chunk of 1, 2 or 3 groups, rows off the 16-byte grid) and rows that
-    fill no tile, in every token tile's range and around its edges: FP32 sums of FP16 products, in any order, stay within
-    columns * 2^-24 of the largest output (F32_TOL is ten times that); a second run gives the same bits. The same holds for
-    blocks that start off the 16-byte grid."""
+    """Widths that are no multiple of 512 (rows off the 16-byte grid) and rows that fill no tile, in every token tile's
+    range and around its edges, within the F32_TOL of the other widths (test_gpu_group_sums.py has the bound that FP32 group
+    sums give); a second run gives the same bits. The same holds for blocks that start off the 16-byte grid."""
     if batch * rows * columns < 1 << 20:
-        pytest.skip("below the tensor-core kernel's range")
+        pytest.skip("the row kernel's")
     from ternel_b200.ops import check_status, tq1_matmul
     blocks, rng = random_blocks(rows, columns, seed=rows + batch, dist="tests")
     x = rng.standard_normal((batch, columns)).astype(np.float16)
@@ -196,8 +195,8 @@ def test_widths_of_whole_groups(rows, columns, batch):
 
 @pytest.mark.parametrize(("rows", "columns", "batch"), ((256, 640, 8), (4099, 128, 2)))
 def test_other_widths_need_no_workspace(rows, columns, batch):
-    """Widths that are no multiple of 512: without a workspace the row kernel computes what the batched kernel does with
-    one. FP32 sums of at most 640 products in two orders: relative difference below 640 * 2^-24 = 4e-5."""
+    """Widths that are no multiple of 512: a call without a workspace gives what a call with one gives, within the
+    relative difference 640 * 2^-24 = 4e-5 of FP32 sums of at most 640 products in two orders."""
     from ternel_b200 import _native
     lib = _native.lib()
     blocks, rng = random_blocks(rows, columns, seed=rows)
