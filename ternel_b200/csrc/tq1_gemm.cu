@@ -17,8 +17,8 @@
 //        pairs of FP16 weights picked out of [0, s_lo, s_hi, s_hi ^ 0x80] -> 32 registers = 64 K columns, stored to the
 //        row's lane of tensor memory.
 //        All groups also read out finished accumulators and store the results.
-//   one warp   issues tcgen05.mma for the halves (64 K columns) in a fixed order: chunk wave, K block, group, half; up to 128
-//        tokens the K blocks take turns on two accumulators, which are added when the segment is read out
+//   one warp   issues tcgen05.mma for the halves (64 K columns) in a fixed order: chunk wave, K block, group, half; the K
+//        blocks take turns on one, two or four accumulators, which are added when the segment is read out
 //   one warp   fetches the activation tiles in the same order
 // Shared memory traffic of the table bounds the decode (two 128-byte wavefronts per 32 code bytes), so decode warps are
 // many and keep no state between chunks. Weights are decoded in natural column order (a byte's five trits straddle
@@ -30,8 +30,8 @@
 // CTA waits for another. A separate launch for these sums cost 3 to 14 us.
 //
 // Precision: the tensor core adds to an accumulator by truncation, so the error grows with the columns that one accumulator
-// covers: 6.3e-7 of the result (2-norm) for 512, 1.2e-6 for 1024, 3.0e-6 for 2560. Two accumulators halve it. Shares of
-// tiles are spread evenly (WorkSplit::first_iter), so that few tiles stay in one piece.
+// covers: 6.3e-7 of the result (2-norm) for 512, 1.2e-6 for 1024, 3.0e-6 for 2560. All of the accumulator area is therefore
+// used, by up to four accumulators that share the columns, and shares of tiles are spread so that few tiles stay in one piece.
 #include <cuda.h>
 #include <math.h>
 
@@ -51,21 +51,20 @@ constexpr uint32_t kSpinLimit = 1u << 20;
 // Variants:
 //   S  up to 32 tokens: two CTAs per SM with two decode groups each hide each other's latencies; the narrow table
 //      (one 8-byte entry per byte and lane pair, 32 KB) leaves room for that
-//   M  33..64, L  65..128 tokens: one CTA per SM, four groups, wide table (even and odd entries, 64 KB); they differ in
-//      how tensor memory is shared between accumulators and decoded weights
+//   L  33..128 tokens: one CTA per SM, four groups, wide table (even and odd entries, 64 KB)
 //   P  larger: CTA pairs (cta_group::2), each CTA holds half of the activation tile, which halves the activation
 //      traffic out of L2 and through shared memory
-template <int CG_, int G_, bool WIDE_, int PACK_STAGES_, int RING_, int MAX_COLS_>
+template <int CG_, int G_, bool WIDE_, int PACK_STAGES_, int RING_, int MAX_COLS_, int ACC_COLS_>
 struct Variant {
     static constexpr int CG = CG_, G = G_, PACK_STAGES = PACK_STAGES_;
     static constexpr bool WIDE = WIDE_;
     static constexpr int RING = RING_;                              // K blocks of decoded weights in tensor memory
-    static constexpr int MAX_COLS = MAX_COLS_;                      // columns of an accumulator
-    static constexpr int ACCS = CG == 1 ? 2 : 1;                    // accumulators that the K blocks take turns on
+    static constexpr int MAX_COLS = MAX_COLS_;                      // tokens of a tile at most
+    static constexpr int ACC_COLS = ACC_COLS_;                      // columns of tensor memory for accumulators
     static constexpr int kDecodeWarps = 4 * G;
     static constexpr int kThreads = 32 * (kDecodeWarps + 2);
     static constexpr int kGroupCols = MAX_COLS / G < 16 ? 16 : MAX_COLS / G;      // columns a group reads out
-    static constexpr int kABase = ACCS * MAX_COLS;
+    static constexpr int kABase = ACC_COLS;
     static constexpr int kTmemCols = G == 2 ? 256 : 512;
     static_assert(kABase + RING * kStageCols <= kTmemCols, "tensor memory budget");
     static constexpr int kMinCtas = G == 2 ? 2 : 1;
@@ -89,10 +88,9 @@ struct Variant {
         return kPackAddr + stage * kPackOne + warp * kPackBytes;
     }
 };
-using VariantS = Variant<1, 2, false, 2, 3, 32>;
-using VariantM = Variant<1, 4, true, 1, 6, 64>;
-using VariantL = Variant<1, 4, true, 1, 4, 128>;
-using VariantP = Variant<2, 4, true, 1, 4, 256>;
+using VariantS = Variant<1, 2, false, 2, 3, 32, 64>;
+using VariantL = Variant<1, 4, true, 1, 4, 128, 256>;
+using VariantP = Variant<2, 4, true, 1, 4, 256, 256>;
 
 // Table entries. An 8-bit selector picks the two bytes of one FP16 weight out of the pool [0x00, s_lo, s_hi, s_hi ^ 0x80]:
 // code 0 -> -s = (1,3), code 1 -> 0 = (0,0), code 2 -> +s = (1,2). A 16-bit selector of two trits is a PRMT control word.
@@ -285,13 +283,14 @@ struct Divisor {
 //     on are cut into equal contiguous ranges of chunks, one per slot (stream-K), so that all slots do the same number.
 struct WorkSplit {
     int total_iters, slots, chunks, splits;
+    int quot, rem;                              // total_iters = slots * quot + rem: `rem` ranges get one more
+    int spread;                                 // those lie between the others, else they come first
     int whole_rounds, whole_tiles;
     int tiles_total;                            // output tiles of the call (a slot's last whole tiles may lie beyond)
     Divisor by_splits, by_chunks, by_slots;
     __host__ __device__ __forceinline__ int first_iter(int slot) const {
         if (slot >= slots) return total_iters;
-        // the shares of one chunk more lie between the others: side by side they would end where tiles end
-        if (splits == 0) return by_slots.div(slot * total_iters);
+        if (splits == 0) return spread ? by_slots.div(slot * total_iters) : slot * quot + (slot < rem ? slot : rem);
         const int tile = by_splits.div(slot), part = slot - tile * splits;
         return tile * chunks + by_splits.div(chunks * part);
     }
@@ -334,6 +333,7 @@ struct GemmParams {
     int tiles_m;              // token tiles; output tile t covers weight tile t / tiles_m, token tile t % tiles_m
     Divisor by_tiles_m;
     int nt;                   // tokens per tile, a multiple of 16 * CG; the last token tile takes what is left
+    int accs, acc_cols;       // accumulators (1, 2 or 4) and the columns from one to the next
     int b_stages, b_rows;     // activation ring: stages and rows per CTA of one stage
     WorkSplit work;
     int y_f32, swiglu;
@@ -473,11 +473,11 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                     const uint32_t a_tmem = tmem_base + (uint32_t)V::kABase + astage * kStageCols;
                     const uint32_t b_addr = wbase + V::kBAddr + bstage * b_bytes;
                     const uint64_t b_lo = umma_desc(b_addr), b_hi = umma_desc(b_addr + b_bytes / 2);
-                    const uint32_t acc = tmem_base + (V::ACCS == 2 && (i & 1) ? (uint32_t)V::MAX_COLS : 0u);
+                    const uint32_t acc = tmem_base + (uint32_t)((i & (prm.accs - 1)) * prm.acc_cols);
 #pragma unroll
                     for (int j = 0; j < 8; ++j)                    // K = 16 steps: four of each 64-wide swizzle atom
                         umma_f16_ts<CG>(acc, a_tmem + 8u * j, (j < 4 ? b_lo : b_hi) + 2u * (j & 3), idesc,
-                                        (i >= V::ACCS || j > 0) ? 1u : 0u);
+                                        (i >= prm.accs || j > 0) ? 1u : 0u);
                     umma_commit<CG>(bar(EMPTY + astage));
                     if (++astage == RING) { astage = 0; aphase ^= 1u; }
                     if (++bstage == (uint32_t)prm.b_stages) { bstage = 0; bphase ^= 1u; }
@@ -634,27 +634,23 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
             mbar_wait(bar(ACC_FULL), seg & 1u, prm.status, dead);
             ++seg;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            constexpr int kStep = V::ACCS == 2 ? 16 : 32;                                      // columns in registers at a time
-            static_assert(V::kGroupCols % kStep == 0, "whole steps");
+            constexpr int kStep = 16;                                                          // columns in registers at a time
             const bool whole = len == chunks;
             const size_t area = (size_t)prm.nt * kTileW;
             float *slot_part = prm.partials + ((size_t)2 * blockIdx.x + part) * area + row_in_tile;
 #pragma unroll
             for (int s0 = 0; s0 < V::kGroupCols; s0 += kStep) {
-                float v[kStep], second[V::ACCS == 2 ? kStep : 1];
+                float v[kStep];
 #pragma unroll
-                for (int c = 0; c < kStep; c += 16)
-                    if (s0 + c < cols) {
-                        tmem_load16(tmem_lane + (uint32_t)(c_begin + s0 + c), v + c);
-                        if (V::ACCS == 2) tmem_load16(tmem_lane + (uint32_t)(V::MAX_COLS + c_begin + s0 + c), second + c);
-                    }
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                for (int c = 0; c < kStep; ++c) v[c] = 0.0f;
+                for (int a = 0; a < prm.accs && s0 < cols; ++a) {
+                    float u[kStep];
+                    tmem_load16(tmem_lane + (uint32_t)(a * prm.acc_cols + c_begin + s0), u);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int c = 0; c < kStep; ++c) {
-                    asm volatile("" : "+f"(v[c]));                                             // no use before the wait
-                    if (V::ACCS == 2) {
-                        asm volatile("" : "+f"(second[c]));
-                        v[c] += second[c];
+                    for (int c = 0; c < kStep; ++c) {
+                        asm volatile("" : "+f"(u[c]));                                         // no use before the wait
+                        v[c] += u[c];
                     }
                 }
                 if (s0 + kStep >= V::kGroupCols) {
@@ -810,7 +806,7 @@ int sm_count_cached() {
     return sm_count[dev];
 }
 
-// The token tile names the variant: 16 and 32 run as S, 64 as M, 128 as L, 256 as P.
+// The token tile names the variant: 16 and 32 run as S, 64 and 128 as L, 256 as P.
 int tile_cg(int tile) { return tile > 128 ? 2 : 1; }
 
 struct Tiling {
@@ -865,6 +861,13 @@ Tiling make_tiling(int tile, int M, int N, int K) {
     }
     w.by_splits.set(w.splits > 0 ? w.splits : 1);
     w.by_chunks.set(w.chunks);
+    w.quot = w.total_iters / w.slots;
+    w.rem = w.total_iters % w.slots;
+    // CTA pairs have one accumulator for most token tiles, and ranges of a whole tile's length side by side would leave a row
+    // of tiles in one piece, each under one accumulator (192 tokens of 17408x5120: 4.5e-6 from the FP64 product, spread
+    // 4.1e-6). Other ranges come first together, which keeps more of the rest on tile boundaries (1024 tokens of 7168x5120:
+    // 67 us, spread 74).
+    w.spread = cg == 2 && w.quot + 1 >= w.chunks;
     w.by_slots.set(w.slots);
     return t;
 }
@@ -879,11 +882,11 @@ struct TileCost { int tile; float fixed, chunk, chunk_token, segment, shared_tok
 int token_tile(int M, int N, int K) {
     if (g_forced_tile) return g_forced_tile;
     if (M <= 16) return 16;
-    static const TileCost costs[5] = {{16, 2.076f, 0.0f, 0.1592f, 0.0f, 0.1997f},
-                                      {32, 4.394f, 2.3991f, 0.0f, 0.9688f, 0.0369f},
-                                      {64, 2.7955f, 1.2087f, 0.0007f, 2.716f, 0.0684f},
-                                      {128, 4.3587f, 0.8426f, 0.0065f, 2.4854f, 0.0441f},
-                                      {256, 5.532f, 0.207f, 0.0102f, 3.4731f, 0.0424f}};
+    static const TileCost costs[5] = {{16, 2.932f, 0.0f, 0.1263f, 1.968f, 0.1093f},
+                                      {32, 0.0f, 0.0f, 0.06457f, 1.932f, 0.1664f},
+                                      {64, 2.805f, 1.073f, 0.0f, 2.893f, 0.04036f},
+                                      {128, 3.198f, 0.8116f, 0.005891f, 2.846f, 0.02803f},
+                                      {256, 3.206f, 0.4634f, 0.009061f, 3.616f, 0.03028f}};
     int best = 128;
     float best_cost = 0.0f;
     for (int i = 0; i < 5; ++i) {
@@ -891,6 +894,8 @@ int token_tile(int M, int N, int K) {
         if (c.tile > 16 && c.tile >= 4 * M) continue;           // a tile mostly of padding
         const Tiling t = make_tiling(c.tile, M, N, K);
         const WorkSplit &w = t.work;
+        // whole tiles on less than half of the chip: a narrower tile splits K over the rest, with shorter accumulators
+        if (c.tile == 256 && w.splits == 1 && 2 * t.ctas() <= sm_count_cached()) continue;
         const float shared = (float)w.total_iters / w.slots;    // chunks of shared tiles per slot
         const float chunks = w.splits ? (float)((w.chunks + w.splits - 1) / w.splits)
                                       : (float)w.whole_rounds * w.chunks + ceilf(shared);
@@ -976,6 +981,9 @@ int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, 
     prm.by_tiles_m.set(t.tiles_m);
     prm.nt = t.nt;
     prm.b_rows = t.nt / cg;
+    const int acc_area = t.tile <= 32 ? VariantS::ACC_COLS : t.tile <= 128 ? VariantL::ACC_COLS : VariantP::ACC_COLS;
+    prm.accs = 4 * t.nt <= acc_area ? 4 : 2 * t.nt <= acc_area ? 2 : 1;       // a segment has at least four K blocks
+    prm.acc_cols = acc_area / prm.accs;
     prm.work = t.work;
     prm.y_f32 = y_f32 ? 1 : 0;
     prm.swiglu = swiglu ? 1 : 0;
@@ -1007,7 +1015,6 @@ int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, 
             return fail(TQ1_ERR_CUDA, "tq1_linear_f16: activation tensor map failed (%d)", (int)res);
     }
     return t.tile <= 32    ? launch_variant<VariantS>(wmap, xmap, prm, t.ctas(), stream)
-           : t.tile <= 64  ? launch_variant<VariantM>(wmap, xmap, prm, t.ctas(), stream)
            : t.tile <= 128 ? launch_variant<VariantL>(wmap, xmap, prm, t.ctas(), stream)
                            : launch_variant<VariantP>(wmap, xmap, prm, t.ctas(), stream);
 }

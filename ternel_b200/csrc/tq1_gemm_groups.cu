@@ -129,11 +129,11 @@ groups_few_kernel(const uint8_t *__restrict__ blocks, const __half *__restrict__
             if (lane + 32 * j < kWords) mine[lane + 32 * j] = next[j];
         __syncwarp();
         load(grp + kFewWarps);
-        float sum[NT][4];
+        float sum[NT][4], half[NT][4];                  // the group's sum so far, that of its second half
 #pragma unroll
         for (int t = 0; t < NT; ++t)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) sum[t][i] = 0.0f;
+            for (int i = 0; i < 4; ++i) sum[t][i] = half[t][i] = 0.0f;
         uint4 xv[4][NT];
 #pragma unroll
         for (int s = 0; s < 4; ++s)
@@ -148,8 +148,12 @@ groups_few_kernel(const uint8_t *__restrict__ blocks, const __half *__restrict__
             decode8(bytes_lo + 2 + a, off, table, lo);
             decode8(bytes_hi + 2 + a, off, table, hi);
 #pragma unroll
-            for (int t = 0; t < NT; ++t) step32(sum[t], lo, hi, xv[s][t]);
+            for (int t = 0; t < NT; ++t) step32(s < 2 ? sum[t] : half[t], lo, hi, xv[s][t]);
         }
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sum[t][i] += half[t][i];
         const float s_lo = __half2float(*reinterpret_cast<const __half *>(bytes_lo));
         const float s_hi = __half2float(*reinterpret_cast<const __half *>(bytes_hi));
 #pragma unroll
@@ -171,15 +175,11 @@ groups_few_kernel(const uint8_t *__restrict__ blocks, const __half *__restrict__
     __syncthreads();
     for (int i = tid; i < 8 * NT * kFewRows; i += kFewWarps * 32) {
         const int r = i % kFewRows, t = i / kFewRows;
-        float v[kFewWarps];
+        double v = 0.0;                                 // one rounding for the sum of the warps' parts
 #pragma unroll
-        for (int w = 0; w < kFewWarps; ++w) v[w] = parts[w][t][r];
-#pragma unroll
-        for (int d = 1; d < kFewWarps; d *= 2)
-#pragma unroll
-            for (int w = 0; w < kFewWarps; w += 2 * d) v[w] += v[w + d];
+        for (int w = 0; w < kFewWarps; ++w) v += (double)parts[w][t][r];
         if (n0 + r < N && m0 + t < M)
-            store_result(y, y_f32, (size_t)(m0 + t) * N + n0 + r, (size_t)M * N, v[0]);
+            store_result(y, y_f32, (size_t)(m0 + t) * N + n0 + r, (size_t)M * N, (float)v);
     }
 }
 

@@ -208,3 +208,24 @@ def test_other_widths_need_no_workspace(rows, columns, batch):
     assert lib.tq1_linear_f16(bd.data_ptr(), xd.data_ptr(), y.data_ptr(), 1, batch, rows, columns, None, 0, stream) == 0
     want = run_linear(blocks, x)
     assert np.abs(y.cpu().numpy() - want).max() <= 4e-5 * np.abs(want).max()
+
+
+@pytest.mark.parametrize(("batch", "rows", "columns", "span"), (
+    (3, 512, 512, 128), (8, 5120, 5120, 256), (16, 17408, 5120, 640), (32, 17408, 5120, 1280), (48, 5120, 17408, 1536),
+    (64, 4096, 4096, 512), (100, 5120, 5120, 1024), (128, 5120, 17408, 3072), (300, 1024, 5120, 512), (512, 1024, 5120, 640),
+    (777, 512, 512, 256), (2048, 17408, 5120, 5120)))
+def test_error_grows_with_the_columns_of_one_accumulator_only(batch, rows, columns, span):
+    """A tensor-core accumulator of `span` columns truncates span / 16 times, on average by half of an ulp of 0.72 * 2^-23 of
+    its value, which grows to the sum from zero (2/3 on the way): a relative error (2-norm) of at most 0.48 * span / 16 *
+    2^-24, whatever the number of accumulators and parts that make up the columns. `span` is what K parts and accumulators
+    leave of the columns in each tile form."""
+    from ternel_b200.ops import tq1_get_rows, tq1_matmul
+    from ternel_b200.stack import random_blocks_device
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(batch)
+    blocks = random_blocks_device(rows, columns, gen, "cuda")
+    x = torch.randn((batch, columns), generator=gen, device="cuda").half()
+    dense = tq1_get_rows(blocks, torch.arange(rows, device="cuda"), dtype=torch.float32).double()
+    want = x.double() @ dense.T
+    got = tq1_matmul(blocks, x, out_dtype=torch.float32).double()
+    assert float((got - want).norm() / want.norm()) < 0.48 * span / 16 * 2.0 ** -24
