@@ -7,16 +7,18 @@
 // these functions it is an output allocation, the stream lookup and the launch.
 //
 // A function here serves only the plain case (CUDA tensors without subclass, mode or gradient, right
-// dtypes and shapes, contiguous, workspace large enough) and returns None for anything else; the
-// caller then takes its ordinary path, which raises the proper error or goes through the dispatcher
-// (fake tensors, torch.compile). Arguments of the C ABI are never invented here: a call either matches
-// what that path would have done or is left to it.
+// dtypes and shapes, contiguous, workspace large enough), in which the dispatcher would do nothing but
+// call the CUDA kernel, and returns None for anything else; the caller then takes its ordinary path, which raises
+// the proper error or goes through the dispatcher (fake tensors, torch.compile, torch.jit.trace, vmap).
+// Arguments of the C ABI are never invented here: a call either matches what that path would have done
+// or is left to it.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
 #include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -61,7 +63,21 @@ int wants_f32(PyObject *dtype) {
     return s == at::kHalf ? 0 : s == at::kFloat ? 1 : -1;
 }
 
-bool modes_active() { return c10::impl::TorchDispatchModeTLS::any_modes_set(); }
+// Whether the dispatcher has something to do for these arguments before the CUDA kernel: tensors that are not what their
+// memory holds (negative views, ...), modes, and what a thread has switched on (tracing, functionalization, transforms).
+// The outputs here are made without the dispatcher, so a tracer would take them for constants.
+bool dispatcher_needed(const at::Tensor &a, const at::Tensor &b) {
+    using c10::DispatchKey;
+    constexpr c10::DispatchKeySet special(
+        {DispatchKey::Python, DispatchKey::Fake, DispatchKey::FuncTorchDynamicLayerBackMode, DispatchKey::Functionalize,
+         DispatchKey::Named, DispatchKey::Conjugate, DispatchKey::Negative, DispatchKey::ZeroTensor, DispatchKey::Tracer,
+         DispatchKey::FuncTorchBatched, DispatchKey::FuncTorchVmapMode, DispatchKey::Batched, DispatchKey::VmapMode,
+         DispatchKey::FuncTorchGradWrapper, DispatchKey::FuncTorchDynamicLayerFrontMode, DispatchKey::PreDispatch,
+         DispatchKey::PythonDispatcher});
+    const c10::impl::LocalDispatchKeySet local = c10::impl::tls_local_dispatch_key_set();
+    return c10::impl::TorchDispatchModeTLS::any_modes_set() ||
+           ((a.key_set() | b.key_set() | local.included_) - local.excluded_).has_any(special);
+}
 
 // linear(blocks, x, out_dtype, swiglu, flat): x of any leading dimensions (exactly two with `flat`)
 PyObject *fast_linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
@@ -71,7 +87,7 @@ PyObject *fast_linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     const bool swiglu = args[3] == Py_True, flat = args[4] == Py_True;
     const int f32 = wants_f32(args[2]);
     int64_t rows, groups;
-    if (f32 < 0 || modes_active() || !canonical_blocks(blocks, rows, groups)) Py_RETURN_NONE;
+    if (f32 < 0 || dispatcher_needed(blocks, x) || !canonical_blocks(blocks, rows, groups)) Py_RETURN_NONE;
     const int64_t columns = groups * TQ1_GROUP, dims = x.dim();
     if (x.scalar_type() != at::kHalf || !plain_cuda(x) || x.device() != blocks.device() || dims < 1 ||
         (flat && dims != 2) || x.size(dims - 1) != columns || x.requires_grad() || (swiglu && rows % 2))
@@ -104,7 +120,7 @@ PyObject *fast_embedding(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     const bool flat = args[3] == Py_True;
     const int f32 = wants_f32(args[2]);
     int64_t rows, groups;
-    if (f32 < 0 || args[2] == Py_None || modes_active() || !canonical_blocks(blocks, rows, groups)) Py_RETURN_NONE;
+    if (f32 < 0 || args[2] == Py_None || dispatcher_needed(blocks, ids) || !canonical_blocks(blocks, rows, groups)) Py_RETURN_NONE;
     if (ids.scalar_type() != at::kLong || !plain_cuda(ids) || ids.device() != blocks.device() ||
         (flat && ids.dim() != 1) || ids.numel() <= 0)
         Py_RETURN_NONE;

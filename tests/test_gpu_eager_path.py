@@ -61,3 +61,24 @@ def test_declines_what_is_not_the_plain_case():
         fake = mode.from_tensor(x)
         assert eager_linear(mode.from_tensor(blocks), fake, None, False, False) is None
         assert tq1_matmul(mode.from_tensor(blocks), fake).shape == (3, 48)
+
+
+def test_what_a_thread_has_switched_on_is_seen():
+    """A trace records the operations and follows its input (a result made outside the dispatcher would be a constant in
+    it), a negative view counts as its values, and functionalization goes through."""
+    from ternel_b200.ops import eager_embedding, eager_linear, tq1_get_rows, tq1_matmul, tq1_swiglu
+    blocks, x = _setup(48, 1024)
+    ids = torch.tensor([3, 0, 47], device="cuda")
+    other, other_ids = torch.randn_like(x), ids.flip(0) - 1
+    tq1_matmul(blocks, x)
+    for op, call, first, second in (("tq1_linear", lambda v: tq1_matmul(blocks, v), x, other),
+                                    ("tq1_linear_swiglu", lambda v: tq1_swiglu(blocks, v), x, other),
+                                    ("tq1_embedding", lambda v: tq1_get_rows(blocks, v), ids, other_ids)):
+        traced = torch.jit.trace(call, (first,))
+        assert f"ternel::{op}" in str(traced.graph)
+        assert torch.equal(traced(second), call(second))
+    assert torch.equal(tq1_matmul(blocks, torch._neg_view(x)), tq1_matmul(blocks, -x))
+    assert eager_linear(blocks, torch._neg_view(x), None, False, True) is None
+    assert torch.equal(torch.func.functionalize(lambda v: tq1_matmul(blocks, v))(x), tq1_matmul(blocks, x))
+    assert eager_linear(blocks, x, None, False, True) is not None               # nothing stays switched on
+    assert eager_embedding(blocks, ids, torch.float16, True) is not None
