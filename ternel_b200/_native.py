@@ -133,8 +133,9 @@ def binding():
         spec = importlib.util.spec_from_file_location("_ternel_torch", BINDING_PATH)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
+        from torch.utils._device import DeviceContext
         module.bind(*(ctypes.cast(getattr(handle, name), c_void_p).value for name in (
-            "tq1_linear_workspace_bytes", "tq1_linear_f16", "tq1_linear_swiglu_f16", "tq1_embedding_f16")))
+            "tq1_linear_workspace_bytes", "tq1_linear_f16", "tq1_linear_swiglu_f16", "tq1_embedding_f16")), DeviceContext)
         _binding = module
     return _binding
 

@@ -15,6 +15,7 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
@@ -23,6 +24,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
+#include <torch/csrc/PyInterpreter.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/ternel_b200.h"
@@ -79,9 +81,21 @@ bool dispatcher_needed(const at::Tensor &a, const at::Tensor &b) {
            ((a.key_set() | b.key_set() | local.included_) - local.excluded_).has_any(special);
 }
 
+PyTypeObject *g_device_context = nullptr;       // torch.utils._device.DeviceContext
+
+// Whether Python wants to see the operation: a TorchFunctionMode other than that of a default device (which looks at
+// factory functions alone), or an argument of a subclass, whose __torch_function__ decides what comes back.
+bool python_watches(PyObject *a, PyObject *b) {
+    if (!THPVariable_CheckExact(a) || !THPVariable_CheckExact(b)) return true;
+    if (!at::impl::torch_function_mode_enabled()) return false;
+    for (int64_t i = 0; i < at::impl::PythonTorchFunctionTLS::stack_len(); ++i)
+        if (Py_TYPE(at::impl::PythonTorchFunctionTLS::get_stack_at(i)->ptr(getPyInterpreter())) != g_device_context) return true;
+    return false;
+}
+
 // linear(blocks, x, out_dtype, swiglu, flat): x of any leading dimensions (exactly two with `flat`)
 PyObject *fast_linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
-    if (nargs != 5 || !g_linear || !THPVariable_Check(args[0]) || !THPVariable_Check(args[1])) Py_RETURN_NONE;
+    if (nargs != 5 || !g_linear || python_watches(args[0], args[1])) Py_RETURN_NONE;
     const at::Tensor &blocks = THPVariable_Unpack(args[0]);
     const at::Tensor &x = THPVariable_Unpack(args[1]);
     const bool swiglu = args[3] == Py_True, flat = args[4] == Py_True;
@@ -114,7 +128,7 @@ PyObject *fast_linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
 
 // embedding(blocks, ids, dtype, flat): ids int64 of any shape (one-dimensional with `flat`)
 PyObject *fast_embedding(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
-    if (nargs != 4 || !g_embedding || !THPVariable_Check(args[0]) || !THPVariable_Check(args[1])) Py_RETURN_NONE;
+    if (nargs != 4 || !g_embedding || python_watches(args[0], args[1])) Py_RETURN_NONE;
     const at::Tensor &blocks = THPVariable_Unpack(args[0]);
     const at::Tensor &ids = THPVariable_Unpack(args[1]);
     const bool flat = args[3] == Py_True;
@@ -143,13 +157,16 @@ PyObject *guarded(PyObject *self, PyObject *const *args, Py_ssize_t nargs) {
     END_HANDLE_TH_ERRORS
 }
 
-// bind(workspace_bytes, linear, swiglu, embedding): addresses of the C ABI functions
+// bind(workspace_bytes, linear, swiglu, embedding, device_context): addresses of the C ABI functions, and the type of the
+// mode that a default device puts up
 PyObject *bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     void *p[4];
-    if (nargs != 4) {
-        PyErr_SetString(PyExc_TypeError, "bind takes four addresses");
+    if (nargs != 5 || !PyType_Check(args[4])) {
+        PyErr_SetString(PyExc_TypeError, "bind takes four addresses and a type");
         return nullptr;
     }
+    Py_INCREF(args[4]);
+    g_device_context = reinterpret_cast<PyTypeObject *>(args[4]);
     for (int i = 0; i < 4; ++i) {
         p[i] = PyLong_AsVoidPtr(args[i]);
         if (!p[i] && PyErr_Occurred()) return nullptr;

@@ -82,3 +82,40 @@ def test_what_a_thread_has_switched_on_is_seen():
     assert torch.equal(torch.func.functionalize(lambda v: tq1_matmul(blocks, v))(x), tq1_matmul(blocks, x))
     assert eager_linear(blocks, x, None, False, True) is not None               # nothing stays switched on
     assert eager_embedding(blocks, ids, torch.float16, True) is not None
+
+
+def test_torch_functions_are_called():
+    """A TorchFunctionMode sees the operation and a subclass gets its own type back, as from any operator; the mode that a
+    default device puts up changes nothing."""
+    from torch.overrides import TorchFunctionMode
+    from ternel_b200.ops import eager_embedding, eager_linear, tq1_get_rows, tq1_matmul
+    blocks, x = _setup()
+    ids = torch.zeros(3, dtype=torch.int64, device="cuda")
+    want = tq1_matmul(blocks, x)
+
+    class Watch(TorchFunctionMode):
+        def __init__(self):
+            super().__init__()
+            self.seen = []
+
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            self.seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    class Named(torch.Tensor):
+        pass
+
+    with Watch() as watch:
+        assert torch.equal(tq1_matmul(blocks, x), want)
+        tq1_get_rows(blocks, ids)
+    assert any("tq1_linear" in f for f in watch.seen) and any("tq1_embedding" in f for f in watch.seen)
+    named = tq1_matmul(blocks, x.as_subclass(Named))
+    assert type(named) is Named and torch.equal(named.as_subclass(torch.Tensor), want)
+    assert type(tq1_get_rows(blocks.as_subclass(Named), ids)) is Named
+    with torch.device("cuda"):
+        assert torch.equal(eager_linear(blocks, x, None, False, True), want)
+        assert eager_embedding(blocks, ids, torch.float16, True) is not None
+        with Watch():
+            assert eager_linear(blocks, x, None, False, True) is None
+    parameter = torch.nn.Parameter(blocks, requires_grad=False)
+    assert torch.equal(eager_linear(parameter, x, None, False, True), want)
