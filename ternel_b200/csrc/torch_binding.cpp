@@ -18,6 +18,7 @@
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/core/Tensor.h>
+#include <ATen/record_function.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
@@ -66,7 +67,7 @@ int wants_f32(PyObject *dtype) {
 }
 
 // Whether the dispatcher has something to do for these arguments before the CUDA kernel: tensors that are not what their
-// memory holds (negative views, ...), modes, and what a thread has switched on (tracing, functionalization, transforms).
+// memory holds (negative views, ...), modes, and what a thread has switched on (tracing, functionalization, transforms, a profiler).
 // The outputs here are made without the dispatcher, so a tracer would take them for constants.
 bool dispatcher_needed(const at::Tensor &a, const at::Tensor &b) {
     using c10::DispatchKey;
@@ -78,6 +79,7 @@ bool dispatcher_needed(const at::Tensor &a, const at::Tensor &b) {
          DispatchKey::PythonDispatcher});
     const c10::impl::LocalDispatchKeySet local = c10::impl::tls_local_dispatch_key_set();
     return c10::impl::TorchDispatchModeTLS::any_modes_set() ||
+           at::getStepCallbacksUnlessEmpty(at::RecordScope::FUNCTION).has_value() ||
            ((a.key_set() | b.key_set() | local.included_) - local.excluded_).has_any(special);
 }
 

@@ -119,3 +119,16 @@ def test_torch_functions_are_called():
             assert eager_linear(blocks, x, None, False, True) is None
     parameter = torch.nn.Parameter(blocks, requires_grad=False)
     assert torch.equal(eager_linear(parameter, x, None, False, True), want)
+
+
+def test_a_profiler_sees_the_operations():
+    from torch.profiler import ProfilerActivity, profile
+    from ternel_b200.ops import eager_linear, tq1_get_rows, tq1_matmul
+    blocks, x = _setup()
+    tq1_matmul(blocks, x)
+    with profile(activities=[ProfilerActivity.CPU]) as record:
+        tq1_matmul(blocks, x)
+        tq1_get_rows(blocks, torch.zeros(3, dtype=torch.int64, device="cuda"))
+    names = {event.key for event in record.key_averages()}
+    assert {"ternel::tq1_linear", "ternel::tq1_embedding"} <= names
+    assert eager_linear(blocks, x, None, False, True) is not None               # and afterwards the short path again
