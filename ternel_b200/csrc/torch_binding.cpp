@@ -27,6 +27,9 @@
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/PyInterpreter.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <array>
 
 #include "../../include/ternel_b200.h"
 
@@ -38,13 +41,11 @@ decltype(&tq1_linear_f16) g_linear = nullptr;
 decltype(&tq1_linear_swiglu_f16) g_swiglu = nullptr;
 decltype(&tq1_embedding_f16) g_embedding = nullptr;
 
-// The per-device workspace that the Python side owns and grows (addresses only; all access under the GIL).
+// The per-device workspace that the Python side makes and grows. The table is only touched under the GIL; a call takes a
+// reference, because it lets the GIL go while it launches and another thread may replace the buffer meanwhile. Never
+// destroyed: at exit the allocator may be gone before it.
 constexpr int kMaxDevices = 64;
-struct Workspace {
-    void *ptr;
-    size_t bytes;
-};
-Workspace g_workspace[kMaxDevices] = {};
+std::array<at::Tensor, kMaxDevices> &g_workspace = *new std::array<at::Tensor, kMaxDevices>();
 
 bool plain_cuda(const at::Tensor &t) {
     return t.is_cuda() && t.layout() == at::kStrided && t.is_contiguous() && !at::isTensorSubclassLike(t);
@@ -111,19 +112,26 @@ PyObject *fast_linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     const int64_t batch = x.numel() / columns;
     const int device = x.device().index();
     if (batch <= 0 || batch > INT32_MAX || device < 0 || device >= kMaxDevices) Py_RETURN_NONE;
-    const Workspace ws = g_workspace[device];
-    const size_t need = g_workspace_bytes((int)batch, (int)rows, (int)columns);
-    if (need > ws.bytes) Py_RETURN_NONE;
-    const c10::cuda::CUDAGuard guard(x.device());
+    const at::Tensor ws = g_workspace[device];
+    const size_t need = g_workspace_bytes((int)batch, (int)rows, (int)columns), have = ws.defined() ? ws.nbytes() : 0;
+    if (need > have) Py_RETURN_NONE;
+    void *scratch = have ? ws.mutable_data_ptr() : nullptr;
     c10::SmallVector<int64_t, 6> shape(x.sizes().begin(), x.sizes().end());
     shape[dims - 1] = swiglu ? rows / 2 : rows;
-    at::Tensor out = at::detail::empty_cuda(shape, f32 ? at::kFloat : at::kHalf, x.device(), std::nullopt);
-    void *stream = c10::cuda::getCurrentCUDAStream(device).stream();
     const auto *w = static_cast<const uint8_t *>(blocks.const_data_ptr());
-    const int rc = swiglu ? g_swiglu(w, x.const_data_ptr(), out.mutable_data_ptr(), f32, (int)batch, (int)(rows / 2),
-                                     (int)columns, ws.ptr, ws.bytes, stream)
-                          : g_linear(w, x.const_data_ptr(), out.mutable_data_ptr(), f32, (int)batch, (int)rows,
-                                     (int)columns, ws.ptr, ws.bytes, stream);
+    at::Tensor out;
+    int rc;
+    {
+        // a launch waits while the stream's queue is full, perhaps for work of another thread that needs the GIL
+        const pybind11::gil_scoped_release no_gil;
+        const c10::cuda::CUDAGuard guard(x.device());
+        out = at::detail::empty_cuda(shape, f32 ? at::kFloat : at::kHalf, x.device(), std::nullopt);
+        void *stream = c10::cuda::getCurrentCUDAStream(device).stream();
+        rc = swiglu ? g_swiglu(w, x.const_data_ptr(), out.mutable_data_ptr(), f32, (int)batch, (int)(rows / 2),
+                               (int)columns, scratch, have, stream)
+                    : g_linear(w, x.const_data_ptr(), out.mutable_data_ptr(), f32, (int)batch, (int)rows,
+                               (int)columns, scratch, have, stream);
+    }
     if (rc != TQ1_OK) Py_RETURN_NONE;
     return THPVariable_Wrap(std::move(out));
 }
@@ -140,14 +148,19 @@ PyObject *fast_embedding(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     if (ids.scalar_type() != at::kLong || !plain_cuda(ids) || ids.device() != blocks.device() ||
         (flat && ids.dim() != 1) || ids.numel() <= 0)
         Py_RETURN_NONE;
-    const c10::cuda::CUDAGuard guard(blocks.device());
     c10::SmallVector<int64_t, 6> shape(ids.sizes().begin(), ids.sizes().end());
     shape.push_back(groups * TQ1_GROUP);
-    at::Tensor out = at::detail::empty_cuda(shape, f32 ? at::kFloat : at::kHalf, blocks.device(), std::nullopt);
-    void *stream = c10::cuda::getCurrentCUDAStream(blocks.device().index()).stream();
-    if (g_embedding(static_cast<const uint8_t *>(blocks.const_data_ptr()), ids.const_data_ptr<int64_t>(),
-                    out.mutable_data_ptr(), f32, ids.numel(), rows, (int)(groups * TQ1_GROUP), stream) != TQ1_OK)
-        Py_RETURN_NONE;
+    at::Tensor out;
+    int rc;
+    {
+        const pybind11::gil_scoped_release no_gil;
+        const c10::cuda::CUDAGuard guard(blocks.device());
+        out = at::detail::empty_cuda(shape, f32 ? at::kFloat : at::kHalf, blocks.device(), std::nullopt);
+        void *stream = c10::cuda::getCurrentCUDAStream(blocks.device().index()).stream();
+        rc = g_embedding(static_cast<const uint8_t *>(blocks.const_data_ptr()), ids.const_data_ptr<int64_t>(),
+                         out.mutable_data_ptr(), f32, ids.numel(), rows, (int)(groups * TQ1_GROUP), stream);
+    }
+    if (rc != TQ1_OK) Py_RETURN_NONE;
     return THPVariable_Wrap(std::move(out));
 }
 
@@ -180,17 +193,15 @@ PyObject *bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     Py_RETURN_NONE;
 }
 
-// set_workspace(device, address, bytes)
+// set_workspace(device, tensor)
 PyObject *set_workspace(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
-    if (nargs != 3) {
-        PyErr_SetString(PyExc_TypeError, "set_workspace takes a device index, an address and a size");
+    if (nargs != 2 || !THPVariable_Check(args[1])) {
+        PyErr_SetString(PyExc_TypeError, "set_workspace takes a device index and a tensor");
         return nullptr;
     }
     const long device = PyLong_AsLong(args[0]);
-    void *ptr = PyLong_AsVoidPtr(args[1]);
-    const size_t bytes = PyLong_AsSize_t(args[2]);
     if (PyErr_Occurred()) return nullptr;
-    if (device >= 0 && device < kMaxDevices) g_workspace[device] = {ptr, bytes};
+    if (device >= 0 && device < kMaxDevices) g_workspace[device] = THPVariable_Unpack(args[1]);
     Py_RETURN_NONE;
 }
 

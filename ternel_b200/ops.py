@@ -50,7 +50,7 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor | None:
     if buf is None or buf.numel() < nbytes:
         buf = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)   # slots start at zero
         _workspaces[index] = buf
-        _native.binding().set_workspace(index, buf.data_ptr(), buf.numel())
+        _native.binding().set_workspace(index, buf)
     return buf
 
 

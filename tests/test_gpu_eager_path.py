@@ -132,3 +132,38 @@ def test_a_profiler_sees_the_operations():
     names = {event.key for event in record.key_averages()}
     assert {"ternel::tq1_linear", "ternel::tq1_embedding"} <= names
     assert eager_linear(blocks, x, None, False, True) is not None               # and afterwards the short path again
+
+
+def test_other_threads_run_while_a_launch_waits():
+    """More launches than a stream's queue holds, behind a kernel that keeps the GPU busy for about a second: the launching
+    thread waits, and another Python thread has to go on meanwhile (the kernel might wait for what it does)."""
+    import threading
+    import time
+    from ternel_b200.ops import tq1_matmul
+    blocks, x = _setup()
+    tq1_matmul(blocks, x)
+    torch.cuda.synchronize()
+    gaps, stop = [], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        torch.cuda._sleep(2_000_000_000)                    # about a second
+        begin = time.perf_counter()
+        for _ in range(3000):
+            tq1_matmul(blocks, x)
+        waited = time.perf_counter() - begin
+    finally:
+        stop.set()
+        thread.join()
+    torch.cuda.synchronize()
+    assert waited > 0.5                                     # the queue did fill up
+    assert max(gaps) < 0.3, max(gaps)
