@@ -30,10 +30,18 @@ ACTIVATION_DTYPES = (torch.float16,)
 OUTPUT_DTYPES = (torch.float16, torch.float32)
 
 _workspaces: dict[int, torch.Tensor] = {}
+_replaced: list[torch.Tensor] = []          # buffers that a larger one has taken over from
 
 
 def _stream_ptr(device: torch.device) -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+
+
+def _new_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
+    """A zero-filled buffer (slots and counters start at zero) of a power of two bytes, at least 1 MiB."""
+    buf = torch.zeros(1 << max(20, (nbytes - 1).bit_length()), dtype=torch.uint8, device=device)
+    torch.cuda.current_stream(device).synchronize()             # whatever stream uses it next
+    return buf
 
 
 def _workspace(device: torch.device, nbytes: int) -> torch.Tensor | None:
@@ -42,13 +50,22 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor | None:
     Calls on one device share it, which is safe because they are ordered on the
     current stream; callers that use several streams per device must pass their
     own workspace through the C ABI instead.
+
+    A captured graph keeps the address it was captured with, and its replays expect the buffer as the last call left it. So
+    a buffer is never given back when a larger one replaces it: sizes are powers of two, so all replaced ones together are smaller
+    than the one in use. A call that is being captured and needs more than there is brings a buffer of its own, which belongs to the
+    graph's memory and is zero-filled by each replay: outside of the graph it would not be zero.
     """
     if nbytes == 0:
         return None
     index = device.index if device.index is not None else torch.cuda.current_device()
     buf = _workspaces.get(index)
     if buf is None or buf.numel() < nbytes:
-        buf = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)   # slots start at zero
+        if torch.cuda.is_current_stream_capturing():
+            return torch.zeros(nbytes, dtype=torch.uint8, device=device)
+        if buf is not None:
+            _replaced.append(buf)
+        buf = _new_workspace(device, nbytes)
         _workspaces[index] = buf
         _native.binding().set_workspace(index, buf)
     return buf

@@ -1,0 +1,40 @@
+"""Scratch buffers of the packed ops on the GPU: what graphs, growth and several streams do to them."""
+
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+GRAPH_SCRIPT = """
+import torch
+from ternel_b200 import ops
+from ternel_b200.graphs import GraphedStep
+from ternel_b200.stack import random_blocks_device
+gen = torch.Generator(device="cuda")
+gen.manual_seed(5)
+small, large = (random_blocks_device(n, 5120, gen, "cuda") for n in (1024, 17408))
+x, other, long = (torch.randn((m, 5120), generator=gen, device="cuda").half() for m in (8, 8, 2048))
+step = GraphedStep(lambda v: ops.tq1_matmul(small, v), [x])             # five K parts: partial tiles and counters in use
+want = step(other).clone()
+first = ops._workspaces[0]
+before = first.data_ptr()
+del first
+ops.tq1_matmul(large, long)                                             # needs more: a larger buffer takes over
+assert ops._workspaces[0].data_ptr() != before
+junk = [torch.full((1 << 20,), 255, dtype=torch.uint8, device="cuda") for _ in range(96)]    # over anything given back
+for _ in range(3):
+    assert torch.equal(step(other), want) and torch.equal(step(x), ops.tq1_matmul(small, x))
+assert all(bool((j == 255).all()) for j in junk)
+ops.check_status()
+print("fine")
+"""
+
+
+def test_a_graph_outlives_the_growth_of_the_workspace():
+    """A process of its own, because the buffer has to start small."""
+    run = subprocess.run([sys.executable, "-c", GRAPH_SCRIPT], capture_output=True, text=True, timeout=300,
+                         cwd=Path(__file__).resolve().parents[1])
+    assert run.returncode == 0 and "fine" in run.stdout, run.stdout + run.stderr
