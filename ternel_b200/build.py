@@ -88,7 +88,7 @@ def build_binding(force: bool = False) -> Path:
            "-isystem", str(root / "include"), "-isystem", str(root / "include/torch/csrc/api/include"),
            "-isystem", str(cuda / "include"), "-isystem", sysconfig.get_paths()["include"],
            str(BINDING_SOURCE), "-o", str(tmp), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu",
-           "-ltorch_cuda", "-lc10", "-lc10_cuda", f"-Wl,-rpath,{root / 'lib'}"]
+           "-ltorch_cuda", "-lc10", "-lc10_cuda", f"-L{cuda / 'lib64'}", "-lcudart", f"-Wl,-rpath,{root / 'lib'}"]
     done = subprocess.run(cmd, capture_output=True, text=True)
     if done.returncode != 0:
         tmp.unlink(missing_ok=True)

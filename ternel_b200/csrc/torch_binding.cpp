@@ -30,6 +30,9 @@
 #include <torch/csrc/utils/pybind.h>
 
 #include <array>
+#include <vector>
+
+#include <cuda_runtime_api.h>
 
 #include "../../include/ternel_b200.h"
 
@@ -41,11 +44,28 @@ decltype(&tq1_linear_f16) g_linear = nullptr;
 decltype(&tq1_linear_swiglu_f16) g_swiglu = nullptr;
 decltype(&tq1_embedding_f16) g_embedding = nullptr;
 
-// The per-device workspace that the Python side makes and grows. The table is only touched under the GIL; a call takes a
-// reference, because it lets the GIL go while it launches and another thread may replace the buffer meanwhile. Never
-// destroyed: at exit the allocator may be gone before it.
+// The workspaces that the Python side makes and grows, per device one for each stream that has called lately. The table is only
+// touched under the GIL; a call takes a reference, because it lets the GIL go while it launches and another thread may
+// replace the buffer meanwhile. Never destroyed: at exit the allocator may be gone before it.
 constexpr int kMaxDevices = 64;
-std::array<at::Tensor, kMaxDevices> &g_workspace = *new std::array<at::Tensor, kMaxDevices>();
+struct Workspace {
+    cudaStream_t stream;
+    at::Tensor buffer;
+};
+std::array<std::vector<Workspace>, kMaxDevices> &g_workspaces = *new std::array<std::vector<Workspace>, kMaxDevices>();
+
+// The buffer for calls on `stream`, undefined where the Python side has to look: no buffer yet, or a capture, whose
+// kernels must not hold a buffer that may be given back (the default stream cannot be captured).
+at::Tensor workspace_of(int device, cudaStream_t stream) {
+    for (const Workspace &w : g_workspaces[device])
+        if (w.stream == stream) {
+            cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+            if (stream && (cudaStreamIsCapturing(stream, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone))
+                return {};
+            return w.buffer;
+        }
+    return {};
+}
 
 bool plain_cuda(const at::Tensor &t) {
     return t.is_cuda() && t.layout() == at::kStrided && t.is_contiguous() && !at::isTensorSubclassLike(t);
@@ -112,7 +132,8 @@ PyObject *fast_linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     const int64_t batch = x.numel() / columns;
     const int device = x.device().index();
     if (batch <= 0 || batch > INT32_MAX || device < 0 || device >= kMaxDevices) Py_RETURN_NONE;
-    const at::Tensor ws = g_workspace[device];
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
+    const at::Tensor ws = workspace_of(device, stream);
     const size_t need = g_workspace_bytes((int)batch, (int)rows, (int)columns), have = ws.defined() ? ws.nbytes() : 0;
     if (need > have) Py_RETURN_NONE;
     void *scratch = have ? ws.mutable_data_ptr() : nullptr;
@@ -126,7 +147,6 @@ PyObject *fast_linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         const pybind11::gil_scoped_release no_gil;
         const c10::cuda::CUDAGuard guard(x.device());
         out = at::detail::empty_cuda(shape, f32 ? at::kFloat : at::kHalf, x.device(), std::nullopt);
-        void *stream = c10::cuda::getCurrentCUDAStream(device).stream();
         rc = swiglu ? g_swiglu(w, x.const_data_ptr(), out.mutable_data_ptr(), f32, (int)batch, (int)(rows / 2),
                                (int)columns, scratch, have, stream)
                     : g_linear(w, x.const_data_ptr(), out.mutable_data_ptr(), f32, (int)batch, (int)rows,
@@ -193,15 +213,23 @@ PyObject *bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     Py_RETURN_NONE;
 }
 
-// set_workspace(device, tensor)
+// set_workspace(device, stream, tensor): None takes the stream's buffer out of the table
 PyObject *set_workspace(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
-    if (nargs != 2 || !THPVariable_Check(args[1])) {
-        PyErr_SetString(PyExc_TypeError, "set_workspace takes a device index and a tensor");
+    if (nargs != 3 || (args[2] != Py_None && !THPVariable_Check(args[2]))) {
+        PyErr_SetString(PyExc_TypeError, "set_workspace takes a device index, a stream and a tensor or None");
         return nullptr;
     }
     const long device = PyLong_AsLong(args[0]);
+    const auto stream = static_cast<cudaStream_t>(PyLong_AsVoidPtr(args[1]));
     if (PyErr_Occurred()) return nullptr;
-    if (device >= 0 && device < kMaxDevices) g_workspace[device] = THPVariable_Unpack(args[1]);
+    if (device < 0 || device >= kMaxDevices) Py_RETURN_NONE;
+    std::vector<Workspace> &table = g_workspaces[device];
+    for (size_t i = 0; i < table.size(); ++i)
+        if (table[i].stream == stream) {
+            table.erase(table.begin() + i);
+            break;
+        }
+    if (args[2] != Py_None) table.push_back({stream, THPVariable_Unpack(args[2])});
     Py_RETURN_NONE;
 }
 
@@ -209,7 +237,7 @@ PyMethodDef methods[] = {
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<fast_linear>)), METH_FASTCALL, nullptr},
     {"embedding", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<fast_embedding>)), METH_FASTCALL, nullptr},
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(bind)), METH_FASTCALL, nullptr},
-    {"set_workspace", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(set_workspace)), METH_FASTCALL, nullptr},
+    {"set_workspace", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<set_workspace>)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_ternel_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

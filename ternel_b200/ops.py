@@ -19,6 +19,7 @@ names and the pre-launch checks of the reference's kernel wrappers
 from __future__ import annotations
 
 import ctypes
+import threading
 
 import torch
 
@@ -29,8 +30,13 @@ from .layout import out_of_range_message
 ACTIVATION_DTYPES = (torch.float16,)
 OUTPUT_DTYPES = (torch.float16, torch.float32)
 
+# Scratch buffers: one per device for calls on its default stream and for captured ones, which hold it for good, and one for
+# each of the last few other streams that have called. Buffers that a larger one has taken over from stay alive.
+MAX_STREAM_WORKSPACES = 8
 _workspaces: dict[int, torch.Tensor] = {}
-_replaced: list[torch.Tensor] = []          # buffers that a larger one has taken over from
+_stream_workspaces: dict[tuple[int, int], torch.Tensor] = {}
+_replaced: dict[int, list[torch.Tensor]] = {}
+_workspace_lock = threading.Lock()
 
 
 def _stream_ptr(device: torch.device) -> ctypes.c_void_p:
@@ -39,40 +45,53 @@ def _stream_ptr(device: torch.device) -> ctypes.c_void_p:
 
 def _new_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     """A zero-filled buffer (slots and counters start at zero) of a power of two bytes, at least 1 MiB."""
-    buf = torch.zeros(1 << max(20, (nbytes - 1).bit_length()), dtype=torch.uint8, device=device)
-    torch.cuda.current_stream(device).synchronize()             # whatever stream uses it next
-    return buf
+    return torch.zeros(1 << max(20, (nbytes - 1).bit_length()), dtype=torch.uint8, device=device)
 
 
 def _workspace(device: torch.device, nbytes: int) -> torch.Tensor | None:
-    """A per-device scratch buffer, grown on demand and reused across calls.
+    """A scratch buffer for a call on the current stream, grown on demand and reused across calls.
 
-    Calls on one device share it, which is safe because they are ordered on the
-    current stream; callers that use several streams per device must pass their
-    own workspace through the C ABI instead.
+    Calls that may overlap need separate buffers, so every stream has its own. Only the last ``MAX_STREAM_WORKSPACES`` streams
+    of a device that asked for one keep it; a buffer that is let go returns to the allocator in the order of its stream.
 
-    A captured graph keeps the address it was captured with, and its replays expect the buffer as the last call left it. So
-    a buffer is never given back when a larger one replaces it: sizes are powers of two, so all replaced ones together are smaller
-    than the one in use. A call that is being captured and needs more than there is brings a buffer of its own, which belongs to the
-    graph's memory and is zero-filled by each replay: outside of the graph it would not be zero.
+    A captured graph keeps the address it was captured with, and its replays expect the buffer as the last call left it.
+    Captured calls therefore take the default stream's buffer, which is at least as large as any other (a warm-up on a side
+    stream has grown it) and is never given back when a larger one replaces it: sizes are powers of two, so all replaced
+    ones together are smaller than the one in use. A captured call that needs more than there is brings a buffer of its own,
+    which belongs to the graph's memory and is zero-filled by each replay. Replays count as calls on the default stream.
     """
     if nbytes == 0:
         return None
     index = device.index if device.index is not None else torch.cuda.current_device()
-    buf = _workspaces.get(index)
-    if buf is None or buf.numel() < nbytes:
-        if torch.cuda.is_current_stream_capturing():
-            return torch.zeros(nbytes, dtype=torch.uint8, device=device)
-        if buf is not None:
-            _replaced.append(buf)
-        buf = _new_workspace(device, nbytes)
-        _workspaces[index] = buf
-        _native.binding().set_workspace(index, buf)
-    return buf
+    stream = torch.cuda.current_stream(device).cuda_stream
+    with torch.cuda.device(index):
+        capturing = torch.cuda.is_current_stream_capturing()
+    with _workspace_lock:
+        shared = _workspaces.get(index)
+        if shared is None or shared.numel() < nbytes:
+            if capturing:
+                return torch.zeros(nbytes, dtype=torch.uint8, device=device)
+            if shared is not None:
+                _replaced.setdefault(index, []).append(shared)
+            with torch.cuda.stream(torch.cuda.default_stream(device)):
+                shared = _workspaces[index] = _new_workspace(device, nbytes)
+            _native.binding().set_workspace(index, 0, shared)
+        if capturing or stream == 0:
+            return shared
+        own = _stream_workspaces.pop((index, stream), None)
+        if own is None or own.numel() < nbytes:
+            own = _new_workspace(device, nbytes)
+            _native.binding().set_workspace(index, stream, own)
+        _stream_workspaces[index, stream] = own                 # the last one used stands last
+        others = [key for key in _stream_workspaces if key[0] == index]
+        if len(others) > MAX_STREAM_WORKSPACES:
+            del _stream_workspaces[others[0]]
+            _native.binding().set_workspace(index, others[0][1], None)
+        return own
 
 
 def check_status(device=None) -> None:
-    """Read the status word of the shared per-device workspace (synchronises the device).
+    """Read the status words of the device's workspaces (synchronises the device).
 
     Zero: every bounded wait inside the kernels was met. 7: results are good but the sequence tags are about
     to wrap, so the workspace is zeroed here. Anything else raises: a wait ran out (the results of the calls
@@ -80,16 +99,19 @@ def check_status(device=None) -> None:
     """
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     index = device.index if device.index is not None else torch.cuda.current_device()
-    buf = _workspaces.get(index)
-    if buf is None:
+    if index not in _workspaces:
         return
     torch.cuda.synchronize(device)
-    status = int(buf[:4].view(torch.int32)[0].item())
-    if status == 0:
-        return
-    buf.zero_()
-    if status != 7:
-        raise RuntimeError(f"a bounded wait inside a packed ternary kernel ran out (status {status}); "
+    buffers = [_workspaces[index], *_replaced.get(index, ()), *(b for k, b in _stream_workspaces.items() if k[0] == index)]
+    failed = 0
+    for buf in buffers:
+        status = int(buf[:4].view(torch.int32)[0].item())
+        if status:
+            buf.zero_()
+            torch.cuda.synchronize(device)      # the buffer may be another stream's
+            failed = status if status != 7 else failed
+    if failed:
+        raise RuntimeError(f"a bounded wait inside a packed ternary kernel ran out (status {failed}); "
                            "the workspace has been reset")
 
 

@@ -5,6 +5,7 @@ import sys
 from pathlib import Path
 
 import pytest
+import torch
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +39,36 @@ def test_a_graph_outlives_the_growth_of_the_workspace():
     run = subprocess.run([sys.executable, "-c", GRAPH_SCRIPT], capture_output=True, text=True, timeout=300,
                          cwd=Path(__file__).resolve().parents[1])
     assert run.returncode == 0 and "fine" in run.stdout, run.stdout + run.stderr
+
+
+def test_streams_may_overlap():
+    """Products that share tiles between different numbers of K parts, on three streams at once and over and over: every one
+    as on the default stream alone, and afterwards the default stream's too."""
+    from ternel_b200 import ops
+    from ternel_b200.stack import random_blocks_device
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(11)
+    shapes = ((8, 5120, 17408), (64, 5120, 17408), (3, 1024, 5120), (1, 5120, 5120), (300, 1024, 5120))
+    cases = [(random_blocks_device(n, k, gen, "cuda"), torch.randn((m, k), generator=gen, device="cuda").half())
+             for m, n, k in shapes]
+    want = [ops.tq1_matmul(b, x) for b, x in cases]
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    torch.cuda.synchronize()
+    got = []
+    for turn in range(30):
+        for s, stream in enumerate(streams):
+            with torch.cuda.stream(stream):
+                which = (turn + 2 * s) % len(cases)
+                got.append((which, ops.tq1_matmul(*cases[which])))
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, want[which]) for which, y in got)
+    for (b, x), y in zip(cases, want):
+        assert torch.equal(ops.tq1_matmul(b, x), y)
+    ops.check_status()
+    assert len(ops._stream_workspaces) <= ops.MAX_STREAM_WORKSPACES
+    for _ in range(2 * ops.MAX_STREAM_WORKSPACES):                      # more streams than keep a buffer
+        with torch.cuda.stream(torch.cuda.Stream()):
+            got = ops.tq1_matmul(*cases[0])
+        torch.cuda.synchronize()
+        assert torch.equal(got, want[0])
+    assert len(ops._stream_workspaces) <= ops.MAX_STREAM_WORKSPACES

@@ -27,7 +27,9 @@ def host(monkeypatch):
     monkeypatch.setattr(torch.cuda, "current_stream",
                         lambda *a: types.SimpleNamespace(cuda_stream=state.stream, synchronize=lambda: None))
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: state.capturing)
-    monkeypatch.setattr(torch.cuda, "device", lambda *a: contextlib.nullcontext())
+    for context in ("device", "stream"):
+        monkeypatch.setattr(torch.cuda, context, lambda *a: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "default_stream", lambda *a: None)
     monkeypatch.setattr(ops._native, "binding", lambda: types.SimpleNamespace(set_workspace=set_workspace))
     for name in ("_workspaces", "_stream_workspaces", "_replaced"):
         if hasattr(ops, name):
@@ -65,3 +67,28 @@ def test_a_captured_call_that_needs_more_brings_its_own_buffer(host):
     assert own is not first and own.numel() >= 40 * MIB
     host.capturing, host.stream = False, 0
     assert get(2 * MIB) is first
+
+
+def test_every_stream_has_a_buffer_of_its_own(host):
+    """Calls on two streams may overlap. Captured calls take the default stream's buffer, however the streams were warmed up,
+    and only the last few streams keep one."""
+    shared = get(2 * MIB)
+    host.stream = 11
+    side = get(2 * MIB)
+    assert side is not shared and get(MIB) is side
+    larger = get(20 * MIB)                              # a warm-up on a side stream
+    assert larger is not side
+    host.capturing = True
+    captured = get(20 * MIB)
+    assert captured is not larger and captured.numel() >= 20 * MIB
+    host.capturing, host.stream = False, 0
+    assert get(20 * MIB) is captured
+    assert host.table[0] is captured and host.table[11] is larger
+    for stream in range(100, 100 + 3 * ops.MAX_STREAM_WORKSPACES):
+        host.stream = stream
+        get(MIB)
+        host.stream = 11
+        assert get(20 * MIB) is larger                  # in use all along, so it is kept
+    assert len(ops._stream_workspaces) == ops.MAX_STREAM_WORKSPACES
+    assert host.table[100] is None                      # let go, also where the short call path looks
+    assert len([buf for buf in host.table.values() if buf is not None]) == ops.MAX_STREAM_WORKSPACES + 1
