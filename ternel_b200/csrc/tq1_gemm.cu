@@ -699,6 +699,7 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                 asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
                 const bool last = before == (unsigned)(hi - lo);
                 if (last) *counter = 0u;                // zero for the next call
+                if (before > (unsigned)(hi - lo)) atomicExch(prm.status, 8u);     // it was not zero when the call began
                 *last_flag = last ? 1u : 0u;
             }
             asm volatile("bar.sync 1, %0;" ::"n"(kDecode * 32) : "memory");

@@ -72,3 +72,34 @@ def test_streams_may_overlap():
         torch.cuda.synchronize()
         assert torch.equal(got, want[0])
     assert len(ops._stream_workspaces) <= ops.MAX_STREAM_WORKSPACES
+
+
+def test_counters_that_are_not_zero_are_reported():
+    """The counters of shared tiles have to be zero when a call begins. One that is beyond its tile's number of parts (here as
+    a stale workspace would leave it) cannot complete the tile: status 8, and good results again after a zero-fill."""
+    import ctypes
+    from ternel_b200 import _native
+    from ternel_b200.dispatch import plan
+    from ternel_b200.ops import tq1_matmul
+    from ternel_b200.stack import random_blocks_device
+    m, n, k = 8, 1024, 5120
+    assert plan(m, n, k).parts > 1
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(2)
+    blocks, x = random_blocks_device(n, k, gen, "cuda"), torch.randn((m, k), generator=gen, device="cuda").half()
+    lib = _native.lib()
+    need = lib.tq1_linear_workspace_bytes(m, n, k)
+    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    slots_end = 256 + (16 << 20)
+    ws[slots_end - 4096:slots_end + 4096].view(torch.int32).fill_(99)       # the counters, and slots and scratch beside them
+    y = torch.zeros((m, n), dtype=torch.float16, device="cuda")
+
+    def call():
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        assert lib.tq1_linear_f16(blocks.data_ptr(), x.data_ptr(), y.data_ptr(), 0, m, n, k, ws.data_ptr(), need, stream) == 0
+        return int(ws[:4].view(torch.int32).item())
+
+    assert call() == 8
+    ws.zero_()
+    assert call() == 0 and torch.equal(y, tq1_matmul(blocks, x))
+    assert call() == 0 and torch.equal(y, tq1_matmul(blocks, x))
