@@ -120,8 +120,9 @@ size_t tq1_linear_workspace_bytes(int M, int N, int K);
  *             a kernel ran out, words 1..4 are counters of the M == 1 kernel),
  *             then 16 MiB of partial-sum slots for M == 1 (eight bytes per row
  *             and 512-wide K chunk: the value and a sequence tag in one 64-bit
- *             word, so nothing is ever cleared), then the scratch of the
- *             M >= 2 kernels. After a non-zero status, zero-fill the workspace
+ *             word, so nothing is ever cleared), then 4 KiB of tile counters
+ *             of the M >= 2 kernel (zero between calls; status 8: one was not)
+ *             and its scratch. After a non-zero status, zero-fill the workspace
  *             again. Status 7 is not a failure: the results are good, but the
  *             32-bit sequence tags have passed 0xF0000000 executed projections
  *             and the workspace must be zero-filled before they wrap.

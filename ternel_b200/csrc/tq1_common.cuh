@@ -17,13 +17,13 @@ constexpr int kMaxFull = 242;
 constexpr int kMaxTail = 26;
 
 // Workspace layout shared by every linear kernel: [control words, 256 B][partial-sum slots of the
-// batch-1 kernel][counters of the batched kernel, 4 KiB; 16 MiB with the slots][scratch of the batched
+// batch-1 kernel, 16 MiB][counters of the batched kernel, 4 KiB][scratch of the batched
 // kernel, or the hand-off words of a chain]. Slots carry sequence tags, so nothing in the slot region ever
 // has to be cleared, and the counters are zero between calls; no other kernel writes to either, so calls of
 // any shape and kind can share one workspace. The workspace must be zero-filled once before its first use.
 constexpr size_t kWsStatusBytes = 256;
 constexpr size_t kWsCounterBytes = 4096;
-constexpr size_t kWsSlotRegionBytes = ((size_t)16 << 20) - kWsCounterBytes;
+constexpr size_t kWsSlotRegionBytes = (size_t)16 << 20;       // 2^21 slots: 131072 rows of 8192 columns are one link
 constexpr size_t kWsCounterOffset = kWsStatusBytes + kWsSlotRegionBytes;
 constexpr size_t kWsScratchOffset = kWsCounterOffset + kWsCounterBytes;
 
