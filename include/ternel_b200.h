@@ -97,7 +97,9 @@ int tq1_validate_codes_device(const uint8_t *codes_dev, int64_t rows, int64_t gp
 int tq1_untile_blocks_device(const uint8_t *codes_dev, const uint16_t *scales_dev, uint8_t *blocks_dev, int64_t rows,
                              int64_t gpr, int64_t tile, void *stream);
 
-/* Scratch the linear entry point needs for this shape (0 when none). The
+/* Scratch the linear entry point needs for this shape (0 when none) and, with
+ * K % 512 == 0, for every shape that is no larger in any of the three, so that
+ * one workspace serves all calls up to the largest. The
  * caller owns the buffer, as the caller of launch_tq1_lut23_smem_streamk owns
  * its workspace (cuda/tq1_lut23_streamk.cu:320-367, lut23_workspace_bytes). */
 size_t tq1_linear_workspace_bytes(int M, int N, int K);

@@ -6,14 +6,23 @@
 
 using namespace tq1;
 
-extern "C" {
-
-size_t tq1_linear_workspace_bytes(int M, int N, int K) {
+// Bytes that a call of this shape uses.
+static size_t linear_scratch_bytes(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0 || K % kGroup) return 0;
     if (M == 1 && gemv_chain_shape_ok(N, K)) return gemv_chain_workspace_bytes(N, K);
     if (gemm_tc_shape_ok(M, N, K)) return gemm_tc_workspace_bytes(M, N, K);
     // the kernel for the other widths runs without a workspace; a caller that has one finds its status word in place
     return gemm_groups_preferred(M, N, K) ? kWsStatusBytes : 0;
+}
+
+extern "C" {
+
+// Bytes that calls of this shape and of every smaller one with K % 512 == 0 use: how many partial tiles a shape leaves does
+// not grow with it (257 tokens take tiles of 144, 256 tokens a tile of 256), but callers make one workspace for the largest.
+size_t tq1_linear_workspace_bytes(int M, int N, int K) {
+    const size_t used = linear_scratch_bytes(M, N, K);
+    if (used == 0 || K % 512) return used;
+    return M == 1 ? gemv_chain_workspace_bound(N, K) : gemm_tc_workspace_bound(M);
 }
 
 int tq1_linear_f16(const uint8_t *blocks, const void *x, void *y, int y_is_f32,
@@ -28,7 +37,7 @@ int tq1_linear_f16(const uint8_t *blocks, const void *x, void *y, int y_is_f32,
         return fail(TQ1_ERR_INVALID, "tq1_linear_f16: blocks must be 4-byte aligned");
     if (reinterpret_cast<uintptr_t>(x) & 15)
         return fail(TQ1_ERR_INVALID, "tq1_linear_f16: x must be 16-byte aligned");
-    const size_t need = tq1_linear_workspace_bytes(M, N, K);
+    const size_t need = linear_scratch_bytes(M, N, K);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (need && K % 512 == 0 && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255)))
         return fail(TQ1_ERR_WORKSPACE, "tq1_linear_f16: workspace of %zu bytes (256-byte aligned) required", need);
@@ -58,7 +67,7 @@ int tq1_linear_swiglu_f16(const uint8_t *blocks, const void *x, void *y, int y_i
     if (!gemv && (M < 2 || K % 512 || (reinterpret_cast<uintptr_t>(blocks) & 15)))
         return fail(TQ1_ERR_INVALID,
                     "tq1_linear_swiglu_f16: needs K %% 512 == 0 and 16-byte aligned blocks (got %dx%d)", rows, K);
-    const size_t need = tq1_linear_workspace_bytes(M, rows, K);
+    const size_t need = linear_scratch_bytes(M, rows, K);
     if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255))
         return fail(TQ1_ERR_WORKSPACE, "tq1_linear_swiglu_f16: workspace of %zu bytes (256-byte aligned) required", need);
     cudaStream_t s = static_cast<cudaStream_t>(stream);

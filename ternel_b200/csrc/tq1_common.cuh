@@ -87,6 +87,7 @@ bool gemv_chain_shape_ok(int N, int K);
 bool gemv_chain_supported(const uint8_t *blocks, int N, int K);
 bool gemv_chain_fits(const uint8_t *blocks, int N, int K);      // also checks the current device's SM count
 size_t gemv_chain_workspace_bytes(int N, int K);
+size_t gemv_chain_workspace_bound(int N, int K);                // for this matrix and every smaller one
 // a few activation rows as M links of one launch over the same weights
 bool gemv_looped_fits(const uint8_t *blocks, int M, int N, int K);
 int launch_gemv_looped(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, bool swiglu,
@@ -105,7 +106,8 @@ int gemv_noalloc_status(unsigned *out_host, cudaStream_t stream);
 
 // Batched linear (M >= 2) on tcgen05 tensor cores; needs K % 512 == 0 and 16-byte aligned pointers.
 bool gemm_tc_shape_ok(int M, int N, int K);
-size_t gemm_tc_workspace_bytes(int M, int N, int K);
+size_t gemm_tc_workspace_bytes(int M, int N, int K);       // what the call uses
+size_t gemm_tc_workspace_bound(int M);                     // what calls of at most M rows use, whatever N and K
 int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K,
                    void *workspace, cudaStream_t stream, bool swiglu = false);
 

@@ -963,6 +963,13 @@ size_t gemm_tc_workspace_bytes(int M, int N, int K) {
     return kWsScratchOffset + align256((size_t)2 * t.ctas() * t.nt * kTileW * sizeof(float));
 }
 
+// The largest such size over all tiles, N and K, and over all smaller batches: token columns in flight on one SM are at most
+// 32 (two 16-token tiles), two 32-token tiles or one tile of the batch's length.
+size_t gemm_tc_workspace_bound(int M) {
+    const int columns = M <= 16 ? 32 : M <= 64 ? 64 : M >= 256 ? 256 : (M + 31) / 32 * 32;
+    return kWsScratchOffset + align256((size_t)2 * sm_count_cached() * columns * kTileW * sizeof(float));
+}
+
 int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K,
                    void *workspace, cudaStream_t stream, bool swiglu) {
     EncodeTiledFn encode = gemm_encode_fn();

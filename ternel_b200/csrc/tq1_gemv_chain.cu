@@ -1308,6 +1308,13 @@ bool gemv_chain_fits(const uint8_t *blocks, int N, int K) {
     return span_ok((rows + kTileRows - 1) / kTileRows, K / kChunkCols, grid);
 }
 
+// The same for every matrix up to this one: a matrix that the region does not hold is cut into equal row ranges, which can be
+// smaller than the whole of a shorter matrix.
+size_t gemv_chain_workspace_bound(int N, int K) {
+    const size_t rows = rows_per_link(N, K, kWsSlotRegionBytes / sizeof(unsigned long long));
+    return rows < (size_t)N ? kWsStatusBytes + kWsSlotRegionBytes : gemv_chain_workspace_bytes(N, K);
+}
+
 size_t gemv_chain_workspace_bytes(int N, int K) {
     const size_t rows = rows_per_link(N, K, kWsSlotRegionBytes / sizeof(unsigned long long));
     const size_t tiles = (rows + kTileRows - 1) / kTileRows;
