@@ -9,7 +9,6 @@
 
 #include <algorithm>
 #include <atomic>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -50,7 +49,7 @@ static void parallel_parts(int64_t n, int64_t grain, const F &f) {
         const int64_t begin = n * i / parts, end = n * (i + 1) / parts;
         try {
             threads[i] = std::thread([&f, i, begin, end] { f(i, begin, end); });
-        } catch (const std::system_error &) {       // no thread to be had: the part runs here
+        } catch (...) {                             // no thread to be had, or no memory for one: the part runs here
             f(i, begin, end);
         }
     }
@@ -80,7 +79,7 @@ static bool checked_parts(int64_t n, int64_t grain, const C &check, const F &act
     for (int i = 1; i < workers; ++i) {
         try {
             threads[i] = std::thread(work);
-        } catch (const std::system_error &) {       // no thread to be had: the others do its pieces
+        } catch (...) {                             // no thread to be had, or no memory for one: the others do its pieces
         }
     }
     work();
