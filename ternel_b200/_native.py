@@ -13,7 +13,7 @@ import os
 from pathlib import Path
 from ctypes import c_char_p, c_int, c_int64, c_size_t, c_void_p, POINTER
 
-from .build import BINDING_PATH, LIB_PATH
+from .build import BINDING_PATH, LIB_PATH, binding_built_for, binding_target
 
 TQ1_OK = 0
 TQ1_ERR_INVALID = -1
@@ -127,8 +127,9 @@ def binding():
     """The eager call path (``_ternel_torch``, built from csrc/torch_binding.cpp), bound to the loaded library."""
     global _binding
     if _binding is None:
-        if not BINDING_PATH.exists():
-            raise NativeLibraryMissing(f"{BINDING_PATH} is missing: build it with `python -m ternel_b200.build`")
+        if binding_built_for() != binding_target():
+            raise NativeLibraryMissing(f"{BINDING_PATH} is missing or built for {binding_built_for()}, not {binding_target()}: "
+                                       "build it with `python -m ternel_b200.build`")
         handle = lib()
         spec = importlib.util.spec_from_file_location("_ternel_torch", BINDING_PATH)
         module = importlib.util.module_from_spec(spec)

@@ -6,6 +6,7 @@ from __future__ import annotations
 import os
 import shutil
 import subprocess
+import sys
 import sysconfig
 from pathlib import Path
 
@@ -72,11 +73,28 @@ def build(force: bool = False, verbose: bool = False, target: Path = LIB_PATH, e
     return target
 
 
+def binding_target() -> str:
+    """What the eager call path has to be built for: its C++ side follows one PyTorch and one Python."""
+    import torch
+
+    return f"torch {torch.__version__}, {sys.implementation.cache_tag}"
+
+
+def binding_built_for() -> "str | None":
+    """What the module in ``_lib`` was built for, None where there is none (or none that says so)."""
+    stamp = BINDING_PATH.with_suffix(".target")
+    return stamp.read_text() if BINDING_PATH.exists() and stamp.exists() else None
+
+
+def binding_is_stale() -> bool:
+    header = PACKAGE_DIR.parent / "include" / "ternel_b200.h"
+    return binding_built_for() != binding_target() or any(
+        p.stat().st_mtime > BINDING_PATH.stat().st_mtime for p in (BINDING_SOURCE, header))
+
+
 def build_binding(force: bool = False) -> Path:
     """Build ``_lib/_ternel_torch.so``, the eager call path, against the installed PyTorch (host code only)."""
-    header = PACKAGE_DIR.parent / "include" / "ternel_b200.h"
-    if not force and BINDING_PATH.exists() and all(
-            p.stat().st_mtime <= BINDING_PATH.stat().st_mtime for p in (BINDING_SOURCE, header)):
+    if not force and not binding_is_stale():
         return BINDING_PATH
     import torch
 
@@ -94,6 +112,7 @@ def build_binding(force: bool = False) -> Path:
         tmp.unlink(missing_ok=True)
         raise RuntimeError(f"g++ failed:\n{done.stdout}\n{done.stderr}")
     os.replace(tmp, BINDING_PATH)
+    BINDING_PATH.with_suffix(".target").write_text(binding_target())
     return BINDING_PATH
 
 

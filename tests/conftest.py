@@ -16,9 +16,10 @@ def pytest_configure(config):
 
 @pytest.fixture(scope="session", autouse=True)
 def _built_library():
-    """Build the C-ABI library (nvcc cross-compiles without a GPU) and the C oracle once."""
-    from ternel_b200.build import build, build_checked
+    """Build the C-ABI library (nvcc cross-compiles without a GPU), the eager call path and the C oracle once."""
+    from ternel_b200.build import build, build_binding, build_checked
     build()
+    build_binding()
     build_checked()
     from oracle import c_oracle
     c_oracle.lib()
