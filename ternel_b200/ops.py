@@ -253,7 +253,8 @@ def validate_device_blocks(blocks: torch.Tensor) -> None:
 def load_tiled_device(blocks: torch.Tensor, codes: torch.Tensor, scales: torch.Tensor, tile: int) -> None:
     """Fill canonical ``blocks`` on the GPU from the tiled pair (``uint8[tiles, groups, 26, tile]`` and 16-bit
     ``[tiles, groups, tile]``, on the host or the GPU): the arrays are uploaded as they are, scanned there, and
-    converted only if every byte is legal (fail closed, as ``validate_packed_codes``)."""
+    converted only if every byte is legal (fail closed, as ``validate_packed_codes``). The blocks are there when the call
+    returns, on whatever stream they are used next."""
     rows, groups = _check_blocks(blocks)
     codes = codes.to(blocks.device).contiguous()
     scales = scales.to(blocks.device).contiguous()
@@ -266,6 +267,7 @@ def load_tiled_device(blocks: torch.Tensor, codes: torch.Tensor, scales: torch.T
             raise FormatError(out_of_range_message(bad_full, bad_tail))
         check(lib.tq1_untile_blocks_device(codes.data_ptr(), scales.data_ptr(), blocks.data_ptr(), rows, groups, tile,
                                            stream))
+        torch.cuda.current_stream().synchronize()
 
 
 def _check_activations(x: torch.Tensor, groups_per_row: int) -> int:

@@ -66,3 +66,27 @@ def test_tiled_pair_is_converted_on_the_gpu(rows, columns):
     with pytest.raises(FormatError, match=r"regular=2 \(max 242\), tail=1 \(max 26\)"):
         module.load_tiled(codes, np.zeros_like(scales))
     assert np.array_equal(module.blocks.cpu().numpy(), blocks)
+
+
+def test_loaded_blocks_are_there_on_every_stream():
+    """A load returns when the blocks are written, as a copy from the host does: nothing is left in flight on the loading
+    stream, so another stream or thread may use the module at once."""
+    from ternel_b200.layout import PackedTensorLayout, pack_blocks
+    from ternel_b200.modules import PackedLinear
+    layout = PackedTensorLayout.for_tensor(17408, 5120)
+    blocks, _ = random_blocks(17408, 5120, seed=1)
+    codes, scales = pack_blocks(blocks, layout=layout)
+    codes, scales = torch.from_numpy(codes).cuda(), torch.from_numpy(scales.view(np.int16)).cuda()
+    module = PackedLinear(layout, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(5):
+        loading, using = torch.cuda.Stream(), torch.cuda.Stream()
+        with torch.cuda.stream(loading):
+            module.load_tiled(codes, scales)
+            assert loading.query()
+        with torch.cuda.stream(using):
+            seen = module.blocks.clone()
+        torch.cuda.synchronize()
+        assert np.array_equal(seen.cpu().numpy(), blocks)
+        module.blocks.zero_()
+        torch.cuda.synchronize()
