@@ -16,6 +16,8 @@ missing or mis-shaped arrays and out-of-range code bytes (fail closed).
 
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import torch
 from torch import nn
@@ -41,13 +43,19 @@ def packed_matmul(blocks: torch.Tensor, x: torch.Tensor, *, layout: PackedTensor
 
 
 def _tensor_of(array) -> "torch.Tensor | None":
-    """A tensor over ``array``'s memory, or None where PyTorch cannot stand over it (byte order, read-only memory)."""
+    """A tensor over ``array``'s memory, which the caller only reads, or None where PyTorch has no such type."""
     if isinstance(array, torch.Tensor):
         return array
     array = np.asarray(array)
-    if not array.dtype.isnative or not array.flags.writeable or array.dtype not in (np.uint8, np.uint16, np.int16):
+    if not array.dtype.isnative or array.dtype not in (np.uint8, np.uint16, np.int16) or array.size == 0:
         return None
-    return torch.from_numpy(np.ascontiguousarray(array))
+    array = np.require(array, requirements=("C", "A"))
+    if array.flags.writeable:
+        return torch.from_numpy(array)
+    # torch.from_numpy warns about memory that cannot be written (a file mapping, a bytes object): stand over its address
+    memory = (ctypes.c_ubyte * array.nbytes).from_address(array.ctypes.data)
+    memory.owner = array                        # lives as long as the tensor does
+    return torch.frombuffer(memory, dtype=getattr(torch, array.dtype.name)).reshape(array.shape)
 
 
 class _PackedBase(nn.Module):

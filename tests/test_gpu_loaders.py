@@ -90,3 +90,17 @@ def test_loaded_blocks_are_there_on_every_stream():
         assert np.array_equal(seen.cpu().numpy(), blocks)
         module.blocks.zero_()
         torch.cuda.synchronize()
+
+
+def test_read_only_arrays_are_converted_on_the_gpu(monkeypatch):
+    """What a file mapping or a bytes object holds takes the same way as arrays that can be written."""
+    from ternel_b200 import modules
+    from ternel_b200.layout import PackedTensorLayout, pack_blocks
+    layout = PackedTensorLayout.for_tensor(768, 1408)
+    blocks, _ = random_blocks(768, 1408, seed=4)
+    codes, scales = pack_blocks(blocks, layout=layout)
+    codes, scales = (np.frombuffer(a.tobytes(), dtype=a.dtype).reshape(a.shape) for a in (codes, scales))
+    module = modules.PackedLinear(layout, device="cuda")
+    monkeypatch.setattr(modules, "unpack_blocks", None)                 # the host converter
+    module.load_tiled(codes, scales)
+    assert np.array_equal(module.blocks.cpu().numpy(), blocks)

@@ -187,3 +187,34 @@ def test_load_packed_model_fills_a_swapped_model(tmp_path):
     with pytest.raises(FormatError, match="head"):
         loaders.load_packed_model(model, loaders.SafetensorsFile(tmp_path / "partial.safetensors"))
     assert torch.is_tensor(model.head.blocks)
+
+
+def test_arrays_that_cannot_be_written_are_read_in_place(tmp_path):
+    """A bytes object, a file mapping, a frozen array: a tensor over the same memory, without a copy or a warning, that keeps
+    the memory alive; odd strides and odd addresses are copied."""
+    import gc
+    import warnings
+    import torch
+    from ternel_b200.modules import _tensor_of
+    values = np.arange(600, dtype=np.uint16)
+    values.tofile(tmp_path / "values")
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        for array in (np.frombuffer(values.tobytes(), dtype=np.uint16).reshape(3, 10, 20),
+                      np.memmap(tmp_path / "values", dtype=np.int16, mode="r", shape=(3, 10, 20)),
+                      np.frombuffer(values.tobytes(), dtype=np.uint8)):
+            assert not array.flags.writeable
+            want, address = array.copy(), array.ctypes.data
+            tensor = _tensor_of(array)
+            assert tensor.data_ptr() == address and tensor.shape == array.shape
+            del array
+            gc.collect()
+            junk = [np.full(600, 77, dtype=np.uint16) for _ in range(50)]
+            assert np.array_equal(tensor.numpy(), want) and len(junk) == 50
+        odd = np.frombuffer(b"x" + values.tobytes(), dtype=np.uint8)[1:].view(np.uint16)
+        strided = np.frombuffer(values.tobytes(), dtype=np.uint16)[::3]
+        for array in (odd, strided):
+            assert np.array_equal(_tensor_of(array).numpy(), array)
+    assert torch.equal(_tensor_of(torch.ones(2)), torch.ones(2))
+    for array in (values.astype(">u2"), values.astype(np.float16), np.zeros((0, 3), np.uint8)):
+        assert _tensor_of(array) is None
