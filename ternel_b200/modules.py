@@ -93,8 +93,9 @@ class _PackedBase(nn.Module):
 
     def load_tiled(self, codes, scales) -> None:
         """Install the reference's tiled ``codes`` / ``scales`` pair. A module on the GPU takes well-formed arrays as
-        they are and scans and converts them there; anything else goes through the host converter and its checks."""
-        if self.blocks.is_cuda and self.blocks.is_contiguous():
+        they are and scans and converts them there; anything else (blocks off the 4-byte grid, for one) goes through the
+        host converter and its checks."""
+        if self.blocks.is_cuda and self.blocks.is_contiguous() and self.blocks.data_ptr() % 4 == 0:
             device_codes, device_scales = _tensor_of(codes), _tensor_of(scales)
             if (device_codes is not None and device_codes.dtype == torch.uint8
                     and device_codes.shape == self.layout.codes_shape

@@ -104,3 +104,18 @@ def test_read_only_arrays_are_converted_on_the_gpu(monkeypatch):
     monkeypatch.setattr(modules, "unpack_blocks", None)                 # the host converter
     module.load_tiled(codes, scales)
     assert np.array_equal(module.blocks.cpu().numpy(), blocks)
+
+
+def test_blocks_off_the_word_grid_are_loaded_too():
+    """A module whose blocks are a view into a flat buffer at an odd address, which the conversion on the GPU does not take."""
+    from ternel_b200.layout import PackedTensorLayout, pack_blocks
+    from ternel_b200.modules import PackedLinear
+    layout = PackedTensorLayout.for_tensor(48, 640)
+    blocks, _ = random_blocks(48, 640, seed=2)
+    module = PackedLinear(layout, device="cuda")
+    flat = torch.zeros(blocks.size + 4, dtype=torch.uint8, device="cuda")
+    for shift in (1, 2, 3, 0):
+        module.blocks = flat[shift:shift + blocks.size].view(blocks.shape)
+        module.load_tiled(*pack_blocks(blocks, layout=layout))
+        assert np.array_equal(module.blocks.cpu().numpy(), blocks)
+        flat.zero_()
