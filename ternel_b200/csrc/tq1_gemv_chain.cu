@@ -382,9 +382,15 @@ __device__ __forceinline__ WarpRange warp_range(int tiles, int units_q, int unit
     return r;
 }
 
-// ALL_PANELS: every link's weights are chunk-major panels, so the 2-D TMA path is compiled out.
-template <bool ALL_PANELS>
+// kPanels: every link's weights are chunk-major panels, so the 2-D TMA path is compiled out.
+// kChain, kAlone: some weights are canonical; a chain of links, and independent products of one matrix. They differ in where
+// non-finite groups are dealt with: in a copy of the unit loop (kAlone, kPanels), or at the end of a unit of the one loop
+// (kChain). Which of the two leaves the compiler's common loop the faster differs from form to form: eight canonical layers
+// 262.7 us with two loops, 259.3 with one; eight panel layers 249.8 and 256.0; 151936x5120 alone 53.6 and 54.3.
+enum Form { kPanels, kChain, kAlone };
+template <Form FORM>
 __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __grid_constant__ ChainParams P) {
+    constexpr bool ALL_PANELS = FORM == kPanels;
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t window = (uint32_t)__cvta_generic_to_shared(smem);
     unsigned char *high = smem + (kWindowEnd - window);
@@ -618,26 +624,28 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
                 mbits = max(mbits, bad[k] ? 0u : __float_as_uint(a));
             }
             mbits = __reduce_max_sync(0xffffffffu, mbits);
-            int group_bad = __any_sync(0xffffffffu, anybad);           // infinite activations, or kGroupNan
-            if (group_bad) {
-                int infs = 0;
-                bool nan = false;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    infs += bad[k] ? 1 : 0;
-                    nan = nan || xv[k] != xv[k];
-                }
-                infs = __reduce_add_sync(0xffffffffu, infs);
-                group_bad = __any_sync(0xffffffffu, nan) ? kGroupNan : infs;
-            }
             // 2^E <= m < 2^(E+1); fixed point xi = round(v * 2^(21-E)), |xi| <= 2^22
             const int e_biased = mbits != 0u ? (int)(mbits >> 23) : 127;
             const float up = __uint_as_float((uint32_t)(275 - e_biased) << 23);                // 2^(21-E)
             int xi[4], s5 = 0;
             uint32_t ent[4];
 #pragma unroll
+            for (int k = 0; k < 4; ++k) xi[k] = __float2int_rn(xv[k] * up);
+            int group_bad = __any_sync(0xffffffffu, anybad);           // infinite activations, or kGroupNan
+            if (group_bad) {                            // rare; a finite group executes nothing of this
+                int infs = 0;
+                bool nan = false;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    infs += bad[k] ? 1 : 0;
+                    nan = nan || xv[k] != xv[k];
+                    xi[k] = bad[k] ? (xv[k] < 0.0f ? -1 : 1) : 0;
+                }
+                infs = __reduce_add_sync(0xffffffffu, infs);
+                group_bad = __any_sync(0xffffffffu, nan) ? kGroupNan : infs;
+            }
+#pragma unroll
             for (int k = 0; k < 4; ++k) {
-                xi[k] = group_bad ? (bad[k] ? (xv[k] < 0.0f ? -1 : 1) : 0) : __float2int_rn(xv[k] * up);
                 xchg[lane + 32 * k] = xi[k];                       // a code byte's first four trits need its fifth
                 ent[k] = preptab[lane + 32 * k];
                 s5 += (ent[k] >> 24) == 0u ? 121 * xi[k] : 0;      // 121 * sum of the fifth-trit activations
@@ -743,16 +751,19 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
             }
             const int seg = min(left, tiles - t);       // units of this chunk
             left -= seg;
-            // One unit. BAD: some group of the chunk holds NaN/Inf activations (rare; kept out of the common loop so that
-            // it costs the common loop neither branches nor registers).
+            // One unit. BAD: some group of the chunk holds NaN/Inf activations (rare; in the forms with two loops kept out of
+            // the common one so that it costs that neither branches nor registers).
             auto unit = [&](auto bad_tag) {
-                constexpr bool BAD = decltype(bad_tag)::value;
+                constexpr bool BAD = decltype(bad_tag)::value, AT_END = FORM == kChain;
                 const uint32_t bar = bar0 + 8u * cstage;
                 uint32_t arrived = mbar_test_wait(bar, cparity);
                 if (!arrived) arrived = slow_wait(bar, cparity);
                 // (arrived >> 8) is zero, but only the hardware knows: the tile loads depend on the wait
                 const uint32_t a1 = ring_warp + cstage * kUnitBytes + (arrived >> 8) + lane_tile_off;
                 float acc1 = 0.0f, acc2 = 0.0f;             // rows g and g+8, this lane's two groups
+                int sums1[2], sums2[2];                     // AT_END: what they were made of
+                float scales1[2], scales2[2];
+                const float inf = __int_as_float(0x7f800000), nan = __int_as_float(0x7fffffff);
 #pragma unroll
                 for (int sub = 0; sub < 2; ++sub) {
                     constexpr int kRow8 = 8 * kChunkBytes;
@@ -794,7 +805,6 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
                     float dot2 = (float)s2 * gpow[sub];
                     if (BAD) {
                         if (gbad[sub]) {
-                            const float inf = __int_as_float(0x7f800000), nan = __int_as_float(0x7fffffff);
                             dot1 = s1 == gbad[sub] ? inf : s1 == -gbad[sub] ? -inf : nan;
                             dot2 = s2 == gbad[sub] ? inf : s2 == -gbad[sub] ? -inf : nan;
                         }
@@ -803,6 +813,20 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
                     const float sc2 = __half2float(__ushort_as_half((unsigned short)(w2a & 0xffffu)));
                     acc1 = fmaf(sc1, dot1, acc1);
                     acc2 = fmaf(sc2, dot2, acc2);
+                    if (AT_END) { sums1[sub] = s1; sums2[sub] = s2; scales1[sub] = sc1; scales2[sub] = sc2; }
+                }
+                if (AT_END && __builtin_expect(chunk_bad, 0)) {
+                    acc1 = acc2 = 0.0f;
+#pragma unroll
+                    for (int sub = 0; sub < 2; ++sub) {
+                        float dot1 = (float)sums1[sub] * gpow[sub], dot2 = (float)sums2[sub] * gpow[sub];
+                        if (gbad[sub]) {
+                            dot1 = sums1[sub] == gbad[sub] ? inf : sums1[sub] == -gbad[sub] ? -inf : nan;
+                            dot2 = sums2[sub] == gbad[sub] ? inf : sums2[sub] == -gbad[sub] ? -inf : nan;
+                        }
+                        acc1 = fmaf(scales1[sub], dot1, acc1);
+                        acc2 = fmaf(scales2[sub], dot2, acc2);
+                    }
                 }
                 // the stage consumed one iteration ago is free: refill it
                 ++consumed;
@@ -820,11 +844,10 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
                 }
                 mine += kTileRows;
             };
-            if (!chunk_bad) {
-                for (int i = 0; i < seg; ++i) unit(std::false_type{});
-            } else {
+            if (FORM != kChain && chunk_bad)
                 for (int i = 0; i < seg; ++i) unit(std::true_type{});
-            }
+            else
+                for (int i = 0; i < seg; ++i) unit(std::false_type{});
             t = 0;
             ++c;
         }
@@ -974,11 +997,10 @@ int device_state(DeviceState **out) {
         int sms = 0;
         err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (err != cudaSuccess || sms <= 0) return cuda_fail(err, "tq1 chain: SM count");
-        err = cudaFuncSetAttribute(tq1_gemv_chain_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(kWindowEnd + kHighBytes));
-        if (err == cudaSuccess)
-            err = cudaFuncSetAttribute(tq1_gemv_chain_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(kWindowEnd + kHighBytes));
+        for (auto kernel : {tq1_gemv_chain_kernel<kPanels>, tq1_gemv_chain_kernel<kChain>, tq1_gemv_chain_kernel<kAlone>}) {
+            err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kWindowEnd + kHighBytes));
+            if (err != cudaSuccess) break;
+        }
         if (err != cudaSuccess) return cuda_fail(err, "tq1 chain: shared memory opt-in");
         st.sm_count = sms;
         st.attr_set = true;
@@ -1173,15 +1195,15 @@ int gemv_chain_describe(const tq1_chain_link *links, int n_links, int rank, int 
     return TQ1_OK;
 }
 
-// True when every link's weights are chunk-major panels (the kernel variant without the 2-D TMA path).
-bool all_panels(const ChainLinkDev *links, int n) {
+// The kernel form for a chain of these links.
+Form chain_form(const ChainLinkDev *links, int n) {
     for (int i = 0; i < n; ++i)
-        if (!(links[i].flags & kFlagPanels)) return false;
-    return n > 0;
+        if (!(links[i].flags & kFlagPanels)) return kChain;
+    return n > 0 ? kPanels : kChain;
 }
 
 int gemv_chain_launch(const ChainLinkDev *table_dev, const ChainLinkDev *inline_links, int n_dev_links,
-                      bool panels_only, unsigned tag_advance, void *workspace, size_t region_slots, int n_regions,
+                      Form form, unsigned tag_advance, void *workspace, size_t region_slots, int n_regions,
                       cudaStream_t stream) {
     DeviceState *st = nullptr;
     int rc = device_state(&st);
@@ -1213,8 +1235,9 @@ int gemv_chain_launch(const ChainLinkDev *table_dev, const ChainLinkDev *inline_
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = use_pdl ? 1 : 0;
-    cudaError_t err = panels_only ? cudaLaunchKernelEx(&cfg, tq1_gemv_chain_kernel<true>, params)
-                                  : cudaLaunchKernelEx(&cfg, tq1_gemv_chain_kernel<false>, params);
+    cudaError_t err = form == kPanels  ? cudaLaunchKernelEx(&cfg, tq1_gemv_chain_kernel<kPanels>, params)
+                      : form == kChain ? cudaLaunchKernelEx(&cfg, tq1_gemv_chain_kernel<kChain>, params)
+                                       : cudaLaunchKernelEx(&cfg, tq1_gemv_chain_kernel<kAlone>, params);
     if (err != cudaSuccess) return cuda_fail(err, "tq1 chain: launch");
     return TQ1_OK;
 }
@@ -1246,7 +1269,7 @@ int launch_gemv_single(const uint8_t *blocks, const __half *x, void *y, bool y_f
     if (rc != TQ1_OK) return rc;
     for (size_t i = 0; i < dev.size(); ++i) {          // row ranges of a very tall matrix: one launch each
         dev[i].tag = 0;
-        rc = gemv_chain_launch(nullptr, &dev[i], 1, all_panels(&dev[i], 1), 1u, workspace, region_slots, 1, stream);
+        rc = gemv_chain_launch(nullptr, &dev[i], 1, kAlone, 1u, workspace, region_slots, 1, stream);
         if (rc != TQ1_OK) return rc;
     }
     return TQ1_OK;
@@ -1275,7 +1298,7 @@ int launch_gemv_looped(const uint8_t *blocks, const __half *x, void *y, bool y_f
     rc = gemv_chain_describe(links, M, 0, 1, nullptr, kRegionSlotsTwo, grid, dev);
     if (rc != TQ1_OK) return rc;
     if ((int)dev.size() != M) return fail(TQ1_ERR_INVALID, "tq1 chain: matrix too tall for the looped path");
-    return gemv_chain_launch(nullptr, dev.data(), M, all_panels(dev.data(), M), (unsigned)M, workspace,
+    return gemv_chain_launch(nullptr, dev.data(), M, kAlone, (unsigned)M, workspace,
                              kRegionSlotsTwo, 2, stream);
 }
 
@@ -1475,7 +1498,7 @@ int tq1_chain_plan_create(const tq1_chain_link *links, int n_links, const tq1_ch
 int tq1_chain_plan_run(const tq1_chain_plan *plan, void *stream) {
     if (!plan) return fail(TQ1_ERR_INVALID, "tq1_chain_plan_run: null plan");
     return gemv_chain_launch(plan->table_dev, nullptr, plan->n_dev_links,
-                             all_panels(plan->host.data(), (int)plan->host.size()), (unsigned)plan->n_links, plan->workspace,
+                             chain_form(plan->host.data(), (int)plan->host.size()), (unsigned)plan->n_links, plan->workspace,
                              gemv_chain_region_slots(), 2, static_cast<cudaStream_t>(stream));
 }
 
@@ -1486,7 +1509,7 @@ int tq1_linear_chain_f16(const tq1_chain_link *links, int n_links, void *workspa
     std::vector<ChainLinkDev> dev;
     int rc = chain_describe_checked(links, n_links, nullptr, workspace, workspace_bytes, dev);
     if (rc != TQ1_OK) return rc;
-    return gemv_chain_launch(nullptr, dev.data(), (int)dev.size(), all_panels(dev.data(), (int)dev.size()),
+    return gemv_chain_launch(nullptr, dev.data(), (int)dev.size(), chain_form(dev.data(), (int)dev.size()),
                              (unsigned)n_links, workspace,
                              gemv_chain_region_slots(), 2, static_cast<cudaStream_t>(stream));
 }

@@ -374,3 +374,32 @@ def test_tags_close_to_wrapping_are_reported_and_results_stay_good():
     linear_chain(links, ws)
     torch.cuda.synchronize()
     assert int(words[0].item()) == 0
+
+
+@pytest.mark.parametrize("panels", (False, True))
+@pytest.mark.parametrize("value", (np.inf, -np.inf, np.nan))
+def test_nonfinite_groups_in_both_chain_forms(panels, value):
+    """Canonical and panel chains deal with non-finite groups in different places of the unit loop: two links that both read
+    an input with such values in one group and in two neighbouring ones (one lane's pair), class by class against the
+    reference's order, and bit for bit the single product. Finite links before and after them are not touched."""
+    from ternel_b200.chain import ChainPlan, Link, blocks_to_panels
+    from ternel_b200.ops import tq1_matmul
+    rows, columns = 720, 2048
+    blocks, rng = random_blocks(rows, columns, seed=91, dist="tests")
+    x = rng.standard_normal((3, columns)).astype(np.float16)
+    x[1, 130] = value
+    x[2, [3, 700, 777]] = value
+    device = to_dev(blocks)
+    weight = {"blocks": blocks_to_panels(device), "panel_rows": rows} if panels else {"blocks": device}
+    order = (0, 1, 2, 1, 0)
+    outs = [torch.zeros(rows, dtype=torch.float32, device="cuda") for _ in order]
+    plan = ChainPlan([Link(x=to_dev(x[i]), y=y, **weight) for i, y in zip(order, outs)])
+    plan.run()
+    torch.cuda.synchronize()
+    with np.errstate(invalid="ignore"):
+        want = o.reference_matmul(blocks, x.astype(np.float32), rows=rows, columns=columns)
+    assert np.isfinite(want[0]).all() and not np.isfinite(want[1]).all()
+    for i, y in zip(order, outs):
+        assert np.array_equal(o.nonfinite_classes(y.cpu().numpy()), o.nonfinite_classes(want[i]))
+        alone = tq1_matmul(device, to_dev(x[i:i + 1]), out_dtype=torch.float32)[0]
+        assert torch.equal(torch.nan_to_num(y), torch.nan_to_num(alone))
