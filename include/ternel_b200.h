@@ -128,8 +128,11 @@ size_t tq1_linear_workspace_bytes(int M, int N, int K);
  *             again. Status 7 is not a failure: the results are good, but the
  *             32-bit sequence tags have passed 0xF0000000 executed projections
  *             and the workspace must be zero-filled before they wrap.
- * The kernel is chosen from M: 1 => streaming GEMV, 2..16 => small-batch
- * split-K GEMV, larger => tiled GEMM. Illegal code bytes must have been
+ * With K % 512 == 0 and 16-byte aligned blocks the kernel is chosen from M:
+ * 1 and 2 => streaming GEMV (exact integer group sums), larger => tcgen05 GEMM
+ * (FP32 accumulators over up to a K part). Other widths and alignments: FP32
+ * group sums on the matrix units from 2^20 products on, the row kernel below
+ * and for M == 1; both need no workspace. Illegal code bytes must have been
  * rejected at load (tq1_validate_blocks*): the kernels carry no clamp. */
 int tq1_linear_f16(const uint8_t *blocks, const void *x, void *y, int y_is_f32,
                    int M, int N, int K, void *workspace, size_t workspace_bytes, void *stream);

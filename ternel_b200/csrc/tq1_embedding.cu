@@ -13,7 +13,7 @@
 // then selected by the trit.
 //
 // What bounds it: up to a wave or two of CTAs the chain id -> code bytes -> table entries -> store, beyond that the stores
-// (8192 tokens of 5120 columns: 21.4 us = 4.35 TB/s in FP16, 38.8 us = 5.3 TB/s in FP32). 2-bit trits unpacked one by one
+// (8192 tokens of 5120 columns: 21.4 us = 4.35 TB/s in FP16, 38.8 us = 4.56 TB/s in FP32). 2-bit trits unpacked one by one
 // took 123 instructions per eight outputs: 6.5 us for 2048 tokens against 6.06 now, 23.1 for 8192.
 #include "tq1_common.cuh"
 
