@@ -167,3 +167,40 @@ def test_other_threads_run_while_a_launch_waits():
     torch.cuda.synchronize()
     assert waited > 0.5                                     # the queue did fill up
     assert max(gaps) < 0.3, max(gaps)
+
+
+FIRST_CALLS = """
+import threading
+import torch
+from ternel_b200.ops import tq1_get_rows, tq1_matmul
+from ternel_b200.stack import random_blocks_device
+gen = torch.Generator(device="cuda")
+gen.manual_seed(1)
+blocks = random_blocks_device(1024, 1024, gen, "cuda")
+xs = [torch.randn((m, 1024), generator=gen, device="cuda").half() for m in (1, 5, 40, 1, 5, 40, 300, 2)]
+torch.cuda.synchronize()
+start, got = threading.Barrier(len(xs)), [None] * len(xs)
+
+def first(i):
+    start.wait()
+    got[i] = tq1_matmul(blocks, xs[i])
+
+threads = [threading.Thread(target=first, args=(i,)) for i in range(len(xs))]
+for t in threads: t.start()
+for t in threads: t.join()
+torch.cuda.synchronize()
+for x, y in zip(xs, got):
+    assert y is not None and torch.equal(y, tq1_matmul(blocks, x))
+print("fine")
+"""
+
+
+def test_the_first_calls_may_come_from_several_threads():
+    """In a process of its own: whatever is looked up or made once is complete for every thread that finds it there."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    for _ in range(3):
+        run = subprocess.run([sys.executable, "-c", FIRST_CALLS], capture_output=True, text=True, timeout=300,
+                             cwd=Path(__file__).resolve().parents[1])
+        assert run.returncode == 0 and "fine" in run.stdout, run.stdout + run.stderr
