@@ -54,16 +54,16 @@ struct Workspace {
 };
 std::array<std::vector<Workspace>, kMaxDevices> &g_workspaces = *new std::array<std::vector<Workspace>, kMaxDevices>();
 
-// The buffer for calls on `stream`, undefined where the Python side has to look: no buffer yet, or a capture, whose
-// kernels must not hold a buffer that may be given back (the default stream cannot be captured).
+// The buffer for calls on `stream`, undefined where there is none yet (the Python side makes it). Captured calls hold the
+// default stream's, which is never given back; the default stream itself cannot be captured.
 at::Tensor workspace_of(int device, cudaStream_t stream) {
+    if (stream) {
+        cudaStreamCaptureStatus status;
+        if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) return {};
+        if (status != cudaStreamCaptureStatusNone) stream = nullptr;
+    }
     for (const Workspace &w : g_workspaces[device])
-        if (w.stream == stream) {
-            cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-            if (stream && (cudaStreamIsCapturing(stream, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone))
-                return {};
-            return w.buffer;
-        }
+        if (w.stream == stream) return w.buffer;
     return {};
 }
 
