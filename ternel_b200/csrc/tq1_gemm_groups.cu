@@ -6,7 +6,7 @@
 // they do there. Weights stay -1, 0, +1 and enter mma.sync.m16n8k16 as its A operand; an accumulator covers 32 columns, the
 // sums of those are FP32 additions on the CUDA cores. The tcgen05 kernel with 4-byte copies had taken these widths with one
 // truncating accumulator over a whole K part: 1.3e-6 from the FP64 product (2-norm, 4099x2176) and 5.3e-6 (300 tokens of
-// 17408x5248) where the row kernel is at 5.7e-8 and 7.2e-8; this one is at 5.8e-8 and 7e-8.
+// 17408x5248) where the row kernel is at 5.7e-8 and 7.2e-8; this one is at 4.2e-8 and 5.3e-8.
 //
 // The contraction may take the columns of a group in any order as long as both operands agree. Here lane q of a quad holds
 // columns 32 s + 8 q .. + 7 of a group for two K = 16 steps: as activations that is one 16-byte load, as weights it is one
@@ -18,8 +18,9 @@
 //   many   a CTA has 128 weight rows and 8 NT tokens; activations come through shared memory (three stages of cp.async)
 //
 // What bounds it: up to 32 tokens the chain of dependent loads and the decode (25 instructions and six table or byte loads
-// per eight weights), beyond that the instructions around the products (700 tokens of 17408x5248: 89 T multiply-adds/s).
-// 5 tokens of 4099x2176 take 6.5 us (row kernel 45, tcgen05 form 10.1), 300 tokens of 4099x2176 56 us (2380, 21).
+// per eight weights), beyond that the products and the instructions around them (700 tokens of 17408x5248: 87 T
+// multiply-adds/s; an SM at work has its mma.sync pipe active for 57% of the time). 5 tokens of 4099x2176 take 5.6 us (row
+// kernel 45, tcgen05 form 11.6), 300 tokens of 4099x2176 60 us (2380, 21), the last of their two waves with 17 CTAs.
 #include "tq1_common.cuh"
 
 namespace tq1 {
@@ -324,8 +325,8 @@ int launch_many(const uint8_t *blocks, const __half *x, void *y, int y_f32, int 
 bool gemm_groups_preferred(int M, int N, int K) { return M >= 2 && (long long)M * N * K >= (1 << 20); }
 
 // The many-row kernel decodes a weight once for all of its tokens, but needs 128 rows a CTA: it takes over where its CTAs
-// fill most of the SMs. Both sides, us: 16 tokens of 17408x5248 38 against 39, of 5120x640 6.5 against 4.5; 32 tokens of
-// 17408x5248 51 against 70, of 4099x2176 22 against 11; 64 tokens of 17408x5248 67 against 136, of 4099x2176 30 against 20;
+// fill most of the SMs. Both sides, us: 16 tokens of 17408x5248 37 against 39, of 5120x640 6.5 against 4.5; 32 tokens of
+// 17408x5248 55 against 70, of 4099x2176 22 against 9; 64 tokens of 17408x5248 71 against 136, of 4099x2176 30 against 15;
 // 129 tokens of 4099x2176 30 against 42, 700 of 383x4224 54 against 31.
 int launch_gemm_groups(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K,
                        cudaStream_t stream) {
