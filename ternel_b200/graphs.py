@@ -23,12 +23,10 @@ class GraphedStep:
 
     def __init__(self, fn: Callable, example_inputs: Sequence[torch.Tensor], warmup: int = 2) -> None:
         self.static_inputs = [t.clone() for t in example_inputs]
-        side = torch.cuda.Stream(device=self.static_inputs[0].device)
-        side.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(side):               # warm up outside capture: workspaces, attributes
-            for _ in range(warmup):
-                fn(*self.static_inputs)
-        torch.cuda.current_stream().wait_stream(side)
+        # Warm up outside capture (workspaces, attributes), on the current stream: every other stream that calls the packed
+        # ops gets a workspace of its own, which a stream made for this alone would only leave behind.
+        for _ in range(warmup):
+            fn(*self.static_inputs)
         torch.cuda.synchronize()
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph):
