@@ -129,8 +129,9 @@ size_t tq1_linear_workspace_bytes(int M, int N, int K);
  *             32-bit sequence tags have passed 0xF0000000 executed projections
  *             and the workspace must be zero-filled before they wrap.
  * With K % 512 == 0 and 16-byte aligned blocks the kernel is chosen from M:
- * 1 and 2 => streaming GEMV (exact integer group sums), larger => tcgen05 GEMM
- * (FP32 accumulators over up to a K part). Other widths and alignments: FP32
+ * 1 and 2 => streaming GEMV (exact integer group sums), 3 to 16 => mma.sync out of
+ * registers where that is faster (FP32 accumulators over 64 columns), else tcgen05
+ * GEMM (FP32 accumulators over up to a K part). Other widths and alignments: FP32
  * group sums on the matrix units from 2^20 products on, the row kernel below
  * and for M == 1; both need no workspace. Illegal code bytes must have been
  * rejected at load (tq1_validate_blocks*): the kernels carry no clamp. */
@@ -152,7 +153,8 @@ int tq1_linear_swiglu_f16(const uint8_t *blocks, const void *x, void *y, int y_i
  * (tests/test_mlx_modules.py:553-1084); here the sweep is ternel_b200/dispatch_sweep_b200.json.
  *   aligned     1 if blocks and x are 16-byte aligned (the fast kernels need it)
  *   kernel      TQ1_KERNEL_*;  token_tile / ctas / parts: tensor-core kernel only (activation rows
- *               per tile, CTAs launched, equal K parts per tile or 0 for the stream-K split) */
+ *               per tile, CTAs launched, equal K parts per tile or 0 for the stream-K split). Up to 16
+ *               rows they describe the tcgen05 form, whose place the mma.sync form takes where it is faster */
 #define TQ1_KERNEL_ROWS 0
 #define TQ1_KERNEL_STREAM_GEMV 1
 #define TQ1_KERNEL_TENSOR_CORE 2

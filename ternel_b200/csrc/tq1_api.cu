@@ -6,6 +6,18 @@
 
 using namespace tq1;
 
+EncodeTiledFn tq1::encode_tiled_fn() {
+    static const EncodeTiledFn fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult qres;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) != cudaSuccess ||
+            qres != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return reinterpret_cast<EncodeTiledFn>(p);
+    }();
+    return fn;
+}
+
 // Bytes that a call of this shape uses.
 static size_t linear_scratch_bytes(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0 || K % kGroup) return 0;
@@ -46,6 +58,8 @@ int tq1_linear_f16(const uint8_t *blocks, const void *x, void *y, int y_is_f32,
                                   kWsSlotRegionBytes, s);
     if (gemv_looped_fits(blocks, M, N, K) && need >= kWsScratchOffset)
         return launch_gemv_looped(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, false, workspace, s);
+    if ((reinterpret_cast<uintptr_t>(blocks) & 15) == 0 && gemm_slices_preferred(M, N, K))
+        return launch_gemm_slices(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, workspace, s);
     if ((reinterpret_cast<uintptr_t>(blocks) & 15) == 0 && gemm_tc_shape_ok(M, N, K))
         return launch_gemm_tc(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, workspace, s);
     if (gemm_groups_preferred(M, N, K))
@@ -74,6 +88,8 @@ int tq1_linear_swiglu_f16(const uint8_t *blocks, const void *x, void *y, int y_i
     if (gemv) return launch_gemv_single(blocks, xh, y, y_is_f32 != 0, rows, K, true, workspace, kWsSlotRegionBytes, s);
     if (gemv_looped_fits(blocks, M, rows, K))
         return launch_gemv_looped(blocks, xh, y, y_is_f32 != 0, M, rows, K, true, workspace, s);
+    if (gemm_slices_preferred(M, rows, K))
+        return launch_gemm_slices(blocks, xh, y, y_is_f32 != 0, M, rows, K, workspace, s, true);
     return launch_gemm_tc(blocks, xh, y, y_is_f32 != 0, M, rows, K, workspace, s, true);
 }
 

@@ -1,5 +1,6 @@
 // Shared constants and helpers for the TQ1_G128 kernels (sm_100a).
 #pragma once
+#include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -33,7 +34,8 @@ constexpr size_t kWsScratchOffset = kWsCounterOffset + kWsCounterBytes;
 // traps nor touches memory it does not own. The reference's analogue is the SAFE build of its Metal kernels,
 // which clamps row indices (src/ternel_mlx/kernels.py:23-27). tq1_debug_bounds() reads the record.
 // Codes: 1x chain kernel (10 slot store, 11 slot read, 12 y, 13 hand-off store, 14 hand-off read),
-// 2x row kernel, 3x gather, 4x batched kernel (40 result, 41 partial tile), 5x panels, 6x shard push.
+// 2x row kernel, 3x gather, 4x batched kernel (40 result, 41 partial tile), 5x panels, 6x shard push,
+// 7x group sums, 8x slice kernel.
 #ifdef TQ1_BOUNDS_CHECK
 extern __device__ unsigned long long g_tq1_bounds[4];
 __device__ __forceinline__ bool tq1_in_bounds(long long index, long long limit, unsigned code) {
@@ -53,6 +55,12 @@ __device__ __forceinline__ bool tq1_in_bounds(long long index, long long limit, 
 // Records a message for tq1_last_error() and returns `code`.
 int fail(int code, const char *fmt, ...);
 int cuda_fail(cudaError_t err, const char *what);
+
+// cuTensorMapEncodeTiled, looked up once (a thread that comes while another one is looking waits for it); null if unavailable.
+typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn encode_tiled_fn();
 
 // Launchers implemented one per .cu file; all enqueue on `stream` and return a status.
 int launch_validate(const uint8_t *blocks, int64_t groups, int64_t *counts, cudaStream_t stream);
@@ -115,6 +123,13 @@ int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, 
 __host__ __device__ inline float swiglu_f32(float gate, float up) { return gate / (1.0f + expf(-gate)) * up; }
 void gemm_tc_plan(int M, int N, int K, int *tile, int *ctas, int *parts);
 int gemm_tc_force_tile(int nt);
+bool gemm_tc_forced();
+float gemm_tc_model_us(int M, int N, int K);                // modelled time of the tile that the kernel takes
+
+// Batched linear of 3 to 16 rows on mma.sync; needs K % 512 == 0 and 16-byte aligned pointers.
+bool gemm_slices_preferred(int M, int N, int K);            // fits, and faster than the tcgen05 kernel
+int launch_gemm_slices(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, void *workspace,
+                       cudaStream_t stream, bool swiglu = false);
 
 // Batched linear (M >= 2) with an FP32 sum per group, for every other width and alignment.
 bool gemm_groups_preferred(int M, int N, int K);

@@ -771,23 +771,6 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
     }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// Looked up once; a thread that comes while another one is looking waits for it.
-EncodeTiledFn gemm_encode_fn() {
-    static const EncodeTiledFn fn = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) != cudaSuccess ||
-            qres != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<EncodeTiledFn>(p);
-    }();
-    return fn;
-}
-
 // Launch state is per DEVICE: the SM count differs between devices and the shared-memory opt-in is an
 // attribute of a function on one device, so a process that drives several GPUs needs one record each.
 constexpr int kMaxDevices = 64;
@@ -879,30 +862,32 @@ Tiling make_tiling(int tile, int M, int N, int K) {
 // case). g_forced_tile overrides the rule while a sweep is being recorded.
 int g_forced_tile = 0;
 struct TileCost { int tile; float fixed, chunk, chunk_token, segment, shared_token; };
+const TileCost g_tile_costs[5] = {{16, 2.932f, 0.0f, 0.1263f, 1.968f, 0.1093f},
+                                  {32, 0.0f, 0.0f, 0.06457f, 1.932f, 0.1664f},
+                                  {64, 2.805f, 1.073f, 0.0f, 2.893f, 0.04036f},
+                                  {128, 3.198f, 0.8116f, 0.005891f, 2.846f, 0.02803f},
+                                  {256, 3.206f, 0.4634f, 0.009061f, 3.616f, 0.03028f}};
+float model_us(const TileCost &c, const Tiling &t) {
+    const WorkSplit &w = t.work;
+    const float shared = (float)w.total_iters / w.slots;        // chunks of shared tiles per slot
+    const float chunks = w.splits ? (float)((w.chunks + w.splits - 1) / w.splits)
+                                  : (float)w.whole_rounds * w.chunks + ceilf(shared);
+    const float segments = w.splits ? 1.0f : (float)w.whole_rounds + (w.total_iters ? shared / w.chunks + 1.0f : 0.0f);
+    const bool sums = w.splits ? w.splits > 1 : w.total_iters > 0;
+    return c.fixed + chunks * (c.chunk + c.chunk_token * t.nt) + segments * c.segment + (sums ? c.shared_token * t.nt : 0.0f);
+}
 int token_tile(int M, int N, int K) {
     if (g_forced_tile) return g_forced_tile;
     if (M <= 16) return 16;
-    static const TileCost costs[5] = {{16, 2.932f, 0.0f, 0.1263f, 1.968f, 0.1093f},
-                                      {32, 0.0f, 0.0f, 0.06457f, 1.932f, 0.1664f},
-                                      {64, 2.805f, 1.073f, 0.0f, 2.893f, 0.04036f},
-                                      {128, 3.198f, 0.8116f, 0.005891f, 2.846f, 0.02803f},
-                                      {256, 3.206f, 0.4634f, 0.009061f, 3.616f, 0.03028f}};
     int best = 128;
     float best_cost = 0.0f;
     for (int i = 0; i < 5; ++i) {
-        const TileCost &c = costs[i];
+        const TileCost &c = g_tile_costs[i];
         if (c.tile > 16 && c.tile >= 4 * M) continue;           // a tile mostly of padding
         const Tiling t = make_tiling(c.tile, M, N, K);
-        const WorkSplit &w = t.work;
         // whole tiles on less than half of the chip: a narrower tile splits K over the rest, with shorter accumulators
-        if (c.tile == 256 && w.splits == 1 && 2 * t.ctas() <= sm_count_cached()) continue;
-        const float shared = (float)w.total_iters / w.slots;    // chunks of shared tiles per slot
-        const float chunks = w.splits ? (float)((w.chunks + w.splits - 1) / w.splits)
-                                      : (float)w.whole_rounds * w.chunks + ceilf(shared);
-        const float segments = w.splits ? 1.0f : (float)w.whole_rounds + (w.total_iters ? shared / w.chunks + 1.0f : 0.0f);
-        const bool sums = w.splits ? w.splits > 1 : w.total_iters > 0;
-        const float cost = c.fixed + chunks * (c.chunk + c.chunk_token * t.nt) + segments * c.segment +
-                           (sums ? c.shared_token * t.nt : 0.0f);
+        if (c.tile == 256 && t.work.splits == 1 && 2 * t.ctas() <= sm_count_cached()) continue;
+        const float cost = model_us(c, t);
         if (i == 0 || cost < best_cost) { best = c.tile; best_cost = cost; }
     }
     return best;
@@ -948,6 +933,15 @@ int gemm_tc_force_tile(int nt) {
     return TQ1_OK;
 }
 
+bool gemm_tc_forced() { return g_forced_tile != 0; }
+
+float gemm_tc_model_us(int M, int N, int K) {
+    const Tiling t = pick_tiling(M, N, K);
+    int i = 0;
+    while (g_tile_costs[i].tile != t.tile) ++i;
+    return model_us(g_tile_costs[i], t);
+}
+
 void gemm_tc_plan(int M, int N, int K, int *tile, int *ctas, int *parts) {
     const Tiling t = pick_tiling(M, N, K);
     *tile = t.tile;
@@ -971,7 +965,7 @@ size_t gemm_tc_workspace_bound(int M) {
 
 int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K,
                    void *workspace, cudaStream_t stream, bool swiglu) {
-    EncodeTiledFn encode = gemm_encode_fn();
+    EncodeTiledFn encode = encode_tiled_fn();
     if (!encode) return fail(TQ1_ERR_CUDA, "tq1_linear_f16: cuTensorMapEncodeTiled is unavailable");
     unsigned char *ws = static_cast<unsigned char *>(workspace);
     const Tiling t = pick_tiling(M, N, K);

@@ -1,0 +1,721 @@
+// Linear of a few activation rows (3 to 16) for widths that are multiples of 512: decoded weights are the A operand of
+// mma.sync.m16n8k16, straight out of registers.
+//
+// The tcgen05 kernel needs 128 weight rows, tensor memory and a K split over CTAs with partial tiles through L2 for such calls:
+// about 7 us before and after the weights, and 311 instructions per 32 rows x 128 columns. Here decoded weights never leave the
+// registers of the warp that decoded them, and a row's sum never leaves the CTA (or its cluster).
+//
+//   slice     a K range of one warp: a 512-column chunk for up to eight tokens, half of one for sixteen (64 registers of
+//             activations either way). Lane (g, q) of a warp takes rows g and g + 8 of a 16-row tile and, in group q of the
+//             chunk, 64 consecutive columns at a time. The contraction may take the columns in any order as long as both operands
+//             agree, so the lane's consecutive weight pairs are the A registers of consecutive MMAs (four columns of each
+//             group of the chunk) and its 128 bytes of activations the B registers.
+//   warp      keeps the activations of its slice in registers and streams row tiles past it
+//   CTA       `slices` warps cover a K range, `subsets` such sets of warps take turns on the row tiles; one more warp fetches
+//             the tiles, 16 rows of the CTA's K range by one TMA box, into a ring (a bulk copy per row, from 16 lanes, took 240
+//             clocks per row to issue). Rows lie an odd number of 16-byte units apart: no bank conflicts between them.
+//   cluster   1, 2, 4 or 8 CTAs split K between them and add their sums through distributed shared memory
+//
+// The slices' sums of a tile meet in shared memory; the set's warps take turns with adding them, two tiles later, in a fixed
+// order (a warp that did nothing else needed 2500 clocks a tile beside twenty that decode, and set the pace).
+//
+// As in the tcgen05 kernel the group scale is folded into the FP16 weight, which is exact, and a code byte becomes PRMT
+// selectors by one lookup in a table with sixteen copies of an entry (src/ternel_mlx/kernels.py:435-440 of the reference
+// folds the scale the same way). A tensor-core accumulator covers 64 columns, everything above is FP32 additions: 1.3e-7 from
+// the FP64 product (2-norm) at every width, where the tcgen05 kernel has 1.8e-7 (512 columns) to 7.5e-7 (17408).
+//
+// What bounds it: few rows, the chain launch - activations - words - lookups - MMAs - sums; many rows, the instructions of the
+// decode with ten warps to hide their latencies (40% of issue slots, ALU 40%, shared memory 40%). 8 tokens, weights out of HBM,
+// against the tcgen05 kernel: 1024x5120 3.7 us (10.2), 4096x4096 5.5 (10.3), 5120x5120 7.9 (11.0), 17408x5120 14.5 (17.6),
+// 34816x5120 23.8 (26.3), 5120x17408 18.3 (18.9). Twenty warps with half a chunk each were as fast (322 instructions instead of
+// 253 per 16 rows x 256 columns); so were four warps for the sums, and fetching a tile's words before the sums before it.
+#include <cuda.h>
+
+#include <type_traits>
+
+#include "tq1_common.cuh"
+
+namespace tq1 {
+
+namespace {
+
+constexpr int kTileRows = 16;
+constexpr int kChunkBytes = 4 * kBlockBytes;                    // a row's bytes of a 512-column chunk
+constexpr int kChain = 4;                                       // MMAs (of 16 columns) under one accumulator
+constexpr uint32_t kSpinLimit = 1u << 20;
+constexpr int kMaxDevices = 64;
+
+constexpr uint32_t kWindow = 1024;                              // shared-window address of dynamic shared memory
+constexpr uint32_t kTableAddr = kWindow;                        // 256 entries of 256 bytes
+constexpr uint32_t kTableBytes = 65536;
+constexpr uint32_t kBarAddr = kTableAddr + kTableBytes;
+constexpr uint32_t kBarBytes = 2048;
+constexpr uint32_t kDataAddr = kBarAddr + kBarBytes;            // activations and later partial sums, sums (split K), ring
+constexpr uint32_t kXBytes = 4096;                              // activations: half a chunk, eight tokens
+constexpr uint32_t kWindowEnd = 227 * 1024;
+constexpr int kTokenPitch = 20;                                 // floats from one token's 16 rows to the next: no conflicts
+constexpr int kTokenTile = 8 * kTokenPitch;                     // floats of eight tokens
+__host__ __device__ constexpr int part_floats(int nt) { return nt * kTokenTile + 8; }      // one slice's sums of a row tile
+constexpr int kLag = 2;                                         // a tile is added up while the second one after it is decoded
+constexpr int kBufs = 2 * kLag;                                 // row tiles whose sums are kept, per set of warps
+constexpr int kMaxStages = 24;
+
+// Warps that decode: 12 warps leave each 168 registers.
+constexpr int kMaxSlices = 11;
+__host__ __device__ constexpr int slice_halves(int nt) { return nt == 1 ? 2 : 1; }          // 64 registers of activations
+constexpr int kExtraWarps = 1;
+
+struct SliceParams {
+    const uint8_t *blocks;
+    const __half *x;
+    void *y;
+    unsigned *status;
+    const unsigned *counters;                                   // of the tcgen05 kernel; zero in a workspace that is in order
+    int M, N, chunks;
+    int tiles, clusters;                                        // row tiles, clusters of the grid
+    int split_log, slices, subsets;                             // the grid's clusters have 2^split_log CTAs
+    int stages, pitch;                                          // ring stages, bytes from row to row
+    int x_bufs;                                                 // 4 KiB pieces of activations that a slice has room for at a time
+    uint32_t sums_addr, ring_addr;
+    int y_f32, swiglu;
+    int wide_y;                                                 // four results of a token may be stored at a time
+};
+
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+    return d;
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Bounded, as in the other kernels: after the limit status 3 is set and the thread waits for nothing any more.
+__device__ __noinline__ bool mbar_wait_more(uint32_t bar, uint32_t parity, unsigned *status) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\t"
+                 "mov.u32 n, %3;\n"
+                 "TRY:\n\t"
+                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 4000;\n\t"
+                 "@p bra DONE;\n\t"
+                 "sub.u32 n, n, 1;\n\t"
+                 "setp.ne.u32 q, n, 0;\n\t"
+                 "@q bra TRY;\n"
+                 "DONE:\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity), "n"(kSpinLimit) : "memory");
+    if (!ok) atomicExch(status, 3u);
+    return !ok;
+}
+__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, unsigned *status, bool &dead) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    if (!ok && !dead) dead = mbar_wait_more(bar, parity, status);
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+template <int OFFSET>
+__device__ __forceinline__ uint32_t lds(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(addr), "n"(OFFSET) : "memory");
+    return v;
+}
+__device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                         uint32_t b1, bool first) {
+    if (first)
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+            : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
+    else
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Table entry of code byte v: PRMT selectors that pick FP16 weights out of [s_lo, s_hi, s_hi ^ 0x80] and zeros, one byte a trit.
+//   even byte (its first trit in the lower half of a register): word0 = (t0,t1) | t4 << 16, word1 = (t2,t3)
+//   odd byte: word0 = (t1,t2) | t0 << 16, word1 = (t3,t4)
+// The 13 values past 242 decode to zero weights: a byte that escaped the load-time scan reads inside the table.
+struct CodeTable { uint2 e[512]; };                             // entry of byte v: e[2 v] even, e[2 v + 1] odd
+constexpr CodeTable make_code_table() {
+    CodeTable t{};
+    for (int v = 0; v < 256; ++v) {
+        uint32_t c[5] = {0x44u, 0x44u, 0x44u, 0x44u, 0x44u};
+        int rest = v;
+        for (int d = 0; d < 5 && v < 243; ++d) {
+            c[d] = rest % 3 == 0 ? 0x20u : rest % 3 == 1 ? 0x44u : 0x10u;
+            rest /= 3;
+        }
+        t.e[2 * v].x = c[0] | (c[1] << 8) | (c[4] << 16);
+        t.e[2 * v].y = c[2] | (c[3] << 8);
+        t.e[2 * v + 1].x = c[1] | (c[2] << 8) | (c[0] << 16);
+        t.e[2 * v + 1].y = c[3] | (c[4] << 8);
+    }
+    return t;
+}
+__device__ __align__(16) const CodeTable g_code_table = make_code_table();
+
+// A lane's 64 weights of one row, 32 registers of two, in the order of the columns. Eager: everything the caller's loop
+// unrolls into; `w` holds the block's words (of half 0 words 0..3, of half 1 words 0 and 3..6).
+struct RowDecoder {
+    const uint32_t *w;
+    uint32_t pool, even_entry, odd_entry;
+    __device__ __forceinline__ void lookup(int j, uint32_t &e0, uint32_t &e1) const {        // code byte j
+        const uint32_t addr = prmt(w[(2 + j) >> 2], j & 1 ? odd_entry : even_entry, 0x7604u | (uint32_t)(((2 + j) & 3) << 4));
+        asm("ld.shared.v2.u32 {%0, %1}, [%2+%3];" : "=r"(e0), "=r"(e1) : "r"(addr), "n"(kTableAddr));
+    }
+    __device__ __forceinline__ uint32_t pick(uint32_t sel) const { return prmt(pool, 0u, sel); }
+    // ten weights of code bytes j (even) and j + 1
+    __device__ __forceinline__ void two_bytes(int j, uint32_t *v) const {
+        uint32_t e0, e1, f0, f1;
+        lookup(j, e0, e1);
+        lookup(j + 1, f0, f1);
+        v[0] = pick(e0);
+        v[1] = pick(e1);
+        v[2] = pick(prmt(e0, f0, 0x0062));
+        v[3] = pick(f0);
+        v[4] = pick(f1);
+    }
+};
+
+// The products of one row tile and half a chunk: added to sum[token tile][..] (rows g and g + 8, tokens 2q and 2q + 1).
+// START: these are the first products of sum.
+template <int NT, int HALF, bool START>
+__device__ __forceinline__ void half_slice(const RowDecoder &lo, const RowDecoder &hi, const uint32_t (&b)[NT][32],
+                                           float (&sum)[NT][4]) {
+    uint32_t va[32], vb[32];
+    float d[NT][4];
+    auto multiply = [&](int i) {                                // the MMA of registers 2i and 2i + 1
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            mma16816(d[t], va[2 * i], vb[2 * i], va[2 * i + 1], vb[2 * i + 1], b[t][2 * i], b[t][2 * i + 1], i % kChain == 0);
+            if (i % kChain == kChain - 1) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sum[t][e] = START && i == kChain - 1 ? d[t][e] : sum[t][e] + d[t][e];
+            }
+        }
+    };
+    if (HALF == 0) {
+#pragma unroll
+        for (int a = 0; a < 6; ++a) {
+            lo.two_bytes(2 * a, va + 5 * a);
+            hi.two_bytes(2 * a, vb + 5 * a);
+#pragma unroll
+            for (int i = 0; i < 15; ++i)
+                if (2 * i + 1 >= 5 * a && 2 * i + 1 < 5 * a + 5) multiply(i);
+        }
+        uint32_t e0, e1;                                        // the first four trits of byte 12
+        lo.lookup(12, e0, e1);
+        va[30] = lo.pick(e0);
+        va[31] = lo.pick(e1);
+        hi.lookup(12, e0, e1);
+        vb[30] = hi.pick(e0);
+        vb[31] = hi.pick(e1);
+        multiply(15);
+    } else {
+        auto first = [](const RowDecoder &r, uint32_t *v) {     // the last trit of byte 12, and byte 13
+            uint32_t e0, e1, f0, f1;
+            r.lookup(12, e0, e1);
+            r.lookup(13, f0, f1);
+            v[0] = r.pick(prmt(e0, f0, 0x0062));
+            v[1] = r.pick(f0);
+            v[2] = r.pick(f1);
+        };
+        first(lo, va);
+        first(hi, vb);
+        multiply(0);
+#pragma unroll
+        for (int a = 0; a < 5; ++a) {
+            lo.two_bytes(14 + 2 * a, va + 3 + 5 * a);
+            hi.two_bytes(14 + 2 * a, vb + 3 + 5 * a);
+#pragma unroll
+            for (int i = 1; i < 14; ++i)
+                if (2 * i + 1 >= 3 + 5 * a && 2 * i + 1 < 8 + 5 * a) multiply(i);
+        }
+        auto last = [](const RowDecoder &r, uint32_t *v) {      // byte 24 and the tail byte's three trits
+            uint32_t e0, e1, f0, f1;
+            r.lookup(24, e0, e1);
+            r.lookup(25, f0, f1);
+            v[0] = r.pick(e0);
+            v[1] = r.pick(e1);
+            v[2] = r.pick(prmt(e0, f0, 0x0062));
+            v[3] = r.pick(f0);
+        };
+        last(lo, va + 28);
+        last(hi, vb + 28);
+        multiply(14);
+        multiply(15);
+    }
+}
+
+// Four neighbouring rows from n of token m: results.
+__device__ __forceinline__ void store_rows(const SliceParams &prm, int n, int m, float4 v) {
+    if (m >= prm.M || n >= prm.N) return;
+    if (prm.swiglu) {                                           // (gate, up) row pairs: silu(gate) * up
+        const size_t o = (size_t)m * (prm.N >> 1) + (n >> 1);
+        const float r[2] = {swiglu_f32(v.x, v.y), swiglu_f32(v.z, v.w)};
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            if (n + 2 * e < prm.N && TQ1_IN_BOUNDS(o + e, (size_t)prm.M * (prm.N >> 1), 80u)) {
+                if (prm.y_f32) static_cast<float *>(prm.y)[o + e] = r[e];
+                else static_cast<__half *>(prm.y)[o + e] = __float2half_rn(r[e]);
+            }
+        return;
+    }
+    const size_t o = (size_t)m * prm.N + n;
+    if (!TQ1_IN_BOUNDS(o + min(4, prm.N - n) - 1, (size_t)prm.M * prm.N, 80u)) return;
+    if (prm.wide_y) {
+        if (prm.y_f32) {
+            *reinterpret_cast<float4 *>(static_cast<float *>(prm.y) + o) = v;
+        } else {
+            const __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
+            *reinterpret_cast<uint2 *>(static_cast<__half *>(prm.y) + o) =
+                make_uint2(reinterpret_cast<const uint32_t &>(lo), reinterpret_cast<const uint32_t &>(hi));
+        }
+        return;
+    }
+    const float r[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        if (n + e < prm.N) {
+            if (prm.y_f32) static_cast<float *>(prm.y)[o + e] = r[e];
+            else static_cast<__half *>(prm.y)[o + e] = __float2half_rn(r[e]);
+        }
+}
+
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+// Sum over the four lanes that differ in bits 3 and 4 of their number, in every one of them.
+__device__ __forceinline__ float4 join4(float4 v) {
+#pragma unroll
+    for (int step = 8; step <= 16; step *= 2)
+        v = add4(v, make_float4(__shfl_xor_sync(0xffffffffu, v.x, step), __shfl_xor_sync(0xffffffffu, v.y, step),
+                                __shfl_xor_sync(0xffffffffu, v.z, step), __shfl_xor_sync(0xffffffffu, v.w, step)));
+    return v;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(32 * (kMaxSlices + kExtraWarps), 1)
+slices_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
+              const __grid_constant__ SliceParams prm) {
+    constexpr int kPart = part_floats(NT), HS = slice_halves(NT);
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const uint32_t window = (uint32_t)__cvta_generic_to_shared(smem);
+    const uint32_t base = window - kWindow;                     // zero, or what names this CTA of a cluster
+    if ((base & 0x00ffffffu) != 0u) {                           // the fixed window addresses do not hold
+        if (threadIdx.x == 0) atomicExch(prm.status, 2u);
+        return;
+    }
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int threads = blockDim.x, warps = threads >> 5, workers = warps - kExtraWarps;
+    const int split_log = prm.split_log, split = 1 << split_log, rank = blockIdx.x & (split - 1), cluster = blockIdx.x >> split_log;
+    // this CTA's slices and row tiles
+    const int all = 2 * prm.chunks / HS, slice_lo = all * rank >> split_log, n_slices = (all * (rank + 1) >> split_log) - slice_lo;
+    const int chunk_lo = slice_lo * HS >> 1;
+    const int tile_lo = (int)((long long)cluster * prm.tiles / prm.clusters);
+    const int n_tiles = (int)((long long)(cluster + 1) * prm.tiles / prm.clusters) - tile_lo;
+    const uint32_t stage_bytes = (uint32_t)(kTileRows * prm.pitch);
+    auto full_bar = [&](int s) { return base + kBarAddr + 8u * (uint32_t)s; };
+    auto empty_bar = [&](int s) { return base + kBarAddr + 8u * (uint32_t)(kMaxStages + s); };
+    auto sum_bar = [&](int s) { return base + kBarAddr + 8u * (uint32_t)(2 * kMaxStages + s); };
+    auto x_bar = [&](int s) { return base + kBarAddr + 8u * (uint32_t)(2 * kMaxStages + kBufs * prm.subsets + s); };
+
+    // ---- set-up that depends on no earlier kernel ---------------------------------------------------------------
+    if (tid == 0) {
+        for (int s = 0; s < prm.stages; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), (uint32_t)n_slices);
+        }
+        for (int s = 0; s < kBufs * prm.subsets; ++s) {
+            mbar_init(sum_bar(s), (uint32_t)n_slices);
+        }
+        for (int s = 0; s < n_slices; ++s) mbar_init(x_bar(s), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    const int word_x = chunk_lo * (kChunkBytes / 8);            // the map's elements are 8 bytes
+    if (tid == 32) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&wmap) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");
+    }
+    if (warp == workers && elect_one())                         // the first tiles: into L2 (a hint, whatever they hold by now)
+        for (int i = 0; i < min(prm.stages, n_tiles); ++i)
+            asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];"
+                         ::"l"(&wmap), "r"(word_x), "r"((tile_lo + i) * kTileRows) : "memory");
+    // Sixteen copies of every entry, two entries of both forms (512 bytes) per warp and step, several loads in flight.
+    constexpr int kSteps = 128, kFlight = 8;
+    for (int j0 = warp; j0 < kSteps; j0 += kFlight * warps) {
+        uint2 e[kFlight];
+#pragma unroll
+        for (int j = 0; j < kFlight; ++j)
+            if (j0 + j * warps < kSteps) e[j] = __ldg(&g_code_table.e[4 * (j0 + j * warps) + (lane >> 3)]);
+#pragma unroll
+        for (int j = 0; j < kFlight; ++j)
+            if (j0 + j * warps < kSteps)
+                *reinterpret_cast<uint4 *>(smem + (kTableAddr - kWindow) + (j0 + j * warps) * 512 + lane * 16) =
+                    make_uint4(e[j].x, e[j].y, e[j].x, e[j].y);
+    }
+    if (split > 1) {                                            // the CTAs of a cluster write into each other's memory
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else {
+        __syncthreads();
+    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    bool dead = false;
+    if (tid == 0 && blockIdx.x == 0 && *prm.counters != 0u) atomicExch(prm.status, 8u);      // a stale workspace
+    if (warp == workers) {
+        // ------------------------------------------------------------------ fetch
+        if (elect_one()) {
+            int stage = 0;
+            uint32_t phase = 1;
+            for (int i = 0; i < n_tiles; ++i) {
+                mbar_wait(empty_bar(stage), phase, prm.status, dead);
+                if (dead) break;
+                mbar_expect_tx(full_bar(stage), stage_bytes);
+                asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                             ::"r"(base + prm.ring_addr + (uint32_t)stage * stage_bytes), "l"(&wmap), "r"(word_x),
+                               "r"((tile_lo + i) * kTileRows), "r"(full_bar(stage)) : "memory");
+                if (++stage == prm.stages) { stage = 0; phase ^= 1u; }
+            }
+        }
+        __syncwarp();
+    } else {
+        // ------------------------------------------------------------------ decode and multiply
+        const int subset = warp / prm.slices, slice = warp - subset * prm.slices, g = lane >> 2, q = lane & 3;
+        const int half0 = (slice_lo + slice) * HS, chunk = half0 >> 1;
+        // This lane's 64 columns of tokens 8t + g: TMA brings the warp's 32 pieces of 128 bytes (16-byte loads from global
+        // memory touch 32 lines each, which took the warps of a CTA 2.7 us).
+        uint32_t b[HS][NT][32];
+        const uint32_t x_addr = base + kDataAddr + (uint32_t)(slice * prm.x_bufs) * kXBytes;
+        if (slice < n_slices) {
+#pragma unroll
+            for (int j = 0; j < HS * NT; ++j) {                 // a half of eight tokens each
+                if (j % prm.x_bufs == 0) {                      // the next x_bufs of them; one set of warps asks for all
+                    if (warp == slice && elect_one()) {
+                        mbar_expect_tx(x_bar(slice), (uint32_t)prm.x_bufs * kXBytes);
+                        for (int u = j; u < j + prm.x_bufs; ++u)
+                            asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes "
+                                         "[%0], [%1, {%2, %3, %4, %5}], [%6];"
+                                         ::"r"(x_addr + (uint32_t)(u - j) * kXBytes), "l"(&xmap), "r"(0),
+                                           "r"(HS == 2 ? u : half0 & 1), "r"(4 * chunk), "r"(HS == 2 ? 0 : 8 * u),
+                                           "r"(x_bar(slice)) : "memory");
+                    }
+                    __syncwarp();
+                    mbar_wait(x_bar(slice), (uint32_t)(j / prm.x_bufs) & 1u, prm.status, dead);
+                }
+                const uint32_t src = x_addr + (uint32_t)(j % prm.x_bufs) * kXBytes + (uint32_t)lane * 128u;
+                uint32_t (&to)[32] = b[HS == 2 ? j : 0][HS == 2 ? 0 : j];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(to[4 * i]), "=r"(to[4 * i + 1]), "=r"(to[4 * i + 2]), "=r"(to[4 * i + 3])
+                                 : "r"(src + (uint32_t)((i ^ (lane & 7)) << 4)) : "memory");
+                __syncwarp();
+            }
+        }
+        asm volatile("bar.sync 1, %0;" ::"r"(workers * 32) : "memory");      // the partial sums take the activations' place
+        if (slice < n_slices) {
+            const uint32_t even_entry = base | ((uint32_t)(lane & 15) * 8u), odd_entry = even_entry | 128u;
+            const uint32_t lane_src = base + prm.ring_addr + (uint32_t)(g * prm.pitch + (chunk - chunk_lo) * kChunkBytes + q * kBlockBytes);
+            float *parts = reinterpret_cast<float *>(smem + (kDataAddr - kWindow)) + subset * (kBufs * prm.slices * kPart);
+            float *lane_dst = parts + slice * kPart + 2 * q * kTokenPitch + g;
+            const uint32_t row8 = 8u * (uint32_t)prm.pitch, own_sum_bar = sum_bar(kBufs * subset);
+            // Adding the slices of the set's k-th row tile is 4 NT passes, number 4 NT k + p: tokens 8 (p / 4) + p % 4 and the
+            // fourth after it, a lane four rows of every fourth slice (the loads of eight lanes fall into different banks). A
+            // fixed order of additions. The set's warps take turns with the passes.
+            constexpr int kPasses = 4 * NT, kMine = (kMaxSlices + 3) / 4;
+            const float *pass_src = parts + (lane >> 3) * kPart + (lane & 4) * kTokenPitch + (lane & 3) * 4;
+            int pass = slice;
+            auto add_passes = [&](int end) {
+                for (; pass < end; pass += n_slices) {
+                    const int k = pass / kPasses, p = pass % kPasses, token = 8 * (p >> 2) + (p & 3);
+                    const float *src = pass_src + k % kBufs * (prm.slices * kPart) + token * kTokenPitch;
+                    float4 total = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+                    for (int s = 0; s < kMine; ++s)
+                        if (4 * s + (lane >> 3) < n_slices) total = add4(total, *reinterpret_cast<const float4 *>(src + 4 * s * kPart));
+                    __syncwarp();
+                    total = join4(total);
+                    if (lane < 8) {
+                        const int i = subset + k * prm.subsets, m = token + (lane & 4), row = (lane & 3) * 4;
+                        if (split_log == 0) {
+                            store_rows(prm, (tile_lo + i) * kTileRows + row, m, total);
+                        } else {                                // to CTA i % split of the cluster, which adds the CTAs' sums
+                            const int slot = (i >> split_log << split_log) + rank;
+                            uint32_t dst;
+                            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst)
+                                         : "r"(base + prm.sums_addr + 4u * (uint32_t)(slot * kPart + m * kTokenPitch + row)), "r"(i & (split - 1)));
+                            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
+                                         ::"r"(dst), "f"(total.x), "f"(total.y), "f"(total.z), "f"(total.w) : "memory");
+                        }
+                    }
+                    __syncwarp();
+                }
+            };
+            auto run = [&](auto half_tag) {
+                constexpr int HALF = decltype(half_tag)::value;
+                int stage = subset, k = 0;
+                uint32_t phase = 0;
+                for (int i = subset; i < n_tiles; i += prm.subsets, ++k) {
+                    uint32_t w_lo[7], w_hi[7];                  // this lane's words of both rows
+                    mbar_wait(full_bar(stage), phase, prm.status, dead);
+                    const uint32_t src = lane_src + (uint32_t)stage * stage_bytes;
+                    auto words = [&](uint32_t (&w)[7], uint32_t at) {
+                        w[0] = lds<0>(at);
+                        if (HS == 2 || HALF == 0) { w[1] = lds<4>(at); w[2] = lds<8>(at); }
+                        w[3] = lds<12>(at);
+                        if (HS == 2 || HALF == 1) { w[4] = lds<16>(at); w[5] = lds<20>(at); w[6] = lds<24>(at); }
+                    };
+                    words(w_lo, src);
+                    words(w_hi, src + row8);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(empty_bar(stage));
+                    stage += prm.subsets;
+                    if (stage >= prm.stages) { stage -= prm.stages; phase ^= 1u; }
+                    auto pool = [](uint32_t w) { return prmt(w, w ^ 0x8000u, 0x0510u); };       // [s_lo, s_hi, s_hi ^ 0x80]
+                    float sum[NT][4];
+                    {
+                        const RowDecoder lo{w_lo, pool(w_lo[0]), even_entry, odd_entry}, hi{w_hi, pool(w_hi[0]), even_entry, odd_entry};
+                        half_slice<NT, HALF, true>(lo, hi, b[0], sum);
+                        if (HS == 2) half_slice<NT, 1, false>(lo, hi, b[HS - 1], sum);
+                    }
+                    // The set's tile kLag before this one is complete by now, or soon will be. That every warp has stored its
+                    // sums of that tile also says that all passes of the one kLag before it are over, whose buffer this tile
+                    // takes.
+                    if (k >= kLag) {
+                        mbar_wait(own_sum_bar + 8u * (uint32_t)((k - kLag) % kBufs), (uint32_t)((k - kLag) / kBufs) & 1u, prm.status, dead);
+                        add_passes((k - kLag + 1) * kPasses);
+                    }
+                    float *dst = lane_dst + k % kBufs * (prm.slices * kPart);
+#pragma unroll
+                    for (int t = 0; t < NT; ++t) {
+                        float *f = dst + t * kTokenTile;
+                        f[0] = sum[t][0];
+                        f[kTokenPitch] = sum[t][1];
+                        f[8] = sum[t][2];
+                        f[kTokenPitch + 8] = sum[t][3];
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(own_sum_bar + 8u * (uint32_t)(k % kBufs));
+                }
+                for (int j = k < kLag ? 0 : k - kLag; j < k; ++j) {
+                    mbar_wait(own_sum_bar + 8u * (uint32_t)(j % kBufs), (uint32_t)(j / kBufs) & 1u, prm.status, dead);
+                    add_passes((j + 1) * kPasses);
+                }
+            };
+            if (HS == 1 && (half0 & 1)) run(std::integral_constant<int, 1>{});
+            else run(std::integral_constant<int, 0>{});
+        }
+    }
+    if (dead)                                                   // a wait ran out: give the copies still in flight time to land
+        for (int i = 0; i < 64; ++i) __nanosleep(20000);
+    if (split > 1) {
+        // CTA r of the cluster has the CTAs' sums of every split-th tile; it adds them in the order of the columns
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const float *sums = reinterpret_cast<const float *>(smem + (prm.sums_addr - kWindow));
+        for (int j = warp; rank + (j / (4 * NT) << split_log) < n_tiles; j += warps) {
+            const int own = j / (4 * NT), p = j % (4 * NT), m = 8 * (p >> 2) + (p & 3) + (lane & 4), row = (lane & 3) * 4;
+            float4 total = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for (int c = lane >> 3; c < split; c += 4)
+                total = add4(total, *reinterpret_cast<const float4 *>(sums + ((own << split_log) + c) * kPart + m * kTokenPitch + row));
+            __syncwarp();
+            total = join4(total);
+            if (lane < 8) store_rows(prm, (tile_lo + rank + (own << split_log)) * kTileRows + row, m, total);
+        }
+    }
+}
+
+// ---- host ---------------------------------------------------------------------------------------------------------
+struct SlicePlan {
+    bool ok;
+    float us;
+    int split, slices, subsets, clusters, stages, pitch;
+    int x_bufs;
+    uint32_t sums_addr, ring_addr, end;
+};
+
+int device_slot() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+    return dev;
+}
+int sm_count() {
+    static int count[kMaxDevices] = {};
+    const int dev = device_slot();
+    if (!count[dev]) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        count[dev] = n;
+    }
+    return count[dev];
+}
+
+// Clusters of `split` CTAs that run at the same time: fewer than SMs / split where the SMs of a GPC are no multiple of it.
+template <int NT>
+int clusters_at_once(int split) {
+    static int known[kMaxDevices][9] = {};
+    const int dev = device_slot();
+    if (split == 1) return sm_count();
+    if (!known[dev][split]) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(sm_count() / split * split));
+        cfg.blockDim = dim3(32 * (kMaxSlices + kExtraWarps));
+        cfg.dynamicSmemBytes = kWindowEnd - kWindow;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = (unsigned)split;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaFuncSetAttribute(slices_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kWindowEnd - kWindow)) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, slices_kernel<NT>, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();                                 // no device, say: planning only
+            n = sm_count() / split;
+        }
+        known[dev][split] = n;
+    }
+    return known[dev][split];
+}
+
+// The K split with the smallest modelled time (us, fitted to graph replays with weights out of HBM): what the SM works through
+// (0.128 per row tile and chunk of eight tokens, twice that for sixteen), or where there are few warps what one of them does
+// one tile after the other, behind launch, table and activations; a cluster's barriers and its exchange on top.
+SlicePlan slice_plan(int nt, int N, int K) {
+    SlicePlan best = {};
+    const int per = slice_halves(nt), halves = K / 256 / per, tiles = (N + kTileRows - 1) / kTileRows;
+    for (int split = 1; split <= 8; split *= 2) {
+        SlicePlan p = {};
+        p.split = split;
+        p.slices = (halves + split - 1) / split;
+        if (halves < split || p.slices > kMaxSlices) continue;
+        const int room = nt == 1 ? clusters_at_once<1>(split) : clusters_at_once<2>(split);
+        p.clusters = tiles < room ? tiles : room;
+        const int per_cluster = (tiles + p.clusters - 1) / p.clusters;
+        p.subsets = kMaxSlices / p.slices;
+        if (p.subsets > per_cluster) p.subsets = per_cluster;
+        // a CTA's slices may begin and end inside a chunk
+        const int most = per == 2 ? p.slices : (p.slices + 2) / 2, chunks = most < K / 512 ? most : K / 512;
+        p.pitch = chunks * kChunkBytes;
+        if (p.pitch / 16 % 2 == 0) p.pitch += 16;
+        p.x_bufs = p.subsets == 1 && nt == 2 ? 1 : 2;           // sets of warps share a slice's activations: all at once
+        const auto aligned = [](int bytes) { return (uint32_t)(bytes + 127) / 128 * 128; };
+        const uint32_t x_room = (uint32_t)(p.slices * p.x_bufs) * kXBytes;
+        const uint32_t part_room = aligned(kBufs * p.subsets * p.slices * part_floats(nt) * 4);
+        p.sums_addr = kDataAddr + (x_room > part_room ? x_room : part_room);
+        p.ring_addr = p.sums_addr + (split > 1 ? aligned((per_cluster + split - 1) / split * split * part_floats(nt) * 4) : 0u);
+        const uint32_t stage_bytes = (uint32_t)(kTileRows * p.pitch);
+        p.stages = p.ring_addr < kWindowEnd ? (int)((kWindowEnd - p.ring_addr) / stage_bytes) : 0;
+        if (p.stages > kMaxStages) p.stages = kMaxStages;
+        if (p.stages > per_cluster) p.stages = per_cluster;
+        if (p.stages < (per_cluster < 2 * p.subsets ? per_cluster : p.subsets + 1)) continue;      // no room to fetch ahead
+        p.end = p.ring_addr + (uint32_t)p.stages * stage_bytes;
+        p.ok = true;
+        const float sm = 0.128f * per_cluster * p.slices, chain = 0.7f * ((per_cluster + p.subsets - 1) / p.subsets);
+        p.us = (split > 1 ? 5.2f : 3.6f) + (sm > chain ? sm : chain);
+        if (!best.ok || p.us < best.us) best = p;
+    }
+    return best;
+}
+
+template <int NT>
+int launch_slices(const CUtensorMap &wmap, const CUtensorMap &xmap, const SliceParams &prm, const SlicePlan &p, cudaStream_t stream) {
+    auto kern = slices_kernel<NT>;
+    static bool attr_set[kMaxDevices] = {};
+    const int dev = device_slot();
+    if (!attr_set[dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kWindowEnd - kWindow));
+        if (e != cudaSuccess) return cuda_fail(e, "tq1_linear_f16: shared memory opt-in (slices)");
+        attr_set[dev] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(p.clusters * p.split));
+    cfg.blockDim = dim3((unsigned)(32 * (p.slices * p.subsets + kExtraWarps)));
+    cfg.dynamicSmemBytes = p.end - kWindow;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)p.split;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = p.split > 1 ? 2 : 1;
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, kern, wmap, xmap, prm);
+    return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: launch (slices)");
+}
+
+}  // namespace
+
+bool gemm_slices_preferred(int M, int N, int K) {
+    if (M < 3 || M > 16 || K % 512 || gemm_tc_forced()) return false;
+    const SlicePlan p = slice_plan(M <= 8 ? 1 : 2, N, K);
+    return p.ok && p.us < gemm_tc_model_us(M, N, K);
+}
+
+int launch_gemm_slices(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, void *workspace,
+                       cudaStream_t stream, bool swiglu) {
+    const int nt = M <= 8 ? 1 : 2;
+    const SlicePlan p = slice_plan(nt, N, K);
+    if (!p.ok) return fail(TQ1_ERR_INVALID, "tq1_linear_f16: %dx%dx%d does not fit the slice kernel", M, N, K);
+    unsigned char *ws = static_cast<unsigned char *>(workspace);
+    SliceParams prm;
+    prm.blocks = blocks;
+    prm.x = x;
+    prm.y = y;
+    prm.status = reinterpret_cast<unsigned *>(ws);
+    prm.counters = reinterpret_cast<const unsigned *>(ws + kWsCounterOffset);
+    prm.M = M;
+    prm.N = N;
+    prm.chunks = K / 512;
+    prm.tiles = (N + kTileRows - 1) / kTileRows;
+    prm.clusters = p.clusters;
+    prm.split_log = p.split == 1 ? 0 : p.split == 2 ? 1 : p.split == 4 ? 2 : 3;
+    prm.slices = p.slices;
+    prm.subsets = p.subsets;
+    prm.stages = p.stages;
+    prm.pitch = p.pitch;
+    prm.x_bufs = p.x_bufs;
+    prm.sums_addr = p.sums_addr;
+    prm.ring_addr = p.ring_addr;
+    prm.y_f32 = y_f32 ? 1 : 0;
+    prm.swiglu = swiglu ? 1 : 0;
+    prm.wide_y = N % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & (y_f32 ? 15 : 7)) == 0 ? 1 : 0;
+    // A row as 8-byte elements; a box is the 16 rows of a tile and a CTA's K range, at most 16 bytes more (another CTA's, or
+    // filled in past the row's end), so that rows lie an odd number of 16-byte units apart.
+    // Activations as [M][K / 128][2][64]: a box is one half of the four groups of a chunk for eight tokens.
+    const EncodeTiledFn encode = encode_tiled_fn();
+    if (!encode) return fail(TQ1_ERR_CUDA, "tq1_linear_f16: cuTensorMapEncodeTiled is unavailable");
+    CUtensorMap wmap, xmap;
+    const cuuint64_t row_bytes = (cuuint64_t)prm.chunks * kChunkBytes;
+    const cuuint64_t w_dims[2] = {row_bytes / 8, (cuuint64_t)N}, w_strides[1] = {row_bytes};
+    const cuuint32_t w_box[2] = {(cuuint32_t)p.pitch / 8, kTileRows}, ones[4] = {1, 1, 1, 1};
+    CUresult res = encode(&wmap, CU_TENSOR_MAP_DATA_TYPE_INT64, 2, const_cast<uint8_t *>(blocks), w_dims, w_strides, w_box, ones,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (res != CUDA_SUCCESS) return fail(TQ1_ERR_CUDA, "tq1_linear_f16: weight tensor map failed (%d)", (int)res);
+    const cuuint64_t x_dims[4] = {64, 2, (cuuint64_t)K / kGroup, (cuuint64_t)M};
+    const cuuint64_t x_strides[3] = {128, 256, (cuuint64_t)K * sizeof(__half)};
+    const cuuint32_t x_box[4] = {64, 1, 4, 8};
+    res = encode(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<__half *>(x), x_dims, x_strides, x_box, ones,
+                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (res != CUDA_SUCCESS) return fail(TQ1_ERR_CUDA, "tq1_linear_f16: activation tensor map failed (%d)", (int)res);
+    return nt == 1 ? launch_slices<1>(wmap, xmap, prm, p, stream) : launch_slices<2>(wmap, xmap, prm, p, stream);
+}
+
+}  // namespace tq1

@@ -961,23 +961,6 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
     }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// Looked up once; a thread that comes while another one is looking waits for it.
-EncodeTiledFn encode_fn() {
-    static const EncodeTiledFn fn = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) != cudaSuccess ||
-            qres != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<EncodeTiledFn>(p);
-    }();
-    return fn;
-}
-
 // Per-device launch state: the shared-memory opt-in is an attribute of the function on ONE device.
 constexpr int kMaxDevices = 64;
 struct DeviceState {
@@ -1047,7 +1030,7 @@ int rows_per_link(int N, int K, size_t region_slots) {
 }
 
 int encode_link_map(CUtensorMap *map, const uint8_t *blocks, int N, int K) {
-    EncodeTiledFn encode = encode_fn();
+    EncodeTiledFn encode = encode_tiled_fn();
     if (!encode) return fail(TQ1_ERR_CUDA, "tq1 chain: cuTensorMapEncodeTiled is unavailable");
     const cuuint64_t row_bytes = (cuuint64_t)(K / kGroup) * kBlockBytes;
     const cuuint64_t dims[2] = {row_bytes, (cuuint64_t)N};

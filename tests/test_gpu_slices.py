@@ -1,0 +1,71 @@
+"""Three to sixteen activation rows (the slice kernel's and, beyond its sizes, the tcgen05 kernel's) against the oracle."""
+
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import tq1_oracle as o
+from tests.gpu_util import random_blocks, run_linear, to_dev
+
+pytestmark = pytest.mark.gpu
+
+# Relative error (2-norm): an accumulator of 64 columns truncates four times, on average half of an ulp of 0.72 * 2^-23 of a
+# value that grows from zero (1.92 * 2^-24 in all), and up to eight FP32 additions in a row, twice (a slice's accumulators,
+# the slices), round by 0.58 * 2^-24 of a sum that grows from zero: 2 * 0.58 * sqrt(8 / 2) * 2^-24.
+BOUND = (1.92 + 2 * 0.58 * 2.0) * 2.0 ** -24
+
+
+@pytest.mark.parametrize("batch", (3, 8, 9, 16))
+@pytest.mark.parametrize(("rows", "columns"), (
+    (1, 512), (15, 1024), (16, 512), (17, 1536),        # a tile and its edges, one to three slices, eleven sets of warps
+    (100, 2560), (4099, 1024), (2400, 5632),            # sets of warps that take turns, eleven slices, rows off the 4-row grid
+    (2369, 5120),                                       # a CTA's second tile, the last one of one row
+    (48, 6144), (264, 17408), (640, 8704)))             # two and more CTAs in a cluster, K parts that begin inside a chunk
+def test_slices_against_float64(rows, columns, batch):
+    blocks, rng = random_blocks(rows, columns, seed=rows + columns + batch)
+    x = rng.standard_normal((batch, columns)).astype(np.float16)
+    want = o.float64_matmul(blocks, x, rows=rows, columns=columns)
+    got = run_linear(blocks, x)
+    assert np.linalg.norm(got - want) <= BOUND * np.linalg.norm(want)
+    assert np.array_equal(run_linear(blocks, x), got)
+    half = run_linear(blocks, x, out_dtype=torch.float16)
+    assert np.array_equal(half, got.astype(np.float16).astype(np.float32))
+
+
+@pytest.mark.parametrize("batch", (3, 16))
+@pytest.mark.parametrize("offset", (1, 2, 4))
+def test_results_off_the_wide_grid(batch, offset):
+    """Results that do not begin on an 8- or 16-byte boundary are stored one by one; the elements around them stay."""
+    from ternel_b200 import _native
+    from ternel_b200.ops import _workspace
+    rows, columns = 100, 1024
+    blocks, rng = random_blocks(rows, columns, seed=offset)
+    x = rng.standard_normal((batch, columns)).astype(np.float16)
+    bd, xd = to_dev(blocks), to_dev(x)
+    lib = _native.lib()
+    need = lib.tq1_linear_workspace_bytes(batch, rows, columns)
+    ws = _workspace(xd.device, need)
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for dtype in (torch.float16, torch.float32):
+        y = torch.full((batch * rows + 2 * offset,), 7.0, dtype=dtype, device="cuda")
+        assert lib.tq1_linear_f16(bd.data_ptr(), xd.data_ptr(), y[offset:].data_ptr(), int(dtype == torch.float32), batch, rows,
+                                  columns, ws.data_ptr(), need, stream) == 0
+        got = y[offset:-offset].float().cpu().numpy().reshape(batch, rows)
+        assert np.array_equal(got, run_linear(blocks, x, out_dtype=dtype))
+        assert bool((y[:offset] == 7).all()) and bool((y[-offset:] == 7).all())
+
+
+@pytest.mark.parametrize("batch", (3, 8, 16))
+@pytest.mark.parametrize(("half_rows", "columns"), ((9, 512), (1001, 5120), (40, 17408)))
+def test_gated_activation(half_rows, columns, batch):
+    """silu(gate) * up of row pairs equals the activation applied to the plain products, which add in the same order."""
+    from ternel_b200.ops import tq1_matmul, tq1_swiglu
+    blocks, rng = random_blocks(2 * half_rows, columns, seed=half_rows)
+    both, x = to_dev(blocks), to_dev(rng.standard_normal((batch, columns)).astype(np.float16))
+    plain = tq1_matmul(both, x, out_dtype=torch.float32).double()
+    want = torch.nn.functional.silu(plain[:, 0::2]) * plain[:, 1::2]
+    got = tq1_swiglu(both, x, out_dtype=torch.float32)
+    # expf, a division and two products in FP32: a few units in the last place of each value
+    assert bool(((got - want).abs() <= 2e-6 * want.abs()).all())
