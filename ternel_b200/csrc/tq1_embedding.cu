@@ -47,7 +47,7 @@ constexpr int kTokensPerThread = 4;
 // barrier behind the copy costs more than lookups through L1 (launch_embedding has the line and the figures).
 template <bool OUT_F32, bool SHARED>
 __global__ void __launch_bounds__(kThreadsPerBlockRow * kBlocksPerCta)
-embedding_kernel(const uint8_t *__restrict__ blocks, const int64_t *__restrict__ ids, void *__restrict__ out,
+embedding_kernel(const uint8_t *blocks, const int64_t *ids, void *out,
                  int64_t T, int64_t V, int gpr) {
     const int j = threadIdx.x & (kThreadsPerBlockRow - 1);      // which eight outputs of the block
     const int g = blockIdx.x * kBlocksPerCta + (threadIdx.x >> 4);
@@ -63,13 +63,14 @@ embedding_kernel(const uint8_t *__restrict__ blocks, const int64_t *__restrict__
     // that follows it for one token only keeps too few bytes in flight to fill the memory system.
     int64_t id[kTokensPerThread];
     bool live[kTokensPerThread];
-#pragma unroll
-    for (int q = 0; q < kTokensPerThread; ++q) id[q] = in_row && t0 + q < T ? ids[t0 + q] : -1;
     if (SHARED) {
 #pragma unroll
         for (int i = 0; i < 256; i += kThreadsPerBlockRow * kBlocksPerCta)
             shared_trits[i + threadIdx.x] = g_trits.e[i + threadIdx.x];
     }
+    grid_dependency_wait();
+#pragma unroll
+    for (int q = 0; q < kTokensPerThread; ++q) id[q] = in_row && t0 + q < T ? ids[t0 + q] : -1;
     const uint8_t *blk[kTokensPerThread];
     uint32_t sbits[kTokensPerThread], b0[kTokensPerThread], b1[kTokensPerThread], b2[kTokensPerThread];
 #pragma unroll
@@ -77,9 +78,9 @@ embedding_kernel(const uint8_t *__restrict__ blocks, const int64_t *__restrict__
         live[q] = id[q] >= 0 && id[q] < V;
         blk[q] = blocks + (size_t)((unsigned)(live[q] ? id[q] : 0) * (unsigned)gpr + (unsigned)(in_row ? g : 0)) * kBlockBytes;
         sbits[q] = *reinterpret_cast<const unsigned short *>(blk[q]);
-        b0[q] = __ldg(blk[q] + 2 + a);
-        b1[q] = __ldg(blk[q] + 3 + a);
-        b2[q] = off >= 3 ? __ldg(blk[q] + 4 + a) : 0u;          // the third byte exists whenever it is needed
+        b0[q] = blk[q][2 + a];
+        b1[q] = blk[q][3 + a];
+        b2[q] = off >= 3 ? blk[q][4 + a] : 0u;          // the third byte exists whenever it is needed
     }
     if (SHARED) __syncthreads();
     if (!in_row) return;
@@ -145,8 +146,8 @@ int launch_embedding(const uint8_t *blocks, const int64_t *ids, void *out, bool 
                               : static_cast<void *>(static_cast<__half *>(out) + t0 * K);
         auto kernel = out_f32 ? (shared ? embedding_kernel<true, true> : embedding_kernel<true, false>)
                               : (shared ? embedding_kernel<false, true> : embedding_kernel<false, false>);
-        kernel<<<grid, kThreadsPerBlockRow * kBlocksPerCta, 0, stream>>>(blocks, ids + t0, first, n, V, gpr);
-        cudaError_t err = cudaGetLastError();
+        const cudaError_t err = launch_dependent(kernel, grid, kThreadsPerBlockRow * kBlocksPerCta, 0, stream, blocks, ids + t0,
+                                                 first, n, V, gpr);
         if (err != cudaSuccess) return cuda_fail(err, "tq1_embedding_f16: launch");
     }
     return TQ1_OK;

@@ -84,7 +84,7 @@ constexpr int kFewWarps = 8, kFewRows = 16;
 
 template <int NT>
 __global__ void __launch_bounds__(kFewWarps * 32)
-groups_few_kernel(const uint8_t *__restrict__ blocks, const __half *__restrict__ x, void *__restrict__ y, int y_f32,
+groups_few_kernel(const uint8_t *blocks, const __half *x, void *y, int y_f32,
                   int M, int N, int groups) {
     __shared__ uint32_t table[256];
     __shared__ uint32_t packed[kFewWarps][kFewRows * kGroupRowWords];
@@ -117,8 +117,9 @@ groups_few_kernel(const uint8_t *__restrict__ blocks, const __half *__restrict__
     uint32_t next[kPerLane];
     auto load = [&](int grp) {
 #pragma unroll
-        for (int j = 0; j < kPerLane; ++j) next[j] = grp < groups ? __ldg(src[j] + (size_t)grp * kGroupRowWords) : 0u;
+        for (int j = 0; j < kPerLane; ++j) next[j] = grp < groups ? src[j][(size_t)grp * kGroupRowWords] : 0u;
     };
+    grid_dependency_wait();
     load(warp);
     __syncthreads();
     uint32_t *mine = packed[warp];
@@ -140,7 +141,7 @@ groups_few_kernel(const uint8_t *__restrict__ blocks, const __half *__restrict__
         for (int s = 0; s < 4; ++s)
 #pragma unroll
             for (int t = 0; t < NT; ++t)
-                xv[s][t] = live[t] ? __ldg(reinterpret_cast<const uint4 *>(xrow[t] + (size_t)grp * kGroup + 32 * s))
+                xv[s][t] = live[t] ? *reinterpret_cast<const uint4 *>(xrow[t] + (size_t)grp * kGroup + 32 * s)
                                    : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
@@ -191,7 +192,7 @@ constexpr size_t many_smem(int nt) {
 
 template <int NT>
 __global__ void __launch_bounds__(kManyWarps * 32, NT == 8 ? 1 : 2)
-groups_many_kernel(const uint8_t *__restrict__ blocks, const __half *__restrict__ x, void *__restrict__ y, int y_f32,
+groups_many_kernel(const uint8_t *blocks, const __half *x, void *y, int y_f32,
                    int M, int N, int groups) {
     constexpr int kTokens = 8 * NT, kStageBytes = kTokens * kGroup * 2, kThreads = kManyWarps * 32;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -228,8 +229,9 @@ groups_many_kernel(const uint8_t *__restrict__ blocks, const __half *__restrict_
     uint32_t next[kPerLane];
     auto load = [&](int grp) {
 #pragma unroll
-        for (int j = 0; j < kPerLane; ++j) next[j] = grp < groups ? __ldg(src[j] + (size_t)grp * kGroupRowWords) : 0u;
+        for (int j = 0; j < kPerLane; ++j) next[j] = grp < groups ? src[j][(size_t)grp * kGroupRowWords] : 0u;
     };
+    grid_dependency_wait();
     load(0);
     request(0);
     request(1);
@@ -304,8 +306,8 @@ groups_many_kernel(const uint8_t *__restrict__ blocks, const __half *__restrict_
 template <int NT>
 int launch_few(const uint8_t *blocks, const __half *x, void *y, int y_f32, int M, int N, int groups, cudaStream_t stream) {
     const long long ctas = (long long)((N + kFewRows - 1) / kFewRows) * ((M + 8 * NT - 1) / (8 * NT));
-    groups_few_kernel<NT><<<(unsigned)ctas, kFewWarps * 32, 0, stream>>>(blocks, x, y, y_f32, M, N, groups);
-    const cudaError_t err = cudaGetLastError();
+    const cudaError_t err = launch_dependent(groups_few_kernel<NT>, dim3((unsigned)ctas), kFewWarps * 32, 0, stream, blocks, x, y,
+                                             y_f32, M, N, groups);
     return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: launch");
 }
 
@@ -315,8 +317,8 @@ int launch_many(const uint8_t *blocks, const __half *x, void *y, int y_f32, int 
     cudaError_t err = cudaFuncSetAttribute(groups_many_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)many_smem(NT));
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: shared memory opt-in");
-    groups_many_kernel<NT><<<(unsigned)ctas, kManyWarps * 32, many_smem(NT), stream>>>(blocks, x, y, y_f32, M, N, groups);
-    err = cudaGetLastError();
+    err = launch_dependent(groups_many_kernel<NT>, dim3((unsigned)ctas), kManyWarps * 32, many_smem(NT), stream, blocks, x, y, y_f32,
+                           M, N, groups);
     return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: launch");
 }
 

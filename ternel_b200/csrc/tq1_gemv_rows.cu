@@ -30,15 +30,13 @@ __device__ __forceinline__ float dot_byte(uint32_t entry, const float *x, int n,
 }
 
 template <int MB, bool OUT_F32>
-__global__ void __launch_bounds__(kRowsThreads) gemv_rows_kernel(const uint8_t *__restrict__ blocks,
-                                                                 const __half *__restrict__ x,
-                                                                 void *__restrict__ y,
-                                                                 int N, int K, int ldy) {
+__global__ void __launch_bounds__(kRowsThreads) gemv_rows_kernel(const uint8_t *blocks, const __half *x, void *y, int N, int K, int ldy) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint16_t *lut = reinterpret_cast<uint16_t *>(smem_raw);          // 256 entries
     float *xs = reinterpret_cast<float *>(smem_raw + 512);           // [MB][K]
 
     for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = (uint16_t)trits_2bit(i);
+    grid_dependency_wait();
     for (int i = threadIdx.x; i < MB * K; i += blockDim.x) xs[i] = __half2float(x[i]);
     __syncthreads();
 
@@ -58,7 +56,7 @@ __global__ void __launch_bounds__(kRowsThreads) gemv_rows_kernel(const uint8_t *
         for (int g0 = 0; g0 < gpr; g0 += 4) {
             const int g = g0 + sub;
             const bool live = g < gpr && pos < kBlockWords;
-            const uint32_t w = live ? __ldg(words + g * kBlockWords + pos) : 0u;
+            const uint32_t w = live ? words[g * kBlockWords + pos] : 0u;
             float sum[MB];
 #pragma unroll
             for (int m = 0; m < MB; ++m) sum[m] = 0.0f;
@@ -116,9 +114,7 @@ static int launch_mb(const uint8_t *blocks, const __half *x, void *y, bool y_f32
     cudaError_t err = cudaFuncSetAttribute(y_f32 ? kern_f : kern_h,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: shared memory opt-in");
-    if (y_f32) kern_f<<<ctas, kRowsThreads, smem, stream>>>(blocks, x, y, N, K, N);
-    else kern_h<<<ctas, kRowsThreads, smem, stream>>>(blocks, x, y, N, K, N);
-    err = cudaGetLastError();
+    err = launch_dependent(y_f32 ? kern_f : kern_h, dim3((unsigned)ctas), kRowsThreads, smem, stream, blocks, x, y, N, K, N);
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: launch");
     return TQ1_OK;
 }
