@@ -62,12 +62,13 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn encode_tiled_fn();
 
-// A launch that may begin while the kernel before it in the stream ends (programmatic dependent launch): the kernel calls
-// grid_dependency_wait() before it touches what an earlier one may have written or may still read, by plain loads: __ldg and
-// __restrict__ tell the compiler that the data were there from the kernel's beginning. Calls back to back: a gather of 2048
+// With `dependent` a launch that may begin while the kernel before it in the stream ends (programmatic dependent launch): it
+// calls grid_dependency_wait() before it touches what an earlier one may have written or may still read, by plain loads: __ldg
+// and __restrict__ tell the compiler that the data were there from the kernel's beginning. Calls back to back: a gather of 2048
 // rows of 5120 columns 8.2 -> 5.7 us, five tokens of 4099x2176 7.2 -> 6.1.
 template <class... P, class... A>
-cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, A... args) {
+cudaError_t launch_dependent(bool dependent, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
+                             A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
@@ -77,14 +78,13 @@ cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, unsigned threads, 
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = dependent ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
-// The next kernel may be launched; then everything before this one has ended and its results are there.
-__device__ __forceinline__ void grid_dependency_wait() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+// The next kernel may be launched where there is room for it (its CTAs then wait beside this kernel's).
+__device__ __forceinline__ void allow_next_grid() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Everything before this kernel has ended and its results are there.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Launchers implemented one per .cu file; all enqueue on `stream` and return a status.
 int launch_validate(const uint8_t *blocks, int64_t groups, int64_t *counts, cudaStream_t stream);

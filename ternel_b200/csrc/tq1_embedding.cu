@@ -43,8 +43,14 @@ constexpr int kTokensPerThread = 4;
 
 }  // namespace
 
+// A dependent launch reads by plain loads.
+template <bool PLAIN>
+__device__ __forceinline__ uint32_t load_byte(const uint8_t *p) { return PLAIN ? *p : __ldg(p); }
+
 // SHARED: a CTA first copies the table to shared memory, which the few CTAs of a short call gain from; in a long one the
-// barrier behind the copy costs more than lookups through L1 (launch_embedding has the line and the figures).
+// barrier behind the copy costs more than lookups through L1 (launch_embedding has the line and the figures). A short call is
+// also a dependent launch; a long one gains nothing from that and loses from the plain loads (8192 tokens, FP32: 38.7 us, 42.7
+// with both).
 template <bool OUT_F32, bool SHARED>
 __global__ void __launch_bounds__(kThreadsPerBlockRow * kBlocksPerCta)
 embedding_kernel(const uint8_t *blocks, const int64_t *ids, void *out,
@@ -68,7 +74,7 @@ embedding_kernel(const uint8_t *blocks, const int64_t *ids, void *out,
         for (int i = 0; i < 256; i += kThreadsPerBlockRow * kBlocksPerCta)
             shared_trits[i + threadIdx.x] = g_trits.e[i + threadIdx.x];
     }
-    grid_dependency_wait();
+    if (SHARED) grid_dependency_wait();
 #pragma unroll
     for (int q = 0; q < kTokensPerThread; ++q) id[q] = in_row && t0 + q < T ? ids[t0 + q] : -1;
     const uint8_t *blk[kTokensPerThread];
@@ -78,11 +84,15 @@ embedding_kernel(const uint8_t *blocks, const int64_t *ids, void *out,
         live[q] = id[q] >= 0 && id[q] < V;
         blk[q] = blocks + (size_t)((unsigned)(live[q] ? id[q] : 0) * (unsigned)gpr + (unsigned)(in_row ? g : 0)) * kBlockBytes;
         sbits[q] = *reinterpret_cast<const unsigned short *>(blk[q]);
-        b0[q] = blk[q][2 + a];
-        b1[q] = blk[q][3 + a];
-        b2[q] = off >= 3 ? blk[q][4 + a] : 0u;          // the third byte exists whenever it is needed
+        b0[q] = load_byte<SHARED>(blk[q] + 2 + a);
+        b1[q] = load_byte<SHARED>(blk[q] + 3 + a);
+        b2[q] = off >= 3 ? load_byte<SHARED>(blk[q] + 4 + a) : 0u;      // the third byte exists whenever it is needed
     }
-    if (SHARED) __syncthreads();
+    if (SHARED) {
+        __syncthreads();
+        // not before the loads: CTAs of the next gather that wait beside this one's take places unevenly
+        allow_next_grid();
+    }
     if (!in_row) return;
     uint32_t sel[kTokensPerThread];                             // eight nibbles, output i at bits 4i..4i+3
 #pragma unroll
@@ -146,7 +156,7 @@ int launch_embedding(const uint8_t *blocks, const int64_t *ids, void *out, bool 
                               : static_cast<void *>(static_cast<__half *>(out) + t0 * K);
         auto kernel = out_f32 ? (shared ? embedding_kernel<true, true> : embedding_kernel<true, false>)
                               : (shared ? embedding_kernel<false, true> : embedding_kernel<false, false>);
-        const cudaError_t err = launch_dependent(kernel, grid, kThreadsPerBlockRow * kBlocksPerCta, 0, stream, blocks, ids + t0,
+        const cudaError_t err = launch_dependent(shared, kernel, grid, kThreadsPerBlockRow * kBlocksPerCta, 0, stream, blocks, ids + t0,
                                                  first, n, V, gpr);
         if (err != cudaSuccess) return cuda_fail(err, "tq1_embedding_f16: launch");
     }

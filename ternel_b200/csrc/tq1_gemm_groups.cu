@@ -167,6 +167,9 @@ groups_few_kernel(const uint8_t *blocks, const __half *x, void *y, int y_f32,
         }
         __syncwarp();                                   // the packed bytes have been read
     }
+    // Not earlier: CTAs of the next call that wait beside this one's take places unevenly (8 tokens of 4099x2176 replayed in a
+    // graph: 6.0 us without the dependent launch, 8.0 with an early one, 5.3 with this).
+    allow_next_grid();
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
         parts[warp][8 * t + 2 * q][g] = acc[t][0];
@@ -294,6 +297,7 @@ groups_many_kernel(const uint8_t *blocks, const __half *x, void *y, int y_f32,
         __syncwarp();                                   // the packed bytes have been read
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
+    allow_next_grid();                                  // not earlier, as above: 16 tokens of 17408x5248 took 62 us instead of 38
 #pragma unroll
     for (int t = 0; t < NT; ++t)
 #pragma unroll
@@ -306,7 +310,10 @@ groups_many_kernel(const uint8_t *blocks, const __half *x, void *y, int y_f32,
 template <int NT>
 int launch_few(const uint8_t *blocks, const __half *x, void *y, int y_f32, int M, int N, int groups, cudaStream_t stream) {
     const long long ctas = (long long)((N + kFewRows - 1) / kFewRows) * ((M + 8 * NT - 1) / (8 * NT));
-    const cudaError_t err = launch_dependent(groups_few_kernel<NT>, dim3((unsigned)ctas), kFewWarps * 32, 0, stream, blocks, x, y,
+    // around one CTA an SM, a call whose first CTAs find places beside the last of the one before takes two places on some SMs
+    // (120 CTAs: 8.7 us alone, 10.1 as a dependent launch; 24 of them 5.9 and 5.3, 257 of them 6.0 and 5.3)
+    const bool dependent = ctas <= 74 || ctas > 148;
+    const cudaError_t err = launch_dependent(dependent, groups_few_kernel<NT>, dim3((unsigned)ctas), kFewWarps * 32, 0, stream, blocks, x, y,
                                              y_f32, M, N, groups);
     return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: launch");
 }
@@ -317,7 +324,7 @@ int launch_many(const uint8_t *blocks, const __half *x, void *y, int y_f32, int 
     cudaError_t err = cudaFuncSetAttribute(groups_many_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)many_smem(NT));
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: shared memory opt-in");
-    err = launch_dependent(groups_many_kernel<NT>, dim3((unsigned)ctas), kManyWarps * 32, many_smem(NT), stream, blocks, x, y, y_f32,
+    err = launch_dependent(true, groups_many_kernel<NT>, dim3((unsigned)ctas), kManyWarps * 32, many_smem(NT), stream, blocks, x, y, y_f32,
                            M, N, groups);
     return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: launch");
 }

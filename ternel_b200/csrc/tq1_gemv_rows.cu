@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(kRowsThreads) gemv_rows_kernel(const uint8_t *
             }
         }
     }
+    allow_next_grid();
 }
 
 template <int MB>
@@ -114,7 +115,9 @@ static int launch_mb(const uint8_t *blocks, const __half *x, void *y, bool y_f32
     cudaError_t err = cudaFuncSetAttribute(y_f32 ? kern_f : kern_h,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: shared memory opt-in");
-    err = launch_dependent(y_f32 ? kern_f : kern_h, dim3((unsigned)ctas), kRowsThreads, smem, stream, blocks, x, y, N, K, N);
+    // as in tq1_gemm_groups.cu: around one CTA an SM the next call's CTAs would double up (125 CTAs: 4.4 us, 8.0 as an early
+    // dependent launch)
+    err = launch_dependent(ctas <= 74 || ctas > 148, y_f32 ? kern_f : kern_h, dim3((unsigned)ctas), kRowsThreads, smem, stream, blocks, x, y, N, K, N);
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: launch");
     return TQ1_OK;
 }
