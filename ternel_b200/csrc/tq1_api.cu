@@ -63,7 +63,9 @@ int tq1_linear_f16(const uint8_t *blocks, const void *x, void *y, int y_is_f32,
     if ((reinterpret_cast<uintptr_t>(blocks) & 15) == 0 && gemm_tc_shape_ok(M, N, K))
         return launch_gemm_tc(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, workspace, s);
     if (gemm_groups_preferred(M, N, K))
-        return launch_gemm_groups(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, s);
+        return launch_gemm_groups(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K,
+                                  workspace && workspace_bytes >= kWsStatusBytes && (reinterpret_cast<uintptr_t>(workspace) & 3) == 0
+                                      ? static_cast<unsigned *>(workspace) : nullptr, s);
     return launch_gemv_rows(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, s);
 }
 

@@ -157,8 +157,12 @@ int launch_gemm_slices(const uint8_t *blocks, const __half *x, void *y, bool y_f
 
 // Batched linear (M >= 2) with an FP32 sum per group, for every other width and alignment.
 bool gemm_groups_preferred(int M, int N, int K);
-int launch_gemm_groups(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K,
+// status: the workspace's first word, or null where the caller has none
+int launch_gemm_groups(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, unsigned *status,
                        cudaStream_t stream);
+float gemm_groups_tc_us(int M, int N, int K);               // modelled time of the tcgen05 form
+int launch_gemm_groups_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, unsigned *status,
+                          cudaStream_t stream);
 
 // Five base-3 digits of a byte packed two bits each (digit i at bits 2i..2i+1).
 __host__ __device__ inline uint32_t trits_2bit(uint32_t byte) {

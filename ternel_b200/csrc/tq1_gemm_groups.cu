@@ -333,23 +333,34 @@ int launch_many(const uint8_t *blocks, const __half *x, void *y, int y_f32, int 
 
 bool gemm_groups_preferred(int M, int N, int K) { return M >= 2 && (long long)M * N * K >= (1 << 20); }
 
-// The many-row kernel decodes a weight once for all of its tokens, but needs 128 rows a CTA: it takes over where its CTAs
-// fill most of the SMs. Both sides, us: 16 tokens of 17408x5248 37 against 39, of 5120x640 6.5 against 4.5; 32 tokens of
-// 17408x5248 55 against 70, of 4099x2176 22 against 9; 64 tokens of 17408x5248 71 against 136, of 4099x2176 30 against 15;
-// 129 tokens of 4099x2176 30 against 42, 700 of 383x4224 54 against 31.
-int launch_gemm_groups(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K,
+// Which of the three takes a call: modelled times (us), fitted to calls with weights out of HBM.
+//   few    a warp works through every eighth group; up to 32 tokens it is taken where `many` would leave SMs empty: 16 tokens of
+//          17408x5248 37 against 39 of `many`, of 5120x640 4.5 against 6.5, 32 tokens of 17408x5248 70 against 55, of 4099x2176
+//          9 against 22
+//   many   a CTA's groups one after the other, 0.85, 1.28 and 1.68 us each at 16, 32 and 64 tokens
+//   tcgen05 form   0.64 us a group up to 32 tokens, 1.13 beyond, behind a longer set-up (its file has both sides)
+int launch_gemm_groups(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, unsigned *status,
                        cudaStream_t stream) {
     const int groups = K / kGroup, f32 = y_f32 ? 1 : 0;
-    const long long row_tiles = (N + kManyRows - 1) / kManyRows;
+    const long long row_tiles = (N + kManyRows - 1) / kManyRows, token_tiles = (M + 63) / 64;
     if (M <= 8) return launch_few<1>(blocks, x, y, f32, M, N, groups, stream);
+    const bool many = M <= 16 ? row_tiles >= 128 : M <= 32 ? row_tiles >= 105 : row_tiles * token_tiles >= 74;
+    const auto rounds = [](long long ctas, int at_once) { return (float)((ctas + at_once - 1) / at_once); };
+    float us = 0.0f;
+    if (many) {
+        us = 3.0f + (float)groups * (M <= 16   ? 0.85f * rounds(row_tiles, 296)
+                                     : M <= 32 ? 1.28f * rounds(row_tiles, 296)
+                                               : 1.68f * rounds(row_tiles * token_tiles, 148));
+    } else if (M > 32) {
+        const long long ctas = (long long)((N + kFewRows - 1) / kFewRows) * ((M + 31) / 32);
+        us = 3.0f + (float)((groups + 7) / 8) * (ctas <= 148 ? 1.1f : 2.1f * rounds(ctas, 296));
+    }
+    if (gemm_groups_tc_us(M, N, K) < us) return launch_gemm_groups_tc(blocks, x, y, y_f32, M, N, K, status, stream);
     if (M <= 16)
-        return row_tiles >= 128 ? launch_many<2>(blocks, x, y, f32, M, N, groups, stream)
-                                : launch_few<2>(blocks, x, y, f32, M, N, groups, stream);
-    if (M <= 32)
-        return row_tiles >= 105 ? launch_many<4>(blocks, x, y, f32, M, N, groups, stream)
-                                : launch_few<4>(blocks, x, y, f32, M, N, groups, stream);
-    return row_tiles * ((M + 63) / 64) >= 74 ? launch_many<8>(blocks, x, y, f32, M, N, groups, stream)
-                                             : launch_few<4>(blocks, x, y, f32, M, N, groups, stream);
+        return many ? launch_many<2>(blocks, x, y, f32, M, N, groups, stream) : launch_few<2>(blocks, x, y, f32, M, N, groups, stream);
+    if (M <= 32 || !many)
+        return many ? launch_many<4>(blocks, x, y, f32, M, N, groups, stream) : launch_few<4>(blocks, x, y, f32, M, N, groups, stream);
+    return launch_many<8>(blocks, x, y, f32, M, N, groups, stream);
 }
 
 }  // namespace tq1

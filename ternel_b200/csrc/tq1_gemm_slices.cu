@@ -34,6 +34,7 @@
 #include <type_traits>
 
 #include "tq1_common.cuh"
+#include "tq1_decode.cuh"
 
 namespace tq1 {
 
@@ -42,13 +43,11 @@ namespace {
 constexpr int kTileRows = 16;
 constexpr int kChunkBytes = 4 * kBlockBytes;                    // a row's bytes of a 512-column chunk
 constexpr int kChain = 4;                                       // MMAs (of 16 columns) under one accumulator
-constexpr uint32_t kSpinLimit = 1u << 20;
 constexpr int kMaxDevices = 64;
 
 constexpr uint32_t kWindow = 1024;                              // shared-window address of dynamic shared memory
 constexpr uint32_t kTableAddr = kWindow;                        // 256 entries of 256 bytes
-constexpr uint32_t kTableBytes = 65536;
-constexpr uint32_t kBarAddr = kTableAddr + kTableBytes;
+constexpr uint32_t kBarAddr = kTableAddr + kCodeTableBytes;
 constexpr uint32_t kBarBytes = 2048;
 constexpr uint32_t kDataAddr = kBarAddr + kBarBytes;            // activations and later partial sums, sums (split K), ring
 constexpr uint32_t kXBytes = 4096;                              // activations: half a chunk, eight tokens
@@ -81,48 +80,6 @@ struct SliceParams {
     int wide_y;                                                 // four results of a token may be stored at a time
 };
 
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t d;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
-    return d;
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// Bounded, as in the other kernels: after the limit status 3 is set and the thread waits for nothing any more.
-__device__ __noinline__ bool mbar_wait_more(uint32_t bar, uint32_t parity, unsigned *status) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\t"
-                 "mov.u32 n, %3;\n"
-                 "TRY:\n\t"
-                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 4000;\n\t"
-                 "@p bra DONE;\n\t"
-                 "sub.u32 n, n, 1;\n\t"
-                 "setp.ne.u32 q, n, 0;\n\t"
-                 "@q bra TRY;\n"
-                 "DONE:\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity), "n"(kSpinLimit) : "memory");
-    if (!ok) atomicExch(status, 3u);
-    return !ok;
-}
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, unsigned *status, bool &dead) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\t"
-                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    if (!ok && !dead) dead = mbar_wait_more(bar, parity, status);
-}
-__device__ __forceinline__ bool elect_one() {
-    uint32_t one;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
-    return one != 0;
-}
 template <int OFFSET>
 __device__ __forceinline__ uint32_t lds(uint32_t addr) {
     uint32_t v;
@@ -141,56 +98,12 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
             : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Table entry of code byte v: PRMT selectors that pick FP16 weights out of [s_lo, s_hi, s_hi ^ 0x80] and zeros, one byte a trit.
-//   even byte (its first trit in the lower half of a register): word0 = (t0,t1) | t4 << 16, word1 = (t2,t3)
-//   odd byte: word0 = (t1,t2) | t0 << 16, word1 = (t3,t4)
-// The 13 values past 242 decode to zero weights: a byte that escaped the load-time scan reads inside the table.
-struct CodeTable { uint2 e[512]; };                             // entry of byte v: e[2 v] even, e[2 v + 1] odd
-constexpr CodeTable make_code_table() {
-    CodeTable t{};
-    for (int v = 0; v < 256; ++v) {
-        uint32_t c[5] = {0x44u, 0x44u, 0x44u, 0x44u, 0x44u};
-        int rest = v;
-        for (int d = 0; d < 5 && v < 243; ++d) {
-            c[d] = rest % 3 == 0 ? 0x20u : rest % 3 == 1 ? 0x44u : 0x10u;
-            rest /= 3;
-        }
-        t.e[2 * v].x = c[0] | (c[1] << 8) | (c[4] << 16);
-        t.e[2 * v].y = c[2] | (c[3] << 8);
-        t.e[2 * v + 1].x = c[1] | (c[2] << 8) | (c[0] << 16);
-        t.e[2 * v + 1].y = c[3] | (c[4] << 8);
-    }
-    return t;
-}
-__device__ __align__(16) const CodeTable g_code_table = make_code_table();
-
-// A lane's 64 weights of one row, 32 registers of two, in the order of the columns. Eager: everything the caller's loop
-// unrolls into; `w` holds the block's words (of half 0 words 0..3, of half 1 words 0 and 3..6).
-struct RowDecoder {
-    const uint32_t *w;
-    uint32_t pool, even_entry, odd_entry;
-    __device__ __forceinline__ void lookup(int j, uint32_t &e0, uint32_t &e1) const {        // code byte j
-        const uint32_t addr = prmt(w[(2 + j) >> 2], j & 1 ? odd_entry : even_entry, 0x7604u | (uint32_t)(((2 + j) & 3) << 4));
-        asm("ld.shared.v2.u32 {%0, %1}, [%2+%3];" : "=r"(e0), "=r"(e1) : "r"(addr), "n"(kTableAddr));
-    }
-    __device__ __forceinline__ uint32_t pick(uint32_t sel) const { return prmt(pool, 0u, sel); }
-    // ten weights of code bytes j (even) and j + 1
-    __device__ __forceinline__ void two_bytes(int j, uint32_t *v) const {
-        uint32_t e0, e1, f0, f1;
-        lookup(j, e0, e1);
-        lookup(j + 1, f0, f1);
-        v[0] = pick(e0);
-        v[1] = pick(e1);
-        v[2] = pick(prmt(e0, f0, 0x0062));
-        v[3] = pick(f0);
-        v[4] = pick(f1);
-    }
-};
-
 // The products of one row tile and half a chunk: added to sum[token tile][..] (rows g and g + 8, tokens 2q and 2q + 1).
+using Decoder = RowDecoder<kTableAddr>;
+
 // START: these are the first products of sum.
 template <int NT, int HALF, bool START>
-__device__ __forceinline__ void half_slice(const RowDecoder &lo, const RowDecoder &hi, const uint32_t (&b)[NT][32],
+__device__ __forceinline__ void half_slice(const Decoder &lo, const Decoder &hi, const uint32_t (&b)[NT][32],
                                            float (&sum)[NT][4]) {
     uint32_t va[32], vb[32];
     float d[NT][4];
@@ -222,7 +135,7 @@ __device__ __forceinline__ void half_slice(const RowDecoder &lo, const RowDecode
         vb[31] = hi.pick(e1);
         multiply(15);
     } else {
-        auto first = [](const RowDecoder &r, uint32_t *v) {     // the last trit of byte 12, and byte 13
+        auto first = [](const Decoder &r, uint32_t *v) {     // the last trit of byte 12, and byte 13
             uint32_t e0, e1, f0, f1;
             r.lookup(12, e0, e1);
             r.lookup(13, f0, f1);
@@ -241,7 +154,7 @@ __device__ __forceinline__ void half_slice(const RowDecoder &lo, const RowDecode
             for (int i = 1; i < 14; ++i)
                 if (2 * i + 1 >= 3 + 5 * a && 2 * i + 1 < 8 + 5 * a) multiply(i);
         }
-        auto last = [](const RowDecoder &r, uint32_t *v) {      // byte 24 and the tail byte's three trits
+        auto last = [](const Decoder &r, uint32_t *v) {      // byte 24 and the tail byte's three trits
             uint32_t e0, e1, f0, f1;
             r.lookup(24, e0, e1);
             r.lookup(25, f0, f1);
@@ -350,19 +263,7 @@ slices_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         for (int i = 0; i < min(prm.stages, n_tiles); ++i)
             asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];"
                          ::"l"(&wmap), "r"(word_x), "r"((tile_lo + i) * kTileRows) : "memory");
-    // Sixteen copies of every entry, two entries of both forms (512 bytes) per warp and step, several loads in flight.
-    constexpr int kSteps = 128, kFlight = 8;
-    for (int j0 = warp; j0 < kSteps; j0 += kFlight * warps) {
-        uint2 e[kFlight];
-#pragma unroll
-        for (int j = 0; j < kFlight; ++j)
-            if (j0 + j * warps < kSteps) e[j] = __ldg(&g_code_table.e[4 * (j0 + j * warps) + (lane >> 3)]);
-#pragma unroll
-        for (int j = 0; j < kFlight; ++j)
-            if (j0 + j * warps < kSteps)
-                *reinterpret_cast<uint4 *>(smem + (kTableAddr - kWindow) + (j0 + j * warps) * 512 + lane * 16) =
-                    make_uint4(e[j].x, e[j].y, e[j].x, e[j].y);
-    }
+    fill_code_table(smem + (kTableAddr - kWindow), warp, warps, lane);
     if (split > 1) {                                            // the CTAs of a cluster write into each other's memory
         __syncwarp();
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -487,7 +388,7 @@ slices_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                     auto pool = [](uint32_t w) { return prmt(w, w ^ 0x8000u, 0x0510u); };       // [s_lo, s_hi, s_hi ^ 0x80]
                     float sum[NT][4];
                     {
-                        const RowDecoder lo{w_lo, pool(w_lo[0]), even_entry, odd_entry}, hi{w_hi, pool(w_hi[0]), even_entry, odd_entry};
+                        const Decoder lo{w_lo, pool(w_lo[0]), even_entry, odd_entry}, hi{w_hi, pool(w_hi[0]), even_entry, odd_entry};
                         half_slice<NT, HALF, true>(lo, hi, b[0], sum);
                         if (HS == 2) half_slice<NT, 1, false>(lo, hi, b[HS - 1], sum);
                     }

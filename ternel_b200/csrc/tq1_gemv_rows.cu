@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(kRowsThreads) gemv_rows_kernel(const uint8_t *
     float *xs = reinterpret_cast<float *>(smem_raw + 512);           // [MB][K]
 
     for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = (uint16_t)trits_2bit(i);
+    allow_next_grid();                                  // early: 82 us for 17408x5248, 92 after the loop
     grid_dependency_wait();
     for (int i = threadIdx.x; i < MB * K; i += blockDim.x) xs[i] = __half2float(x[i]);
     __syncthreads();
@@ -99,7 +100,6 @@ __global__ void __launch_bounds__(kRowsThreads) gemv_rows_kernel(const uint8_t *
             }
         }
     }
-    allow_next_grid();
 }
 
 template <int MB>

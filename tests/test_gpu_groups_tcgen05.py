@@ -1,0 +1,73 @@
+"""Group sums on tcgen05 (widths that are no multiple of 512, and blocks off the 16-byte grid) at the edges of its tiles."""
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import tq1_oracle as o
+from tests.gpu_util import random_blocks, run_linear, to_dev
+
+pytestmark = pytest.mark.gpu
+
+# Relative error (2-norm): two truncating steps per accumulator, on average half an ulp of 0.72 * 2^-23 each of a value that
+# grows from zero (0.96 * 2^-24), two FP32 additions of four accumulators (0.58 * 2^-24 each, in quadrature 0.82), and one
+# rounding of the carried sum (0.58).
+BOUND = (0.96 + 0.82 + 0.58) * 2.0 ** -24
+
+
+@pytest.mark.parametrize(("rows", "columns", "batch"), (
+    (17408, 2688, 12), (17000, 1408, 16),               # one unit, of 16 tokens
+    (17408, 1664, 17), (14000, 2688, 32),               # of 32, rows that fill no tile
+    (4099, 2176, 33), (2000, 4224, 64),                 # two units, a cluster per tile
+    (4099, 2176, 65), (9000, 640, 129), (13313, 384, 200)))        # several token tiles, more tiles than SMs, three groups
+@pytest.mark.parametrize("shift", (0, 4))
+def test_against_float64(rows, columns, batch, shift):
+    from ternel_b200.ops import check_status, tq1_get_rows, tq1_matmul
+    blocks, rng = random_blocks(rows, columns, seed=rows + batch)
+    backing = torch.zeros(blocks.size + 16, dtype=torch.uint8, device="cuda")
+    bd = backing[shift:shift + blocks.size].view(blocks.shape)
+    bd.copy_(torch.from_numpy(blocks))
+    x = torch.from_numpy(rng.standard_normal((batch, columns)).astype(np.float16)).cuda()
+    dense = tq1_get_rows(bd, torch.arange(rows, device="cuda"), dtype=torch.float32).double()
+    want = x.double() @ dense.T
+    got = tq1_matmul(bd, x, out_dtype=torch.float32)
+    assert float((got.double() - want).norm() / want.norm()) <= BOUND
+    assert torch.equal(tq1_matmul(bd, x, out_dtype=torch.float32), got)
+    assert torch.equal(tq1_matmul(bd, x), got.half())
+    check_status()
+
+
+@pytest.mark.parametrize(("rows", "columns", "batch"), ((16500, 640, 16), (4099, 2176, 48), (9000, 640, 100)))
+@pytest.mark.parametrize("kind", ("scales", "activations", "infinite sum"))
+def test_nonfinite_values(rows, columns, batch, kind):
+    """Whole activations: infinities of a sum's sign, NaN for 0 * Inf and Inf - Inf, and a sum that has become infinite stays so."""
+    blocks, rng = random_blocks(rows, columns, seed=batch)
+    x = rng.integers(-3, 4, (batch, columns)).astype(np.float16)
+    scales = blocks.reshape(rows, columns // 128, 28)[:, :, :2].copy().view(np.float16)[:, :, 0]
+    if kind == "scales":
+        hit = rng.random(scales.shape) < 0.1
+        scales[hit] = rng.choice(np.array([np.inf, -np.inf, np.nan, 0.0], dtype=np.float16), hit.sum())
+    elif kind == "activations":
+        hit = rng.random(x.shape) < 0.5 / columns
+        x[hit] = rng.choice(np.array([np.inf, -np.inf, np.nan], dtype=np.float16), hit.sum())
+    else:
+        scales[:, 0], x[0, :128] = np.inf, 1.0
+    blocks[:, :, :2] = scales[:, :, None].copy().view(np.uint8)
+    few = rng.choice(rows, 300, replace=False)          # the oracle takes its time
+    with np.errstate(invalid="ignore", over="ignore"):
+        want = o.reference_matmul(np.ascontiguousarray(blocks[few]), x.astype(np.float32), rows=300, columns=columns)
+    got = run_linear(blocks, x)[:, few]
+    assert not np.isfinite(want).all()
+    assert np.array_equal(o.nonfinite_classes(got), o.nonfinite_classes(want))
+
+
+def test_no_workspace_is_needed():
+    from ternel_b200 import _native
+    rows, columns, batch = 4099, 2176, 64
+    blocks, rng = random_blocks(rows, columns, seed=5)
+    x = rng.standard_normal((batch, columns)).astype(np.float16)
+    bd, xd = to_dev(blocks), to_dev(x)
+    y = torch.empty((batch, rows), dtype=torch.float32, device="cuda")
+    assert _native.lib().tq1_linear_f16(bd.data_ptr(), xd.data_ptr(), y.data_ptr(), 1, batch, rows, columns, None, 0,
+                                        torch.cuda.current_stream().cuda_stream) == 0
+    assert np.array_equal(y.cpu().numpy(), run_linear(blocks, x))
