@@ -493,9 +493,16 @@ int clusters_at_once(int split) {
     return known[dev][split];
 }
 
-// The K split with the smallest modelled time (us, fitted to graph replays with weights out of HBM): what the SM works through
-// (0.128 per row tile and chunk of eight tokens, twice that for sixteen), or where there are few warps what one of them does
-// one tile after the other, behind launch, table and activations; a cluster's barriers and its exchange on top.
+// Modelled time (us, fitted to graph replays with weights out of HBM): what the SM works through (0.128 per row tile and chunk of
+// eight tokens, twice that for sixteen), or where there are few warps what one of them does one tile after the other, behind
+// launch, table and activations; a cluster's barriers and its exchange on top.
+float slice_us(int split, int slices, int per_cluster) {
+    const int subsets = kMaxSlices / slices < per_cluster ? kMaxSlices / slices : per_cluster;
+    const float sm = 0.128f * (float)(per_cluster * slices), chain = 0.7f * (float)((per_cluster + subsets - 1) / subsets);
+    return (split > 1 ? 5.2f : 3.6f) + (sm > chain ? sm : chain);
+}
+
+// The K split with the smallest modelled time.
 SlicePlan slice_plan(int nt, int N, int K) {
     SlicePlan best = {};
     const int per = slice_halves(nt), halves = K / 256 / per, tiles = (N + kTileRows - 1) / kTileRows;
@@ -504,6 +511,8 @@ SlicePlan slice_plan(int nt, int N, int K) {
         p.split = split;
         p.slices = (halves + split - 1) / split;
         if (halves < split || p.slices > kMaxSlices) continue;
+        // how many clusters run at once is asked of the driver (milliseconds, the first time) only where this split could win
+        if (best.ok && slice_us(split, p.slices, (tiles + sm_count() / split - 1) / (sm_count() / split)) >= best.us) continue;
         const int room = nt == 1 ? clusters_at_once<1>(split) : clusters_at_once<2>(split);
         p.clusters = tiles < room ? tiles : room;
         const int per_cluster = (tiles + p.clusters - 1) / p.clusters;
@@ -526,8 +535,7 @@ SlicePlan slice_plan(int nt, int N, int K) {
         if (p.stages < (per_cluster < 2 * p.subsets ? per_cluster : p.subsets + 1)) continue;      // no room to fetch ahead
         p.end = p.ring_addr + (uint32_t)p.stages * stage_bytes;
         p.ok = true;
-        const float sm = 0.128f * per_cluster * p.slices, chain = 0.7f * ((per_cluster + p.subsets - 1) / p.subsets);
-        p.us = (split > 1 ? 5.2f : 3.6f) + (sm > chain ? sm : chain);
+        p.us = slice_us(split, p.slices, per_cluster);
         if (!best.ok || p.us < best.us) best = p;
     }
     return best;
