@@ -19,8 +19,8 @@
 //
 // What bounds it: up to 32 tokens the chain of dependent loads and the decode (25 instructions and six table or byte loads
 // per eight weights), beyond that the products and the instructions around them (700 tokens of 17408x5248: 87 T
-// multiply-adds/s; an SM at work has its mma.sync pipe active for 57% of the time). 5 tokens of 4099x2176 take 5.6 us (row
-// kernel 45, tcgen05 form 11.6), 300 tokens of 4099x2176 60 us (2380, 21), the last of their two waves with 17 CTAs.
+// multiply-adds/s; an SM at work has its mma.sync pipe active for 57% of the time). 5 tokens of 4099x2176 take 5.1 us (row
+// kernel 45). Longer calls go to the tcgen05 form (tq1_gemm_groups_tc.cu).
 #include "tq1_common.cuh"
 
 namespace tq1 {
