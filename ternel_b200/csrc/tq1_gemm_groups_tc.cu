@@ -16,11 +16,12 @@
 // Two units' accumulators (256 columns of tensor memory) alternate. Few tiles: a cluster of CTAs splits the groups of a tile and
 // adds its sums through distributed shared memory; no workspace is needed.
 //
-// What bounds it: the round trip of a unit, MMAs - accumulators read and added - slot free again, with two slots: 0.64 us a
-// K block of one unit, 1.13 of two (without the sums 0.5 and 0.75, without the decode or the MMAs hardly less than with
-// them; one MMA warp, or half as many warps with twice the tokens for the sums, 3% more). Weights out of HBM, against the
-// mma.sync forms: 16 / 64 / 700 tokens of 17408x5248 31.6 / 51.6 / 523 us (37.8 / 72 / 735), 64 / 129 / 700 of 4099x2176
-// 12.5 / 23.1 / 66 (15.7 / 31.3 / 89).
+// What bounds it: issue slots (69% used; 6400 instructions per K block of two units, 900 of them the decode, the rest for the
+// sums of its 32768 accumulator values) and the round trip of a unit, MMAs - accumulators read and added - slot free again, with
+// two slots: 0.64 us a K block of one unit, 1.13 of two (without the sums 0.5 and 0.75; without the decode, or with one of eight
+// MMAs, hardly less than with them; one MMA warp, or half as many warps with twice the tokens for the sums, 3% more). Weights
+// out of HBM, against the mma.sync forms: 16 / 64 / 700 tokens of 17408x5248 31.8 / 51.8 / 525 us (37.8 / 72 / 735),
+// 64 / 129 / 700 of 4099x2176 12.5 / 23.2 / 66.5 (15.7 / 31.3 / 89).
 #include <cuda.h>
 
 #include "tq1_common.cuh"
