@@ -65,11 +65,8 @@ __host__ __device__ constexpr int slice_halves(int nt) { return nt == 1 ? 2 : 1;
 constexpr int kExtraWarps = 1;
 
 struct SliceParams {
-    const uint8_t *blocks;
-    const __half *x;
     void *y;
     unsigned *status;
-    const unsigned *counters;                                   // of the tcgen05 kernel; zero in a workspace that is in order
     int M, N, chunks;
     int tiles, clusters;                                        // row tiles, clusters of the grid
     int split_log, slices, subsets;                             // the grid's clusters have 2^split_log CTAs
@@ -275,7 +272,6 @@ slices_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     bool dead = false;
-    if (tid == 0 && blockIdx.x == 0 && *prm.counters != 0u) atomicExch(prm.status, 8u);      // a stale workspace
     if (warp == workers) {
         // ------------------------------------------------------------------ fetch
         if (elect_one()) {
@@ -581,13 +577,9 @@ int launch_gemm_slices(const uint8_t *blocks, const __half *x, void *y, bool y_f
     const int nt = M <= 8 ? 1 : 2;
     const SlicePlan p = slice_plan(nt, N, K);
     if (!p.ok) return fail(TQ1_ERR_INVALID, "tq1_linear_f16: %dx%dx%d does not fit the slice kernel", M, N, K);
-    unsigned char *ws = static_cast<unsigned char *>(workspace);
     SliceParams prm;
-    prm.blocks = blocks;
-    prm.x = x;
     prm.y = y;
-    prm.status = reinterpret_cast<unsigned *>(ws);
-    prm.counters = reinterpret_cast<const unsigned *>(ws + kWsCounterOffset);
+    prm.status = static_cast<unsigned *>(workspace);
     prm.M = M;
     prm.N = N;
     prm.chunks = K / 512;

@@ -69,3 +69,22 @@ def test_gated_activation(half_rows, columns, batch):
     got = tq1_swiglu(both, x, out_dtype=torch.float32)
     # expf, a division and two products in FP32: a few units in the last place of each value
     assert bool(((got - want).abs() <= 2e-6 * want.abs()).all())
+
+
+@pytest.mark.parametrize("batch", (8, 16))
+def test_counters_of_other_kernels_do_not_matter(batch):
+    """The slice kernel adds nothing up in the workspace: counters that another kernel is using, or has left behind, are no
+    fault of its results."""
+    from ternel_b200 import _native
+    rows, columns = 1024, 5120
+    blocks, rng = random_blocks(rows, columns, seed=4)
+    x = rng.standard_normal((batch, columns)).astype(np.float16)
+    bd, xd = to_dev(blocks), to_dev(x)
+    lib = _native.lib()
+    ws = torch.full((lib.tq1_linear_workspace_bytes(batch, rows, columns),), 99, dtype=torch.uint8, device="cuda")
+    ws[:256].zero_()
+    y = torch.zeros((batch, rows), dtype=torch.float32, device="cuda")
+    assert lib.tq1_linear_f16(bd.data_ptr(), xd.data_ptr(), y.data_ptr(), 1, batch, rows, columns, ws.data_ptr(), ws.numel(),
+                              ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    assert int(ws[:4].view(torch.int32).item()) == 0 and bool((ws[256:] == 99).all())
+    assert np.array_equal(y.cpu().numpy(), run_linear(blocks, x))

@@ -17,7 +17,7 @@ from ternel_b200.stack import random_blocks_device
 gen = torch.Generator(device="cuda")
 gen.manual_seed(5)
 small, large = (random_blocks_device(n, 5120, gen, "cuda") for n in (1024, 17408))
-x, other, long = (torch.randn((m, 5120), generator=gen, device="cuda").half() for m in (8, 8, 2048))
+x, other, long = (torch.randn((m, 5120), generator=gen, device="cuda").half() for m in (17, 17, 2048))
 step = GraphedStep(lambda v: ops.tq1_matmul(small, v), [x])             # five K parts: partial tiles and counters in use
 want = step(other).clone()
 first = ops._workspaces[0]
@@ -48,7 +48,8 @@ def test_streams_may_overlap():
     from ternel_b200.stack import random_blocks_device
     gen = torch.Generator(device="cuda")
     gen.manual_seed(11)
-    shapes = ((8, 5120, 17408), (64, 5120, 17408), (3, 1024, 5120), (1, 5120, 5120), (300, 1024, 5120))
+    shapes = ((8, 5120, 17408), (64, 5120, 17408), (3, 1024, 5120), (1, 5120, 5120), (300, 1024, 5120),
+              (17, 1024, 5120), (48, 1024, 5120))
     cases = [(random_blocks_device(n, k, gen, "cuda"), torch.randn((m, k), generator=gen, device="cuda").half())
              for m, n, k in shapes]
     want = [ops.tq1_matmul(b, x) for b, x in cases]
@@ -82,8 +83,8 @@ def test_counters_that_are_not_zero_are_reported():
     from ternel_b200.dispatch import plan
     from ternel_b200.ops import tq1_matmul
     from ternel_b200.stack import random_blocks_device
-    m, n, k = 8, 1024, 5120
-    assert plan(m, n, k).parts > 1
+    m, n, k = 17, 1024, 5120
+    assert plan(m, n, k).kernel == "tensor_core" and plan(m, n, k).parts > 1
     gen = torch.Generator(device="cuda")
     gen.manual_seed(2)
     blocks, x = random_blocks_device(n, k, gen, "cuda"), torch.randn((m, k), generator=gen, device="cuda").half()
