@@ -133,8 +133,12 @@ size_t tq1_linear_workspace_bytes(int M, int N, int K);
  * registers where that is faster (FP32 accumulators over 64 columns), else tcgen05
  * GEMM (FP32 accumulators over up to a K part). Other widths and alignments: FP32
  * group sums on the matrix units from 2^20 products on, the row kernel below
- * and for M == 1; both need no workspace. Illegal code bytes must have been
- * rejected at load (tq1_validate_blocks*): the kernels carry no clamp. */
+ * and for M == 1; neither needs a workspace. With one, of at least
+ * tq1_linear_workspace_bytes (4-byte aligned, nothing but its first word is
+ * touched), long calls run the group sums on tcgen05, whose bounded waits report
+ * there; without one they stay on kernels that wait for nothing. Illegal code
+ * bytes must have been rejected at load (tq1_validate_blocks*): the kernels carry
+ * no clamp. */
 int tq1_linear_f16(const uint8_t *blocks, const void *x, void *y, int y_is_f32,
                    int M, int N, int K, void *workspace, size_t workspace_bytes, void *stream);
 

@@ -33,7 +33,7 @@ static __device__ __noinline__ bool mbar_wait_more(uint32_t bar, uint32_t parity
                  "@q bra TRY;\n"
                  "DONE:\n\t"
                  "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity), "n"(kSpinLimit) : "memory");
-    if (!ok && status) atomicExch(status, 3u);
+    if (!ok) atomicExch(status, 3u);
     return !ok;
 }
 __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, unsigned *status, bool &dead) {

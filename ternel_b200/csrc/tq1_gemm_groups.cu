@@ -355,7 +355,8 @@ int launch_gemm_groups(const uint8_t *blocks, const __half *x, void *y, bool y_f
         const long long ctas = (long long)((N + kFewRows - 1) / kFewRows) * ((M + 31) / 32);
         us = 3.0f + (float)((groups + 7) / 8) * (ctas <= 148 ? 1.1f : 2.1f * rounds(ctas, 296));
     }
-    if (gemm_groups_tc_us(M, N, K) < us) return launch_gemm_groups_tc(blocks, x, y, y_f32, M, N, K, status, stream);
+    // the tcgen05 form waits on barriers, with a limit: only for a caller that can be told that a wait ran out
+    if (status && gemm_groups_tc_us(M, N, K) < us) return launch_gemm_groups_tc(blocks, x, y, y_f32, M, N, K, status, stream);
     if (M <= 16)
         return many ? launch_many<2>(blocks, x, y, f32, M, N, groups, stream) : launch_few<2>(blocks, x, y, f32, M, N, groups, stream);
     if (M <= 32 || !many)

@@ -54,7 +54,7 @@ static_assert(kABase + kRing * 64 <= 512, "tensor memory");
 struct GroupParams {
     const uint8_t *blocks;
     void *y;
-    unsigned *status;                                           // null: the caller has no workspace
+    unsigned *status;
     int M, N, groups;
     int tiles_m, tiles, clusters, split_log, nt;                // nt: tokens of a tile, the last token tile has what is left
     int y_f32;
@@ -122,7 +122,7 @@ groups_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
     const uint32_t window = (uint32_t)__cvta_generic_to_shared(smem);
     const uint32_t base = window - kWindow;                     // zero, or what names this CTA of a cluster
     if ((base & 0x00ffffffu) != 0u) {                           // the fixed window addresses do not hold
-        if (threadIdx.x == 0 && prm.status) atomicExch(prm.status, 2u);
+        if (threadIdx.x == 0) atomicExch(prm.status, 2u);
         return;
     }
     constexpr int FULL_A = 0, FULL_B = FULL_A + kRing, EMPTY = FULL_B + kRing, ACC_FULL = EMPTY + kRing, ACC_FREE = ACC_FULL + 2;

@@ -61,7 +61,9 @@ def test_nonfinite_values(rows, columns, batch, kind):
     assert np.array_equal(o.nonfinite_classes(got), o.nonfinite_classes(want))
 
 
-def test_no_workspace_is_needed():
+def test_without_a_workspace_nothing_waits():
+    """A caller without a status word cannot be told that a wait ran out, so its calls stay on the forms that have none: the
+    results are those of a few tokens at a time, which take the same sums in the same order."""
     from ternel_b200 import _native
     rows, columns, batch = 4099, 2176, 64
     blocks, rng = random_blocks(rows, columns, seed=5)
@@ -70,4 +72,8 @@ def test_no_workspace_is_needed():
     y = torch.empty((batch, rows), dtype=torch.float32, device="cuda")
     assert _native.lib().tq1_linear_f16(bd.data_ptr(), xd.data_ptr(), y.data_ptr(), 1, batch, rows, columns, None, 0,
                                         torch.cuda.current_stream().cuda_stream) == 0
-    assert np.array_equal(y.cpu().numpy(), run_linear(blocks, x))
+    got = y.cpu().numpy()
+    assert np.array_equal(got, np.concatenate([run_linear(blocks, x[i:i + 8]) for i in range(0, batch, 8)]))
+    with_workspace = run_linear(blocks, x)
+    assert not np.array_equal(got, with_workspace)
+    assert np.linalg.norm(got - with_workspace) <= 2 * 2.3e-7 * np.linalg.norm(got)       # the forms' bounds
