@@ -193,7 +193,7 @@ groups_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
         // ------------------------------------------------------------------ MMAs: every second unit, and one of the two slots
         if (elect_one()) {
             const uint32_t slot = (uint32_t)(warp - kMmaWarp);
-            uint32_t i = 0, unit = 0;
+            uint32_t i = 0, unit = 0, last_bar = 0, last_phase = 0;
             for (int tile = cluster; tile < prm.tiles && !dead; tile += prm.clusters) {
                 const int m0 = token0(tile), units = units_of(m0);
                 for (int kb = 0; kb < blocks_k; ++kb, ++i, unit += (uint32_t)units) {
@@ -217,10 +217,13 @@ groups_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
                     umma_commit(bar(EMPTY + (int)stage));
                     if (units == 1) umma_commit(bar(EMPTY + (int)stage));
                     mbar_arrive(bar(ACC_FULL + (int)slot));
+                    last_bar = bar(EMPTY + (int)stage);
+                    last_phase = phase;
                 }
             }
-            // nothing of the tensor core arrives after this
-            if (i > 0) mbar_wait(bar(EMPTY + (int)((i - 1) % kRing)), (i - 1) / kRing & 1u, prm.status, dead);
+            // Nothing of this warp's commits arrives after the last of them, which this phase has to have. With one unit per
+            // block that is not the last block's: the warps take turns, and commits of different threads come in any order.
+            if (last_bar) mbar_wait(last_bar, last_phase, prm.status, dead);
         }
     } else if (warp < kDecodeWarps) {
         // ------------------------------------------------------------------ decode

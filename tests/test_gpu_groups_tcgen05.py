@@ -18,6 +18,7 @@ BOUND = (0.96 + 0.82 + 0.58) * 2.0 ** -24
 @pytest.mark.parametrize(("rows", "columns", "batch"), (
     (17408, 2688, 12), (17000, 1408, 16),               # one unit, of 16 tokens
     (17408, 1664, 17), (14000, 2688, 32),               # of 32, rows that fill no tile
+    (17408, 1408, 24), (38000, 1408, 24),               # one unit and an odd number of groups, in one tile and in three
     (4099, 2176, 33), (2000, 4224, 64),                 # two units, a cluster per tile
     (4099, 2176, 65), (9000, 640, 129), (13313, 384, 200)))        # several token tiles, more tiles than SMs, three groups
 @pytest.mark.parametrize("shift", (0, 4))
