@@ -18,6 +18,57 @@ EncodeTiledFn tq1::encode_tiled_fn() {
     return fn;
 }
 
+int tq1::device_slot() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+    return dev;
+}
+
+int tq1::sm_count() {
+    static std::atomic<int> count[kMaxDevices];
+    const int dev = device_slot();
+    int n = count[dev].load(std::memory_order_relaxed);
+    if (!n) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        count[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+cudaError_t tq1::opt_in(KernelRecord &record, const void *kernel, size_t smem) {
+    std::atomic<bool> &done = record.opted_in[device_slot()];
+    if (done.load(std::memory_order_acquire)) return cudaSuccess;
+    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err == cudaSuccess) done.store(true, std::memory_order_release);
+    return err;
+}
+
+int tq1::clusters_at_once(KernelRecord &record, const void *kernel, unsigned threads, size_t smem, int split_log) {
+    if (split_log == 0) return sm_count();
+    std::atomic<int> &known = record.clusters[device_slot()][split_log];
+    int n = known.load(std::memory_order_relaxed);
+    if (!n) {
+        const int split = 1 << split_log;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(sm_count() / split * split));
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = (unsigned)split;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        if (opt_in(record, kernel, smem) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();                                 // no device, say: planning only
+            const int of_b200[4] = {148, 74, 33, 15};
+            n = of_b200[split_log];
+        }
+        known.store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 // Bytes that a call of this shape uses.
 static size_t linear_scratch_bytes(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0 || K % kGroup) return 0;

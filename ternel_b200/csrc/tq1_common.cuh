@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/ternel_b200.h"
 
 namespace tq1 {
@@ -61,6 +63,21 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn encode_tiled_fn();
+
+// What launches keep per device: the SM count differs between devices, and the shared-memory opt-in is an attribute of a
+// function on one device. A record is filled by whoever comes first; threads that come together write the same.
+constexpr int kMaxDevices = 64;
+int device_slot();                                      // the current device's
+int sm_count();                                         // the current device's, 148 on a machine without one (planning)
+struct KernelRecord {
+    std::atomic<bool> opted_in[kMaxDevices];
+    std::atomic<int> clusters[kMaxDevices][4];          // of 1, 2, 4 and 8 CTAs that run at once
+};
+// The kernel may have `smem` bytes of dynamic shared memory.
+cudaError_t opt_in(KernelRecord &record, const void *kernel, size_t smem);
+// Clusters of 2^split_log CTAs of a kernel with one CTA per SM that run at the same time: fewer than SMs / CTAs where the SMs of
+// a GPC are no multiple of it (74, 33 and 15 on this part).
+int clusters_at_once(KernelRecord &record, const void *kernel, unsigned threads, size_t smem, int split_log);
 
 // With `dependent` a launch that may begin while the kernel before it in the stream ends (programmatic dependent launch): it
 // calls grid_dependency_wait() before it touches what an earlier one may have written or may still read, by plain loads: __ldg

@@ -771,24 +771,6 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
     }
 }
 
-// Launch state is per DEVICE: the SM count differs between devices and the shared-memory opt-in is an
-// attribute of a function on one device, so a process that drives several GPUs needs one record each.
-constexpr int kMaxDevices = 64;
-int current_device_slot() {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
-    return dev;
-}
-int sm_count_cached() {
-    static int sm_count[kMaxDevices] = {};
-    const int dev = current_device_slot();
-    if (!sm_count[dev]) {
-        if (cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count[dev] <= 0)
-            sm_count[dev] = 148;
-    }
-    return sm_count[dev];
-}
-
 // The token tile names the variant: 16 and 32 run as S, 64 and 128 as L, 256 as P.
 int tile_cg(int tile) { return tile > 128 ? 2 : 1; }
 
@@ -809,7 +791,7 @@ Tiling make_tiling(int tile, int M, int N, int K) {
     t.nt = (even + 16 * cg - 1) / (16 * cg) * (16 * cg);
     t.tiles_m = (M + t.nt - 1) / t.nt;
     const long long tiles = (long long)((N + kTileW * cg - 1) / (kTileW * cg)) * t.tiles_m;
-    const long long slots = (long long)sm_count_cached() * (tile <= 32 ? 2 : 1) / cg;
+    const long long slots = (long long)sm_count() * (tile <= 32 ? 2 : 1) / cg;
     WorkSplit &w = t.work;
     w.chunks = (K / kGroup + kChunkGroups - 1) / kChunkGroups;
     w.total_iters = (int)(tiles * w.chunks);
@@ -886,7 +868,7 @@ int token_tile(int M, int N, int K) {
         if (c.tile > 16 && c.tile >= 4 * M) continue;           // a tile mostly of padding
         const Tiling t = make_tiling(c.tile, M, N, K);
         // whole tiles on less than half of the chip: a narrower tile splits K over the rest, with shorter accumulators
-        if (c.tile == 256 && t.work.splits == 1 && 2 * t.ctas() <= sm_count_cached()) continue;
+        if (c.tile == 256 && t.work.splits == 1 && 2 * t.ctas() <= sm_count()) continue;
         const float cost = model_us(c, t);
         if (i == 0 || cost < best_cost) { best = c.tile; best_cost = cost; }
     }
@@ -901,13 +883,9 @@ int launch_variant(const CUtensorMap &wmap, const CUtensorMap &xmap, GemmParams 
     const int stages = (int)(V::kBRoom / ((uint32_t)prm.b_rows * 256u));
     prm.b_stages = stages < V::RING ? stages : V::RING;
     auto kern = tq1_gemm_kernel<V>;
-    static bool attr_set[kMaxDevices] = {};
-    const int dev = current_device_slot();
-    if (!attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)V::kSmemBytes);
-        if (e != cudaSuccess) return cuda_fail(e, "tq1_linear_f16: shared memory opt-in (GEMM)");
-        attr_set[dev] = true;
-    }
+    static KernelRecord record;
+    const cudaError_t e = opt_in(record, reinterpret_cast<const void *>(kern), V::kSmemBytes);
+    if (e != cudaSuccess) return cuda_fail(e, "tq1_linear_f16: shared memory opt-in (GEMM)");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(V::kThreads);
@@ -960,7 +938,7 @@ size_t gemm_tc_workspace_bytes(int M, int N, int K) {
 // 32 (two 16-token tiles), two 32-token tiles or one tile of the batch's length.
 size_t gemm_tc_workspace_bound(int M) {
     const int columns = M <= 16 ? 32 : M <= 64 ? 64 : M >= 256 ? 256 : (M + 31) / 32 * 32;
-    return kWsScratchOffset + align256((size_t)2 * sm_count_cached() * columns * kTileW * sizeof(float));
+    return kWsScratchOffset + align256((size_t)2 * sm_count() * columns * kTileW * sizeof(float));
 }
 
 int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K,

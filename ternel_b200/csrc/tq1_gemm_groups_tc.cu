@@ -35,7 +35,6 @@ constexpr int kTileW = 128, kUnit = 32, kUnits = 2, kTokens = kUnit * kUnits;
 constexpr int kRing = 4, kScaleRing = 8, kPackRing = 4;         // a scale outlives its ring stage by two K blocks at most
 constexpr int kDecodeWarps = 8, kSumWarps = 16, kMmaWarps = 2;
 constexpr int kMmaWarp = kDecodeWarps + kSumWarps, kXWarp = kMmaWarp + kMmaWarps, kThreads = 32 * (kXWarp + 1);
-constexpr int kMaxDevices = 64;
 constexpr uint32_t kPackBytes = 32 * kBlockBytes;               // a warp's rows of a K block
 constexpr uint32_t kWindow = 1024;                              // shared-window address of dynamic shared memory
 constexpr uint32_t kBarAddr = kWindow;
@@ -431,46 +430,9 @@ groups_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
 }
 
 // ---- host ---------------------------------------------------------------------------------------------------------
-int device_slot() {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
-    return dev;
-}
-
-cudaError_t opt_in() {
-    static bool done[kMaxDevices] = {};
-    const int dev = device_slot();
-    if (done[dev]) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(groups_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemEnd - kWindow));
-    if (e == cudaSuccess) done[dev] = true;
-    return e;
-}
-
-// Clusters of `split` CTAs that run at the same time.
-int clusters_at_once(int split) {
-    static int known[kMaxDevices][9] = {};
-    const int dev = device_slot();
-    if (!known[dev][split]) {
-        int n = 0, sms = 0;
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-        if (split > 1) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)(sms / split * split));
-            cfg.blockDim = dim3(kThreads);
-            cfg.dynamicSmemBytes = kSmemEnd - kWindow;
-            cudaLaunchAttribute attr;
-            attr.id = cudaLaunchAttributeClusterDimension;
-            attr.val.clusterDim.x = (unsigned)split;
-            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-            cfg.attrs = &attr;
-            cfg.numAttrs = 1;
-            if (opt_in() != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, groups_tc_kernel, &cfg) != cudaSuccess) n = 0;
-            cudaGetLastError();
-        }
-        known[dev][split] = n > 0 ? n : sms / split;
-    }
-    return known[dev][split];
-}
+KernelRecord g_record;
+const void *const kKernel = reinterpret_cast<const void *>(groups_tc_kernel);
+int clusters_at_once(int split_log) { return tq1::clusters_at_once(g_record, kKernel, kThreads, kSmemEnd - kWindow, split_log); }
 
 struct GroupPlan { int nt, tiles_m, tiles, clusters, split; float us; };
 
@@ -481,9 +443,10 @@ GroupPlan group_plan(int M, int N, int groups) {
     p.nt = ((M + p.tiles_m - 1) / p.tiles_m + 15) / 16 * 16;
     p.tiles_m = (M + p.nt - 1) / p.nt;
     p.tiles = (N + kTileW - 1) / kTileW * p.tiles_m;
-    p.split = 1;
-    while (p.split < 8 && p.tiles <= clusters_at_once(2 * p.split) && groups >= 8 * p.split) p.split *= 2;
-    const int room = clusters_at_once(p.split);
+    int split_log = 0;
+    while (split_log < 3 && p.tiles <= clusters_at_once(split_log + 1) && groups >= 8 << split_log) ++split_log;
+    p.split = 1 << split_log;
+    const int room = clusters_at_once(split_log);
     p.clusters = p.tiles < room ? p.tiles : room;
     const int blocks = (p.tiles + p.clusters - 1) / p.clusters * ((groups + p.split - 1) / p.split);
     p.us = p.nt <= kUnit ? 5.4f + 0.64f * (float)blocks : 6.5f + 1.13f * (float)blocks;
@@ -519,7 +482,7 @@ int launch_gemm_groups_tc(const uint8_t *blocks, const __half *x, void *y, bool 
                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (res != CUDA_SUCCESS) return fail(TQ1_ERR_CUDA, "tq1_linear_f16: activation tensor map failed (%d)", (int)res);
-    cudaError_t err = opt_in();
+    cudaError_t err = opt_in(g_record, kKernel, kSmemEnd - kWindow);
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: shared memory opt-in (group sums)");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(p.clusters * p.split));

@@ -43,7 +43,6 @@ namespace {
 constexpr int kTileRows = 16;
 constexpr int kChunkBytes = 4 * kBlockBytes;                    // a row's bytes of a 512-column chunk
 constexpr int kChain = 4;                                       // MMAs (of 16 columns) under one accumulator
-constexpr int kMaxDevices = 64;
 
 constexpr uint32_t kWindow = 1024;                              // shared-window address of dynamic shared memory
 constexpr uint32_t kTableAddr = kWindow;                        // 256 entries of 256 bytes
@@ -445,48 +444,9 @@ struct SlicePlan {
     uint32_t sums_addr, ring_addr, end;
 };
 
-int device_slot() {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
-    return dev;
-}
-int sm_count() {
-    static int count[kMaxDevices] = {};
-    const int dev = device_slot();
-    if (!count[dev]) {
-        int n = 0;
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        count[dev] = n;
-    }
-    return count[dev];
-}
-
-// Clusters of `split` CTAs that run at the same time: fewer than SMs / split where the SMs of a GPC are no multiple of it.
-template <int NT>
-int clusters_at_once(int split) {
-    static int known[kMaxDevices][9] = {};
-    const int dev = device_slot();
-    if (split == 1) return sm_count();
-    if (!known[dev][split]) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(sm_count() / split * split));
-        cfg.blockDim = dim3(32 * (kMaxSlices + kExtraWarps));
-        cfg.dynamicSmemBytes = kWindowEnd - kWindow;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = (unsigned)split;
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaFuncSetAttribute(slices_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kWindowEnd - kWindow)) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, slices_kernel<NT>, &cfg) != cudaSuccess || n < 1) {
-            cudaGetLastError();                                 // no device, say: planning only
-            n = sm_count() / split;
-        }
-        known[dev][split] = n;
-    }
-    return known[dev][split];
+KernelRecord g_records[2];                                      // of slices_kernel<1> and <2>
+const void *kernel_of(int nt) {
+    return nt == 1 ? reinterpret_cast<const void *>(slices_kernel<1>) : reinterpret_cast<const void *>(slices_kernel<2>);
 }
 
 // Modelled time (us, fitted to graph replays with weights out of HBM): what the SM works through (0.128 per row tile and chunk of
@@ -502,14 +462,15 @@ float slice_us(int split, int slices, int per_cluster) {
 SlicePlan slice_plan(int nt, int N, int K) {
     SlicePlan best = {};
     const int per = slice_halves(nt), halves = K / 256 / per, tiles = (N + kTileRows - 1) / kTileRows;
-    for (int split = 1; split <= 8; split *= 2) {
+    for (int log = 0; log <= 3; ++log) {
+        const int split = 1 << log;
         SlicePlan p = {};
         p.split = split;
         p.slices = (halves + split - 1) / split;
         if (halves < split || p.slices > kMaxSlices) continue;
         // how many clusters run at once is asked of the driver (milliseconds, the first time) only where this split could win
         if (best.ok && slice_us(split, p.slices, (tiles + sm_count() / split - 1) / (sm_count() / split)) >= best.us) continue;
-        const int room = nt == 1 ? clusters_at_once<1>(split) : clusters_at_once<2>(split);
+        const int room = clusters_at_once(g_records[nt - 1], kernel_of(nt), 32 * (kMaxSlices + kExtraWarps), kWindowEnd - kWindow, log);
         p.clusters = tiles < room ? tiles : room;
         const int per_cluster = (tiles + p.clusters - 1) / p.clusters;
         p.subsets = kMaxSlices / p.slices;
@@ -540,13 +501,8 @@ SlicePlan slice_plan(int nt, int N, int K) {
 template <int NT>
 int launch_slices(const CUtensorMap &wmap, const CUtensorMap &xmap, const SliceParams &prm, const SlicePlan &p, cudaStream_t stream) {
     auto kern = slices_kernel<NT>;
-    static bool attr_set[kMaxDevices] = {};
-    const int dev = device_slot();
-    if (!attr_set[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kWindowEnd - kWindow));
-        if (e != cudaSuccess) return cuda_fail(e, "tq1_linear_f16: shared memory opt-in (slices)");
-        attr_set[dev] = true;
-    }
+    const cudaError_t e = opt_in(g_records[NT - 1], kernel_of(NT), kWindowEnd - kWindow);
+    if (e != cudaSuccess) return cuda_fail(e, "tq1_linear_f16: shared memory opt-in (slices)");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(p.clusters * p.split));
     cfg.blockDim = dim3((unsigned)(32 * (p.slices * p.subsets + kExtraWarps)));

@@ -962,7 +962,6 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
 }
 
 // Per-device launch state: the shared-memory opt-in is an attribute of the function on ONE device.
-constexpr int kMaxDevices = 64;
 struct DeviceState {
     int sm_count;
     bool attr_set;
