@@ -69,6 +69,41 @@ int tq1::clusters_at_once(KernelRecord &record, const void *kernel, unsigned thr
     return n;
 }
 
+namespace {
+
+struct GraphTail { unsigned long long capture; cudaGraphNode_t node; };
+// The last kernel of this library that this thread has captured: in which capture, which node.
+thread_local GraphTail t_own = {};
+
+// Whether the stream is being captured; `tail` is the node that the next one will depend on, if there is one such.
+bool capturing(cudaStream_t stream, GraphTail *tail) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    *tail = {};
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+        cudaGetLastError();                                     // the launch will say so
+        return false;
+    }
+    if (status != cudaStreamCaptureStatusActive) return false;
+    const cudaGraphNode_t *nodes = nullptr;
+    const cudaGraphEdgeData *edges = nullptr;
+    size_t n = 0;
+    if (cudaStreamGetCaptureInfo_v3(stream, &status, &tail->capture, nullptr, &nodes, &edges, &n) != cudaSuccess) cudaGetLastError();
+    else if (n == 1) tail->node = nodes[0];
+    return true;
+}
+
+}  // namespace
+
+bool tq1::behind_own_kernel(cudaStream_t stream) {
+    GraphTail tail;
+    return !capturing(stream, &tail) || (tail.node && tail.capture == t_own.capture && tail.node == t_own.node);
+}
+
+void tq1::note_kernel(cudaStream_t stream) {
+    GraphTail tail;
+    if (capturing(stream, &tail)) t_own = tail;
+}
+
 // Bytes that a call of this shape uses.
 static size_t linear_scratch_bytes(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0 || K % kGroup) return 0;

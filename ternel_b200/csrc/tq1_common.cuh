@@ -79,13 +79,22 @@ cudaError_t opt_in(KernelRecord &record, const void *kernel, size_t smem);
 // a GPC are no multiple of it (74, 33 and 15 on this part).
 int clusters_at_once(KernelRecord &record, const void *kernel, unsigned threads, size_t smem, int split_log);
 
-// With `dependent` a launch that may begin while the kernel before it in the stream ends (programmatic dependent launch): it
-// calls grid_dependency_wait() before it touches what an earlier one may have written or may still read, by plain loads: __ldg
-// and __restrict__ tell the compiler that the data were there from the kernel's beginning. Calls back to back: a gather of 2048
-// rows of 5120 columns 8.2 -> 5.7 us, five tokens of 4099x2176 7.2 -> 6.1.
+// A launch may begin while the kernel before it in the stream ends (programmatic dependent launch): that kernel lets it in
+// (allow_next_grid), and it calls grid_dependency_wait() before it touches what an earlier one may have written or may still
+// read, by plain loads: __ldg and __restrict__ tell the compiler that the data were there from the kernel's beginning. Calls back
+// to back: a gather of 2048 rows of 5120 columns 8.2 -> 5.7 us, five tokens of 4099x2176 7.2 -> 6.1.
+//
+// Not in a graph behind a kernel that is not this library's and lets nothing in: there the edge alone costs some 0.3 us and up
+// to 0.7 (512 rows gathered 3.1 us as an ordinary launch, 3.4 as a dependent one; five tokens of 4099x2176 6.3 and 6.9). Outside
+// a graph such a launch gains all the same: the launch itself is brought forward (the gather 4.1 -> 3.1).
+bool behind_own_kernel(cudaStream_t stream);            // false: the stream is being captured, and the last node is another's
+void note_kernel(cudaStream_t stream);                  // a kernel of this library that lets the next one in has been launched
+
+// `dependent` where overlapping is asked for and pays, else `plain`, its form for an ordinary launch.
 template <class... P, class... A>
-cudaError_t launch_dependent(bool dependent, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
-                             A... args) {
+cudaError_t launch_either(bool overlap, void (*dependent)(P...), void (*plain)(P...), dim3 grid, unsigned threads, size_t smem,
+                          cudaStream_t stream, A... args) {
+    overlap = overlap && behind_own_kernel(stream);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
@@ -95,9 +104,12 @@ cudaError_t launch_dependent(bool dependent, void (*kernel)(P...), dim3 grid, un
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = dependent ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, overlap ? dependent : plain, static_cast<P>(args)...);
 }
+// Read-only data, in a kernel of either form.
+template <bool DEPENDENT, class T>
+__device__ __forceinline__ T load_input(const T *p) { return DEPENDENT ? *p : __ldg(p); }
 // The next kernel may be launched where there is room for it (its CTAs then wait beside this kernel's).
 __device__ __forceinline__ void allow_next_grid() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Everything before this kernel has ended and its results are there.

@@ -43,15 +43,12 @@ constexpr int kTokensPerThread = 4;
 
 }  // namespace
 
-// A dependent launch reads by plain loads.
-template <bool PLAIN>
-__device__ __forceinline__ uint32_t load_byte(const uint8_t *p) { return PLAIN ? *p : __ldg(p); }
-
 // SHARED: a CTA first copies the table to shared memory, which the few CTAs of a short call gain from; in a long one the
-// barrier behind the copy costs more than lookups through L1 (launch_embedding has the line and the figures). A short call is
-// also a dependent launch; a long one gains nothing from that and loses from the plain loads (8192 tokens, FP32: 38.7 us, 42.7
-// with both).
-template <bool OUT_F32, bool SHARED>
+// barrier behind the copy costs more than lookups through L1 (launch_embedding has the line and the figures).
+// DEPENDENT: the form for a programmatic dependent launch, of a short call: a long one gains nothing from that and loses from
+// the plain loads (8192 tokens, FP32: 38.7 us, 42.7 with both). The ordinary form asks for the ids before the table, whose copy
+// the dependent one has done by the time that the kernel before it ends.
+template <bool OUT_F32, bool SHARED, bool DEPENDENT>
 __global__ void __launch_bounds__(kThreadsPerBlockRow * kBlocksPerCta)
 embedding_kernel(const uint8_t *blocks, const int64_t *ids, void *out,
                  int64_t T, int64_t V, int gpr) {
@@ -69,24 +66,31 @@ embedding_kernel(const uint8_t *blocks, const int64_t *ids, void *out,
     // that follows it for one token only keeps too few bytes in flight to fill the memory system.
     int64_t id[kTokensPerThread];
     bool live[kTokensPerThread];
+    auto load_ids = [&] {
+#pragma unroll
+        for (int q = 0; q < kTokensPerThread; ++q)
+            id[q] = in_row && t0 + q < T ? load_input<DEPENDENT>(reinterpret_cast<const long long *>(ids) + t0 + q) : -1;
+    };
+    if (!DEPENDENT) load_ids();
     if (SHARED) {
 #pragma unroll
         for (int i = 0; i < 256; i += kThreadsPerBlockRow * kBlocksPerCta)
             shared_trits[i + threadIdx.x] = g_trits.e[i + threadIdx.x];
     }
-    if (SHARED) grid_dependency_wait();
-#pragma unroll
-    for (int q = 0; q < kTokensPerThread; ++q) id[q] = in_row && t0 + q < T ? ids[t0 + q] : -1;
+    if (DEPENDENT) {
+        grid_dependency_wait();
+        load_ids();
+    }
     const uint8_t *blk[kTokensPerThread];
     uint32_t sbits[kTokensPerThread], b0[kTokensPerThread], b1[kTokensPerThread], b2[kTokensPerThread];
 #pragma unroll
     for (int q = 0; q < kTokensPerThread; ++q) {
         live[q] = id[q] >= 0 && id[q] < V;
         blk[q] = blocks + (size_t)((unsigned)(live[q] ? id[q] : 0) * (unsigned)gpr + (unsigned)(in_row ? g : 0)) * kBlockBytes;
-        sbits[q] = *reinterpret_cast<const unsigned short *>(blk[q]);
-        b0[q] = load_byte<SHARED>(blk[q] + 2 + a);
-        b1[q] = load_byte<SHARED>(blk[q] + 3 + a);
-        b2[q] = off >= 3 ? load_byte<SHARED>(blk[q] + 4 + a) : 0u;      // the third byte exists whenever it is needed
+        sbits[q] = load_input<DEPENDENT>(reinterpret_cast<const unsigned short *>(blk[q]));
+        b0[q] = load_input<DEPENDENT>(blk[q] + 2 + a);
+        b1[q] = load_input<DEPENDENT>(blk[q] + 3 + a);
+        b2[q] = off >= 3 ? load_input<DEPENDENT>(blk[q] + 4 + a) : 0u;  // the third byte exists whenever it is needed
     }
     if (SHARED) {
         __syncthreads();
@@ -154,11 +158,13 @@ int launch_embedding(const uint8_t *blocks, const int64_t *ids, void *out, bool 
         const bool shared = (long long)grid.x * grid.y <= kSharedTableCtas;
         void *first = out_f32 ? static_cast<void *>(static_cast<float *>(out) + t0 * K)
                               : static_cast<void *>(static_cast<__half *>(out) + t0 * K);
-        auto kernel = out_f32 ? (shared ? embedding_kernel<true, true> : embedding_kernel<true, false>)
-                              : (shared ? embedding_kernel<false, true> : embedding_kernel<false, false>);
-        const cudaError_t err = launch_dependent(shared, kernel, grid, kThreadsPerBlockRow * kBlocksPerCta, 0, stream, blocks, ids + t0,
-                                                 first, n, V, gpr);
+        auto dependent = out_f32 ? embedding_kernel<true, true, true> : embedding_kernel<false, true, true>;
+        auto plain = out_f32 ? (shared ? embedding_kernel<true, true, false> : embedding_kernel<true, false, false>)
+                             : (shared ? embedding_kernel<false, true, false> : embedding_kernel<false, false, false>);
+        const cudaError_t err = launch_either(shared, dependent, plain, grid, kThreadsPerBlockRow * kBlocksPerCta, 0, stream, blocks,
+                                              ids + t0, first, n, V, gpr);
         if (err != cudaSuccess) return cuda_fail(err, "tq1_embedding_f16: launch");
+        if (shared) note_kernel(stream);
     }
     return TQ1_OK;
 }

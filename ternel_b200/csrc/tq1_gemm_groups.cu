@@ -79,10 +79,10 @@ __device__ __forceinline__ void store_result(void *y, int y_f32, size_t o, size_
     else static_cast<__half *>(y)[o] = __float2half_rn(v);
 }
 
-// NT: token tiles of eight per CTA.
+// NT: token tiles of eight per CTA; DEPENDENT: the form for a programmatic dependent launch.
 constexpr int kFewWarps = 8, kFewRows = 16;
 
-template <int NT>
+template <int NT, bool DEPENDENT>
 __global__ void __launch_bounds__(kFewWarps * 32)
 groups_few_kernel(const uint8_t *blocks, const __half *x, void *y, int y_f32,
                   int M, int N, int groups) {
@@ -117,9 +117,10 @@ groups_few_kernel(const uint8_t *blocks, const __half *x, void *y, int y_f32,
     uint32_t next[kPerLane];
     auto load = [&](int grp) {
 #pragma unroll
-        for (int j = 0; j < kPerLane; ++j) next[j] = grp < groups ? src[j][(size_t)grp * kGroupRowWords] : 0u;
+        for (int j = 0; j < kPerLane; ++j)
+            next[j] = grp < groups ? load_input<DEPENDENT>(src[j] + (size_t)grp * kGroupRowWords) : 0u;
     };
-    grid_dependency_wait();
+    if (DEPENDENT) grid_dependency_wait();
     load(warp);
     __syncthreads();
     uint32_t *mine = packed[warp];
@@ -141,7 +142,7 @@ groups_few_kernel(const uint8_t *blocks, const __half *x, void *y, int y_f32,
         for (int s = 0; s < 4; ++s)
 #pragma unroll
             for (int t = 0; t < NT; ++t)
-                xv[s][t] = live[t] ? *reinterpret_cast<const uint4 *>(xrow[t] + (size_t)grp * kGroup + 32 * s)
+                xv[s][t] = live[t] ? load_input<DEPENDENT>(reinterpret_cast<const uint4 *>(xrow[t] + (size_t)grp * kGroup + 32 * s))
                                    : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
@@ -193,7 +194,7 @@ constexpr size_t many_smem(int nt) {
     return (size_t)kManyStages * 8 * nt * kGroup * 2 + kManyWarps * 16 * kBlockBytes + 1024;
 }
 
-template <int NT>
+template <int NT, bool DEPENDENT>
 __global__ void __launch_bounds__(kManyWarps * 32, NT == 8 ? 1 : 2)
 groups_many_kernel(const uint8_t *blocks, const __half *x, void *y, int y_f32,
                    int M, int N, int groups) {
@@ -232,9 +233,10 @@ groups_many_kernel(const uint8_t *blocks, const __half *x, void *y, int y_f32,
     uint32_t next[kPerLane];
     auto load = [&](int grp) {
 #pragma unroll
-        for (int j = 0; j < kPerLane; ++j) next[j] = grp < groups ? src[j][(size_t)grp * kGroupRowWords] : 0u;
+        for (int j = 0; j < kPerLane; ++j)
+            next[j] = grp < groups ? load_input<DEPENDENT>(src[j] + (size_t)grp * kGroupRowWords) : 0u;
     };
-    grid_dependency_wait();
+    if (DEPENDENT) grid_dependency_wait();
     load(0);
     request(0);
     request(1);
@@ -312,21 +314,27 @@ int launch_few(const uint8_t *blocks, const __half *x, void *y, int y_f32, int M
     const long long ctas = (long long)((N + kFewRows - 1) / kFewRows) * ((M + 8 * NT - 1) / (8 * NT));
     // around one CTA an SM, a call whose first CTAs find places beside the last of the one before takes two places on some SMs
     // (120 CTAs: 8.7 us alone, 10.1 as a dependent launch; 24 of them 5.9 and 5.3, 257 of them 6.0 and 5.3)
-    const bool dependent = ctas <= 74 || ctas > 148;
-    const cudaError_t err = launch_dependent(dependent, groups_few_kernel<NT>, dim3((unsigned)ctas), kFewWarps * 32, 0, stream, blocks, x, y,
-                                             y_f32, M, N, groups);
-    return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: launch");
+    const bool overlap = ctas <= sm_count() / 2 || ctas > sm_count();
+    const cudaError_t err = launch_either(overlap, groups_few_kernel<NT, true>, groups_few_kernel<NT, false>, dim3((unsigned)ctas),
+                                          kFewWarps * 32, 0, stream, blocks, x, y, y_f32, M, N, groups);
+    if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: launch");
+    note_kernel(stream);
+    return TQ1_OK;
 }
 
 template <int NT>
 int launch_many(const uint8_t *blocks, const __half *x, void *y, int y_f32, int M, int N, int groups, cudaStream_t stream) {
     const long long ctas = (long long)((N + kManyRows - 1) / kManyRows) * ((M + 8 * NT - 1) / (8 * NT));
-    cudaError_t err = cudaFuncSetAttribute(groups_many_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)many_smem(NT));
+    cudaError_t err = cudaSuccess;
+    for (auto kernel : {groups_many_kernel<NT, true>, groups_many_kernel<NT, false>})
+        if (err == cudaSuccess)
+            err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)many_smem(NT));
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: shared memory opt-in");
-    err = launch_dependent(true, groups_many_kernel<NT>, dim3((unsigned)ctas), kManyWarps * 32, many_smem(NT), stream, blocks, x, y, y_f32,
-                           M, N, groups);
-    return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: launch");
+    err = launch_either(true, groups_many_kernel<NT, true>, groups_many_kernel<NT, false>, dim3((unsigned)ctas), kManyWarps * 32,
+                        many_smem(NT), stream, blocks, x, y, y_f32, M, N, groups);
+    if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: launch");
+    note_kernel(stream);
+    return TQ1_OK;
 }
 
 }  // namespace

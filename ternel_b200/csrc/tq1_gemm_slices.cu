@@ -509,14 +509,15 @@ int launch_slices(const CUtensorMap &wmap, const CUtensorMap &xmap, const SliceP
     cfg.dynamicSmemBytes = p.end - kWindow;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = (unsigned)p.split;
-    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)p.split;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = p.split > 1 ? 2 : 1;
+    cfg.numAttrs = behind_own_kernel(stream) ? 2 : 1;
     const cudaError_t err = cudaLaunchKernelEx(&cfg, kern, wmap, xmap, prm);
+    if (err == cudaSuccess) note_kernel(stream);
     return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: launch (slices)");
 }
 

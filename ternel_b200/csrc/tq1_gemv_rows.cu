@@ -29,7 +29,7 @@ __device__ __forceinline__ float dot_byte(uint32_t entry, const float *x, int n,
     return sum;
 }
 
-template <int MB, bool OUT_F32>
+template <int MB, bool OUT_F32, bool DEPENDENT>
 __global__ void __launch_bounds__(kRowsThreads) gemv_rows_kernel(const uint8_t *blocks, const __half *x, void *y, int N, int K, int ldy) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint16_t *lut = reinterpret_cast<uint16_t *>(smem_raw);          // 256 entries
@@ -37,8 +37,9 @@ __global__ void __launch_bounds__(kRowsThreads) gemv_rows_kernel(const uint8_t *
 
     for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = (uint16_t)trits_2bit(i);
     allow_next_grid();                                  // early: 82 us for 17408x5248, 92 after the loop
-    grid_dependency_wait();
-    for (int i = threadIdx.x; i < MB * K; i += blockDim.x) xs[i] = __half2float(x[i]);
+    if (DEPENDENT) grid_dependency_wait();
+    for (int i = threadIdx.x; i < MB * K; i += blockDim.x)
+        xs[i] = __half2float(__ushort_as_half(load_input<DEPENDENT>(reinterpret_cast<const unsigned short *>(x) + i)));
     __syncthreads();
 
     const int lane = threadIdx.x & 31;
@@ -57,7 +58,7 @@ __global__ void __launch_bounds__(kRowsThreads) gemv_rows_kernel(const uint8_t *
         for (int g0 = 0; g0 < gpr; g0 += 4) {
             const int g = g0 + sub;
             const bool live = g < gpr && pos < kBlockWords;
-            const uint32_t w = live ? words[g * kBlockWords + pos] : 0u;
+            const uint32_t w = live ? load_input<DEPENDENT>(words + g * kBlockWords + pos) : 0u;
             float sum[MB];
 #pragma unroll
             for (int m = 0; m < MB; ++m) sum[m] = 0.0f;
@@ -109,16 +110,19 @@ static int launch_mb(const uint8_t *blocks, const __half *x, void *y, bool y_f32
     if (smem > 227 * 1024)
         return fail(TQ1_ERR_INVALID, "tq1_linear_f16: K=%d too large for the row kernel's shared memory", K);
     int ctas = (N + 7) / 8;
-    if (ctas > 148 * 2) ctas = 148 * 2;
-    auto kern_h = gemv_rows_kernel<MB, false>;
-    auto kern_f = gemv_rows_kernel<MB, true>;
-    cudaError_t err = cudaFuncSetAttribute(y_f32 ? kern_f : kern_h,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (ctas > 2 * sm_count()) ctas = 2 * sm_count();
+    auto dependent = y_f32 ? gemv_rows_kernel<MB, true, true> : gemv_rows_kernel<MB, false, true>;
+    auto plain = y_f32 ? gemv_rows_kernel<MB, true, false> : gemv_rows_kernel<MB, false, false>;
+    cudaError_t err = cudaSuccess;
+    for (auto kernel : {dependent, plain})
+        if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: shared memory opt-in");
     // as in tq1_gemm_groups.cu: around one CTA an SM the next call's CTAs would double up (125 CTAs: 4.4 us, 8.0 as an early
     // dependent launch)
-    err = launch_dependent(ctas <= 74 || ctas > 148, y_f32 ? kern_f : kern_h, dim3((unsigned)ctas), kRowsThreads, smem, stream, blocks, x, y, N, K, N);
+    const bool overlap = ctas <= sm_count() / 2 || ctas > sm_count();
+    err = launch_either(overlap, dependent, plain, dim3((unsigned)ctas), kRowsThreads, smem, stream, blocks, x, y, N, K, N);
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: launch");
+    note_kernel(stream);
     return TQ1_OK;
 }
 

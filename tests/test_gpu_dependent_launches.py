@@ -40,3 +40,77 @@ def test_a_chain_of_calls_equals_one_call_at_a_time(batch, columns):
     assert len(torch.unique(want)) > 1
     for _ in range(5):
         assert torch.equal(run(False), want)
+
+
+def test_a_captured_call_depends_fully_on_another_library_s_kernel():
+    """In a graph a programmatic edge pays behind a kernel that lets the next one in. Behind any other kernel it costs time: a
+    call there is an ordinary node, whichever stream and capture came before."""
+    import ctypes
+    from ternel_b200.ops import tq1_get_rows, tq1_matmul
+    table, weight, ragged = (to_dev(random_blocks(n, k, seed=n)[0]) for n, k in ((500, 1024), (1024, 1024), (500, 640)))
+    ids, x, other = torch.arange(16, device="cuda"), torch.ones((8, 1024), device="cuda").half(), torch.zeros(32, device="cuda")
+    short = x[:, :640].contiguous()
+    # gather, slice kernel, group sums of few rows, row kernel
+    calls = (lambda: tq1_get_rows(table, ids), lambda: tq1_matmul(weight, x), lambda: tq1_matmul(ragged, short),
+             lambda: tq1_matmul(ragged, short[:1]))
+    cudart = ctypes.CDLL("libcudart.so.12")
+
+    def edges(run):
+        """Programmatic edges and all edges of the graph that `run` is captured as."""
+        run()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            run()
+        raw, count = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(0)
+        assert cudart.cudaGraphGetEdges_v2(raw, None, None, None, ctypes.byref(count)) == 0
+        nodes, data = (ctypes.c_void_p * (2 * count.value))(), (ctypes.c_uint8 * (8 * count.value))()
+        assert cudart.cudaGraphGetEdges_v2(raw, nodes, ctypes.byref(nodes, 8 * count.value), data, ctypes.byref(count)) == 0
+        return sum(data[8 * i + 2] != 0 for i in range(count.value)), count.value       # .type: 0 is a full dependency
+
+    for call in calls:
+        def apart():
+            for _ in range(4):
+                other.add_(1)
+                call()
+
+        def in_a_row():
+            other.add_(1)
+            for _ in range(4):
+                call()
+
+        assert edges(apart)[0] == 0
+        assert edges(in_a_row) == (3, 4)
+        assert edges(apart)[0] == 0
+
+
+@pytest.mark.parametrize("tokens", (1, 3, 2049))
+def test_gathers_of_both_forms_are_the_same(tokens):
+    """The first gather of a graph is an ordinary launch, the ones behind it are dependent ones."""
+    from ternel_b200.ops import tq1_get_rows
+    table = to_dev(random_blocks(3000, 640, seed=8)[0])
+    ids = torch.randint(-5, 3005, (tokens,), device="cuda")
+    for dtype in (torch.float16, torch.float32):
+        want = tq1_get_rows(table, ids, dtype=dtype)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = [tq1_get_rows(table, ids, dtype=dtype) for _ in range(3)]
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(g, want) for g in got)
+
+
+@pytest.mark.parametrize(("batch", "rows", "columns"), ((1, 300, 640), (5, 4099, 640), (16, 2400, 1408), (32, 4800, 640), (64, 9600, 640)))
+def test_products_of_both_forms_are_the_same(batch, rows, columns):
+    from ternel_b200.ops import tq1_matmul
+    blocks, rng = random_blocks(rows, columns, seed=batch)
+    w, x = to_dev(blocks), to_dev(rng.standard_normal((batch, columns)).astype(np.float16))
+    want = tq1_matmul(w, x, out_dtype=torch.float32)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = [tq1_matmul(w, x, out_dtype=torch.float32) for _ in range(3)]
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(g, want) for g in got)
