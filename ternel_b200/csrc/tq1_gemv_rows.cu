@@ -117,9 +117,12 @@ static int launch_mb(const uint8_t *blocks, const __half *x, void *y, bool y_f32
     for (auto kernel : {dependent, plain})
         if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: shared memory opt-in");
-    // as in tq1_gemm_groups.cu: around one CTA an SM the next call's CTAs would double up (125 CTAs: 4.4 us, 8.0 as an early
-    // dependent launch)
-    const bool overlap = ctas <= sm_count() / 2 || ctas > sm_count();
+    // The calls that follow are let in at once and fill the SMs up, so they have to come in whole grids: as many CTAs on every SM.
+    // Two an SM, and room for an even number of them (eight by their threads), or so few that each has an SM to itself. Otherwise
+    // some SMs have two CTAs of a call and others none: calls in a row, us, as ordinary launches / as dependent ones: 125 CTAs of
+    // 1408 columns 4.4 / 8.0, 256 of 2176 7.1 / 13.1, 296 of 9856 (five an SM) 46 / 70; 296 of 640 4.9 / 4.5, of 5248 26 / 25.
+    const int sms = sm_count(), room = (int)(228 * 1024 / (smem + 1024)), per_sm = room < 8 ? room : 8;
+    const bool overlap = ctas <= sms / 2 || (ctas == 2 * sms && per_sm % 2 == 0);
     err = launch_either(overlap, dependent, plain, dim3((unsigned)ctas), kRowsThreads, smem, stream, blocks, x, y, N, K, N);
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: launch");
     note_kernel(stream);
