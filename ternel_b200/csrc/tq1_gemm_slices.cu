@@ -62,13 +62,16 @@ constexpr int kMaxStages = 24;
 constexpr int kMaxSlices = 11;
 __host__ __device__ constexpr int slice_halves(int nt) { return nt == 1 ? 2 : 1; }          // 64 registers of activations
 constexpr int kExtraWarps = 1;
+// Fewer warps than this would be long at filling the table (two of them: 1.1 us more than six; 8 tokens of 2048x512 6.5 us apart
+// from other calls, 5.4 with six, 5.2 with nine). Six leave half of the registers to the next call's CTAs: in a row 3.8, 3.1 and 3.9.
+constexpr int kFillWarps = 6;
 
 struct SliceParams {
     void *y;
     unsigned *status;
     int M, N, chunks;
     int tiles, clusters;                                        // row tiles, clusters of the grid
-    int split_log, slices, subsets;                             // the grid's clusters have 2^split_log CTAs
+    int split_log, slices, subsets, workers;                    // the grid's clusters have 2^split_log CTAs; workers: slices * subsets
     int stages, pitch;                                          // ring stages, bytes from row to row
     int x_bufs;                                                 // 4 KiB pieces of activations that a slice has room for at a time
     uint32_t sums_addr, ring_addr;
@@ -224,7 +227,7 @@ slices_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         return;
     }
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const int threads = blockDim.x, warps = threads >> 5, workers = warps - kExtraWarps;
+    const int warps = blockDim.x >> 5, workers = prm.workers;
     const int split_log = prm.split_log, split = 1 << split_log, rank = blockIdx.x & (split - 1), cluster = blockIdx.x >> split_log;
     // this CTA's slices and row tiles
     const int all = 2 * prm.chunks / HS, slice_lo = all * rank >> split_log, n_slices = (all * (rank + 1) >> split_log) - slice_lo;
@@ -287,7 +290,7 @@ slices_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             }
         }
         __syncwarp();
-    } else {
+    } else if (warp < workers) {
         // ------------------------------------------------------------------ decode and multiply
         const int subset = warp / prm.slices, slice = warp - subset * prm.slices, g = lane >> 2, q = lane & 3;
         const int half0 = (slice_lo + slice) * HS, chunk = half0 >> 1;
@@ -505,7 +508,8 @@ int launch_slices(const CUtensorMap &wmap, const CUtensorMap &xmap, const SliceP
     if (e != cudaSuccess) return cuda_fail(e, "tq1_linear_f16: shared memory opt-in (slices)");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(p.clusters * p.split));
-    cfg.blockDim = dim3((unsigned)(32 * (p.slices * p.subsets + kExtraWarps)));
+    const int warps = prm.workers + kExtraWarps;
+    cfg.blockDim = dim3((unsigned)(32 * (warps > kFillWarps ? warps : kFillWarps)));
     cfg.dynamicSmemBytes = p.end - kWindow;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -545,6 +549,7 @@ int launch_gemm_slices(const uint8_t *blocks, const __half *x, void *y, bool y_f
     prm.split_log = p.split == 1 ? 0 : p.split == 2 ? 1 : p.split == 4 ? 2 : 3;
     prm.slices = p.slices;
     prm.subsets = p.subsets;
+    prm.workers = p.slices * p.subsets;
     prm.stages = p.stages;
     prm.pitch = p.pitch;
     prm.x_bufs = p.x_bufs;
