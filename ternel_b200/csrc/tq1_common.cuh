@@ -177,7 +177,7 @@ __host__ __device__ inline float swiglu_f32(float gate, float up) { return gate 
 void gemm_tc_plan(int M, int N, int K, int *tile, int *ctas, int *parts);
 int gemm_tc_force_tile(int nt);
 bool gemm_tc_forced();
-float gemm_tc_model_us(int M, int N, int K);                // modelled time of the tile that the kernel takes
+float gemm_tc_few_us(int N, int K);                         // modelled time of a call of up to 16 rows
 
 // Batched linear of 3 to 16 rows on mma.sync; needs K % 512 == 0 and 16-byte aligned pointers.
 bool gemm_slices_preferred(int M, int N, int K);            // fits, and faster than the tcgen05 kernel

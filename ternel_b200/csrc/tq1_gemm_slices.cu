@@ -452,9 +452,9 @@ const void *kernel_of(int nt) {
     return nt == 1 ? reinterpret_cast<const void *>(slices_kernel<1>) : reinterpret_cast<const void *>(slices_kernel<2>);
 }
 
-// Modelled time (us, fitted to graph replays with weights out of HBM): what the SM works through (0.128 per row tile and chunk of
-// eight tokens, twice that for sixteen), or where there are few warps what one of them does one tile after the other, behind
-// launch, table and activations; a cluster's barriers and its exchange on top.
+// Modelled time (us) by which a K split is chosen: what the SM works through (0.128 per row tile and chunk of eight tokens, twice
+// that for sixteen), or where there are few warps what one of them does one tile after the other, behind launch, table and
+// activations; a cluster's barriers and its exchange on top.
 float slice_us(int split, int slices, int per_cluster) {
     const int subsets = kMaxSlices / slices < per_cluster ? kMaxSlices / slices : per_cluster;
     const float sm = 0.128f * (float)(per_cluster * slices), chain = 0.7f * (float)((per_cluster + subsets - 1) / subsets);
@@ -501,6 +501,19 @@ SlicePlan slice_plan(int nt, int N, int K) {
     return best;
 }
 
+// Modelled time (us) of a call behind another kernel, which this kernel has to beat the tcgen05 kernel at too: it gains 2 us from
+// a call of this library before it, that one 1. Fitted to 1022 calls, weights out of HBM, within 6% (2-norm): launch, table and
+// activations, a cluster's exchange, the turns of the sets of warps and the row tiles that go through a CTA. Of these calls the
+// kernel that is chosen is within 2% of the better one, both in a row and apart, for all but 32, and never 9% behind in either
+// (beyond eight tokens the line lies where it would lose as much to leave this kernel, 20% in a row, as to take it).
+float call_us(const SlicePlan &p, int nt, int tiles) {
+    const int per = (tiles + p.clusters - 1) / p.clusters, turns = (per + p.subsets - 1) / p.subsets;
+    const float exchange = p.split == 1 ? 0.0f : p.split == 2 ? (nt == 1 ? 1.58f : 1.82f)
+                         : p.split == 4 ? (nt == 1 ? 0.93f : 1.29f) : (nt == 1 ? 0.58f : 0.93f);
+    return nt == 1 ? 4.47f + exchange + 0.329f * (float)turns + (float)per * (0.153f + 0.104f * (float)p.slices)
+                   : 4.47f + exchange + 0.624f * (float)turns + (float)per * (0.231f + 0.043f * (float)p.slices);
+}
+
 template <int NT>
 int launch_slices(const CUtensorMap &wmap, const CUtensorMap &xmap, const SliceParams &prm, const SlicePlan &p, cudaStream_t stream) {
     auto kern = slices_kernel<NT>;
@@ -529,8 +542,9 @@ int launch_slices(const CUtensorMap &wmap, const CUtensorMap &xmap, const SliceP
 
 bool gemm_slices_preferred(int M, int N, int K) {
     if (M < 3 || M > 16 || K % 512 || gemm_tc_forced()) return false;
-    const SlicePlan p = slice_plan(M <= 8 ? 1 : 2, N, K);
-    return p.ok && p.us < gemm_tc_model_us(M, N, K);
+    const int nt = M <= 8 ? 1 : 2;
+    const SlicePlan p = slice_plan(nt, N, K);
+    return p.ok && call_us(p, nt, (N + kTileRows - 1) / kTileRows) < (nt == 1 ? 1.0f : 1.04f) * gemm_tc_few_us(N, K);
 }
 
 int launch_gemm_slices(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, void *workspace,

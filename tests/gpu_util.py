@@ -35,3 +35,23 @@ def run_linear(blocks, x, *, out_dtype=torch.float32):
     y = tq1_matmul(to_dev(blocks), xd, out_dtype=out_dtype)
     torch.cuda.synchronize()
     return y.float().cpu().numpy()
+
+
+def graph_ms(run, calls=40):
+    """Best time of a graph of ``calls`` calls of ``run(i)``."""
+    run(0)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for i in range(calls):
+            run(i)
+    graph.replay()
+    best = float("inf")
+    for _ in range(5):
+        start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        graph.replay()
+        stop.record()
+        torch.cuda.synchronize()
+        best = min(best, start.elapsed_time(stop))
+    return best

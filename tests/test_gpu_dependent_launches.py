@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from tests.gpu_util import random_blocks, to_dev
+from tests.gpu_util import graph_ms, random_blocks, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -125,28 +125,10 @@ def test_calls_in_a_row_are_no_slower_than_calls_apart(batch, rows, columns):
     from ternel_b200.ops import tq1_matmul
     blocks, rng = random_blocks(rows, columns, seed=3)
     weight, x = to_dev(blocks), to_dev(rng.standard_normal((batch, columns)).astype(np.float16))
-    other, calls = torch.zeros(32, device="cuda"), 40
-    tq1_matmul(weight, x)
-    torch.cuda.synchronize()
+    other = torch.zeros(32, device="cuda")
 
-    def timed(run):
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph):
-            for _ in range(calls):
-                run()
-        graph.replay()
-        best = float("inf")
-        for _ in range(5):
-            start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            start.record()
-            graph.replay()
-            stop.record()
-            torch.cuda.synchronize()
-            best = min(best, start.elapsed_time(stop))
-        return best
-
-    def apart():
+    def apart(_):
         other.add_(1)
         tq1_matmul(weight, x)
 
-    assert timed(lambda: tq1_matmul(weight, x)) <= 1.1 * timed(apart)
+    assert graph_ms(lambda _: tq1_matmul(weight, x)) <= 1.1 * graph_ms(apart)

@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from oracle import tq1_oracle as o
-from tests.gpu_util import random_blocks, run_linear, to_dev
+from tests.gpu_util import graph_ms, random_blocks, run_linear, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -88,3 +88,34 @@ def test_counters_of_other_kernels_do_not_matter(batch):
                               ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
     assert int(ws[:4].view(torch.int32).item()) == 0 and bool((ws[256:] == 99).all())
     assert np.array_equal(y.cpu().numpy(), run_linear(blocks, x))
+
+
+@pytest.mark.parametrize(("batch", "rows", "columns"), (
+    (8, 2048, 512), (8, 34816, 512), (16, 17408, 1536), (16, 4096, 4096), (8, 12000, 6144), (8, 1024, 5120)))
+def test_the_choice_is_not_the_slower_kernel(batch, rows, columns):
+    """In a row of calls and behind another kernel, weights out of HBM: the kernel that is chosen against the tcgen05 kernel."""
+    from ternel_b200 import _native
+    from ternel_b200.ops import tq1_matmul
+    from ternel_b200.stack import random_blocks_device
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(3)
+    first = random_blocks_device(rows, columns, gen, "cuda")
+    weights = [first.clone() for _ in range(min(40, 260_000_000 // first.numel() + 1))]
+    x, other = torch.randn((batch, columns), generator=gen, device="cuda").half(), torch.zeros(32, device="cuda")
+
+    def in_a_row(i):
+        tq1_matmul(weights[i % len(weights)], x)
+
+    def apart(i):
+        other.add_(1)
+        tq1_matmul(weights[i % len(weights)], x)
+
+    lib = _native.lib()
+    lib.tq1_debug_force_token_tile.argtypes = [ctypes.c_int]
+    chosen = [graph_ms(in_a_row), graph_ms(apart)]
+    try:
+        assert lib.tq1_debug_force_token_tile(16) == 0
+        tcgen05 = [graph_ms(in_a_row), graph_ms(apart)]
+    finally:
+        assert lib.tq1_debug_force_token_tile(0) == 0
+    assert all(a <= 1.07 * b for a, b in zip(chosen, tcgen05)), (chosen, tcgen05)
