@@ -346,35 +346,58 @@ int launch_many(const uint8_t *blocks, const __half *x, void *y, int y_f32, int 
 
 bool gemm_groups_preferred(int M, int N, int K) { return M >= 2 && (long long)M * N * K >= (1 << 20); }
 
-// Which of the three takes a call: modelled times (us), fitted to calls with weights out of HBM.
-//   few    a warp works through every eighth group; up to 32 tokens it is taken where `many` would leave SMs empty: 16 tokens of
-//          17408x5248 37 against 39 of `many`, of 5120x640 4.5 against 6.5, 32 tokens of 17408x5248 70 against 55, of 4099x2176
-//          9 against 22
-//   many   a CTA's groups one after the other, 0.85, 1.28 and 1.68 us each at 16, 32 and 64 tokens
-//   tcgen05 form   0.64 us a group up to 32 tokens, 1.13 beyond, behind a longer set-up (its file has both sides)
+// Which of the three takes a call, by modelled times (us) with weights out of HBM. Up to 32 tokens fitted to 400 calls behind
+// another kernel, within 8% (few), 3% (many) and 5% (tcgen05 form), the choice 1% above the best on average:
+//   few    a warp works through every eighth group; what it takes grows with the CTAs on an SM
+//   many   a CTA's groups one after the other; only where it fills most SMs, and its sums are the least exact of the three
+//          (5.3e-8, few 4.2e-8, tcgen05 form 4.0e-8), so the tcgen05 form is preferred to it up to 10% behind
+// 16 tokens of 17408x5248 41 us few, 37.5 many, 32 tcgen05 form; 16 of 8192x8320 40, 55 and 28; 32 of 5120x17280 68, 172 and 58;
+// 16 of 4099x2176 7.5, 16 and 9.1; 16 of 34816x640 15.8, 10.7 and 13.
+// Beyond 32 tokens: a few row takes 1.1 or (two CTAs an SM) 2.1 a group of eight, many 1.68 a group, the tcgen05 form 1.13.
+// Without a status word the tcgen05 form, which waits on barriers with a limit, is left out: nobody would learn of a wait that
+// ran out.
+enum class GroupForm { few, many, tcgen05 };
+static GroupForm group_form(int M, int N, int K, bool status) {
+    if (M <= 8) return GroupForm::few;
+    const int sms = sm_count();
+    const auto rounds = [](long long ctas, int at_once) { return (float)((ctas + at_once - 1) / at_once); };
+    const long long few_tiles = (N + kFewRows - 1) / kFewRows, row_tiles = (N + kManyRows - 1) / kManyRows;
+    const float groups = (float)(K / kGroup), turns = (float)((K / kGroup + 7) / 8);
+    bool many;
+    float us, behind = 1.0f;
+    if (M <= 32) {
+        const float per_sm = (float)few_tiles / (float)sms;
+        us = M <= 16 ? 1.62f + turns * (0.494f + 0.264f * rounds(few_tiles, sms) + 0.366f * per_sm + 0.497f * rounds(few_tiles, 3 * sms))
+                     : 2.03f + turns * (0.073f + 0.633f * rounds(few_tiles, sms) + 0.263f * per_sm + 0.563f * rounds(few_tiles, 2 * sms));
+        const float many_us = M <= 16 ? 2.14f + groups * (0.04f + 0.80f * rounds(row_tiles, sms))
+                                      : 2.41f + groups * (0.35f + 0.92f * rounds(row_tiles, sms));
+        many = row_tiles * 100 >= sms * (M <= 16 ? 86 : 70) && many_us < us;
+        if (many) { us = many_us; behind = 1.1f; }
+    } else {
+        const long long token_tiles = (M + 63) / 64, few_ctas = few_tiles * ((M + 31) / 32);
+        many = 2 * row_tiles * token_tiles >= sms;
+        us = 3.0f + (many ? groups * 1.68f * rounds(row_tiles * token_tiles, sms)
+                          : turns * (few_ctas <= sms ? 1.1f : 2.1f * rounds(few_ctas, 2 * sms)));
+    }
+    if (status && gemm_groups_tc_us(M, N, K) < behind * us) return GroupForm::tcgen05;
+    return many ? GroupForm::many : GroupForm::few;
+}
+
 int launch_gemm_groups(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, unsigned *status,
                        cudaStream_t stream) {
     const int groups = K / kGroup, f32 = y_f32 ? 1 : 0;
-    const long long row_tiles = (N + kManyRows - 1) / kManyRows, token_tiles = (M + 63) / 64;
-    if (M <= 8) return launch_few<1>(blocks, x, y, f32, M, N, groups, stream);
-    const bool many = M <= 16 ? row_tiles >= 128 : M <= 32 ? row_tiles >= 105 : row_tiles * token_tiles >= 74;
-    const auto rounds = [](long long ctas, int at_once) { return (float)((ctas + at_once - 1) / at_once); };
-    float us = 0.0f;
-    if (many) {
-        us = 3.0f + (float)groups * (M <= 16   ? 0.85f * rounds(row_tiles, 296)
-                                     : M <= 32 ? 1.28f * rounds(row_tiles, 296)
-                                               : 1.68f * rounds(row_tiles * token_tiles, 148));
-    } else if (M > 32) {
-        const long long ctas = (long long)((N + kFewRows - 1) / kFewRows) * ((M + 31) / 32);
-        us = 3.0f + (float)((groups + 7) / 8) * (ctas <= 148 ? 1.1f : 2.1f * rounds(ctas, 296));
+    switch (group_form(M, N, K, status != nullptr)) {
+        case GroupForm::tcgen05:
+            return launch_gemm_groups_tc(blocks, x, y, y_f32, M, N, K, status, stream);
+        case GroupForm::many:
+            return M <= 16   ? launch_many<2>(blocks, x, y, f32, M, N, groups, stream)
+                   : M <= 32 ? launch_many<4>(blocks, x, y, f32, M, N, groups, stream)
+                             : launch_many<8>(blocks, x, y, f32, M, N, groups, stream);
+        default:
+            return M <= 8    ? launch_few<1>(blocks, x, y, f32, M, N, groups, stream)
+                   : M <= 16 ? launch_few<2>(blocks, x, y, f32, M, N, groups, stream)
+                             : launch_few<4>(blocks, x, y, f32, M, N, groups, stream);
     }
-    // the tcgen05 form waits on barriers, with a limit: only for a caller that can be told that a wait ran out
-    if (status && gemm_groups_tc_us(M, N, K) < us) return launch_gemm_groups_tc(blocks, x, y, y_f32, M, N, K, status, stream);
-    if (M <= 16)
-        return many ? launch_many<2>(blocks, x, y, f32, M, N, groups, stream) : launch_few<2>(blocks, x, y, f32, M, N, groups, stream);
-    if (M <= 32 || !many)
-        return many ? launch_many<4>(blocks, x, y, f32, M, N, groups, stream) : launch_few<4>(blocks, x, y, f32, M, N, groups, stream);
-    return launch_many<8>(blocks, x, y, f32, M, N, groups, stream);
 }
 
 }  // namespace tq1

@@ -448,8 +448,10 @@ GroupPlan group_plan(int M, int N, int groups) {
     p.split = 1 << split_log;
     const int room = clusters_at_once(split_log);
     p.clusters = p.tiles < room ? p.tiles : room;
-    const int blocks = (p.tiles + p.clusters - 1) / p.clusters * ((groups + p.split - 1) / p.split);
-    p.us = p.nt <= kUnit ? 5.4f + 0.64f * (float)blocks : 6.5f + 1.13f * (float)blocks;
+    const int tiles = (p.tiles + p.clusters - 1) / p.clusters, blocks = tiles * ((groups + p.split - 1) / p.split);
+    p.us = p.nt <= kUnit ? 4.37f + 1.41f * (float)tiles + 0.643f * (float)blocks + (p.split > 1 ? 1.1f : 0.0f) +
+                               55.5e-9f * (float)N * (float)(groups * kGroup)
+                         : 6.5f + 1.13f * (float)blocks;
     return p;
 }
 

@@ -78,3 +78,23 @@ def test_without_a_workspace_nothing_waits():
     with_workspace = run_linear(blocks, x)
     assert not np.array_equal(got, with_workspace)
     assert np.linalg.norm(got - with_workspace) <= 2 * 2.3e-7 * np.linalg.norm(got)       # the forms' bounds
+
+
+@pytest.mark.parametrize(("rows", "columns", "batch"), ((8192, 8320, 12), (8192, 8320, 24), (8192, 8320, 32), (5120, 17280, 24)))
+def test_long_calls_of_nine_to_32_tokens_take_it(rows, columns, batch):
+    """Where this form is faster by a quarter it has to be the one that runs: the sums are not those of the form for a caller
+    without a workspace, and no less exact."""
+    from ternel_b200 import _native
+    from ternel_b200.ops import tq1_get_rows, tq1_matmul
+    from ternel_b200.stack import random_blocks_device
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(6)
+    bd = random_blocks_device(rows, columns, gen, "cuda")
+    x = torch.randn((batch, columns), generator=gen, device="cuda").half()
+    other = torch.empty((batch, rows), dtype=torch.float32, device="cuda")
+    assert _native.lib().tq1_linear_f16(bd.data_ptr(), x.data_ptr(), other.data_ptr(), 1, batch, rows, columns, None, 0,
+                                        torch.cuda.current_stream().cuda_stream) == 0
+    got = tq1_matmul(bd, x, out_dtype=torch.float32)
+    assert not torch.equal(got, other)
+    want = x.double() @ tq1_get_rows(bd, torch.arange(rows, device="cuda"), dtype=torch.float32).double().T
+    assert float((got.double() - want).norm() / want.norm()) <= BOUND
