@@ -158,12 +158,22 @@ int tq1_linear_swiglu_f16(const uint8_t *blocks, const void *x, void *y, int y_i
  *   aligned     1 if blocks and x are 16-byte aligned (the fast kernels need it)
  *   kernel      TQ1_KERNEL_*;  token_tile / ctas / parts: tensor-core kernel only (activation rows
  *               per tile, CTAs launched, equal K parts per tile or 0 for the stream-K split). Up to 16
- *               rows they describe the tcgen05 form, whose place the mma.sync form takes where it is faster */
+ *               rows they describe the tcgen05 form, whose place the mma.sync form takes where it is faster:
+ *               tq1_linear_form tells them apart, and the forms of the group sums */
 #define TQ1_KERNEL_ROWS 0
 #define TQ1_KERNEL_STREAM_GEMV 1
 #define TQ1_KERNEL_TENSOR_CORE 2
 #define TQ1_KERNEL_GROUP_SUMS 3
+#define TQ1_FORM_ROWS 0
+#define TQ1_FORM_STREAM_GEMV 1
+#define TQ1_FORM_TCGEN05 2              /* of TQ1_KERNEL_TENSOR_CORE */
+#define TQ1_FORM_SLICES 3               /* of TQ1_KERNEL_TENSOR_CORE: mma.sync out of registers, 3 to 16 rows */
+#define TQ1_FORM_GROUPS_FEW 4           /* of TQ1_KERNEL_GROUP_SUMS: mma.sync, 16 weight rows a CTA */
+#define TQ1_FORM_GROUPS_MANY 5          /* mma.sync, 128 weight rows a CTA */
+#define TQ1_FORM_GROUPS_TCGEN05 6       /* needs a workspace */
 int tq1_linear_plan(int M, int N, int K, int aligned, int *kernel, int *token_tile, int *ctas, int *parts);
+/* The kernel that runs: TQ1_FORM_* of a call with a workspace or (has_workspace = 0) without one. */
+int tq1_linear_form(int M, int N, int K, int aligned, int has_workspace, int *form);
 
 /* ---- row-sharded linear over several GPUs -------------------------------- */
 

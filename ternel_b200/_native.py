@@ -42,6 +42,7 @@ SIGNATURES = {
                                       c_void_p, c_size_t, c_void_p]),
     "tq1_linear_plan": (c_int, [c_int, c_int, c_int, c_int, POINTER(c_int), POINTER(c_int), POINTER(c_int),
                                 POINTER(c_int)]),
+    "tq1_linear_form": (c_int, [c_int, c_int, c_int, c_int, c_int, POINTER(c_int)]),
     "tq1_linear_sharded_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
     "tq1_shard_advance_epoch": (c_int, [c_void_p, ctypes.c_uint32, c_void_p]),
     "tq1_linear_f16_sharded": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_size_t,

@@ -144,14 +144,18 @@ int tq1_linear_f16(const uint8_t *blocks, const void *x, void *y, int y_is_f32,
                                   kWsSlotRegionBytes, s);
     if (gemv_looped_fits(blocks, M, N, K) && need >= kWsScratchOffset)
         return launch_gemv_looped(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, false, workspace, s);
-    if ((reinterpret_cast<uintptr_t>(blocks) & 15) == 0 && gemm_slices_preferred(M, N, K))
-        return launch_gemm_slices(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, workspace, s);
+    int status = TQ1_OK;
+    if ((reinterpret_cast<uintptr_t>(blocks) & 15) == 0 &&
+        try_gemm_slices(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, workspace, s, false, &status))
+        return status;
     if ((reinterpret_cast<uintptr_t>(blocks) & 15) == 0 && gemm_tc_shape_ok(M, N, K))
         return launch_gemm_tc(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, workspace, s);
-    if (gemm_groups_preferred(M, N, K))
-        return launch_gemm_groups(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K,
-                                  workspace && workspace_bytes >= kWsStatusBytes && (reinterpret_cast<uintptr_t>(workspace) & 3) == 0
-                                      ? static_cast<unsigned *>(workspace) : nullptr, s);
+    if (gemm_groups_preferred(M, N, K)) {
+        unsigned *word = workspace && workspace_bytes >= kWsStatusBytes && (reinterpret_cast<uintptr_t>(workspace) & 3) == 0
+                             ? static_cast<unsigned *>(workspace) : nullptr;
+        return launch_gemm_groups(gemm_groups_form(M, N, K, word != nullptr), blocks, static_cast<const __half *>(x), y,
+                                  y_is_f32 != 0, M, N, K, word, s);
+    }
     return launch_gemv_rows(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, s);
 }
 
@@ -176,8 +180,8 @@ int tq1_linear_swiglu_f16(const uint8_t *blocks, const void *x, void *y, int y_i
     if (gemv) return launch_gemv_single(blocks, xh, y, y_is_f32 != 0, rows, K, true, workspace, kWsSlotRegionBytes, s);
     if (gemv_looped_fits(blocks, M, rows, K))
         return launch_gemv_looped(blocks, xh, y, y_is_f32 != 0, M, rows, K, true, workspace, s);
-    if (gemm_slices_preferred(M, rows, K))
-        return launch_gemm_slices(blocks, xh, y, y_is_f32 != 0, M, rows, K, workspace, s, true);
+    int status = TQ1_OK;
+    if (try_gemm_slices(blocks, xh, y, y_is_f32 != 0, M, rows, K, workspace, s, true, &status)) return status;
     return launch_gemm_tc(blocks, xh, y, y_is_f32 != 0, M, rows, K, workspace, s, true);
 }
 
@@ -198,6 +202,18 @@ int tq1_linear_plan(int M, int N, int K, int aligned, int *kernel, int *token_ti
     return TQ1_OK;
 }
 
+int tq1_linear_form(int M, int N, int K, int aligned, int has_workspace, int *form) {
+    int kernel, token_tile, ctas, parts;
+    if (!form) return fail(TQ1_ERR_INVALID, "tq1_linear_form: null pointer");
+    const int rc = tq1_linear_plan(M, N, K, aligned, &kernel, &token_tile, &ctas, &parts);
+    if (rc != TQ1_OK) return rc;
+    *form = kernel == TQ1_KERNEL_TENSOR_CORE   ? (gemm_slices_preferred(M, N, K) ? TQ1_FORM_SLICES : TQ1_FORM_TCGEN05)
+            : kernel == TQ1_KERNEL_GROUP_SUMS  ? gemm_groups_form(M, N, K, has_workspace != 0)
+            : kernel == TQ1_KERNEL_STREAM_GEMV ? TQ1_FORM_STREAM_GEMV
+                                               : TQ1_FORM_ROWS;
+    return TQ1_OK;
+}
+
 // Sweep recording only (ternel_b200/dispatch.py binds it by name): forces the tensor-core kernel's token tile
 // for every later call of this process; 0 restores the rule. Process-global and not thread-safe, which is why
 // it is not part of the public header.
@@ -206,6 +222,21 @@ int tq1_debug_set_loop_tokens(int tokens) {
     if (gemv_set_loop_tokens(tokens) != TQ1_OK)
         return fail(TQ1_ERR_INVALID, "tq1_debug_set_loop_tokens: %d is not in 0..8", tokens);
     return TQ1_OK;
+}
+
+// Sweep recording only: the product by one of the forms that share calls between them (TQ1_FORM_SLICES with K % 512 == 0 and
+// aligned blocks, or one of the group sums), whichever the rules would take. Arguments as those of tq1_linear_f16, checked less.
+int tq1_debug_linear_as(int form, const uint8_t *blocks, const void *x, void *y, int y_is_f32, int M, int N, int K,
+                        void *workspace, void *stream) {
+    if (!blocks || !x || !y || !workspace || M <= 0 || N <= 0 || K <= 0 || K % kGroup)
+        return fail(TQ1_ERR_INVALID, "tq1_debug_linear_as: bad call");
+    const __half *xh = static_cast<const __half *>(x);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (form == TQ1_FORM_SLICES && K % 512 == 0 && M >= 3 && M <= 16 && (reinterpret_cast<uintptr_t>(blocks) & 15) == 0)
+        return launch_gemm_slices(blocks, xh, y, y_is_f32 != 0, M, N, K, workspace, s);
+    if (form >= TQ1_FORM_GROUPS_FEW && form <= TQ1_FORM_GROUPS_TCGEN05 && M >= 2)
+        return launch_gemm_groups(form, blocks, xh, y, y_is_f32 != 0, M, N, K, static_cast<unsigned *>(workspace), s);
+    return fail(TQ1_ERR_INVALID, "tq1_debug_linear_as: form %d does not take %dx%dx%d", form, M, N, K);
 }
 
 int tq1_debug_force_token_tile(int token_tile) {

@@ -183,11 +183,15 @@ float gemm_tc_few_us(int N, int K);                         // modelled time of 
 bool gemm_slices_preferred(int M, int N, int K);            // fits, and faster than the tcgen05 kernel
 int launch_gemm_slices(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, void *workspace,
                        cudaStream_t stream, bool swiglu = false);
+// Launches it (`status` is what came of that) and returns true where it is preferred.
+bool try_gemm_slices(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, void *workspace,
+                     cudaStream_t stream, bool swiglu, int *status);
 
 // Batched linear (M >= 2) with an FP32 sum per group, for every other width and alignment.
 bool gemm_groups_preferred(int M, int N, int K);
-// status: the workspace's first word, or null where the caller has none
-int launch_gemm_groups(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, unsigned *status,
+// The form that takes a call (TQ1_FORM_GROUPS_*); status: the call has a status word, the workspace's first.
+int gemm_groups_form(int M, int N, int K, bool status);
+int launch_gemm_groups(int form, const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, unsigned *status,
                        cudaStream_t stream);
 float gemm_groups_tc_us(int M, int N, int K);               // modelled time of the tcgen05 form
 int launch_gemm_groups_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, unsigned *status,

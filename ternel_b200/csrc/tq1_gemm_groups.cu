@@ -356,9 +356,8 @@ bool gemm_groups_preferred(int M, int N, int K) { return M >= 2 && (long long)M 
 // Beyond 32 tokens: a few row takes 1.1 or (two CTAs an SM) 2.1 a group of eight, many 1.68 a group, the tcgen05 form 1.13.
 // Without a status word the tcgen05 form, which waits on barriers with a limit, is left out: nobody would learn of a wait that
 // ran out.
-enum class GroupForm { few, many, tcgen05 };
-static GroupForm group_form(int M, int N, int K, bool status) {
-    if (M <= 8) return GroupForm::few;
+int gemm_groups_form(int M, int N, int K, bool status) {
+    if (M <= 8) return TQ1_FORM_GROUPS_FEW;
     const int sms = sm_count();
     const auto rounds = [](long long ctas, int at_once) { return (float)((ctas + at_once - 1) / at_once); };
     const long long few_tiles = (N + kFewRows - 1) / kFewRows, row_tiles = (N + kManyRows - 1) / kManyRows;
@@ -379,17 +378,17 @@ static GroupForm group_form(int M, int N, int K, bool status) {
         us = 3.0f + (many ? groups * 1.68f * rounds(row_tiles * token_tiles, sms)
                           : turns * (few_ctas <= sms ? 1.1f : 2.1f * rounds(few_ctas, 2 * sms)));
     }
-    if (status && gemm_groups_tc_us(M, N, K) < behind * us) return GroupForm::tcgen05;
-    return many ? GroupForm::many : GroupForm::few;
+    if (status && gemm_groups_tc_us(M, N, K) < behind * us) return TQ1_FORM_GROUPS_TCGEN05;
+    return many ? TQ1_FORM_GROUPS_MANY : TQ1_FORM_GROUPS_FEW;
 }
 
-int launch_gemm_groups(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, unsigned *status,
+int launch_gemm_groups(int form, const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, unsigned *status,
                        cudaStream_t stream) {
     const int groups = K / kGroup, f32 = y_f32 ? 1 : 0;
-    switch (group_form(M, N, K, status != nullptr)) {
-        case GroupForm::tcgen05:
+    switch (form) {
+        case TQ1_FORM_GROUPS_TCGEN05:
             return launch_gemm_groups_tc(blocks, x, y, y_f32, M, N, K, status, stream);
-        case GroupForm::many:
+        case TQ1_FORM_GROUPS_MANY:
             return M <= 16   ? launch_many<2>(blocks, x, y, f32, M, N, groups, stream)
                    : M <= 32 ? launch_many<4>(blocks, x, y, f32, M, N, groups, stream)
                              : launch_many<8>(blocks, x, y, f32, M, N, groups, stream);

@@ -540,18 +540,20 @@ int launch_slices(const CUtensorMap &wmap, const CUtensorMap &xmap, const SliceP
 
 }  // namespace
 
-bool gemm_slices_preferred(int M, int N, int K) {
-    if (M < 3 || M > 16 || K % 512 || gemm_tc_forced()) return false;
+// The plan of a call, not `ok` where the tcgen05 kernel is preferred.
+static SlicePlan preferred_plan(int M, int N, int K) {
+    if (M < 3 || M > 16 || K % 512 || gemm_tc_forced()) return {};
     const int nt = M <= 8 ? 1 : 2;
-    const SlicePlan p = slice_plan(nt, N, K);
-    return p.ok && call_us(p, nt, (N + kTileRows - 1) / kTileRows) < (nt == 1 ? 1.0f : 1.04f) * gemm_tc_few_us(N, K);
+    SlicePlan p = slice_plan(nt, N, K);
+    p.ok = p.ok && call_us(p, nt, (N + kTileRows - 1) / kTileRows) < (nt == 1 ? 1.0f : 1.04f) * gemm_tc_few_us(N, K);
+    return p;
 }
 
-int launch_gemm_slices(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, void *workspace,
-                       cudaStream_t stream, bool swiglu) {
+bool gemm_slices_preferred(int M, int N, int K) { return preferred_plan(M, N, K).ok; }
+
+static int launch_plan(const SlicePlan &p, const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K,
+                       void *workspace, cudaStream_t stream, bool swiglu) {
     const int nt = M <= 8 ? 1 : 2;
-    const SlicePlan p = slice_plan(nt, N, K);
-    if (!p.ok) return fail(TQ1_ERR_INVALID, "tq1_linear_f16: %dx%dx%d does not fit the slice kernel", M, N, K);
     SliceParams prm;
     prm.y = y;
     prm.status = static_cast<unsigned *>(workspace);
@@ -593,6 +595,20 @@ int launch_gemm_slices(const uint8_t *blocks, const __half *x, void *y, bool y_f
                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (res != CUDA_SUCCESS) return fail(TQ1_ERR_CUDA, "tq1_linear_f16: activation tensor map failed (%d)", (int)res);
     return nt == 1 ? launch_slices<1>(wmap, xmap, prm, p, stream) : launch_slices<2>(wmap, xmap, prm, p, stream);
+}
+
+int launch_gemm_slices(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, void *workspace,
+                       cudaStream_t stream, bool swiglu) {
+    const SlicePlan p = slice_plan(M <= 8 ? 1 : 2, N, K);
+    if (!p.ok) return fail(TQ1_ERR_INVALID, "tq1_linear_f16: %dx%dx%d does not fit the slice kernel", M, N, K);
+    return launch_plan(p, blocks, x, y, y_f32, M, N, K, workspace, stream, swiglu);
+}
+
+bool try_gemm_slices(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, void *workspace,
+                     cudaStream_t stream, bool swiglu, int *status) {
+    const SlicePlan p = preferred_plan(M, N, K);
+    if (p.ok) *status = launch_plan(p, blocks, x, y, y_f32, M, N, K, workspace, stream, swiglu);
+    return p.ok;
 }
 
 }  // namespace tq1

@@ -4,7 +4,8 @@ reference replays its dispatch rules against committed sweeps (tests/test_mlx_mo
 
 import pytest
 
-from ternel_b200.dispatch import LOOPED_MAX, SWEEP_BATCHES, SWEEP_SHAPES, chosen_over_best, load_sweep, plan
+from ternel_b200.dispatch import (GROUP_BATCHES, GROUP_SHAPES, LOOPED_MAX, SWEEP_BATCHES, SWEEP_SHAPES, chosen_over_best,
+                                  load_sweep, plan)
 
 
 def test_rule_is_near_the_best_recorded_option_everywhere():
@@ -12,7 +13,8 @@ def test_rule_is_near_the_best_recorded_option_everywhere():
     assert len(sweep["cases"]) == len(SWEEP_BATCHES) * len(SWEEP_SHAPES)
     worst = 1.0
     for case in sweep["cases"]:
-        assert ("us_looped" in case) == (case["batch"] <= LOOPED_MAX)       # both arms recorded where both exist
+        assert ("us_looped" in case) == (case["batch"] <= LOOPED_MAX)       # every arm recorded where it exists
+        assert ("us_by_form" in case) == (3 <= case["batch"] <= 16)
         ratio, chosen = chosen_over_best(case)
         assert chosen.kernel in ("tensor_core", "stream_gemv")
         assert ratio <= 1.10, (case, chosen)
@@ -54,3 +56,28 @@ def test_two_rows_of_any_matrix_take_the_exact_kernel():
     assert setter(before) == 0
     for rows, columns in shapes:
         assert plan(2, rows, columns).kernel == "stream_gemv"
+
+
+def test_rule_between_the_forms_of_the_group_sums():
+    """The line is drawn by times behind another kernel, where the tcgen05 form begins 1 to 2 us later than it does in the recorded
+    rows of calls: up to 20% of the shortest calls (383 rows), 10% of the others."""
+    cases = load_sweep()["group_cases"]
+    assert len(cases) == len(GROUP_BATCHES) * len(GROUP_SHAPES)
+    for case in cases:
+        ratio, chosen = chosen_over_best(case)
+        assert chosen.kernel == "group_sums"
+        assert ratio <= (1.20 if case["rows"] < 1000 else 1.10), (case, chosen)
+
+
+def test_plan_names_the_kernel_that_runs():
+    assert plan(1, 5120, 5120).form == plan(2, 5120, 5120).form == "stream_gemv"
+    assert plan(1, 5120, 640).form == plan(4, 100, 640).form == "rows"
+    for batch in range(3, 9):                                  # few rows: mma.sync out of registers, not tcgen05
+        assert plan(batch, 1024, 5120).form == "slices" and plan(batch, 1024, 5120).kernel == "tensor_core"
+    assert plan(8, 34816, 512).form == plan(16, 17408, 5120).form == plan(17, 1024, 5120).form == "tcgen05"
+    assert plan(8, 4099, 2176).form == plan(16, 4099, 2176).form == "groups_few"
+    assert plan(16, 34816, 640).form == "groups_many"
+    for batch in (12, 32, 300):                                # without a status word nothing may wait
+        assert plan(batch, 8192, 8320).form == "groups_tcgen05"
+        assert plan(batch, 8192, 8320, workspace=False).form in ("groups_few", "groups_many")
+    assert plan(8, 1024, 5120, aligned=False).form == "groups_few"
