@@ -72,6 +72,8 @@ def stream():
     (1, 1, 128), (1, 1, 512), (1, 7, 640), (1, 17, 512), (1, 16, 1024), (1, 100, 1536), (1, 1000, 512),
     (2, 1, 128), (3, 17, 256), (5, 100, 640), (8, 31, 512), (16, 16, 128), (17, 33, 384), (33, 129, 512),
     (64, 1, 128), (129, 200, 256),
+    # the slice kernel in clusters of 2 and 8, and the group sums on tcgen05: a cluster of 8 and of 2, CTAs by themselves
+    (3, 33, 6144), (9, 17, 17408), (48, 1500, 5248), (65, 4099, 2176), (17, 17408, 1408),
 ])
 def test_linear_stays_inside_its_buffers(batch, rows, columns):
     lib = native().lib()
@@ -182,6 +184,7 @@ def test_chain_stays_inside_its_buffers():
 SMALL_CASE_MODULES = [
     "tests/test_gpu_chain.py", "tests/test_gpu_linear.py", "tests/test_gpu_swiglu.py", "tests/test_gpu_embedding.py",
     "tests/test_gpu_gemv_stream.py", "tests/test_gpu_gemm.py", "tests/test_gpu_sharded.py", "tests/test_gpu_loaders.py",
+    "tests/test_gpu_slices.py", "tests/test_gpu_groups_tcgen05.py", "tests/test_gpu_dependent_launches.py",
 ]
 
 

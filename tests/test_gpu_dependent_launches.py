@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize(("batch", "columns"), (
     (1, 640),           # row kernel
     (5, 640),           # group sums, few rows
-    (70, 1408),         # group sums, many rows
+    (70, 1408),         # group sums on tcgen05
     (8, 1024)))         # mma.sync out of registers
 def test_a_chain_of_calls_equals_one_call_at_a_time(batch, columns):
     """gather -> product -> rows for the next gather, buffers reused: without a synchronisation between the calls the results
@@ -132,3 +132,60 @@ def test_calls_in_a_row_are_no_slower_than_calls_apart(batch, rows, columns):
         tq1_matmul(weight, x)
 
     assert graph_ms(lambda _: tq1_matmul(weight, x)) <= 1.1 * graph_ms(apart)
+
+
+@pytest.mark.parametrize(("batch", "rows", "columns", "form"), (
+    (1, 4096, 640, "rows"), (5, 4096, 640, "groups_few"), (100, 9000, 640, "groups_many"), (48, 4099, 2176, "groups_tcgen05"),
+    (8, 4096, 1024, "slices"), (64, 1024, 1024, "tcgen05"), (1, 1024, 1024, "stream_gemv")))
+def test_no_kernel_writes_what_an_earlier_one_reads(batch, rows, columns, form):
+    """Nothing but this library's kernels on a stream: a gather overwrites the activations that the product before it reads, two
+    products in a row read them, and the second one's results are overwritten each time. As with a synchronisation after every
+    call, eagerly and as a graph."""
+    import ctypes
+    from ternel_b200 import _native
+    from ternel_b200.dispatch import plan
+    assert plan(batch, rows, columns).form == form
+    lib, turns = _native.lib(), 12
+    table, weight = (to_dev(random_blocks(n, columns, seed=n)[0]) for n in (500, rows))
+    ids = torch.randint(0, 500, (turns, batch), device="cuda")
+    x = torch.zeros((batch, columns), dtype=torch.float16, device="cuda")
+    last, kept = torch.zeros((batch, rows), device="cuda"), torch.zeros((turns, batch, rows), device="cuda")
+    need = lib.tq1_linear_workspace_bytes(batch, rows, columns)
+    scratch = torch.zeros(max(need, 256), dtype=torch.uint8, device="cuda")
+
+    def run(wait):
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+        def done(status):
+            assert status == 0
+            if wait:
+                torch.cuda.synchronize()
+
+        def product(y):
+            done(lib.tq1_linear_f16(weight.data_ptr(), x.data_ptr(), y.data_ptr(), 1, batch, rows, columns, scratch.data_ptr(),
+                                    need, stream))
+
+        for i in range(turns):
+            done(lib.tq1_embedding_f16(table.data_ptr(), ids[i].data_ptr(), x.data_ptr(), 0, batch, 500, columns, stream))
+            product(kept[i])
+            product(last)
+
+    run(True)
+    want, want_last = kept.clone(), last.clone()
+    assert torch.equal(want[-1], want_last) and not torch.equal(want[0], want[1])
+
+    def check(go):
+        kept.zero_()
+        last.zero_()
+        go()
+        torch.cuda.synchronize()
+        assert torch.equal(kept, want) and torch.equal(last, want_last)
+
+    for _ in range(10):
+        check(lambda: run(False))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run(False)
+    for _ in range(10):
+        check(graph.replay)
+    assert int(scratch[:4].view(torch.int32).item()) == 0

@@ -16,14 +16,16 @@ BOUND = (0.96 + 0.82 + 0.58) * 2.0 ** -24
 
 
 @pytest.mark.parametrize(("rows", "columns", "batch"), (
-    (17408, 2688, 12), (17000, 1408, 16),               # one unit, of 16 tokens
+    (9000, 3200, 12), (17408, 3200, 16),                # one unit, of 16 tokens; a cluster of 2
     (17408, 1664, 17), (14000, 2688, 32),               # of 32, rows that fill no tile
     (17408, 1408, 24), (38000, 1408, 24),               # one unit and an odd number of groups, in one tile and in three
-    (4099, 2176, 33), (2000, 4224, 64),                 # two units, a cluster per tile
+    (4099, 2176, 33), (1500, 5248, 48), (383, 4224, 255),       # two units, clusters of 4, 8 and 8
     (4099, 2176, 65), (9000, 640, 129), (13313, 384, 200)))        # several token tiles, more tiles than SMs, three groups
 @pytest.mark.parametrize("shift", (0, 4))
 def test_against_float64(rows, columns, batch, shift):
+    from ternel_b200.dispatch import plan
     from ternel_b200.ops import check_status, tq1_get_rows, tq1_matmul
+    assert plan(batch, rows, columns).form == "groups_tcgen05"
     blocks, rng = random_blocks(rows, columns, seed=rows + batch)
     backing = torch.zeros(blocks.size + 16, dtype=torch.uint8, device="cuda")
     bd = backing[shift:shift + blocks.size].view(blocks.shape)
@@ -38,10 +40,15 @@ def test_against_float64(rows, columns, batch, shift):
     check_status()
 
 
-@pytest.mark.parametrize(("rows", "columns", "batch"), ((16500, 640, 16), (4099, 2176, 48), (9000, 640, 100)))
+@pytest.mark.parametrize(("rows", "columns", "batch", "form"), (
+    (17408, 3200, 12, "tcgen05"), (17408, 1408, 32, "tcgen05"),         # one unit, CTAs by themselves
+    (4099, 2176, 48, "tcgen05"), (4099, 2176, 129, "tcgen05"),          # a cluster of 4, several token tiles
+    (16500, 640, 16, "many"), (9000, 640, 100, "many")))
 @pytest.mark.parametrize("kind", ("scales", "activations", "infinite sum"))
-def test_nonfinite_values(rows, columns, batch, kind):
+def test_nonfinite_values(rows, columns, batch, form, kind):
     """Whole activations: infinities of a sum's sign, NaN for 0 * Inf and Inf - Inf, and a sum that has become infinite stays so."""
+    from ternel_b200.dispatch import plan
+    assert plan(batch, rows, columns).form == "groups_" + form
     blocks, rng = random_blocks(rows, columns, seed=batch)
     x = rng.integers(-3, 4, (batch, columns)).astype(np.float16)
     scales = blocks.reshape(rows, columns // 128, 28)[:, :, :2].copy().view(np.float16)[:, :, 0]

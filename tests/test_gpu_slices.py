@@ -1,4 +1,4 @@
-"""Three to sixteen activation rows (the slice kernel's and, beyond its sizes, the tcgen05 kernel's) against the oracle."""
+"""Three to sixteen activation rows where the slice kernel takes them, against the oracle."""
 
 import ctypes
 
@@ -24,6 +24,8 @@ BOUND = (1.92 + 2 * 0.58 * 2.0) * 2.0 ** -24
     (2369, 5120),                                       # a CTA's second tile, the last one of one row
     (48, 6144), (264, 17408), (640, 8704)))             # two and more CTAs in a cluster, K parts that begin inside a chunk
 def test_slices_against_float64(rows, columns, batch):
+    from ternel_b200.dispatch import plan
+    assert plan(batch, rows, columns).form == "slices"
     blocks, rng = random_blocks(rows, columns, seed=rows + columns + batch)
     x = rng.standard_normal((batch, columns)).astype(np.float16)
     want = o.float64_matmul(blocks, x, rows=rows, columns=columns)
@@ -119,3 +121,25 @@ def test_the_choice_is_not_the_slower_kernel(batch, rows, columns):
     finally:
         assert lib.tq1_debug_force_token_tile(0) == 0
     assert all(a <= 1.07 * b for a, b in zip(chosen, tcgen05)), (chosen, tcgen05)
+
+
+@pytest.mark.parametrize("batch", (3, 16, 17))          # slice kernel, and the tcgen05 kernel, which has the same rule
+def test_nonfinite_scales_are_folded_into_the_weights(batch):
+    """A weight is -s, 0 or s: an infinite or NaN scale makes infinities and NaN of the products with trits other than zero, and
+    with activations of zero; the products with zero trits stay zero."""
+    rows, columns = 300, 1024
+    blocks, rng = random_blocks(rows, columns, seed=12)
+    scales, trits = o.decode_blocks(blocks.reshape(-1, 28))
+    values = scales.copy().view(np.float16)[:, 0]
+    hit = rng.random(values.shape) < 0.02
+    values[hit] = rng.choice(np.array([np.inf, -np.inf, np.nan], dtype=np.float16), hit.sum())
+    trits = trits.copy()
+    trits[hit] = np.where(rng.random((int(hit.sum()), 128)) < 0.985, 1, trits[hit])       # few products decide: infinities remain
+    blocks = o.encode_blocks(values.view(np.uint8).reshape(-1, 2), trits).reshape(rows, columns // 128, 28)
+    x = rng.integers(-3, 4, (batch, columns)).astype(np.float16)
+    with np.errstate(invalid="ignore", over="ignore"):
+        weights = np.where(trits == 1, 0.0, (trits.astype(np.float64) - 1.0) * values.astype(np.float64)[:, None])
+        want = x.astype(np.float64) @ weights.reshape(rows, columns).T
+    classes = o.nonfinite_classes(want)
+    assert len(np.unique(classes)) == 4                 # finite, NaN, and infinities of both signs
+    assert np.array_equal(o.nonfinite_classes(run_linear(blocks, x)), classes)
