@@ -87,14 +87,17 @@ int clusters_at_once(KernelRecord &record, const void *kernel, unsigned threads,
 // Not in a graph behind a kernel that is not this library's and lets nothing in: there the edge alone costs some 0.3 us and up
 // to 0.7 (512 rows gathered 3.1 us as an ordinary launch, 3.4 as a dependent one; five tokens of 4099x2176 6.3 and 6.9). Outside
 // a graph such a launch gains all the same: the launch itself is brought forward (the gather 4.1 -> 3.1).
-bool behind_own_kernel(cudaStream_t stream);            // false: the stream is being captured, and the last node is another's
-void note_kernel(cudaStream_t stream);                  // a kernel of this library that lets the next one in has been launched
+bool stream_captured(cudaStream_t stream);              // is being captured; asked once per launch
+bool behind_own_kernel(cudaStream_t stream);            // the node that the next one captured depends on is one that was noted
+void note_captured_kernel(cudaStream_t stream);         // a kernel of this library that lets the next one in has been captured
 
-// `dependent` where overlapping is asked for and pays, else `plain`, its form for an ordinary launch.
+// `dependent` where overlapping is asked for and pays, else `plain`, its form for an ordinary launch. lets_in: it calls
+// allow_next_grid().
 template <class... P, class... A>
-cudaError_t launch_either(bool overlap, void (*dependent)(P...), void (*plain)(P...), dim3 grid, unsigned threads, size_t smem,
-                          cudaStream_t stream, A... args) {
-    overlap = overlap && behind_own_kernel(stream);
+cudaError_t launch_either(bool overlap, bool lets_in, void (*dependent)(P...), void (*plain)(P...), dim3 grid, unsigned threads,
+                          size_t smem, cudaStream_t stream, A... args) {
+    const bool captured = stream_captured(stream);
+    overlap = overlap && (!captured || behind_own_kernel(stream));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
@@ -105,7 +108,9 @@ cudaError_t launch_either(bool overlap, void (*dependent)(P...), void (*plain)(P
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = overlap ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, overlap ? dependent : plain, static_cast<P>(args)...);
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, overlap ? dependent : plain, static_cast<P>(args)...);
+    if (captured && lets_in && err == cudaSuccess) note_captured_kernel(stream);
+    return err;
 }
 // Read-only data, in a kernel of either form.
 template <bool DEPENDENT, class T>

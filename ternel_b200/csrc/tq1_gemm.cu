@@ -900,7 +900,7 @@ int launch_variant(const CUtensorMap &wmap, const CUtensorMap &xmap, GemmParams 
     cfg.attrs = attr;
     cfg.numAttrs = V::CG > 1 ? 2 : 1;
     const cudaError_t err = cudaLaunchKernelEx(&cfg, kern, wmap, xmap, prm);
-    if (err == cudaSuccess) note_kernel(stream);
+    if (err == cudaSuccess && stream_captured(stream)) note_captured_kernel(stream);
     return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: GEMM launch");
 }
 

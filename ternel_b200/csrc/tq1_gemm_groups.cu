@@ -320,11 +320,9 @@ int launch_few(const uint8_t *blocks, const __half *x, void *y, int y_f32, int M
     const long long sms = sm_count();
     const bool uneven = NT == 2 && ((2 * ctas > 3 * sms && ctas <= 2 * sms) || (ctas > 3 * sms && ctas <= 5 * sms && groups > 8));
     const bool overlap = ctas <= sms / 2 || (ctas > sms && !uneven);
-    const cudaError_t err = launch_either(overlap, groups_few_kernel<NT, true>, groups_few_kernel<NT, false>, dim3((unsigned)ctas),
+    const cudaError_t err = launch_either(overlap, true, groups_few_kernel<NT, true>, groups_few_kernel<NT, false>, dim3((unsigned)ctas),
                                           kFewWarps * 32, 0, stream, blocks, x, y, y_f32, M, N, groups);
-    if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: launch");
-    note_kernel(stream);
-    return TQ1_OK;
+    return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: launch");
 }
 
 template <int NT>
@@ -335,11 +333,9 @@ int launch_many(const uint8_t *blocks, const __half *x, void *y, int y_f32, int 
         if (err == cudaSuccess)
             err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)many_smem(NT));
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: shared memory opt-in");
-    err = launch_either(true, groups_many_kernel<NT, true>, groups_many_kernel<NT, false>, dim3((unsigned)ctas), kManyWarps * 32,
+    err = launch_either(true, true, groups_many_kernel<NT, true>, groups_many_kernel<NT, false>, dim3((unsigned)ctas), kManyWarps * 32,
                         many_smem(NT), stream, blocks, x, y, y_f32, M, N, groups);
-    if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: launch");
-    note_kernel(stream);
-    return TQ1_OK;
+    return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: launch");
 }
 
 }  // namespace

@@ -498,9 +498,10 @@ int launch_gemm_groups_tc(const uint8_t *blocks, const __half *x, void *y, bool 
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = behind_own_kernel(stream) ? 2 : 1;
+    const bool captured = stream_captured(stream);
+    cfg.numAttrs = !captured || behind_own_kernel(stream) ? 2 : 1;
     err = cudaLaunchKernelEx(&cfg, groups_tc_kernel, xmap, prm);
-    if (err == cudaSuccess) note_kernel(stream);
+    if (captured && err == cudaSuccess) note_captured_kernel(stream);
     return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: launch (group sums)");
 }
 

@@ -532,9 +532,10 @@ int launch_slices(const CUtensorMap &wmap, const CUtensorMap &xmap, const SliceP
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = behind_own_kernel(stream) ? 2 : 1;
+    const bool captured = stream_captured(stream);
+    cfg.numAttrs = !captured || behind_own_kernel(stream) ? 2 : 1;
     const cudaError_t err = cudaLaunchKernelEx(&cfg, kern, wmap, xmap, prm);
-    if (err == cudaSuccess) note_kernel(stream);
+    if (captured && err == cudaSuccess) note_captured_kernel(stream);
     return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: launch (slices)");
 }
 

@@ -1220,7 +1220,7 @@ int gemv_chain_launch(const ChainLinkDev *table_dev, const ChainLinkDev *inline_
                       : form == kChain ? cudaLaunchKernelEx(&cfg, tq1_gemv_chain_kernel<kChain>, params)
                                        : cudaLaunchKernelEx(&cfg, tq1_gemv_chain_kernel<kAlone>, params);
     if (err != cudaSuccess) return cuda_fail(err, "tq1 chain: launch");
-    note_kernel(stream);
+    if (stream_captured(stream)) note_captured_kernel(stream);
     return TQ1_OK;
 }
 

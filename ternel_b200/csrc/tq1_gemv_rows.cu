@@ -123,9 +123,8 @@ static int launch_mb(const uint8_t *blocks, const __half *x, void *y, bool y_f32
     // 1408 columns 4.4 / 8.0, 256 of 2176 7.1 / 13.1, 296 of 9856 (five an SM) 46 / 70; 296 of 640 4.9 / 4.5, of 5248 26 / 25.
     const int sms = sm_count(), room = (int)(228 * 1024 / (smem + 1024)), per_sm = room < 8 ? room : 8;
     const bool overlap = ctas <= sms / 2 || (ctas == 2 * sms && per_sm % 2 == 0);
-    err = launch_either(overlap, dependent, plain, dim3((unsigned)ctas), kRowsThreads, smem, stream, blocks, x, y, N, K, N);
+    err = launch_either(overlap, true, dependent, plain, dim3((unsigned)ctas), kRowsThreads, smem, stream, blocks, x, y, N, K, N);
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: launch");
-    note_kernel(stream);
     return TQ1_OK;
 }
 
