@@ -1,24 +1,11 @@
 // What the kernels share that turn code bytes into FP16 weights by a table of PRMT selectors in shared memory.
 #pragma once
-#include "tq1_common.cuh"
+#include "tq1_async.cuh"
 
 namespace tq1 {
 
-constexpr uint32_t kSpinLimit = 1u << 20;
-
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t d;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
-    return d;
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 // Bounded, as in the other kernels: after the limit status 3 is set and the thread waits for nothing any more.
 static __device__ __noinline__ bool mbar_wait_more(uint32_t bar, uint32_t parity, unsigned *status) {
@@ -43,11 +30,7 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, unsigne
                  "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     if (!ok && !dead) dead = mbar_wait_more(bar, parity, status);
 }
-__device__ __forceinline__ bool elect_one() {
-    uint32_t one;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
-    return one != 0;
-}
+
 // Table entry of code byte v: PRMT selectors that pick FP16 weights out of [s_lo, s_hi, s_hi ^ 0x80] and zeros, one byte a trit.
 //   even byte (its first trit in the lower half of a register): word0 = (t0,t1) | t4 << 16, word1 = (t2,t3)
 //   odd byte: word0 = (t1,t2) | t0 << 16, word1 = (t3,t4)

@@ -35,7 +35,7 @@
 #include <cuda.h>
 #include <math.h>
 
-#include "tq1_common.cuh"
+#include "tq1_async.cuh"
 
 namespace tq1 {
 
@@ -46,7 +46,6 @@ constexpr int kChunkGroups = 4;
 constexpr int kChunkBytes = kChunkGroups * kBlockBytes;             // 112 packed bytes per row
 constexpr int kPackBytes = 32 * kChunkBytes;                        // a warp's rows of a chunk: 3584
 constexpr int kStageCols = 64;                                      // tensor-memory columns of a K block of FP16 weights
-constexpr uint32_t kSpinLimit = 1u << 20;
 
 // Variants:
 //   S  up to 32 tokens: two CTAs per SM with two decode groups each hide each other's latencies; the narrow table
@@ -135,17 +134,6 @@ constexpr NarrowTable make_narrow() {
 __device__ __align__(128) const WideTable g_wide = make_wide();
 __device__ __align__(128) const NarrowTable g_narrow = make_narrow();
 
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t d;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
-    return d;
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
 // Address, in the cluster's shared window, of `addr` in the leading CTA of the pair.
 __device__ __forceinline__ uint32_t leader_addr(uint32_t addr) {
     uint32_t d;
@@ -180,14 +168,6 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, unsigne
         dead = true;
     }
 }
-// One lane of a converged warp. Branching on it (and not on the lane number) tells the compiler that a single thread
-// runs the branch, so the operands of tcgen05.mma stay in uniform registers: 25 clocks per MMA issued instead of 134
-// (a loop over the lanes that might hold different operands), which had paced every token tile below 256.
-__device__ __forceinline__ bool elect_one() {
-    uint32_t one;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
-    return one != 0;
-}
 // Activation tile half: {64 columns, box rows} at (x, y). With a CTA pair the bytes count on the leader's barrier.
 template <int CG>
 __device__ __forceinline__ void tma_load_x(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
@@ -210,11 +190,6 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row groups 1024 B apart.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
-    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
-           (2ull << 61);
-}
 // A operand in tensor memory (lane = weight row, 8 columns per K = 16 step), B in shared memory.
 template <int CG>
 __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
@@ -236,17 +211,6 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
                      ::"r"(bar), "h"((uint16_t)3) : "memory");
     else
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_store32(uint32_t taddr, const uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-        "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
-          "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
-          "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-        : "memory");
 }
 __device__ __forceinline__ void tmem_load16(uint32_t taddr, float *v) {
     uint32_t u[16];
