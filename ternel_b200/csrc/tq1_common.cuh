@@ -82,7 +82,7 @@ int clusters_at_once(KernelRecord &record, const void *kernel, unsigned threads,
 // A launch may begin while the kernel before it in the stream ends (programmatic dependent launch): that kernel lets it in
 // (allow_next_grid), and it calls grid_dependency_wait() before it touches what an earlier one may have written or may still
 // read, by plain loads: __ldg and __restrict__ tell the compiler that the data were there from the kernel's beginning. Calls back
-// to back: a gather of 2048 rows of 5120 columns 8.2 -> 5.7 us, five tokens of 4099x2176 7.2 -> 6.1.
+// to back through the Python modules: a gather of 2048 rows of 5120 columns 8.2 -> 5.5 us, five tokens of 4099x2176 7.2 -> 5.9.
 //
 // Not in a graph behind a kernel that is not this library's and lets nothing in: there the edge alone costs some 0.3 us and up
 // to 0.7 (512 rows gathered 3.1 us as an ordinary launch, 3.4 as a dependent one; five tokens of 4099x2176 6.3 and 6.9). Outside

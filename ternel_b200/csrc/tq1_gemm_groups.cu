@@ -17,10 +17,10 @@
 //          short call is load, decode, product and one sum through shared memory
 //   many   a CTA has 128 weight rows and 8 NT tokens; activations come through shared memory (three stages of cp.async)
 //
-// What bounds it: up to 32 tokens the chain of dependent loads and the decode (25 instructions and six table or byte loads
-// per eight weights), beyond that the products and the instructions around them (700 tokens of 17408x5248: 87 T
-// multiply-adds/s; an SM at work has its mma.sync pipe active for 57% of the time). 5 tokens of 4099x2176 take 5.1 us (row
-// kernel 45). Longer calls go to the tcgen05 form (tq1_gemm_groups_tc.cu).
+// What bounds it: the chain of dependent loads and the decode (25 instructions and six table or byte loads per eight weights).
+// 5 tokens of 4099x2176 take 5.2 us in a row of calls (6.3 behind another kernel, 5.9 through the Python module; row kernel 45).
+// A `many` CTA of 64 tokens is bound by its products (the mma.sync pipe is active for 57% of the time); most calls of that length
+// go to the tcgen05 form (tq1_gemm_groups_tc.cu).
 #include "tq1_common.cuh"
 
 namespace tq1 {
@@ -328,10 +328,9 @@ int launch_few(const uint8_t *blocks, const __half *x, void *y, int y_f32, int M
 template <int NT>
 int launch_many(const uint8_t *blocks, const __half *x, void *y, int y_f32, int M, int N, int groups, cudaStream_t stream) {
     const long long ctas = (long long)((N + kManyRows - 1) / kManyRows) * ((M + 8 * NT - 1) / (8 * NT));
-    cudaError_t err = cudaSuccess;
-    for (auto kernel : {groups_many_kernel<NT, true>, groups_many_kernel<NT, false>})
-        if (err == cudaSuccess)
-            err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)many_smem(NT));
+    static KernelRecord records[2];
+    cudaError_t err = opt_in(records[0], reinterpret_cast<const void *>(groups_many_kernel<NT, true>), many_smem(NT));
+    if (err == cudaSuccess) err = opt_in(records[1], reinterpret_cast<const void *>(groups_many_kernel<NT, false>), many_smem(NT));
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: shared memory opt-in");
     err = launch_either(true, true, groups_many_kernel<NT, true>, groups_many_kernel<NT, false>, dim3((unsigned)ctas), kManyWarps * 32,
                         many_smem(NT), stream, blocks, x, y, y_f32, M, N, groups);

@@ -109,19 +109,23 @@ static int launch_mb(const uint8_t *blocks, const __half *x, void *y, bool y_f32
     const size_t smem = 512 + sizeof(float) * (size_t)MB * K;
     if (smem > 227 * 1024)
         return fail(TQ1_ERR_INVALID, "tq1_linear_f16: K=%d too large for the row kernel's shared memory", K);
+    const int sms = sm_count();
     int ctas = (N + 7) / 8;
-    if (ctas > 2 * sm_count()) ctas = 2 * sm_count();
+    if (ctas > 2 * sms) ctas = 2 * sms;
     auto dependent = y_f32 ? gemv_rows_kernel<MB, true, true> : gemv_rows_kernel<MB, false, true>;
     auto plain = y_f32 ? gemv_rows_kernel<MB, true, false> : gemv_rows_kernel<MB, false, false>;
     cudaError_t err = cudaSuccess;
-    for (auto kernel : {dependent, plain})
-        if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: shared memory opt-in");
+    if (smem > 48 * 1024) {
+        static KernelRecord records[2][2];
+        err = opt_in(records[y_f32][0], reinterpret_cast<const void *>(dependent), 227 * 1024);
+        if (err == cudaSuccess) err = opt_in(records[y_f32][1], reinterpret_cast<const void *>(plain), 227 * 1024);
+        if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: shared memory opt-in");
+    }
     // The calls that follow are let in at once and fill the SMs up, so they have to come in whole grids: as many CTAs on every SM.
     // Two an SM, and room for an even number of them (eight by their threads), or so few that each has an SM to itself. Otherwise
     // some SMs have two CTAs of a call and others none: calls in a row, us, as ordinary launches / as dependent ones: 125 CTAs of
     // 1408 columns 4.4 / 8.0, 256 of 2176 7.1 / 13.1, 296 of 9856 (five an SM) 46 / 70; 296 of 640 4.9 / 4.5, of 5248 26 / 25.
-    const int sms = sm_count(), room = (int)(228 * 1024 / (smem + 1024)), per_sm = room < 8 ? room : 8;
+    const int room = (int)(228 * 1024 / (smem + 1024)), per_sm = room < 8 ? room : 8;
     const bool overlap = ctas <= sms / 2 || (ctas == 2 * sms && per_sm % 2 == 0);
     err = launch_either(overlap, true, dependent, plain, dim3((unsigned)ctas), kRowsThreads, smem, stream, blocks, x, y, N, K, N);
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: launch");
