@@ -91,13 +91,12 @@ bool stream_captured(cudaStream_t stream);              // is being captured; as
 bool behind_own_kernel(cudaStream_t stream);            // the node that the next one captured depends on is one that was noted
 void note_captured_kernel(cudaStream_t stream);         // a kernel of this library that lets the next one in has been captured
 
-// `dependent` where overlapping is asked for and pays, else `plain`, its form for an ordinary launch. lets_in: it calls
-// allow_next_grid().
+// `dependent` where overlapping is asked for (by calls of a stream, by captured ones) and pays, else `plain`, its form for an
+// ordinary launch. lets_in: it calls allow_next_grid().
 template <class... P, class... A>
-cudaError_t launch_either(bool overlap, bool lets_in, void (*dependent)(P...), void (*plain)(P...), dim3 grid, unsigned threads,
-                          size_t smem, cudaStream_t stream, A... args) {
-    const bool captured = stream_captured(stream);
-    overlap = overlap && (!captured || behind_own_kernel(stream));
+cudaError_t launch_either(bool in_stream, bool in_graph, bool lets_in, void (*dependent)(P...), void (*plain)(P...), dim3 grid,
+                          unsigned threads, size_t smem, cudaStream_t stream, A... args) {
+    const bool captured = stream_captured(stream), overlap = captured ? in_graph && behind_own_kernel(stream) : in_stream;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);

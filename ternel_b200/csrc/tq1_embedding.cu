@@ -161,7 +161,7 @@ int launch_embedding(const uint8_t *blocks, const int64_t *ids, void *out, bool 
         auto dependent = out_f32 ? embedding_kernel<true, true, true> : embedding_kernel<false, true, true>;
         auto plain = out_f32 ? (shared ? embedding_kernel<true, true, false> : embedding_kernel<true, false, false>)
                              : (shared ? embedding_kernel<false, true, false> : embedding_kernel<false, false, false>);
-        const cudaError_t err = launch_either(shared, shared, dependent, plain, grid, kThreadsPerBlockRow * kBlocksPerCta, 0, stream, blocks,
+        const cudaError_t err = launch_either(shared, shared, shared, dependent, plain, grid, kThreadsPerBlockRow * kBlocksPerCta, 0, stream, blocks,
                                               ids + t0, first, n, V, gpr);
         if (err != cudaSuccess) return cuda_fail(err, "tq1_embedding_f16: launch");
     }

@@ -314,14 +314,15 @@ int launch_few(const uint8_t *blocks, const __half *x, void *y, int y_f32, int M
     const long long ctas = (long long)((N + kFewRows - 1) / kFewRows) * ((M + 8 * NT - 1) / (8 * NT));
     // around one CTA an SM, a call whose first CTAs find places beside the last of the one before takes two places on some SMs
     // (120 CTAs: 8.7 us alone, 10.1 as a dependent launch; 24 of them 5.9 and 5.3, 257 of them 6.0 and 5.3)
-    // (nor does it gain with two token tiles, three CTAs an SM: between one and a half and two of them on an SM a few places are
-    // left to the next call, and between three and five the plain loads weigh more. 16 tokens, calls in a row, ordinary /
-    // dependent: 275 CTAs of 1408 columns 5.35 / 5.81, of 9856 22.6 / 24.6, 625 of 2176 13.6 / 14.6, 175 of 640 3.46 / 2.78)
+    // (nor does it gain in a graph with two token tiles, three CTAs an SM: between one and a half and two of them on an SM a few
+    // places are left to the next call, and between three and five the plain loads weigh more. 16 tokens, calls in a row, ordinary /
+    // dependent: 275 CTAs of 1408 columns 5.35 / 5.81, of 9856 22.6 / 24.6, 625 of 2176 13.6 / 14.6, 175 of 640 3.46 / 2.78. Outside
+    // a graph, where the launch itself costs 2 us: 275 of 1408 6.3 / 6.0, of 9856 24.5 / 25.8, 625 of 2176 15.8 / 14.6)
     const long long sms = sm_count();
     const bool uneven = NT == 2 && ((2 * ctas > 3 * sms && ctas <= 2 * sms) || (ctas > 3 * sms && ctas <= 5 * sms && groups > 8));
-    const bool overlap = ctas <= sms / 2 || (ctas > sms && !uneven);
-    const cudaError_t err = launch_either(overlap, true, groups_few_kernel<NT, true>, groups_few_kernel<NT, false>, dim3((unsigned)ctas),
-                                          kFewWarps * 32, 0, stream, blocks, x, y, y_f32, M, N, groups);
+    const bool overlap = ctas <= sms / 2 || ctas > sms;
+    const cudaError_t err = launch_either(overlap, overlap && !uneven, true, groups_few_kernel<NT, true>, groups_few_kernel<NT, false>,
+                                          dim3((unsigned)ctas), kFewWarps * 32, 0, stream, blocks, x, y, y_f32, M, N, groups);
     return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: launch");
 }
 
@@ -332,7 +333,7 @@ int launch_many(const uint8_t *blocks, const __half *x, void *y, int y_f32, int 
     cudaError_t err = opt_in(records[0], reinterpret_cast<const void *>(groups_many_kernel<NT, true>), many_smem(NT));
     if (err == cudaSuccess) err = opt_in(records[1], reinterpret_cast<const void *>(groups_many_kernel<NT, false>), many_smem(NT));
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: shared memory opt-in");
-    err = launch_either(true, true, groups_many_kernel<NT, true>, groups_many_kernel<NT, false>, dim3((unsigned)ctas), kManyWarps * 32,
+    err = launch_either(true, true, true, groups_many_kernel<NT, true>, groups_many_kernel<NT, false>, dim3((unsigned)ctas), kManyWarps * 32,
                         many_smem(NT), stream, blocks, x, y, y_f32, M, N, groups);
     return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: launch");
 }

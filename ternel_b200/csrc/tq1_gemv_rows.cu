@@ -30,13 +30,14 @@ __device__ __forceinline__ float dot_byte(uint32_t entry, const float *x, int n,
 }
 
 template <int MB, bool OUT_F32, bool DEPENDENT>
-__global__ void __launch_bounds__(kRowsThreads) gemv_rows_kernel(const uint8_t *blocks, const __half *x, void *y, int N, int K, int ldy) {
+__global__ void __launch_bounds__(kRowsThreads) gemv_rows_kernel(const uint8_t *blocks, const __half *x, void *y, int N, int K, int ldy,
+                                                                 int lets_in) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint16_t *lut = reinterpret_cast<uint16_t *>(smem_raw);          // 256 entries
     float *xs = reinterpret_cast<float *>(smem_raw + 512);           // [MB][K]
 
     for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = (uint16_t)trits_2bit(i);
-    allow_next_grid();                                  // early: 82 us for 17408x5248, 92 after the loop
+    if (lets_in) allow_next_grid();                     // early: 82 us for 17408x5248, 92 after the loop
     if (DEPENDENT) grid_dependency_wait();
     for (int i = threadIdx.x; i < MB * K; i += blockDim.x)
         xs[i] = __half2float(__ushort_as_half(load_input<DEPENDENT>(reinterpret_cast<const unsigned short *>(x) + i)));
@@ -124,10 +125,12 @@ static int launch_mb(const uint8_t *blocks, const __half *x, void *y, bool y_f32
     // The calls that follow are let in at once and fill the SMs up, so they have to come in whole grids: as many CTAs on every SM.
     // Two an SM, and room for an even number of them (eight by their threads), or so few that each has an SM to itself. Otherwise
     // some SMs have two CTAs of a call and others none: calls in a row, us, as ordinary launches / as dependent ones: 125 CTAs of
-    // 1408 columns 4.4 / 8.0, 256 of 2176 7.1 / 13.1, 296 of 9856 (five an SM) 46 / 70; 296 of 640 4.9 / 4.5, of 5248 26 / 25.
+    // 1408 columns 4.4 / 8.0, 256 of 2176 7.1 / 13.1, 296 of 9856 (five an SM) 46 / 70; 296 of 640 4.9 / 4.5, of 5248 26 / 25. Such
+    // a call lets nothing in; outside a graph it is a dependent launch all the same, which hides the launch behind any kernel.
     const int room = (int)(228 * 1024 / (smem + 1024)), per_sm = room < 8 ? room : 8;
-    const bool overlap = ctas <= sms / 2 || (ctas == 2 * sms && per_sm % 2 == 0);
-    err = launch_either(overlap, true, dependent, plain, dim3((unsigned)ctas), kRowsThreads, smem, stream, blocks, x, y, N, K, N);
+    const bool lets_in = ctas <= sms / 2 || (ctas == 2 * sms && per_sm % 2 == 0);
+    err = launch_either(true, lets_in, lets_in, dependent, plain, dim3((unsigned)ctas), kRowsThreads, smem, stream, blocks, x, y, N, K, N,
+                        lets_in ? 1 : 0);
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: launch");
     return TQ1_OK;
 }
