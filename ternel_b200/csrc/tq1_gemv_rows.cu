@@ -123,12 +123,13 @@ static int launch_mb(const uint8_t *blocks, const __half *x, void *y, bool y_f32
         if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: shared memory opt-in");
     }
     // The calls that follow are let in at once and fill the SMs up, so they have to come in whole grids: as many CTAs on every SM.
-    // Two an SM, and room for an even number of them (eight by their threads), or so few that each has an SM to itself. Otherwise
+    // Two an SM, and room for an even number of them (eight by their threads), or so few that each has an SM to itself, and short
+    // (64 CTAs of 640 columns 3.0 us as ordinary launches, 2.6 as dependent ones, of 7424 15.0 / 15.7, of 9856 20.3 / 21.9). Otherwise
     // some SMs have two CTAs of a call and others none: calls in a row, us, as ordinary launches / as dependent ones: 125 CTAs of
     // 1408 columns 4.4 / 8.0, 256 of 2176 7.1 / 13.1, 296 of 9856 (five an SM) 46 / 70; 296 of 640 4.9 / 4.5, of 5248 26 / 25. Such
     // a call lets nothing in; outside a graph it is a dependent launch all the same, which hides the launch behind any kernel.
     const int room = (int)(228 * 1024 / (smem + 1024)), per_sm = room < 8 ? room : 8;
-    const bool lets_in = ctas <= sms / 2 || (ctas == 2 * sms && per_sm % 2 == 0);
+    const bool lets_in = (ctas <= sms / 2 && per_sm == 8) || (ctas == 2 * sms && per_sm % 2 == 0);
     err = launch_either(true, lets_in, lets_in, dependent, plain, dim3((unsigned)ctas), kRowsThreads, smem, stream, blocks, x, y, N, K, N,
                         lets_in ? 1 : 0);
     if (err != cudaSuccess) return cuda_fail(err, "tq1_linear_f16: launch");

@@ -117,7 +117,7 @@ def test_products_of_both_forms_are_the_same(batch, rows, columns):
 
 
 @pytest.mark.parametrize(("batch", "rows", "columns"), (
-    (1, 1000, 1408), (1, 2048, 2176), (1, 4400, 9856), (1, 3300, 13184), (1, 5120, 17280), (1, 4400, 5248),       # row kernel
+    (1, 1000, 1408), (1, 2048, 2176), (1, 4400, 9856), (1, 3300, 13184), (1, 5120, 17280), (1, 4400, 5248), (1, 512, 9856),
     (16, 4400, 9856), (16, 10000, 2176)))               # group sums of few rows
 def test_calls_in_a_row_are_no_slower_than_calls_apart(batch, rows, columns):
     """Calls that come in while the one before them ends must not crowd on some SMs: in a row they take no longer than with a
