@@ -6,22 +6,26 @@
 
 using namespace tq1;
 
+// A function of the driver, null where there is none.
+template <class F>
+static F driver_function(const char *name) {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &qres) != cudaSuccess || qres != cudaDriverEntryPointSuccess) p = nullptr;
+    return reinterpret_cast<F>(p);
+}
+
 EncodeTiledFn tq1::encode_tiled_fn() {
-    static const EncodeTiledFn fn = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) != cudaSuccess ||
-            qres != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<EncodeTiledFn>(p);
-    }();
+    static const EncodeTiledFn fn = driver_function<EncodeTiledFn>("cuTensorMapEncodeTiled");
     return fn;
 }
 
 int tq1::device_slot() {
+    // asked several times per launch: of the driver where a context is current, which answers sooner than the runtime
+    static const auto ask = driver_function<CUresult (*)(CUdevice *)>("cuCtxGetDevice");
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
-    return dev;
+    if ((!ask || ask(&dev) != CUDA_SUCCESS) && cudaGetDevice(&dev) != cudaSuccess) return 0;
+    return dev >= 0 && dev < kMaxDevices ? dev : 0;
 }
 
 int tq1::sm_count() {
@@ -91,15 +95,7 @@ GraphTail tail_of(cudaStream_t stream) {
 
 // Whether the stream is being captured. Asked by every launch, so of the driver, which answers in 17 ns (the runtime in 46).
 bool tq1::stream_captured(cudaStream_t stream) {
-    typedef CUresult (*IsCapturingFn)(CUstream, CUstreamCaptureStatus *);
-    static const IsCapturingFn ask = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuStreamIsCapturing", &p, cudaEnableDefault, &qres) != cudaSuccess ||
-            qres != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<IsCapturingFn>(p);
-    }();
+    static const auto ask = driver_function<CUresult (*)(CUstream, CUstreamCaptureStatus *)>("cuStreamIsCapturing");
     CUstreamCaptureStatus status = CU_STREAM_CAPTURE_STATUS_NONE;
     return ask && ask(stream, &status) == CUDA_SUCCESS && status == CU_STREAM_CAPTURE_STATUS_ACTIVE;
 }
