@@ -35,6 +35,8 @@
 #include <cuda.h>
 #include <math.h>
 
+#include <type_traits>
+
 #include "tq1_async.cuh"
 
 namespace tq1 {
@@ -67,6 +69,10 @@ struct Variant {
     static constexpr int kTmemCols = G == 2 ? 256 : 512;
     static_assert(kABase + RING * kStageCols <= kTmemCols, "tensor memory budget");
     static constexpr int kMinCtas = G == 2 ? 2 : 1;
+    // P reads a segment's results out after the first K block of the next one is decoded. S and L read them out at once: their
+    // pace is the decode's, which loses by the interruption (16 tokens of 17408x5120 18.1 us, 19.9 otherwise; 48 of 5120x17408
+    // 21.4 and 21.9; only the most tiles gain, 128 of 34816x5120 45.2 and 44.2).
+    static constexpr bool kDecodeAhead = CG == 2;
     static constexpr uint32_t kTableBytes = WIDE ? 65536 : 32768;
     // shared-memory window addresses; the wide table sits at a 64 KiB multiple so that one PRMT builds an entry address
     static constexpr uint32_t kBase = 1024;
@@ -262,26 +268,24 @@ struct WorkSplit {
 
 // A slot's segments in order: its whole tiles, then the pieces of its range of the shared tiles.
 struct SegmentWalk {
-    const Divisor &by_chunks;
-    int chunks, whole_rounds, whole_tiles, tiles_total, slot, round, it, end, pieces;
-    __device__ __forceinline__ SegmentWalk(const WorkSplit &work, int slot_)
-        : by_chunks(work.by_chunks), chunks(work.chunks), whole_rounds(work.whole_rounds), whole_tiles(work.whole_tiles),
-          tiles_total(work.tiles_total), slot(slot_), round(0), it(work.first_iter(slot_)),
-          end(work.first_iter(slot_ + 1)), pieces(0) {}
-    // part: which of the slot's two partial-tile areas a partial segment is stored to
-    __device__ __forceinline__ bool next(int &tile, int &c0, int &len, int &part) {
-        if (round < whole_rounds && slot * whole_rounds + round < tiles_total) {
-            tile = slot * whole_rounds + round++;
+    const WorkSplit &work;                      // kernel parameters: read where they are used, not kept in registers
+    int slot, round, it, pieces;
+    __device__ __forceinline__ SegmentWalk(const WorkSplit &work_, int slot_)
+        : work(work_), slot(slot_), round(0), it(work_.first_iter(slot_)), pieces(0) {}
+    // end: work.first_iter(slot + 1); part: which of the slot's two partial-tile areas a partial segment is stored to
+    __device__ __forceinline__ bool next(int end, int &tile, int &c0, int &len, int &part) {
+        if (round < work.whole_rounds && slot * work.whole_rounds + round < work.tiles_total) {
+            tile = slot * work.whole_rounds + round++;
             c0 = 0;
-            len = chunks;
+            len = work.chunks;
             part = 0;
             return true;
         }
         if (it >= end) return false;
-        const int t = by_chunks.div(it);
-        c0 = it - t * chunks;
-        len = min(chunks - c0, end - it);
-        tile = whole_tiles + t;
+        const int t = work.by_chunks.div(it);
+        c0 = it - t * work.chunks;
+        len = min(work.chunks - c0, end - it);
+        tile = work.whole_tiles + t;
         part = pieces++ == 0 ? 0 : 1;
         it += len;
         return true;
@@ -300,10 +304,13 @@ struct GemmParams {
     int accs, acc_cols;       // accumulators (1, 2 or 4) and the columns from one to the next
     int b_stages, b_rows;     // activation ring: stages and rows per CTA of one stage
     WorkSplit work;
-    int y_f32, swiglu;
+    int y_f32;
+    int pair_y;               // FP16 results of two neighbouring rows may be stored at a time
 };
 
-template <class V>
+// GATED: the rows are (gate, up) pairs. A kernel of its own: the gates' code in the common one cost 3% of long prompts (777 tokens
+// of 34816x5120 without gates 204 us, 199 apart) and 7% of the shortest calls (17 of 1000x1024 5.8 us, 5.4).
+template <class V, bool GATED>
 __global__ void __launch_bounds__(V::kThreads, V::kMinCtas)
 tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
                 const __grid_constant__ GemmParams prm) {
@@ -317,8 +324,11 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         if (threadIdx.x == 0) atomicExch(prm.status, 2u);
         return;
     }
+    // EMPTY[i % READ_BARS]: the MMAs of K block i have read both operands. A barrier tells one phase from the next only; with
+    // four per ring stage a group knows a block that is up to four uses of the stage ahead of the last one it waited for.
+    constexpr int READ_BARS = V::kDecodeAhead ? 4 * RING : RING;
     constexpr int TAB = 0, PACK = 1, FULL_A = PACK + kDecode * V::PACK_STAGES, FULL_B = FULL_A + RING,
-                  EMPTY = FULL_B + RING, ACC_FULL = EMPTY + RING, ACC_FREE = ACC_FULL + 1, NUM_BARS = ACC_FREE + 1;
+                  EMPTY = FULL_B + RING, ACC_FULL = EMPTY + READ_BARS, ACC_FREE = ACC_FULL + 1, NUM_BARS = ACC_FREE + 1;
     static_assert(NUM_BARS * 8 <= 1000, "barrier area");
     auto bar = [wbase](int i) { return wbase + V::kBarAddr + 8u * (uint32_t)i; };
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(smem + (V::kBarAddr - V::kBase) + 1008);
@@ -326,7 +336,6 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
 
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int slot = CG == 2 ? blockIdx.x >> 1 : blockIdx.x, rank = CG == 2 ? blockIdx.x & 1 : 0;
-    const int chunks = prm.work.chunks;
 
     // ---- set-up that depends on no earlier kernel: barriers, decode table, tensor memory ---------------------
     if (tid == 0) {
@@ -335,8 +344,8 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         for (int i = 0; i < RING; ++i) {
             mbar_init(bar(FULL_A + i), 4 * CG);
             mbar_init(bar(FULL_B + i), 1);
-            mbar_init(bar(EMPTY + i), 1);
         }
+        for (int i = 0; i < READ_BARS; ++i) mbar_init(bar(EMPTY + i), 1);
         mbar_init(bar(ACC_FULL), 1);
         mbar_init(bar(ACC_FREE), kDecode * CG);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -371,6 +380,7 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
 
     bool dead = false;
     SegmentWalk walk(prm.work, slot);
+    const int end_iter = prm.work.first_iter(slot + 1);
     int tile, c0, len, part;
 
     auto weight_tile = [&](int t) { return prm.by_tiles_m.div(t); };
@@ -382,16 +392,16 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
     };
 
     // K blocks are numbered in the order the MMA warp takes them, over all segments: block i of a CTA uses stage i % RING of
-    // the decoded weights and stage i % b_stages (<= RING) of the activations. EMPTY[i % RING] completes when its MMAs have
-    // read both, one commit for decoders and activations alike.
+    // the decoded weights and stage i % b_stages (<= RING) of the activations. One commit (EMPTY) says to decoders and
+    // activations alike that its MMAs have read both.
     // A wave is the G chunks (fewer at a segment's end) that the groups decode side by side; its blocks are ordered by K
     // block first.
     if (warp == kXWarp) {
         // ------------------------------------------------------------------ activation tiles
         if (elect_one()) {
-            uint32_t stage = 0, freed = 0, phase = 0, filled = 0;      // freed: stage of the block that used this buffer before
+            uint32_t stage = 0, freed = 0, phase = 0, filled = 0;      // freed: barrier of the block that used this buffer before
             const uint32_t bytes = (uint32_t)prm.b_rows * 256u;
-            while (walk.next(tile, c0, len, part)) {
+            while (walk.next(end_iter, tile, c0, len, part)) {
                 const int m0 = token_tile0(tile);
                 const int row = m0 + (CG == 2 ? rank * (tile_tokens(m0) / 2) : 0);
                 for (int u0 = 0; u0 < len; u0 += G) {
@@ -403,7 +413,7 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                                 ++filled;
                             } else {
                                 mbar_wait(bar(EMPTY + freed), phase, prm.status, dead);
-                                if (++freed == RING) { freed = 0; phase ^= 1u; }
+                                if (++freed == READ_BARS) { freed = 0; phase ^= 1u; }
                             }
                             if (dead) break;
                             const uint32_t full = CG == 2 ? leader_addr(bar(FULL_B + stage)) : bar(FULL_B + stage);
@@ -420,9 +430,9 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
     } else if (warp == kMmaWarp) {
         // ------------------------------------------------------------------ MMA issue (leading CTA of a pair)
         if (rank == 0 && elect_one()) {
-            uint32_t bstage = 0, bphase = 0, astage = 0, aphase = 0, seg = 0;
+            uint32_t bstage = 0, bphase = 0, astage = 0, aphase = 0, read = 0, seg = 0;
             const uint32_t b_bytes = (uint32_t)prm.b_rows * 256u;
-            while (walk.next(tile, c0, len, part)) {
+            while (walk.next(end_iter, tile, c0, len, part)) {
                 const int n_tok = tile_tokens(token_tile0(tile));
                 // FP32 accumulate, FP16 A and B, both K-major, M = 128 per CTA, N = tokens
                 const uint32_t idesc = (1u << 4) | ((uint32_t)(n_tok >> 3) << 17) | ((uint32_t)(kTileW * CG >> 4) << 24);
@@ -442,7 +452,8 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                     for (int j = 0; j < 8; ++j)                    // K = 16 steps: four of each 64-wide swizzle atom
                         umma_f16_ts<CG>(acc, a_tmem + 8u * j, (j < 4 ? b_lo : b_hi) + 2u * (j & 3), idesc,
                                         (i >= prm.accs || j > 0) ? 1u : 0u);
-                    umma_commit<CG>(bar(EMPTY + astage));
+                    umma_commit<CG>(bar(EMPTY + read));
+                    if (++read == READ_BARS) read = 0;
                     if (++astage == RING) { astage = 0; aphase ^= 1u; }
                     if (++bstage == (uint32_t)prm.b_stages) { bstage = 0; bphase ^= 1u; }
                 }
@@ -463,7 +474,7 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         uint32_t requested = 0, consumed = 0;
         auto request = [&]() {
             while (p_unit >= p_len) {
-                if (!pwalk.next(p_tile, p_c0, p_len, p_part)) { p_len = 0; return; }
+                if (!pwalk.next(end_iter, p_tile, p_c0, p_len, p_part)) { p_len = 0; return; }
                 p_unit = group;
             }
             const uint32_t s = requested % V::PACK_STAGES;
@@ -477,37 +488,211 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         for (int s = 0; s < V::PACK_STAGES; ++s) request();
 
         int block0 = 0;                                                 // number of the wave's first K block
+        int seen = -1;                                                  // the newest K block waited for: its MMAs have read it
+        auto wait_read = [&](int block) {
+            if (block < 0) return;
+            seen = block;
+            mbar_wait(bar(EMPTY + block % READ_BARS), (uint32_t)(block / READ_BARS) & 1u, prm.status, dead);
+        };
         uint32_t seg = 0;
         mbar_wait(bar(TAB), 0, prm.status, dead);
 
-        while (walk.next(tile, c0, len, part)) {
+        // Reads out a segment's accumulators and stores its results.
+        auto finish = [&](int tile, int len, int part) {
+            const int m0 = token_tile0(tile), n_tok = tile_tokens(m0);
+            const int n = (weight_tile(tile) * CG + rank) * kTileW + row_in_tile;
+            const int per_group = (n_tok / 16 + G - 1) / G * 16;
+            const int c_begin = group * per_group, cols = min(per_group, n_tok - c_begin);     // cols <= 0: none
+            const bool whole = len == prm.work.chunks;
+            // the slots that share this tile, worked out while the last products are still being added
+            const int shared_tile = tile - prm.work.whole_tiles, it0 = shared_tile * prm.work.chunks;
+            int lo = slot, hi = slot;
+            if (!whole && prm.work.splits > 0) {
+                lo = shared_tile * prm.work.splits;
+                hi = lo + prm.work.splits - 1;
+            } else if (!whole) {
+                while (prm.work.first_iter(lo) > it0) --lo;
+                while (prm.work.first_iter(hi + 1) < it0 + prm.work.chunks) ++hi;
+            }
+            mbar_wait(bar(ACC_FULL), seg & 1u, prm.status, dead);
+            ++seg;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            constexpr int kStep = 16;                                                          // columns in registers at a time
+            auto read_step = [&](int s0, float (&v)[kStep]) {
+#pragma unroll
+                for (int c = 0; c < kStep; ++c) v[c] = 0.0f;
+                for (int a = 0; a < prm.accs && s0 < cols; ++a) {
+                    float u[kStep];
+                    tmem_load16(tmem_lane + (uint32_t)(a * prm.acc_cols + c_begin + s0), u);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int c = 0; c < kStep; ++c) {
+                        asm volatile("" : "+f"(u[c]));                                         // no use before the wait
+                        v[c] += u[c];
+                    }
+                }
+            };
+            auto release = [&]() {                      // the next segment may overwrite the accumulators
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive_leader<CG>(CG == 2 ? leader_addr(bar(ACC_FREE)) : bar(ACC_FREE));
+            };
+            const int tokens = min(cols, prm.M - (m0 + c_begin));                              // of the group's columns
+            const int out_n = GATED ? prm.N >> 1 : prm.N;
+            if (!whole) {                               // a part of the tile's K range: kept as FP32
+                const size_t area = (size_t)prm.nt * kTileW;
+                float *slot_part = prm.partials + ((size_t)2 * blockIdx.x + part) * area + row_in_tile;
+#pragma unroll 1
+                for (int s0 = 0; s0 < V::kGroupCols; s0 += kStep) {
+                    float v[kStep];
+                    read_step(s0, v);
+                    if (s0 + kStep >= V::kGroupCols) release();
+                    const int col0 = c_begin + s0;
+#pragma unroll
+                    for (int c = 0; c < kStep; ++c)
+                        if (s0 + c < tokens && TQ1_IN_BOUNDS((size_t)(col0 + c) * kTileW + row_in_tile, area, 41u))
+                            __stcg(slot_part + (size_t)(col0 + c) * kTileW, v[c]);
+                }
+                // The slot that completes the tile's count adds the parts.
+                asm volatile("bar.sync 1, %0;" ::"n"(kDecode * 32) : "memory");
+                if (tid == 0) {
+                    // the barrier orders the other warps' stores before this thread's release, and its acquire before their reads
+                    unsigned *counter = prm.counters + shared_tile * CG + rank, before;
+                    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
+                    const bool last = before == (unsigned)(hi - lo);
+                    if (last) *counter = 0u;                // zero for the next call
+                    if (before > (unsigned)(hi - lo)) atomicExch(prm.status, 8u);     // it was not zero when the call began
+                    *last_flag = last ? 1u : 0u;
+                }
+                asm volatile("bar.sync 1, %0;" ::"n"(kDecode * 32) : "memory");
+                if (*last_flag == 0u) return;
+                const int all = min(n_tok, prm.M - m0), quads = all * (kTileW / 4);      // four rows of a column each
+                constexpr int kThreadsR = kDecode * 32, kFlight = 4;
+                const int tile_n0 = (weight_tile(tile) * CG + rank) * kTileW;
+                for (int i0 = tid; i0 < quads; i0 += kThreadsR * kFlight) {
+                    float4 total[kFlight];
+#pragma unroll
+                    for (int f = 0; f < kFlight; ++f) total[f] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 2
+                    for (int sl = lo; sl <= hi; ++sl) {
+                        // the tile is that slot's first segment of shared tiles if its range starts inside the tile
+                        const int which = prm.work.splits > 0 || prm.work.first_iter(sl) >= it0 ? 0 : 1;
+                        const float4 *src = reinterpret_cast<const float4 *>(
+                            prm.partials + ((size_t)2 * (sl * CG + rank) + which) * area);
+#pragma unroll
+                        for (int f = 0; f < kFlight; ++f) {
+                            const int i = i0 + f * kThreadsR;
+                            const float4 p = i < quads ? __ldcg(src + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                            total[f].x += p.x; total[f].y += p.y; total[f].z += p.z; total[f].w += p.w;
+                        }
+                    }
+#pragma unroll
+                    for (int f = 0; f < kFlight; ++f) {
+                        const int i = i0 + f * kThreadsR, m = m0 + (i >> 5), nq = tile_n0 + (i & 31) * 4;
+                        if (i >= quads) break;
+                        float r[4] = {total[f].x, total[f].y, total[f].z, total[f].w};
+                        int count = min(4, prm.N - nq);
+                        size_t o = (size_t)m * prm.N + nq;
+                        size_t limit = (size_t)prm.M * prm.N;
+                        if (GATED) {
+                            r[0] = swiglu_f32(r[0], r[1]);
+                            r[1] = swiglu_f32(r[2], r[3]);
+                            count >>= 1;
+                            o = (size_t)m * (prm.N >> 1) + (nq >> 1);
+                            limit >>= 1;
+                        }
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            if (e < count && TQ1_IN_BOUNDS(o + e, limit, 40u)) {
+                                if (prm.y_f32) static_cast<float *>(prm.y)[o + e] = r[e];
+                                else static_cast<__half *>(prm.y)[o + e] = __float2half_rn(r[e]);
+                            }
+                        }
+                    }
+                }
+                return;
+            }
+            if (GATED || (!prm.y_f32 && prm.pair_y)) {
+                // Neighbouring rows are neighbouring results, and neighbouring lanes. Two lanes exchange columns, so that the even
+                // one has both rows of column c and the odd one of column c + 1: half as many stores, and with gate and up rows
+                // every lane has a result to work out. Results wait in registers until the accumulators are given back; gate and
+                // up themselves, twice as many, spill (777 tokens of 34816x5120 without gates 203 -> 216 us, as one kernel).
+                const int odd = lane & 1, row = n - odd;
+                uint32_t held[V::kGroupCols / 2];
+#pragma unroll
+                for (int s0 = 0; s0 < V::kGroupCols; s0 += kStep) {
+                    float v[kStep];
+                    read_step(s0, v);
+#pragma unroll
+                    for (int c = 0; c < kStep; c += 2) {
+                        const float other = __shfl_xor_sync(0xffffffffu, odd ? v[c] : v[c + 1], 1);
+                        const float first = odd ? other : v[c], second = odd ? v[c + 1] : other;
+                        uint32_t &result = held[(s0 + c) / 2];
+                        if (GATED) {
+                            const float out = swiglu_f32(first, second);
+                            result = prm.y_f32 ? __float_as_uint(out) : (uint32_t)__half_as_ushort(__float2half_rn(out));
+                        } else {
+                            const __half2 out = __floats2half2_rn(first, second);
+                            result = reinterpret_cast<const uint32_t &>(out);
+                        }
+                    }
+                }
+                release();
+                size_t o = (size_t)(m0 + c_begin + odd) * out_n + (GATED ? row >> 1 : row);
+                const bool in_rows = row + 1 < prm.N;                  // N is even here
+#pragma unroll
+                for (int c = 0; c < V::kGroupCols; c += 2) {
+                    if (c + odd < tokens && in_rows && TQ1_IN_BOUNDS(o + (GATED ? 0 : 1), (size_t)prm.M * out_n, 40u)) {
+                        if (!GATED) *reinterpret_cast<uint32_t *>(static_cast<__half *>(prm.y) + o) = held[c / 2];
+                        else if (prm.y_f32) static_cast<float *>(prm.y)[o] = __uint_as_float(held[c / 2]);
+                        else static_cast<__half *>(prm.y)[o] = __ushort_as_half((unsigned short)held[c / 2]);
+                    }
+                    o += 2 * (size_t)out_n;
+                }
+                return;
+            }
+            if constexpr (!GATED) {
+#pragma unroll 1
+                for (int s0 = 0; s0 < V::kGroupCols; s0 += kStep) {
+                    float v[kStep];
+                    read_step(s0, v);
+                    if (s0 + kStep >= V::kGroupCols) release();
+                    const size_t o = (size_t)(m0 + c_begin + s0) * prm.N + n;
+#pragma unroll
+                    for (int c = 0; c < kStep; ++c) {
+                        if (n < prm.N && s0 + c < tokens && TQ1_IN_BOUNDS(o + (size_t)c * prm.N, (size_t)prm.M * prm.N, 40u)) {
+                            if (prm.y_f32) static_cast<float *>(prm.y)[o + (size_t)c * prm.N] = v[c];
+                            else static_cast<__half *>(prm.y)[o + (size_t)c * prm.N] = __float2half_rn(v[c]);
+                        }
+                    }
+                }
+            }
+        };
+
+        // A segment's results are read out when the group has decoded its first K block of the next one: the ring is full
+        // again by then, and the MMAs go on as soon as the accumulators are in registers, over the stores too (2048 tokens of
+        // 17408x5120 253 us with the results first, 240 now; 777 of 34816x5120 213 and 199, with gates 251 and 219).
+        int done_tile = 0, done_len = 0, done_part = 0;                 // the segment that waits for it (length 0: none)
+        for (;;) {
+            const bool more = walk.next(end_iter, tile, c0, len, part);
+            if (!more) len = V::kDecodeAhead ? 1 : 0;                   // one more turn, for the last segment's results
             for (int u0 = 0; u0 < len; u0 += G) {
                 const int width = min(G, len - u0), unit = u0 + group;
                 const int wave0 = block0;
                 block0 += width * kChunkGroups;
-                if (unit >= len) continue;
-                const uint32_t s = consumed % V::PACK_STAGES;
-                mbar_wait(bar(PACK + warp * V::PACK_STAGES + (int)s), (consumed / V::PACK_STAGES) & 1u, prm.status, dead);
-                // This row's 112 bytes come into registers in two steps (all at once spills); after the second the
-                // buffer is free for the next request.
+                const bool active = more && unit < len;
+                // This row's 112 bytes come into registers in three steps (all at once spills); after the last the buffer is
+                // free for the next request.
                 uint32_t words[4 * 7];
+                const uint32_t s = consumed % V::PACK_STAGES;
                 const uint32_t src = wbase + V::pack_addr(warp, (int)s) + (uint32_t)lane * kChunkBytes;
                 auto fetch = [&](int i) {
                     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                                  : "=r"(words[4 * i]), "=r"(words[4 * i + 1]), "=r"(words[4 * i + 2]), "=r"(words[4 * i + 3])
                                  : "r"(src + 16u * i) : "memory");
                 };
-#pragma unroll
-                for (int i = 0; i < 4; ++i) fetch(i);
-                ++consumed;
-#pragma unroll
-                for (int b = 0; b < kChunkGroups; ++b) {
-                    if (b == 2) {
-#pragma unroll
-                        for (int i = 4; i < 7; ++i) fetch(i);
-                        __syncwarp();
-                        request();
-                    }
+                auto decode = [&](auto block_tag) {                     // K block b of the chunk
+                    constexpr int b = decltype(block_tag)::value;
                     const uint32_t *w = words + 7 * b;
                     const uint32_t pool = (w[0] << 16 >> 8) | (((w[0] & 0xff00u) ^ 0x8000u) << 16);
                     // table entry of code byte j
@@ -528,7 +713,7 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                     // trit 4 of an even byte beside trit 0 of the odd byte after it
                     auto straddle = [&](uint32_t p0, uint32_t q0) { return pick(prmt(p0, q0, V::WIDE ? 0x0062 : 0x0042)); };
                     const uint32_t number = (uint32_t)(wave0 + b * width + group);
-                    const uint32_t stage = number % RING, use = number / RING;
+                    const uint32_t stage = number % RING;
                     const uint32_t a_addr = tmem_lane + (uint32_t)V::kABase + stage * kStageCols;
                     uint32_t m0w, m1w;                                  // byte 12 belongs to both halves
                     {
@@ -544,7 +729,8 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                         }
                         lookup(12, m0w, m1w);
                         even(m0w, m1w, v[30], v[31]);
-                        mbar_wait(bar(EMPTY + (int)stage), (use & 1u) ^ 1u, prm.status, dead);
+                        if (V::kDecodeAhead) wait_read((int)number - RING);
+                        else mbar_wait(bar(EMPTY + (int)stage), (number / RING & 1u) ^ 1u, prm.status, dead);
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         tmem_store32(a_addr, v);
                     }
@@ -575,143 +761,46 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                         const uint32_t full = bar(FULL_A + (int)stage);
                         if (lane == 0) mbar_arrive_leader<CG>(CG == 2 ? leader_addr(full) : full);
                     }
-                }
-            }
-
-            // ---- the segment's accumulator -------------------------------------------------------------------
-            const int m0 = token_tile0(tile), n_tok = tile_tokens(m0);
-            const int n = (weight_tile(tile) * CG + rank) * kTileW + row_in_tile;
-            const int per_group = (n_tok / 16 + G - 1) / G * 16;
-            const int c_begin = group * per_group, cols = min(per_group, n_tok - c_begin);     // cols <= 0: none
-            // the slots that share this tile, worked out while the last products are still being added
-            const int shared_tile = tile - prm.work.whole_tiles, it0 = shared_tile * chunks;
-            int lo = slot, hi = slot;
-            if (len != chunks) {
-                if (prm.work.splits > 0) {
-                    lo = shared_tile * prm.work.splits;
-                    hi = lo + prm.work.splits - 1;
-                } else {
-                    while (prm.work.first_iter(lo) > it0) --lo;
-                    while (prm.work.first_iter(hi + 1) < it0 + chunks) ++hi;
-                }
-            }
-            mbar_wait(bar(ACC_FULL), seg & 1u, prm.status, dead);
-            ++seg;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            constexpr int kStep = 16;                                                          // columns in registers at a time
-            const bool whole = len == chunks;
-            const size_t area = (size_t)prm.nt * kTileW;
-            float *slot_part = prm.partials + ((size_t)2 * blockIdx.x + part) * area + row_in_tile;
+                };
+                auto first_block = [&]() {
+                    mbar_wait(bar(PACK + warp * V::PACK_STAGES + (int)s), (consumed / V::PACK_STAGES) & 1u, prm.status, dead);
 #pragma unroll
-            for (int s0 = 0; s0 < V::kGroupCols; s0 += kStep) {
-                float v[kStep];
-#pragma unroll
-                for (int c = 0; c < kStep; ++c) v[c] = 0.0f;
-                for (int a = 0; a < prm.accs && s0 < cols; ++a) {
-                    float u[kStep];
-                    tmem_load16(tmem_lane + (uint32_t)(a * prm.acc_cols + c_begin + s0), u);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                    for (int c = 0; c < kStep; ++c) {
-                        asm volatile("" : "+f"(u[c]));                                         // no use before the wait
-                        v[c] += u[c];
+                    for (int i = 0; i < (V::kDecodeAhead ? 2 : 4); ++i) fetch(i);
+                    decode(std::integral_constant<int, 0>{});
+                };
+                if (V::kDecodeAhead) {
+                    // Not where the group had no chunk for so long that the wait for its ring stage could take a phase for an
+                    // older one: then the results, and with them the end of all earlier products, come first.
+                    const bool early = done_len == 0 || wave0 + group - RING - seen <= READ_BARS;
+#pragma unroll 1
+                    for (int turn = 0; turn < 2; ++turn) {
+                        if (active && early == (turn == 0)) first_block();
+                        if (done_len) {
+                            finish(done_tile, done_len, done_part);
+                            done_len = 0;
+                        }
                     }
+                } else if (active) {
+                    first_block();
                 }
-                if (s0 + kStep >= V::kGroupCols) {
-                    // the columns are in registers: the next segment may overwrite them while the results are stored
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                if (active) {
+                    if (V::kDecodeAhead) {
+#pragma unroll
+                        for (int i = 1; i < 4; ++i) fetch(i);
+                    }
+                    decode(std::integral_constant<int, 1>{});
+#pragma unroll
+                    for (int i = 4; i < 7; ++i) fetch(i);
+                    ++consumed;
                     __syncwarp();
-                    if (lane == 0) mbar_arrive_leader<CG>(CG == 2 ? leader_addr(bar(ACC_FREE)) : bar(ACC_FREE));
-                }
-                const int col0 = c_begin + s0, tokens = min(cols - s0, prm.M - (m0 + col0));   // of this step's columns
-                if (!whole) {
-                    // a part of the tile's K range: kept as FP32
-#pragma unroll
-                    for (int c = 0; c < kStep; ++c)
-                        if (c < tokens && TQ1_IN_BOUNDS((size_t)(col0 + c) * kTileW + row_in_tile, area, 41u))
-                            __stcg(slot_part + (size_t)(col0 + c) * kTileW, v[c]);
-                } else if (prm.swiglu) {                // (gate, up) row pairs: the even row stores silu(gate) * up
-                    const int out_n = prm.N >> 1;
-#pragma unroll
-                    for (int c = 0; c < kStep; ++c) {
-                        const float up = __shfl_down_sync(0xffffffffu, v[c], 1);
-                        if (c < tokens && (lane & 1) == 0 && n + 1 < prm.N) {
-                            const float out = swiglu_f32(v[c], up);
-                            const size_t o = (size_t)(m0 + col0 + c) * out_n + (n >> 1);
-                            if (!TQ1_IN_BOUNDS(o, (size_t)prm.M * out_n, 40u)) continue;
-                            if (prm.y_f32) static_cast<float *>(prm.y)[o] = out;
-                            else static_cast<__half *>(prm.y)[o] = __float2half_rn(out);
-                        }
-                    }
-                } else if (n < prm.N) {
-                    const size_t o = (size_t)(m0 + col0) * prm.N + n;
-#pragma unroll
-                    for (int c = 0; c < kStep; ++c) {
-                        if (c < tokens && TQ1_IN_BOUNDS(o + (size_t)c * prm.N, (size_t)prm.M * prm.N, 40u)) {
-                            if (prm.y_f32) static_cast<float *>(prm.y)[o + (size_t)c * prm.N] = v[c];
-                            else static_cast<__half *>(prm.y)[o + (size_t)c * prm.N] = __float2half_rn(v[c]);
-                        }
-                    }
+                    request();
+                    decode(std::integral_constant<int, 2>{});
+                    decode(std::integral_constant<int, 3>{});
                 }
             }
-            if (whole) continue;
-            // The slot that completes the tile's count adds the parts.
-            asm volatile("bar.sync 1, %0;" ::"n"(kDecode * 32) : "memory");
-            if (tid == 0) {
-                // the barrier orders the other warps' stores before this thread's release, and its acquire before their reads
-                unsigned *counter = prm.counters + shared_tile * CG + rank, before;
-                asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
-                const bool last = before == (unsigned)(hi - lo);
-                if (last) *counter = 0u;                // zero for the next call
-                if (before > (unsigned)(hi - lo)) atomicExch(prm.status, 8u);     // it was not zero when the call began
-                *last_flag = last ? 1u : 0u;
-            }
-            asm volatile("bar.sync 1, %0;" ::"n"(kDecode * 32) : "memory");
-            if (*last_flag == 0u) continue;
-            const int all = min(n_tok, prm.M - m0), quads = all * (kTileW / 4);      // four rows of a column each
-            constexpr int kThreadsR = kDecode * 32, kFlight = 4;
-            const int tile_n0 = (weight_tile(tile) * CG + rank) * kTileW;
-            for (int i0 = tid; i0 < quads; i0 += kThreadsR * kFlight) {
-                float4 total[kFlight];
-#pragma unroll
-                for (int f = 0; f < kFlight; ++f) total[f] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 2
-                for (int sl = lo; sl <= hi; ++sl) {
-                    // the tile is that slot's first segment of shared tiles if its range starts inside the tile
-                    const int which = prm.work.splits > 0 || prm.work.first_iter(sl) >= it0 ? 0 : 1;
-                    const float4 *src = reinterpret_cast<const float4 *>(
-                        prm.partials + ((size_t)2 * (sl * CG + rank) + which) * area);
-#pragma unroll
-                    for (int f = 0; f < kFlight; ++f) {
-                        const int i = i0 + f * kThreadsR;
-                        const float4 p = i < quads ? __ldcg(src + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        total[f].x += p.x; total[f].y += p.y; total[f].z += p.z; total[f].w += p.w;
-                    }
-                }
-#pragma unroll
-                for (int f = 0; f < kFlight; ++f) {
-                    const int i = i0 + f * kThreadsR, m = m0 + (i >> 5), nq = tile_n0 + (i & 31) * 4;
-                    if (i >= quads) break;
-                    float r[4] = {total[f].x, total[f].y, total[f].z, total[f].w};
-                    int count = min(4, prm.N - nq);
-                    size_t o = (size_t)m * prm.N + nq;
-                    size_t limit = (size_t)prm.M * prm.N;
-                    if (prm.swiglu) {
-                        r[0] = swiglu_f32(r[0], r[1]);
-                        r[1] = swiglu_f32(r[2], r[3]);
-                        count >>= 1;
-                        o = (size_t)m * (prm.N >> 1) + (nq >> 1);
-                        limit >>= 1;
-                    }
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        if (e < count && TQ1_IN_BOUNDS(o + e, limit, 40u)) {
-                            if (prm.y_f32) static_cast<float *>(prm.y)[o + e] = r[e];
-                            else static_cast<__half *>(prm.y)[o + e] = __float2half_rn(r[e]);
-                        }
-                    }
-                }
-            }
+            if (!more) break;
+            if (V::kDecodeAhead) { done_tile = tile; done_len = len; done_part = part; }
+            else finish(tile, len, part);
         }
     }
 
@@ -842,11 +931,11 @@ Tiling pick_tiling(int M, int N, int K) { return make_tiling(token_tile(M, N, K)
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
-template <class V>
+template <class V, bool GATED>
 int launch_variant(const CUtensorMap &wmap, const CUtensorMap &xmap, GemmParams &prm, int ctas, cudaStream_t stream) {
     const int stages = (int)(V::kBRoom / ((uint32_t)prm.b_rows * 256u));
     prm.b_stages = stages < V::RING ? stages : V::RING;
-    auto kern = tq1_gemm_kernel<V>;
+    auto kern = tq1_gemm_kernel<V, GATED>;
     static KernelRecord record;
     const cudaError_t e = opt_in(record, reinterpret_cast<const void *>(kern), V::kSmemBytes);
     if (e != cudaSuccess) return cuda_fail(e, "tq1_linear_f16: shared memory opt-in (GEMM)");
@@ -935,7 +1024,7 @@ int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, 
     prm.acc_cols = acc_area / prm.accs;
     prm.work = t.work;
     prm.y_f32 = y_f32 ? 1 : 0;
-    prm.swiglu = swiglu ? 1 : 0;
+    prm.pair_y = N % 2 == 0 && (reinterpret_cast<uintptr_t>(y) & 3) == 0 ? 1 : 0;
 
     CUtensorMap wmap, xmap;
     const cuuint32_t estr[2] = {1, 1};
@@ -963,9 +1052,13 @@ int launch_gemm_tc(const uint8_t *blocks, const __half *x, void *y, bool y_f32, 
         if (res != CUDA_SUCCESS)
             return fail(TQ1_ERR_CUDA, "tq1_linear_f16: activation tensor map failed (%d)", (int)res);
     }
-    return t.tile <= 32    ? launch_variant<VariantS>(wmap, xmap, prm, t.ctas(), stream)
-           : t.tile <= 128 ? launch_variant<VariantL>(wmap, xmap, prm, t.ctas(), stream)
-                           : launch_variant<VariantP>(wmap, xmap, prm, t.ctas(), stream);
+    const auto launch = [&](auto gated) {
+        constexpr bool GATED = decltype(gated)::value;
+        return t.tile <= 32    ? launch_variant<VariantS, GATED>(wmap, xmap, prm, t.ctas(), stream)
+               : t.tile <= 128 ? launch_variant<VariantL, GATED>(wmap, xmap, prm, t.ctas(), stream)
+                               : launch_variant<VariantP, GATED>(wmap, xmap, prm, t.ctas(), stream);
+    };
+    return swiglu ? launch(std::true_type{}) : launch(std::false_type{});
 }
 
 }  // namespace tq1

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from oracle import c_oracle, tq1_oracle as o
-from tests.gpu_util import POWERS, random_blocks, run_linear
+from tests.gpu_util import POWERS, random_blocks, run_linear, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -229,3 +229,25 @@ def test_error_grows_with_the_columns_of_one_accumulator_only(batch, rows, colum
     want = x.double() @ dense.T
     got = tq1_matmul(blocks, x, out_dtype=torch.float32).double()
     assert float((got - want).norm() / want.norm()) < 0.48 * span / 16 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("columns", (512, 1536, 2560, 3584))
+def test_segments_that_follow_one_another(columns):
+    """Several tiles per CTA, of one, three, five and seven chunks: the decoding groups go on to the next tile before the
+    results of this one are read out, and some have no chunk in it. Whole numbers, so every sum is exact."""
+    from ternel_b200.ops import tq1_matmul, tq1_swiglu
+    rows = 40008
+    rng = np.random.default_rng(columns)
+    trits = rng.integers(0, 3, size=(rows * columns // 128, 128), dtype=np.uint8)
+    blocks = to_dev(o.encode_blocks(ones_scale(rows * columns // 128), trits).reshape(rows, columns // 128, 28))
+    dense = to_dev(trits.reshape(rows, columns)).float() - 1
+    for batch in (24, 100, 300):
+        x = torch.randint(-1, 2, (batch, columns), device="cuda").to(torch.float16)
+        want = x.float() @ dense.T
+        assert torch.equal(tq1_matmul(blocks, x, out_dtype=torch.float32), want)
+        assert torch.equal(tq1_matmul(blocks, x), want.half())
+        assert torch.equal(tq1_matmul(blocks[:rows - 1], x), want[:, :rows - 1].half())
+        gate, up = want[:, 0::2], want[:, 1::2]
+        # silu in FP32: exp and the division differ from PyTorch's by a few units in the last place
+        torch.testing.assert_close(tq1_swiglu(blocks, x, out_dtype=torch.float32), torch.nn.functional.silu(gate) * up,
+                                   rtol=2e-6, atol=1e-30)
