@@ -37,7 +37,7 @@ constexpr size_t kWsScratchOffset = kWsCounterOffset + kWsCounterBytes;
 // which clamps row indices (src/ternel_mlx/kernels.py:23-27). tq1_debug_bounds() reads the record.
 // Codes: 1x chain kernel (10 slot store, 11 slot read, 12 y, 13 hand-off store, 14 hand-off read),
 // 2x row kernel, 3x gather, 4x batched kernel (40 result, 41 partial tile), 5x panels, 6x shard push,
-// 7x group sums, 8x slice kernel.
+// 7x group sums, 8x slice kernel, 9x tile kernel.
 #ifdef TQ1_BOUNDS_CHECK
 extern __device__ unsigned long long g_tq1_bounds[4];
 __device__ __forceinline__ bool tq1_in_bounds(long long index, long long limit, unsigned code) {
@@ -162,6 +162,10 @@ int gemv_set_loop_tokens(int tokens);       // sweep recording only; process-glo
 // slot_bytes: room for partial-sum slots behind the workspace's control words
 int launch_gemv_single(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int N, int K, bool swiglu,
                        void *workspace, size_t slot_bytes, cudaStream_t stream);
+// One or two activation rows with a row's whole sum inside a CTA or a cluster. Launches it (`status` is what came of that; the
+// workspace's first word is the status word) and returns true where it takes the call.
+bool try_gemv_tiles(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, bool swiglu, void *workspace,
+                    cudaStream_t stream, int *status);
 int launch_shard_wait(const ShardDev &shard, unsigned *status, cudaStream_t stream);
 int launch_shard_push(const __half *local, int M, int n_local, const ShardDev &shard, cudaStream_t stream);
 int launch_epoch_advance(unsigned *epoch_base, unsigned delta, cudaStream_t stream);

@@ -53,17 +53,12 @@
 #include <type_traits>
 #include <vector>
 
-#include "tq1_common.cuh"
+#include "tq1_gemv_unit.cuh"
 
 namespace tq1 {
 
 namespace {
 
-constexpr int kTileRows = 16;
-constexpr int kChunkGroups = 4;
-constexpr int kChunkCols = kChunkGroups * kGroup;             // 512
-constexpr int kChunkBytes = kChunkGroups * kBlockBytes;       // 112
-constexpr int kUnitBytes = kTileRows * kChunkBytes;           // 1792
 #ifndef TQ1_GEMV_WARPS
 #define TQ1_GEMV_WARPS 16
 #endif
@@ -75,18 +70,7 @@ constexpr int kWarps = TQ1_GEMV_WARPS;           // warp w < 4 * (chunks of the 
 constexpr int kThreads = kWarps * 32;
 constexpr int kMaxChunksPerCta = 3;
 constexpr int kPrepWarps = 4 * kMaxChunksPerCta;               // one warp per 128-activation group
-constexpr int kRegsPerSub = 18;                                // A/B registers per lane per sub-unit
 static_assert(kWarps >= kPrepWarps, "one warp per activation group of the CTA's chunks");
-
-// Per activation group, written by the warp that prepared it: 121 * (sum of the fifth-trit activations),
-// 2^(E-21) for the group's exponent E, and how many of its activations are Inf (kGroupNan: one is NaN).
-constexpr int kGroupNan = 1 << 30;
-struct alignas(16) GroupConst {
-    int sum;
-    float pow;
-    int bad;
-    int pad;
-};
 
 // Shared-memory window layout (addresses relative to the CTA's shared window). The table sits
 // at a 64 KiB multiple so that PRMT can build a complete lookup address
@@ -96,16 +80,15 @@ constexpr uint32_t kLutWindowAddr = 131072;
 constexpr uint32_t kLutBytes = 256 * 256;                     // 256 entries x (2 x 32 lanes x 4 B)
 constexpr uint32_t kWindowEnd = kLutWindowAddr + kLutBytes;   // 196608
 constexpr uint32_t kRingBytes = kWarps * kStages * kUnitBytes;                     // 114688
-constexpr uint32_t kBtabChunk = 2 * kRegsPerSub * 32 * 4;                          // 4608: digit planes of one chunk
-constexpr uint32_t kBtabOne = kMaxChunksPerCta * kBtabChunk;                       // 13824 per buffer
+constexpr uint32_t kBtabChunk = kPlaneChunk;
+constexpr uint32_t kBtabOne = kMaxChunksPerCta * kBtabChunk;                       // per buffer
 constexpr uint32_t kBtabBytes = 2 * kBtabOne;                                      // two links in flight
 constexpr uint32_t kMbarBytes = 8 * (kWarps * kStages + 2);
 constexpr uint32_t kGconstOne = kPrepWarps * sizeof(GroupConst);
 constexpr uint32_t kGconstBytes = 2 * kGconstOne;
 constexpr uint32_t kXchgBytes = kPrepWarps * kGroup * 4;                           // a warp's fixed-point activations
-constexpr uint32_t kPrepTabBytes = kGroup * 4;                                     // where activation e of a group goes
 constexpr uint32_t kMiscBytes = 16;
-constexpr uint32_t kHighBytes = kBtabBytes + kMbarBytes + kGconstBytes + kXchgBytes + kPrepTabBytes + kMiscBytes;
+constexpr uint32_t kHighBytes = kBtabBytes + kMbarBytes + kGconstBytes + kXchgBytes + kMiscBytes;
 static_assert(kRingBytes + 1024 + 128 <= kLutWindowAddr, "the ring must end below the table's fixed address");
 static_assert(kWindowEnd + kHighBytes <= 227 * 1024, "shared memory budget");
 constexpr uint32_t kMaxWaitSpins = 1u << 21;
@@ -195,50 +178,6 @@ constexpr LutImage make_lut_image() {
 __device__ __align__(128) const LutImage g_chain_lut = make_lut_image();
 static_assert(sizeof(LutImage) == kLutBytes, "table image size");
 
-template <uint32_t SEL>
-__device__ __forceinline__ uint32_t prmt_imm(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "n"(SEL));
-    return d;
-}
-// Ring-buffer words. Not volatile: the address depends on the value returned by the barrier wait,
-// which keeps the loads behind it while leaving the compiler free to interleave the two sub-units.
-template <int OFF>
-__device__ __forceinline__ uint32_t lds_off(uint32_t addr) {
-    uint32_t v;
-    asm("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(addr), "n"(OFF));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds_lut(uint32_t addr) {
-    uint32_t v;
-    asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-    return v;
-}
-
-template <bool SIGNED_A, bool ZERO_C>
-__device__ __forceinline__ void mma_bytes(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                          uint32_t b0, uint32_t b1) {
-    if (ZERO_C) {
-        if (SIGNED_A)
-            asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
-                : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
-                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0), "r"(0), "r"(0), "r"(0));
-        else
-            asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-                : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
-                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
-    } else {
-        if (SIGNED_A)
-            asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-        else
-            asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    }
-}
-
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
@@ -283,31 +222,6 @@ __device__ __forceinline__ void elected_tma_load_2d(uint32_t dst, const CUtensor
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-
-// One lane-stream (half a block: 14 code-byte slots in four words, wa holding slots 0,1 in its
-// upper half) becomes 18 A registers: 14 table entries (weights of trits 0..3 of each slot) and
-// the four raw words (the code bytes themselves, paired with the fifth trit's activation).
-__device__ __forceinline__ void decode_stream(uint32_t wa, uint32_t wb, uint32_t wc, uint32_t wd,
-                                              uint32_t lane_base, uint32_t (&r)[kRegsPerSub]) {
-    r[0] = lds_lut(prmt_imm<0x7624>(wa, lane_base));
-    r[1] = lds_lut(prmt_imm<0x7634>(wa, lane_base));
-    r[2] = lds_lut(prmt_imm<0x7604>(wb, lane_base));
-    r[3] = lds_lut(prmt_imm<0x7614>(wb, lane_base));
-    r[4] = lds_lut(prmt_imm<0x7624>(wb, lane_base));
-    r[5] = lds_lut(prmt_imm<0x7634>(wb, lane_base));
-    r[6] = lds_lut(prmt_imm<0x7604>(wc, lane_base));
-    r[7] = lds_lut(prmt_imm<0x7614>(wc, lane_base));
-    r[8] = lds_lut(prmt_imm<0x7624>(wc, lane_base));
-    r[9] = lds_lut(prmt_imm<0x7634>(wc, lane_base));
-    r[10] = lds_lut(prmt_imm<0x7604>(wd, lane_base));
-    r[11] = lds_lut(prmt_imm<0x7614>(wd, lane_base));
-    r[12] = lds_lut(prmt_imm<0x7624>(wd, lane_base));
-    r[13] = lds_lut(prmt_imm<0x7634>(wd, lane_base));
-    r[14] = wa;
-    r[15] = wb;
-    r[16] = wc;
-    r[17] = wd;
 }
 
 // 64-bit words {payload, tag}: a 64-bit store is a single access, so a reader that finds the tag
@@ -386,7 +300,8 @@ __device__ __forceinline__ WarpRange warp_range(int tiles, int units_q, int unit
 // kChain, kAlone: some weights are canonical; a chain of links, and independent products of one matrix. They differ in where
 // non-finite groups are dealt with: in a copy of the unit loop (kAlone, kPanels), or at the end of a unit of the one loop
 // (kChain). Which of the two leaves the compiler's common loop the faster differs from form to form: eight canonical layers
-// 262.7 us with two loops, 259.3 with one; eight panel layers 249.8 and 256.0; 151936x5120 alone 53.6 and 54.3.
+// 262.7 us with two loops, 259.3 with one; eight panel layers 249.8 and 256.0; 151936x5120 alone 53.6 and 54.3. Products of one
+// matrix come here only where the tile kernel (tq1_gemv_tiles.cu) has no room for their sums.
 enum Form { kPanels, kChain, kAlone };
 template <Form FORM>
 __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __grid_constant__ ChainParams P) {
@@ -395,12 +310,11 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
     const uint32_t window = (uint32_t)__cvta_generic_to_shared(smem);
     unsigned char *high = smem + (kWindowEnd - window);
     uint32_t *btab_all = reinterpret_cast<uint32_t *>(high);
+    const uint32_t btab_addr = kWindowEnd;
     uint64_t *mbars = reinterpret_cast<uint64_t *>(high + kBtabBytes);
     GroupConst *gconst_all = reinterpret_cast<GroupConst *>(high + kBtabBytes + kMbarBytes);      // [buffer][group]
     int *xchg = reinterpret_cast<int *>(high + kBtabBytes + kMbarBytes + kGconstBytes) + (threadIdx.x >> 5) * kGroup;
-    uint32_t *preptab = reinterpret_cast<uint32_t *>(high + kBtabBytes + kMbarBytes + kGconstBytes + kXchgBytes);
-    volatile int *region_ok = reinterpret_cast<volatile int *>(high + kBtabBytes + kMbarBytes + kGconstBytes +
-                                                               kXchgBytes + kPrepTabBytes);
+    volatile int *region_ok = reinterpret_cast<volatile int *>(high + kBtabBytes + kMbarBytes + kGconstBytes + kXchgBytes);
     unsigned *ctl = P.ctl;
     if (window + kRingBytes > kLutWindowAddr) {      // the fixed-address table would overlap the ring
         if (threadIdx.x == 0) atomicExch(ctl + kCtlStatus, 2u);
@@ -493,27 +407,8 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
     // byte offset of this lane's first half-block inside a tile (sub-unit 0, row g)
     const uint32_t lane_tile_off = (uint32_t)(((g * kChunkGroups + 2 * cls) * kBlockWords + 3 * h) * 4);
 
-    // Where activation e of a group goes. Trits 0..3 of code byte j sit in the table-entry register of the
-    // byte's slot; a fifth trit pairs with the raw word. Entry: byte offset of digit 0 inside a group's planes
-    // (bits 0..15), index of the byte's fifth-trit activation (16..23, 255: the tail byte has none) and 3^i
-    // (24..31, 0 for a fifth trit).
-    if (tid < kGroup) {
-        const int el = tid;
-        const int bj = el < 125 ? el / 5 : 25;             // code byte
-        const int bi = el < 125 ? el - 5 * bj : el - 125;  // trit within the byte
-        const bool is_fifth = el < 125 && bi == 4;
-        const int hh = bj < 14 ? 0 : 1;                    // which half-block lane decodes the byte
-        const int slot = hh ? bj - 12 : bj;
-        const int reg = !is_fifth ? slot : slot < 2 ? 14 : 15 + ((slot - 2) >> 2);
-        const int pos = !is_fifth ? bi : slot < 2 ? slot + 2 : ((slot - 2) & 3);
-        const uint32_t off = (uint32_t)((reg * 32 + hh) * 4 + pos);
-        const uint32_t fifth = el < 125 ? (uint32_t)(5 * bj + 4) : 255u;
-        const uint32_t pow3 = is_fifth ? 0u : bi == 0 ? 1u : bi == 1 ? 3u : bi == 2 ? 9u : 27u;
-        preptab[el] = off | (fifth << 16) | (pow3 << 24);
-    }
     if (tid == 0) *region_ok = 0;
-    // planes of group gi of a chunk: sub-unit gi & 1, B lanes 18 * (gi >> 1) + {0, 1} (+ 4 per digit plane)
-    const uint32_t warp_plane_off = (uint32_t)(((warp & 1) * kRegsPerSub * 32 + 18 * ((warp >> 1) & 1)) * 4);
+    const int warp_plane_off = plane_group(warp & 3);
 
     bool dead = false;                                 // a bounded wait ran out: stop waiting, finish quickly
     __syncthreads();                                   // barriers initialised, planes zeroed, table written
@@ -541,10 +436,10 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
         if (warp < 4 * (chunk_hi - chunk_lo + 1)) {
             const int cl = warp >> 2;
             const size_t x0 = (size_t)(chunk_lo + cl) * kChunkCols + (size_t)(warp & 3) * kGroup + lane;
-            float xv[4];
+            float xv[1][4];
             if (xin == nullptr) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) xv[k] = __half2float(xh[x0 + 32 * k]);
+                for (int k = 0; k < 4; ++k) xv[0][k] = __half2float(xh[x0 + 32 * k]);
                 // The activation loads are in flight: now top up this warp's weight tiles (issued the other
                 // way round the few activation bytes queue behind megabytes of weight traffic).
                 while (issued - consumed < kStages - 1 && issue_one()) {}
@@ -557,7 +452,7 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
                 const int parts = max(1, (int)((flags >> kFlagSrcPartsShift) & 15u));
                 const size_t part_stride = (size_t)L.src_stride;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) xv[k] = 0.0f;
+                for (int k = 0; k < 4; ++k) xv[0][k] = 0.0f;
                 // one pass per rank that contributed a partial sum (a single pass for an ordinary source); the
                 // partial sums are added in rank order, so the result does not depend on arrival order
                 if (parts == 2) {
@@ -581,7 +476,7 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
                         if (spins > kMaxWaitSpins) { atomicExch(ctl + kCtlStatus, 4u); dead = true; }
                     }
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) xv[k] = (0.0f + word_value(wa[k], src_f32)) + word_value(wb[k], src_f32);
+                    for (int k = 0; k < 4; ++k) xv[0][k] = (0.0f + word_value(wa[k], src_f32)) + word_value(wb[k], src_f32);
                 } else
                 for (int r = 0; r < parts; ++r) {
                     const unsigned long long *src = xin + (size_t)r * part_stride + x0;
@@ -605,77 +500,17 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
                         if (spins > kMaxWaitSpins) { atomicExch(ctl + kCtlStatus, 4u); dead = true; }
                     }
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) xv[k] += word_value(wv[k], src_f32);
+                    for (int k = 0; k < 4; ++k) xv[0][k] += word_value(wv[k], src_f32);
                 }
                 if (src_f32) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) xv[k] = round_to_half(xv[k]);
+                    for (int k = 0; k < 4; ++k) xv[0][k] = round_to_half(xv[0][k]);
                 }
             }
             PHASE(0)
-            // non-negative floats order like their bit patterns: one redux instruction for the group maximum
-            unsigned mbits = 0u;
-            bool bad[4], anybad = false;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float a = fabsf(xv[k]);
-                bad[k] = !(a <= 65504.0f);                         // NaN or Inf
-                anybad = anybad || bad[k];
-                mbits = max(mbits, bad[k] ? 0u : __float_as_uint(a));
-            }
-            mbits = __reduce_max_sync(0xffffffffu, mbits);
-            // 2^E <= m < 2^(E+1); fixed point xi = round(v * 2^(21-E)), |xi| <= 2^22
-            const int e_biased = mbits != 0u ? (int)(mbits >> 23) : 127;
-            const float up = __uint_as_float((uint32_t)(275 - e_biased) << 23);                // 2^(21-E)
-            int xi[4], s5 = 0;
-            uint32_t ent[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) xi[k] = __float2int_rn(xv[k] * up);
-            int group_bad = __any_sync(0xffffffffu, anybad);           // infinite activations, or kGroupNan
-            if (group_bad) {                            // rare; a finite group executes nothing of this
-                int infs = 0;
-                bool nan = false;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    infs += bad[k] ? 1 : 0;
-                    nan = nan || xv[k] != xv[k];
-                    xi[k] = bad[k] ? (xv[k] < 0.0f ? -1 : 1) : 0;
-                }
-                infs = __reduce_add_sync(0xffffffffu, infs);
-                group_bad = __any_sync(0xffffffffu, nan) ? kGroupNan : infs;
-            }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                xchg[lane + 32 * k] = xi[k];                       // a code byte's first four trits need its fifth
-                ent[k] = preptab[lane + 32 * k];
-                s5 += (ent[k] >> 24) == 0u ? 121 * xi[k] : 0;      // 121 * sum of the fifth-trit activations
-            }
-            s5 = __reduce_add_sync(0xffffffffu, s5);
-            if (lane == 0) {
-                GroupConst gc;
-                gc.sum = s5;
-                gc.pow = __uint_as_float((uint32_t)(e_biased - 21) << 23);                     // 2^(E-21)
-                gc.bad = group_bad;
-                gc.pad = 0;
-                gconst[warp] = gc;
-            }
-            __syncwarp();
-            unsigned char *planes = reinterpret_cast<unsigned char *>(btab) + cl * kBtabChunk + warp_plane_off;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                // value paired with this k-slot: x_4 for the raw byte, 81 x_i - 3^i x_4 for trit i < 4
-                const uint32_t fifth = (ent[k] >> 16) & 0xffu;
-                const int x4 = fifth != 255u ? xchg[fifth] : 0;
-                const int pw = (int)(ent[k] >> 24);
-                const int v = pw ? 81 * xi[k] - pw * x4 : xi[k];
-                // four signed byte digits: the bytes of v + 0x80808080 are the digits plus 128
-                const uint32_t d = ((uint32_t)v + 0x80808080u) ^ 0x80808080u;
-                unsigned char *base = planes + (ent[k] & 0xffffu);
-                base[0] = (unsigned char)d;
-                base[16] = (unsigned char)(d >> 8);
-                base[32] = (unsigned char)(d >> 16);
-                base[48] = (unsigned char)(d >> 24);
-            }
+            unsigned char *const planes[1] = {reinterpret_cast<unsigned char *>(btab) + cl * kBtabChunk + warp_plane_off};
+            GroupConst *const consts[1] = {gconst + warp};
+            prepare_groups<1, false>(xv, 1, lane, xchg, planes, consts);
         } else {
             while (issued - consumed < kStages - 1 && issue_one()) {}
             PHASE(0)
@@ -709,7 +544,7 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
 
         // ---- per-warp streaming loop -------------------------------------------------------------------
         unsigned long long *slots = P.slots + (P.n_regions > 1 ? (size_t)(p & 1) * P.region_slots : 0);
-        uint32_t breg[2][kRegsPerSub];
+        uint32_t breg[2 * kRegsPerSub];
         int gsum[2];
         float gpow[2];
         int gbad[2];
@@ -731,11 +566,9 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
         for (int left = n_units; left > 0;) {
             // ---- (re)load the B fragments and the group constants of this K chunk ----------------------
             const int cl = c - chunk_lo;
+            load_planes(breg, btab_addr + (uint32_t)(buf * kBtabOne + cl * kBtabChunk), lane);
 #pragma unroll
             for (int sub = 0; sub < 2; ++sub) {
-#pragma unroll
-                for (int r = 0; r < kRegsPerSub; ++r)
-                    breg[sub][r] = btab[((cl * 2 + sub) * kRegsPerSub + r) * 32 + lane];
                 const GroupConst gc = gconst[cl * 4 + sub + 2 * cls];
                 gsum[sub] = gc.sum;
                 gpow[sub] = gc.pow;
@@ -776,20 +609,20 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
                     const uint32_t w2c = sub ? lds_off<kRow8 + 36>(a1) : lds_off<kRow8 + 8>(a1);
                     const uint32_t w2d = sub ? lds_off<kRow8 + 40>(a1) : lds_off<kRow8 + 12>(a1);
                     uint32_t r1[kRegsPerSub], r2[kRegsPerSub];
-                    decode_stream(w1a, w1b, w1c, w1d, lane_base, r1);
-                    decode_stream(w2a, w2b, w2c, w2d, lane_base, r2);
+                    decode_stream<0>(w1a, w1b, w1c, w1d, lane_base, r1);
+                    decode_stream<0>(w2a, w2b, w2c, w2d, lane_base, r2);
                     // One accumulator chain (splitting it in two or three measured the same and costs registers and
                     // additions); register pairs 0..6 hold signed weights, pairs 7,8 the raw (unsigned) code bytes.
                     int acc[4];
-                    mma_bytes<true, true>(acc, r1[0], r2[0], r1[1], r2[1], breg[sub][0], breg[sub][1]);
-                    mma_bytes<true, false>(acc, r1[2], r2[2], r1[3], r2[3], breg[sub][2], breg[sub][3]);
-                    mma_bytes<true, false>(acc, r1[4], r2[4], r1[5], r2[5], breg[sub][4], breg[sub][5]);
-                    mma_bytes<true, false>(acc, r1[6], r2[6], r1[7], r2[7], breg[sub][6], breg[sub][7]);
-                    mma_bytes<true, false>(acc, r1[8], r2[8], r1[9], r2[9], breg[sub][8], breg[sub][9]);
-                    mma_bytes<true, false>(acc, r1[10], r2[10], r1[11], r2[11], breg[sub][10], breg[sub][11]);
-                    mma_bytes<true, false>(acc, r1[12], r2[12], r1[13], r2[13], breg[sub][12], breg[sub][13]);
-                    mma_bytes<false, false>(acc, r1[14], r2[14], r1[15], r2[15], breg[sub][14], breg[sub][15]);
-                    mma_bytes<false, false>(acc, r1[16], r2[16], r1[17], r2[17], breg[sub][16], breg[sub][17]);
+                    mma_bytes<true, true>(acc, r1[0], r2[0], r1[1], r2[1], breg[sub * kRegsPerSub + 0], breg[sub * kRegsPerSub + 1]);
+                    mma_bytes<true, false>(acc, r1[2], r2[2], r1[3], r2[3], breg[sub * kRegsPerSub + 2], breg[sub * kRegsPerSub + 3]);
+                    mma_bytes<true, false>(acc, r1[4], r2[4], r1[5], r2[5], breg[sub * kRegsPerSub + 4], breg[sub * kRegsPerSub + 5]);
+                    mma_bytes<true, false>(acc, r1[6], r2[6], r1[7], r2[7], breg[sub * kRegsPerSub + 6], breg[sub * kRegsPerSub + 7]);
+                    mma_bytes<true, false>(acc, r1[8], r2[8], r1[9], r2[9], breg[sub * kRegsPerSub + 8], breg[sub * kRegsPerSub + 9]);
+                    mma_bytes<true, false>(acc, r1[10], r2[10], r1[11], r2[11], breg[sub * kRegsPerSub + 10], breg[sub * kRegsPerSub + 11]);
+                    mma_bytes<true, false>(acc, r1[12], r2[12], r1[13], r2[13], breg[sub * kRegsPerSub + 12], breg[sub * kRegsPerSub + 13]);
+                    mma_bytes<false, false>(acc, r1[14], r2[14], r1[15], r2[15], breg[sub * kRegsPerSub + 14], breg[sub * kRegsPerSub + 15]);
+                    mma_bytes<false, false>(acc, r1[16], r2[16], r1[17], r2[17], breg[sub * kRegsPerSub + 16], breg[sub * kRegsPerSub + 17]);
                     // columns: lane q=0 holds planes 0,1 of the first group, q=1 planes 2,3; q=2/3 the second group.
                     // Combine each lane's plane pair first, then one shuffle per row brings the upper pair over.
                     const uint32_t pair1 = (uint32_t)acc[0] + ((uint32_t)acc[1] << 8);
@@ -1238,8 +1071,10 @@ size_t gemv_chain_link_bytes() { return sizeof(ChainLinkDev); }
 // One product through the chain kernel (a chain of one link per row range).
 int launch_gemv_single(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int N, int K, bool swiglu,
                        void *workspace, size_t slot_bytes, cudaStream_t stream) {
+    int rc;
+    if (try_gemv_tiles(blocks, x, y, y_f32, 1, N, K, swiglu, workspace, stream, &rc)) return rc;
     int grid = 0;
-    int rc = gemv_chain_grid(&grid);
+    rc = gemv_chain_grid(&grid);
     if (rc != TQ1_OK) return rc;
     // single links never run ahead of one another inside a launch, so one region holds all the slots
     const size_t region_slots = slot_bytes / sizeof(unsigned long long);
@@ -1258,13 +1093,14 @@ int launch_gemv_single(const uint8_t *blocks, const __half *x, void *y, bool y_f
 }
 
 
-// A few activation rows through the batch-1 kernel: one launch of M independent links over the same weights
-// (the second and later passes read them from L2). Faster than the batched kernel while M passes cost less
-// than its decode-to-tensor-memory pipeline; the crossover is recorded by the dispatch sweep.
+// Two activation rows: the tile kernel, else (and for more rows, while a sweep is recorded) one launch of M independent links over
+// the same weights, of which the second and later passes read them from L2.
 int launch_gemv_looped(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, bool swiglu,
                        void *workspace, cudaStream_t stream) {
+    int rc;
+    if (try_gemv_tiles(blocks, x, y, y_f32, M, N, K, swiglu, workspace, stream, &rc)) return rc;
     int grid = 0;
-    int rc = gemv_chain_grid(&grid);
+    rc = gemv_chain_grid(&grid);
     if (rc != TQ1_OK) return rc;
     if (M < 1 || M > kInlineLinks) return fail(TQ1_ERR_INVALID, "tq1 chain: %d activation rows do not fit one launch", M);
     tq1_chain_link links[kInlineLinks];
@@ -1286,8 +1122,8 @@ int launch_gemv_looped(const uint8_t *blocks, const __half *x, void *y, bool y_f
 
 // Largest M that tq1_linear_f16 sends through launch_gemv_looped (0 or 1: none). Every matrix that the batch-1 kernel takes
 // goes this way, because its sums are exact integers per group: two tokens of 5120x5120 are 7e-8 from the FP64 result
-// (2-norm) against 1.2e-6 of the batched kernel's FP32 accumulators. Two tokens, weights out of HBM, this path and the
-// batched kernel: 1024x5120 8.9 and 9.7 us, 5120x5120 11.6 and 10.8, 17408x5120 19.0 and 17.9.
+// (2-norm) against 1.2e-6 of the batched kernel's FP32 accumulators. Two tokens, weights out of HBM, the tile kernel, two links of
+// the chain kernel and the batched kernel: 1024x5120 4.8, 8.9 and 9.7 us, 5120x5120 9.0, 11.6 and 10.8, 17408x5120 14.7, 19.0 and 17.9.
 static int g_loop_tokens = 2;
 bool gemv_loop_preferred(int M) { return M >= 2 && M <= g_loop_tokens; }
 int gemv_set_loop_tokens(int tokens) {

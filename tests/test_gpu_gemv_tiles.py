@@ -1,0 +1,90 @@
+"""One and two activation rows by the tile kernel: bit for bit what the chain kernel gives for one link. Needs a B200."""
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import tq1_oracle as o
+from tests.gpu_util import random_blocks, to_dev
+
+pytestmark = pytest.mark.gpu
+
+# (rows, columns): one row, tile remainders, twenty sets of one chunk and fewer; the widest K range of one CTA (18 chunks), and
+# clusters of two (19 chunks: uneven halves, 34), four (two activation rows of 34) and eight (128 chunks: the most); several tiles
+# per set, more tiles than ring stages
+SHAPES = ((1, 512), (15, 512), (2375, 512), (50002, 512), (33, 1536), (4100, 4096), (12018, 5120), (2400, 9216), (2390, 9728),
+          (1202, 17408), (49, 65536))
+
+
+def single_links(blocks, x, swiglu):
+    from ternel_b200.chain import ChainPlan, Link
+    rows = blocks.shape[0] // 2 if swiglu else blocks.shape[0]
+    y = torch.empty((x.shape[0], rows), dtype=torch.float32, device="cuda")
+    for m in range(x.shape[0]):
+        ChainPlan([Link(blocks=blocks, x=x[m], y=y[m], swiglu=swiglu)]).run()
+    torch.cuda.synchronize()
+    return y
+
+
+@pytest.mark.parametrize(("rows", "columns"), SHAPES)
+def test_equals_the_chain_kernel(rows, columns):
+    from ternel_b200.ops import tq1_matmul, tq1_swiglu
+    host, rng = random_blocks(rows, columns, seed=rows + columns, dist="tests")
+    blocks = to_dev(host)
+    x = to_dev(rng.standard_normal((2, columns)).astype(np.float16))
+    x[1, ::3] *= 2.0 ** -9                      # groups of a wide range
+    want = single_links(blocks, x, False)
+    if rows * columns < 6_000_000:
+        exact = o.float64_matmul(host, x.cpu().numpy(), rows=rows, columns=columns)
+        assert o.normalised_error(want.cpu().numpy(), exact) < 1e-5
+    for batch in (1, 2):
+        assert torch.equal(tq1_matmul(blocks, x[:batch], out_dtype=torch.float32), want[:batch])
+        assert torch.equal(tq1_matmul(blocks, x[:batch]), want[:batch].half())
+    if rows % 2 == 0:
+        gated = single_links(blocks, x, True)
+        for batch in (1, 2):
+            assert torch.equal(tq1_swiglu(blocks, x[:batch], out_dtype=torch.float32), gated[:batch])
+
+
+@pytest.mark.parametrize("value", (np.inf, -np.inf, np.nan))
+@pytest.mark.parametrize(("rows", "columns"), ((70, 1024), (40, 10240)))
+def test_non_finite_groups(rows, columns, value):
+    """In the first, in the middle and in the last group, of either activation row."""
+    from ternel_b200.ops import tq1_matmul
+    host, rng = random_blocks(rows, columns, seed=3)
+    blocks = to_dev(host)
+    x = rng.standard_normal((2, columns)).astype(np.float16)
+    x[0, 5] = x[0, columns // 2 + 130] = x[1, columns - 1] = value
+    x = to_dev(x)
+    want = single_links(blocks, x, False)
+    assert not torch.isfinite(want).all()
+    got = tq1_matmul(blocks, x, out_dtype=torch.float32)
+    torch.testing.assert_close(got, want, rtol=0, atol=0, equal_nan=True)
+    torch.testing.assert_close(tq1_matmul(blocks, x[:1], out_dtype=torch.float32), want[:1], rtol=0, atol=0, equal_nan=True)
+
+
+def test_calls_that_follow_one_another_and_replays():
+    """Back to back on a stream and in a graph, each call reading what the one before wrote."""
+    from ternel_b200.ops import tq1_matmul
+    host, rng = random_blocks(2560, 2560, seed=9)
+    blocks = to_dev(host)
+    x = to_dev((rng.standard_normal((1, 2560)) * 0.05).astype(np.float16))
+
+    def chain():
+        y = x
+        for _ in range(12):
+            y = tq1_matmul(blocks, y)
+        return y
+
+    want = x
+    for _ in range(12):
+        want = tq1_matmul(blocks, want)
+        torch.cuda.synchronize()
+    assert torch.equal(chain(), want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = chain()
+    for _ in range(3):
+        y.zero_()
+        graph.replay()
+        assert torch.equal(y, want)
