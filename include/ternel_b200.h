@@ -96,6 +96,15 @@ int tq1_validate_codes_device(const uint8_t *codes_dev, int64_t rows, int64_t gp
                               void *stream);
 int tq1_untile_blocks_device(const uint8_t *codes_dev, const uint16_t *scales_dev, uint8_t *blocks_dev, int64_t rows,
                              int64_t gpr, int64_t tile, void *stream);
+/* Two host arrays to device memory, through `staging` (pinned host memory, at least 64 KiB): threads of the call's own fill it
+ * piece by piece while the copies are enqueued on `stream`. The sources may change when the call returns, the staging when the
+ * stream has come to that point. */
+int tq1_upload_pair(void *dst0, const void *src0, size_t bytes0, void *dst1, const void *src1, size_t bytes1,
+                    void *staging, size_t staging_bytes, void *stream);
+/* Both without a look at the counts in between: the blocks are written only if the counts (two device words, as above) come
+ * out zero, and stay as they are otherwise. */
+int tq1_load_tiled_device(const uint8_t *codes_dev, const uint16_t *scales_dev, uint8_t *blocks_dev, int64_t rows,
+                          int64_t gpr, int64_t tile, int64_t *counts_dev, void *stream);
 
 /* Scratch the linear entry point needs for this shape (0 when none) and, with
  * K % 512 == 0, for every shape that is no larger in any of the three, so that

@@ -34,6 +34,8 @@ SIGNATURES = {
     "tq1_untile_blocks": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64]),
     "tq1_validate_blocks_device": (c_int, [c_void_p, c_int64, c_void_p, c_void_p]),
     "tq1_validate_codes_device": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_void_p, c_void_p]),
+    "tq1_upload_pair": (c_int, [c_void_p, c_void_p, c_size_t, c_void_p, c_void_p, c_size_t, c_void_p, c_size_t, c_void_p]),
+    "tq1_load_tiled_device": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_void_p, c_void_p]),
     "tq1_untile_blocks_device": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_void_p]),
     "tq1_linear_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
     "tq1_linear_f16": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,

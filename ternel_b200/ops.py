@@ -250,24 +250,39 @@ def validate_device_blocks(blocks: torch.Tensor) -> None:
         raise FormatError(f"invalid base-3 bytes: regular={bad_full}, tail={bad_tail}")
 
 
+_STAGING_BYTES = 8 << 20            # pinned memory of an upload at most
+
+
+def _upload(first: torch.Tensor, second: torch.Tensor, device: torch.device) -> tuple[torch.Tensor, torch.Tensor]:
+    """Contiguous copies of both on the current device, complete in the order of its current stream. Ordinary host memory goes
+    through pinned staging, filled by several threads while the transfer runs (``tq1_upload_pair``)."""
+    arrays = [array.contiguous() for array in (first, second)]
+    if any(array.device.type != "cpu" or array.is_pinned() for array in arrays):
+        return tuple(array.to(device) for array in arrays)
+    sizes = [array.numel() * array.element_size() for array in arrays]
+    copies = [torch.empty(array.shape, dtype=array.dtype, device=device) for array in arrays]
+    staging = torch.empty(min(sum(sizes) + (1 << 20), _STAGING_BYTES), dtype=torch.uint8, pin_memory=True)
+    check(_native.lib().tq1_upload_pair(copies[0].data_ptr(), arrays[0].data_ptr(), sizes[0],
+                                        copies[1].data_ptr(), arrays[1].data_ptr(), sizes[1],
+                                        staging.data_ptr(), staging.numel(), _stream_ptr(device)))
+    return tuple(copies)
+
+
 def load_tiled_device(blocks: torch.Tensor, codes: torch.Tensor, scales: torch.Tensor, tile: int) -> None:
     """Fill canonical ``blocks`` on the GPU from the tiled pair (``uint8[tiles, groups, 26, tile]`` and 16-bit
     ``[tiles, groups, tile]``, on the host or the GPU): the arrays are uploaded as they are, scanned there, and
     converted only if every byte is legal (fail closed, as ``validate_packed_codes``). The blocks are there when the call
     returns, on whatever stream they are used next."""
     rows, groups = _check_blocks(blocks)
-    codes = codes.to(blocks.device).contiguous()
-    scales = scales.to(blocks.device).contiguous()
-    counts = torch.empty(2, dtype=torch.int64, device=blocks.device)
-    lib, stream = _native.lib(), _stream_ptr(blocks.device)
     with torch.cuda.device(blocks.device):
-        check(lib.tq1_validate_codes_device(codes.data_ptr(), rows, groups, tile, counts.data_ptr(), stream))
+        codes, scales = _upload(codes, scales, blocks.device)
+        counts = torch.empty(2, dtype=torch.int64, device=blocks.device)
+        # scanned and, where nothing was found, converted: one wait for both, by reading the counts
+        check(_native.lib().tq1_load_tiled_device(codes.data_ptr(), scales.data_ptr(), blocks.data_ptr(), rows, groups, tile,
+                                                  counts.data_ptr(), _stream_ptr(blocks.device)))
         bad_full, bad_tail = counts.tolist()
-        if bad_full or bad_tail:
-            raise FormatError(out_of_range_message(bad_full, bad_tail))
-        check(lib.tq1_untile_blocks_device(codes.data_ptr(), scales.data_ptr(), blocks.data_ptr(), rows, groups, tile,
-                                           stream))
-        torch.cuda.current_stream().synchronize()
+    if bad_full or bad_tail:
+        raise FormatError(out_of_range_message(bad_full, bad_tail))
 
 
 def _check_activations(x: torch.Tensor, groups_per_row: int) -> int:

@@ -119,3 +119,22 @@ def test_blocks_off_the_word_grid_are_loaded_too():
         module.load_tiled(*pack_blocks(blocks, layout=layout))
         assert np.array_equal(module.blocks.cpu().numpy(), blocks)
         flat.zero_()
+
+
+@pytest.mark.parametrize("staging_bytes", (65536, 100_000, 8 << 20))
+@pytest.mark.parametrize("sizes", ((1, 0), (16384, 1), (65537, 5), (700_001, 70_000), (5_324_800, 409_600), (0, 9_000_001)))
+def test_upload_through_staging_of_any_size(sizes, staging_bytes):
+    """Fewer bytes than a piece, ends inside a piece, many turns of the staging, and the pieces of two arrays side by side."""
+    from ternel_b200 import _native
+    rng = np.random.default_rng(sum(sizes))
+    hosts = [rng.integers(0, 256, size + 3, dtype=np.uint8)[3:] for size in sizes]         # off the 16-byte grid
+    devices = [torch.zeros(size + 64, dtype=torch.uint8, device="cuda") for size in sizes]
+    staging = torch.empty(staging_bytes, dtype=torch.uint8, pin_memory=True)
+    lib, stream = _native.lib(), torch.cuda.current_stream().cuda_stream
+    rc = lib.tq1_upload_pair(devices[0].data_ptr(), hosts[0].ctypes.data, sizes[0], devices[1].data_ptr(), hosts[1].ctypes.data,
+                             sizes[1], staging.data_ptr(), staging.numel(), stream)
+    assert rc == 0
+    for host, device in zip(hosts, devices):
+        got = device.cpu().numpy()
+        assert np.array_equal(got[:host.size], host) and not got[host.size:].any()
+    assert lib.tq1_upload_pair(devices[0].data_ptr(), hosts[0].ctypes.data, 1, None, None, 0, staging.data_ptr(), 1024, stream) != 0
