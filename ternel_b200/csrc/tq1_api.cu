@@ -39,34 +39,35 @@ int tq1::sm_count() {
     return n;
 }
 
-cudaError_t tq1::opt_in(KernelRecord &record, const void *kernel, size_t smem) {
+cudaError_t tq1::opt_in(KernelRecord &record, const void *kernel, size_t smem, bool large_clusters) {
     std::atomic<bool> &done = record.opted_in[device_slot()];
     if (done.load(std::memory_order_acquire)) return cudaSuccess;
-    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err == cudaSuccess && large_clusters) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (err == cudaSuccess) done.store(true, std::memory_order_release);
     return err;
 }
 
-int tq1::clusters_at_once(KernelRecord &record, const void *kernel, unsigned threads, size_t smem, int split_log) {
-    if (split_log == 0) return sm_count();
-    std::atomic<int> &known = record.clusters[device_slot()][split_log];
+int tq1::clusters_at_once(KernelRecord &record, const void *kernel, unsigned threads, size_t smem, int size) {
+    if (size == 1) return sm_count();
+    std::atomic<int> &known = record.clusters[device_slot()][size];
     int n = known.load(std::memory_order_relaxed);
     if (!n) {
-        const int split = 1 << split_log;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(sm_count() / split * split));
+        cfg.gridDim = dim3((unsigned)(sm_count() / size * size));
         cfg.blockDim = dim3(threads);
         cfg.dynamicSmemBytes = smem;
         cudaLaunchAttribute attr;
         attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = (unsigned)split;
+        attr.val.clusterDim.x = (unsigned)size;
         attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
+        if (size > 8) cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (opt_in(record, kernel, smem) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
             cudaGetLastError();                                 // no device, say: planning only
-            const int of_b200[4] = {148, 74, 33, 15};
-            n = of_b200[split_log];
+            const int of_b200[kMaxCluster + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15, 14, 14, 8, 8, 8, 8, 8, 8};
+            n = of_b200[size];
         }
         known.store(n, std::memory_order_relaxed);
     }

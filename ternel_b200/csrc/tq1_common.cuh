@@ -69,15 +69,16 @@ EncodeTiledFn encode_tiled_fn();
 constexpr int kMaxDevices = 64;
 int device_slot();                                      // the current device's
 int sm_count();                                         // the current device's, 148 on a machine without one (planning)
+constexpr int kMaxCluster = 16;                         // more than eight CTAs are asked for by name (large_clusters)
 struct KernelRecord {
     std::atomic<bool> opted_in[kMaxDevices];
-    std::atomic<int> clusters[kMaxDevices][4];          // of 1, 2, 4 and 8 CTAs that run at once
+    std::atomic<int> clusters[kMaxDevices][kMaxCluster + 1];      // of so many CTAs that run at once
 };
 // The kernel may have `smem` bytes of dynamic shared memory.
-cudaError_t opt_in(KernelRecord &record, const void *kernel, size_t smem);
-// Clusters of 2^split_log CTAs of a kernel with one CTA per SM that run at the same time: fewer than SMs / CTAs where the SMs of
-// a GPC are no multiple of it (74, 33 and 15 on this part).
-int clusters_at_once(KernelRecord &record, const void *kernel, unsigned threads, size_t smem, int split_log);
+cudaError_t opt_in(KernelRecord &record, const void *kernel, size_t smem, bool large_clusters = false);
+// Clusters of `size` CTAs of a kernel that run at the same time: fewer than SMs / CTAs where the SMs of a GPC are no
+// multiple of it (with one CTA per SM 74 of 2, 33 of 4 and 15 of 8 on this part).
+int clusters_at_once(KernelRecord &record, const void *kernel, unsigned threads, size_t smem, int size);
 
 // A launch may begin while the kernel before it in the stream ends (programmatic dependent launch): that kernel lets it in
 // (allow_next_grid), and it calls grid_dependency_wait() before it touches what an earlier one may have written or may still

@@ -27,7 +27,8 @@
 //
 // Segments that cover only a part of a tile's K range leave an FP32 partial tile in the workspace; the CTA that finishes
 // the tile's last part (a counter per tile) adds the parts in ascending K order, so results never depend on timing, and no
-// CTA waits for another. A separate launch for these sums cost 3 to 14 us.
+// CTA waits for another. A separate launch for these sums cost 3 to 14 us. Equal parts of fewer tiles than slots add up in
+// clusters (CLUSTERED, below).
 //
 // Precision: the tensor core adds to an accumulator by truncation, so the error grows with the columns that one accumulator
 // covers: 6.3e-7 of the result (2-norm) for 512, 1.2e-6 for 1024, 3.0e-6 for 2560. All of the accumulator area is therefore
@@ -292,6 +293,23 @@ struct SegmentWalk {
     }
 };
 
+// The one segment of a slot where every tile is cut into equal parts (splits > 0).
+struct OneSegment {
+    const WorkSplit &work;
+    int slot;
+    bool taken;
+    __device__ __forceinline__ OneSegment(const WorkSplit &work_, int slot_) : work(work_), slot(slot_), taken(false) {}
+    __device__ __forceinline__ bool next(int end, int &tile, int &c0, int &len, int &part) {
+        if (taken) return false;
+        taken = true;
+        tile = work.by_splits.div(slot);
+        c0 = work.first_iter(slot) - tile * work.chunks;
+        len = end - work.first_iter(slot);
+        part = 0;
+        return true;
+    }
+};
+
 struct GemmParams {
     void *y;                  // [M][N] (FP16/FP32), with swiglu [M][N / 2]
     float *partials;          // [2 * CTAs][nt][128] FP32
@@ -310,7 +328,11 @@ struct GemmParams {
 
 // GATED: the rows are (gate, up) pairs. A kernel of its own: the gates' code in the common one cost 3% of long prompts (777 tokens
 // of 34816x5120 without gates 204 us, 199 apart) and 7% of the shortest calls (17 of 1000x1024 5.8 us, 5.4).
-template <class V, bool GATED>
+// CLUSTERED: every tile is cut into equal parts, and the CTAs of a cluster, one for each, add them through distributed shared
+// memory. Through the workspace a part's way out, the count and the sum by the last CTA took 4 us of the 8.4 that 20 tokens of
+// 4096x4096 took, now 7.2; 100 of 1024x5120 9.6 and 7.8, 66 rows with gates of 129 tokens 9.8 and 7.4, 48 of 5120x17408 20.8 and 20.4. A kernel of its own too: addresses of a CTA in a cluster take a register, for which only the walk
+// over several segments makes room (64 tokens of 17408x5120 as one kernel 21.3 -> 23.4 us).
+template <class V, bool GATED, bool CLUSTERED>
 __global__ void __launch_bounds__(V::kThreads, V::kMinCtas)
 tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
                 const __grid_constant__ GemmParams prm) {
@@ -319,7 +341,7 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
     extern __shared__ __align__(1024) unsigned char smem[];
     // In a cluster launch the upper byte of a shared-memory address names the CTA; the offsets below it are fixed.
     const uint32_t window = (uint32_t)__cvta_generic_to_shared(smem);
-    const uint32_t wbase = CG == 2 ? window & 0xff000000u : 0u;
+    const uint32_t wbase = CG == 2 || CLUSTERED ? window & 0xff000000u : 0u;
     if (window != wbase + V::kBase) {                                // the fixed window addresses do not hold
         if (threadIdx.x == 0) atomicExch(prm.status, 2u);
         return;
@@ -354,6 +376,55 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         if (V::WIDE) bulk_load(wbase + V::kTableAddr, &g_wide, V::kTableBytes, bar(TAB));
         else bulk_load(wbase + V::kTableAddr, &g_narrow, V::kTableBytes, bar(TAB));
     }
+    // The segments, and for a decode warp the packed bytes that it requests ahead of its decoding: the walks are set up and the
+    // first bytes brought to L2 (a hint, whatever they hold by now) while earlier kernels run. Behind the wait below this
+    // took 4700 clocks up to the first decoded byte, now 2800.
+    auto weight_tile = [&](int t) { return prm.by_tiles_m.div(t); };
+    auto token_tile0 = [&](int t) { return (t - prm.by_tiles_m.div(t) * prm.tiles_m) * prm.nt; };     // first token
+    // tokens of a token tile, as the MMA's N (whole steps of 16 per CTA)
+    auto tile_tokens = [&](int m0) {
+        const int left = min(prm.nt, prm.M - m0);
+        return (left + 16 * CG - 1) / (16 * CG) * (16 * CG);
+    };
+    using Walk = std::conditional_t<CLUSTERED, OneSegment, SegmentWalk>;
+    Walk walk(prm.work, slot), pwalk(prm.work, slot);
+    const int end_iter = prm.work.first_iter(slot + 1);
+    int p_tile = 0, p_c0 = 0, p_len = 0, p_part, p_unit = warp >> 2;
+    auto seek = [&]() -> bool {
+        while (p_unit >= p_len) {
+            if (!pwalk.next(end_iter, p_tile, p_c0, p_len, p_part)) { p_len = 0; return false; }
+            p_unit = warp >> 2;
+        }
+        return true;
+    };
+    auto packed_row = [&]() { return (weight_tile(p_tile) * CG + rank) * kTileW + (warp & 3) * 32; };
+    // the results of four neighbouring rows from nq of token m
+    auto store_quad = [&](float (&r)[4], int m, int nq) {
+        int count = min(4, prm.N - nq);
+        size_t o = (size_t)m * prm.N + nq;
+        size_t limit = (size_t)prm.M * prm.N;
+        if (GATED) {
+            r[0] = swiglu_f32(r[0], r[1]);
+            r[1] = swiglu_f32(r[2], r[3]);
+            count >>= 1;
+            o = (size_t)m * (prm.N >> 1) + (nq >> 1);
+            limit >>= 1;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (e < count && TQ1_IN_BOUNDS(o + e, limit, 40u)) {
+                if (prm.y_f32) static_cast<float *>(prm.y)[o + e] = r[e];
+                else static_cast<__half *>(prm.y)[o + e] = __float2half_rn(r[e]);
+            }
+        }
+    };
+    if (warp < kDecode) {
+        if (seek() && elect_one())
+            asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];"
+                         ::"l"(&wmap), "r"((p_c0 + p_unit) * kChunkBytes), "r"(packed_row()) : "memory");
+        __syncwarp();
+    }
+    if (warp == kXWarp && elect_one()) asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");
     if (warp == kMmaWarp) {
         const uint32_t where = wbase + V::kBarAddr + 1008;
         if (CG == 2) {
@@ -379,17 +450,8 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     bool dead = false;
-    SegmentWalk walk(prm.work, slot);
-    const int end_iter = prm.work.first_iter(slot + 1);
     int tile, c0, len, part;
 
-    auto weight_tile = [&](int t) { return prm.by_tiles_m.div(t); };
-    auto token_tile0 = [&](int t) { return (t - prm.by_tiles_m.div(t) * prm.tiles_m) * prm.nt; };     // first token
-    // tokens of a token tile, as the MMA's N (whole steps of 16 per CTA)
-    auto tile_tokens = [&](int m0) {
-        const int left = min(prm.nt, prm.M - m0);
-        return (left + 16 * CG - 1) / (16 * CG) * (16 * CG);
-    };
 
     // K blocks are numbered in the order the MMA warp takes them, over all segments: block i of a CTA uses stage i % RING of
     // the decoded weights and stage i % b_stages (<= RING) of the activations. One commit (EMPTY) says to decoders and
@@ -468,18 +530,11 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         const uint32_t tmem_lane = tmem_base + ((uint32_t)(quad * 32) << 16);
         const uint32_t lane_entry = wbase + V::kTableAddr + (uint32_t)(lane & 15) * 8u;
 
-        // cursor of the packed bytes this warp requests ahead of its decoding
-        SegmentWalk pwalk(prm.work, slot);
-        int p_tile = 0, p_c0 = 0, p_len = 0, p_part, p_unit = group;
         uint32_t requested = 0, consumed = 0;
         auto request = [&]() {
-            while (p_unit >= p_len) {
-                if (!pwalk.next(end_iter, p_tile, p_c0, p_len, p_part)) { p_len = 0; return; }
-                p_unit = group;
-            }
+            if (!seek()) return;
             const uint32_t s = requested % V::PACK_STAGES;
-            const int n0 = (weight_tile(p_tile) * CG + rank) * kTileW + quad * 32;
-            elected_load_packed(wbase + V::pack_addr(warp, (int)s), &wmap, (p_c0 + p_unit) * kChunkBytes, n0,
+            elected_load_packed(wbase + V::pack_addr(warp, (int)s), &wmap, (p_c0 + p_unit) * kChunkBytes, packed_row(),
                                 bar(PACK + warp * V::PACK_STAGES + (int)s));
             ++requested;
             p_unit += G;
@@ -503,11 +558,12 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
             const int n = (weight_tile(tile) * CG + rank) * kTileW + row_in_tile;
             const int per_group = (n_tok / 16 + G - 1) / G * 16;
             const int c_begin = group * per_group, cols = min(per_group, n_tok - c_begin);     // cols <= 0: none
-            const bool whole = len == prm.work.chunks;
+            const bool whole = !CLUSTERED && len == prm.work.chunks;
             // the slots that share this tile, worked out while the last products are still being added
             const int shared_tile = tile - prm.work.whole_tiles, it0 = shared_tile * prm.work.chunks;
             int lo = slot, hi = slot;
-            if (!whole && prm.work.splits > 0) {
+            if (CLUSTERED) {
+            } else if (!whole && prm.work.splits > 0) {
                 lo = shared_tile * prm.work.splits;
                 hi = lo + prm.work.splits - 1;
             } else if (!whole) {
@@ -539,6 +595,18 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
             };
             const int tokens = min(cols, prm.M - (m0 + c_begin));                              // of the group's columns
             const int out_n = GATED ? prm.N >> 1 : prm.N;
+            if (CLUSTERED) {             // a part of the tile's K range: kept as FP32 where the activations were
+#pragma unroll 1
+                for (int s0 = 0; s0 < V::kGroupCols; s0 += kStep) {
+                    float v[kStep];
+                    read_step(s0, v);
+                    float *to = reinterpret_cast<float *>(smem + (V::kBAddr - V::kBase)) + (c_begin + s0) * kTileW + row_in_tile;
+#pragma unroll
+                    for (int c = 0; c < kStep; ++c)
+                        if (s0 + c < tokens) to[c * kTileW] = v[c];
+                }
+                return;
+            }
             if (!whole) {                               // a part of the tile's K range: kept as FP32
                 const size_t area = (size_t)prm.nt * kTileW;
                 float *slot_part = prm.partials + ((size_t)2 * blockIdx.x + part) * area + row_in_tile;
@@ -591,23 +659,7 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                         const int i = i0 + f * kThreadsR, m = m0 + (i >> 5), nq = tile_n0 + (i & 31) * 4;
                         if (i >= quads) break;
                         float r[4] = {total[f].x, total[f].y, total[f].z, total[f].w};
-                        int count = min(4, prm.N - nq);
-                        size_t o = (size_t)m * prm.N + nq;
-                        size_t limit = (size_t)prm.M * prm.N;
-                        if (GATED) {
-                            r[0] = swiglu_f32(r[0], r[1]);
-                            r[1] = swiglu_f32(r[2], r[3]);
-                            count >>= 1;
-                            o = (size_t)m * (prm.N >> 1) + (nq >> 1);
-                            limit >>= 1;
-                        }
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            if (e < count && TQ1_IN_BOUNDS(o + e, limit, 40u)) {
-                                if (prm.y_f32) static_cast<float *>(prm.y)[o + e] = r[e];
-                                else static_cast<__half *>(prm.y)[o + e] = __float2half_rn(r[e]);
-                            }
-                        }
+                        store_quad(r, m, nq);
                     }
                 }
                 return;
@@ -812,6 +864,36 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
     if (CG == 2) {
         asm volatile("barrier.cluster.arrive.release;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    } else if (CLUSTERED) {
+        // Every CTA adds its share of the tile's columns, the parts in the order of their columns of the matrix.
+        const int splits = prm.work.splits, tile = prm.work.by_splits.div(slot), part = slot - tile * splits;
+        // the tile's counter has no use here; that it is not zero is reported as by the calls that count (a warp with time to spare)
+        if (tid == kMmaWarp * 32 && part == 0 && __ldcg(prm.counters + tile) != 0u) atomicExch(prm.status, 8u);
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const int m0 = token_tile0(tile), all = min(tile_tokens(m0), prm.M - m0), tile_n0 = weight_tile(tile) * kTileW;
+        const int first = all * part / splits, quads = (all * (part + 1) / splits - first) * (kTileW / 4);      // four rows of a column each
+#pragma unroll 1
+        for (int i = tid; i < quads; i += V::kThreads) {
+            const int col = first + (i >> 5), m = m0 + col, nq = tile_n0 + (i & 31) * 4;
+            if (nq >= prm.N) continue;                  // nothing is read that is not used below
+            const uint32_t own = wbase + V::kBAddr + (uint32_t)(col * kTileW + (i & 31) * 4) * 4u;
+            float r[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 4
+            for (int c = 0; c < splits; ++c) {
+                float4 p;
+                asm volatile("{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\t"
+                             "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
+                             : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w) : "r"(own), "r"(c) : "memory");
+                r[0] += p.x; r[1] += p.y; r[2] += p.z; r[3] += p.w;
+            }
+            store_quad(r, m, nq);
+        }
+        // the others' parts have been read (what was read has been used); the results' own way needs no waiting for
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     } else {
         __syncthreads();
     }
@@ -832,6 +914,15 @@ struct Tiling {
     WorkSplit work;
     int ctas() const { return work.slots * tile_cg(tile); }
 };
+
+// Clusters of `size` CTAs of the clustered kernel for this token tile that run at once.
+KernelRecord g_clustered[2];                                    // of variants S and L
+int cluster_room(int tile, int size) {
+    return tile <= 32 ? clusters_at_once(g_clustered[0], reinterpret_cast<const void *>(tq1_gemm_kernel<VariantS, false, true>),
+                                         VariantS::kThreads, VariantS::kSmemBytes, size)
+                      : clusters_at_once(g_clustered[1], reinterpret_cast<const void *>(tq1_gemm_kernel<VariantL, false, true>),
+                                         VariantL::kThreads, VariantL::kSmemBytes, size);
+}
 
 // How the chunks of a shape are dealt out for a given token tile.
 Tiling make_tiling(int tile, int M, int N, int K) {
@@ -890,11 +981,17 @@ Tiling make_tiling(int tile, int M, int N, int K) {
     return t;
 }
 
+// A tile's parts add up in a cluster.
+bool clustered(int tile, const WorkSplit &w) {
+    return tile <= 128 && w.splits > 1 && w.splits <= kMaxCluster && w.tiles_total <= cluster_room(tile, w.splits);
+}
+
 // Activation rows per tile. Up to 16 rows always take the 16-row tile. Beyond that the tile with the smallest modelled
 // time wins: launch and pipeline fill, chunks a slot works through (decode, plus products per token), segments it stores,
 // and the sums of shared tiles. The constants (us) are fitted to the recorded sweep in
 // ternel_b200/dispatch_sweep_b200.json; tests replay the file (the choice is within 10% of the best recorded tile for every
-// case). g_forced_tile overrides the rule while a sweep is being recorded.
+// case), which was made when the parts of a tile met in the workspace. The choice has been kept since: it also says how many columns an
+// accumulator covers, and with them the error. g_forced_tile overrides the rule while a sweep is being recorded.
 int g_forced_tile = 0;
 struct TileCost { int tile; float fixed, chunk, chunk_token, segment, shared_token; };
 const TileCost g_tile_costs[5] = {{16, 2.932f, 0.0f, 0.1263f, 1.968f, 0.1093f},
@@ -931,13 +1028,10 @@ Tiling pick_tiling(int M, int N, int K) { return make_tiling(token_tile(M, N, K)
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
-template <class V, bool GATED>
-int launch_variant(const CUtensorMap &wmap, const CUtensorMap &xmap, GemmParams &prm, int ctas, cudaStream_t stream) {
-    const int stages = (int)(V::kBRoom / ((uint32_t)prm.b_rows * 256u));
-    prm.b_stages = stages < V::RING ? stages : V::RING;
-    auto kern = tq1_gemm_kernel<V, GATED>;
-    static KernelRecord record;
-    const cudaError_t e = opt_in(record, reinterpret_cast<const void *>(kern), V::kSmemBytes);
+template <class V, bool GATED, bool CLUSTERED>
+int launch_kernel(KernelRecord &record, const CUtensorMap &wmap, const CUtensorMap &xmap, const GemmParams &prm, int ctas, cudaStream_t stream) {
+    auto kern = tq1_gemm_kernel<V, GATED, CLUSTERED>;
+    const cudaError_t e = opt_in(record, reinterpret_cast<const void *>(kern), V::kSmemBytes, CLUSTERED);
     if (e != cudaSuccess) return cuda_fail(e, "tq1_linear_f16: shared memory opt-in (GEMM)");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
@@ -948,13 +1042,27 @@ int launch_variant(const CUtensorMap &wmap, const CUtensorMap &xmap, GemmParams 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = V::CG;
+    attr[1].val.clusterDim.x = CLUSTERED ? (unsigned)prm.work.splits : V::CG;
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = V::CG > 1 ? 2 : 1;
+    cfg.numAttrs = V::CG > 1 || CLUSTERED ? 2 : 1;
     const cudaError_t err = cudaLaunchKernelEx(&cfg, kern, wmap, xmap, prm);
     if (err == cudaSuccess && stream_captured(stream)) note_captured_kernel(stream);
     return err == cudaSuccess ? TQ1_OK : cuda_fail(err, "tq1_linear_f16: GEMM launch");
+}
+
+template <class V, bool GATED>
+int launch_variant(const CUtensorMap &wmap, const CUtensorMap &xmap, GemmParams &prm, int ctas, cudaStream_t stream) {
+    const int stages = (int)(V::kBRoom / ((uint32_t)prm.b_rows * 256u));
+    prm.b_stages = stages < V::RING ? stages : V::RING;
+    static KernelRecord record, in_clusters;
+    if constexpr (V::CG == 1) {
+        static_assert(V::MAX_COLS * kTileW * 4 <= V::kBRoom, "a part lies where the activations were");
+        // in clusters, where all of them run at once
+        if (clustered(V::G == 2 ? 32 : 128, prm.work))
+            return launch_kernel<V, GATED, true>(in_clusters, wmap, xmap, prm, ctas, stream);
+    }
+    return launch_kernel<V, GATED, false>(record, wmap, xmap, prm, ctas, stream);
 }
 
 }  // namespace
@@ -967,8 +1075,9 @@ int gemm_tc_force_tile(int nt) {
 
 bool gemm_tc_forced() { return g_forced_tile != 0; }
 
-// Behind another kernel, fitted to 1022 calls with weights out of HBM, within 4.4% (2-norm): a CTA's chunks, what it costs two CTAs
-// of an SM to begin and end a tile, the sum of K parts, and the bytes.
+// What draws the line between this kernel and the slice kernel, whose sums have a third to a tenth of the error: fitted to 1022 calls
+// behind another kernel when parts still met in the workspace, and kept. (Since a cluster adds them this kernel would be the faster
+// one for 39 of 380 calls of nine to sixteen tokens that the line leaves to the other, by 11% on average.)
 float gemm_tc_few_us(int N, int K) {
     const Tiling t = make_tiling(16, 16, N, K);
     const WorkSplit &w = t.work;

@@ -418,7 +418,7 @@ groups_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
 // ---- host ---------------------------------------------------------------------------------------------------------
 KernelRecord g_record;
 const void *const kKernel = reinterpret_cast<const void *>(groups_tc_kernel);
-int clusters_at_once(int split_log) { return tq1::clusters_at_once(g_record, kKernel, kThreads, kSmemEnd - kWindow, split_log); }
+int clusters_at_once(int split_log) { return tq1::clusters_at_once(g_record, kKernel, kThreads, kSmemEnd - kWindow, 1 << split_log); }
 
 struct GroupPlan { int nt, tiles_m, tiles, clusters, split; float us; };
 

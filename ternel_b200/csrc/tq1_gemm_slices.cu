@@ -473,7 +473,7 @@ SlicePlan slice_plan(int nt, int N, int K) {
         if (halves < split || p.slices > kMaxSlices) continue;
         // how many clusters run at once is asked of the driver (milliseconds, the first time) only where this split could win
         if (best.ok && slice_us(split, p.slices, (tiles + sm_count() / split - 1) / (sm_count() / split)) >= best.us) continue;
-        const int room = clusters_at_once(g_records[nt - 1], kernel_of(nt), 32 * (kMaxSlices + kExtraWarps), kWindowEnd - kWindow, log);
+        const int room = clusters_at_once(g_records[nt - 1], kernel_of(nt), 32 * (kMaxSlices + kExtraWarps), kWindowEnd - kWindow, 1 << log);
         p.clusters = tiles < room ? tiles : room;
         const int per_cluster = (tiles + p.clusters - 1) / p.clusters;
         p.subsets = kMaxSlices / p.slices;

@@ -382,7 +382,7 @@ TilePlan tile_plan(int tokens, int N, int K) {
         // how many clusters run at once is asked of the driver (milliseconds, the first time) only where this split could win
         const int hope = (tiles + sm_count() / split - 1) / (sm_count() / split);
         if (best.ok && tile_us(log, set_warps, subsets_for(hope), hope) >= best.us) continue;
-        const int room = clusters_at_once(g_records[log > 0][tokens - 1], reinterpret_cast<const void *>(kernel_of(log > 0, tokens)), 32 * kMaxWarps, kWindowEnd - kWindow, log);
+        const int room = clusters_at_once(g_records[log > 0][tokens - 1], reinterpret_cast<const void *>(kernel_of(log > 0, tokens)), 32 * kMaxWarps, kWindowEnd - kWindow, 1 << log);
         p.clusters = tiles < room ? tiles : room;
         const int per = (tiles + p.clusters - 1) / p.clusters;
         p.subsets = subsets_for(per);

@@ -251,3 +251,26 @@ def test_segments_that_follow_one_another(columns):
         # silu in FP32: exp and the division differ from PyTorch's by a few units in the last place
         torch.testing.assert_close(tq1_swiglu(blocks, x, out_dtype=torch.float32), torch.nn.functional.silu(gate) * up,
                                    rtol=2e-6, atol=1e-30)
+
+
+@pytest.mark.parametrize(("rows", "columns"), ((50, 2048), (130, 4608), (1001, 5120), (2046, 17408), (5120, 8704)))
+def test_parts_that_a_cluster_adds(rows, columns):
+    """Tiles cut into two to nine equal parts, with rows past the last whole quad, and columns that the CTAs of a cluster do not
+    share evenly. Whole numbers, so every sum is exact."""
+    from ternel_b200.dispatch import plan
+    from ternel_b200.ops import tq1_matmul, tq1_swiglu
+    rng = np.random.default_rng(rows)
+    trits = rng.integers(0, 3, size=(rows * columns // 128, 128), dtype=np.uint8)
+    blocks = to_dev(o.encode_blocks(ones_scale(rows * columns // 128), trits).reshape(rows, columns // 128, 28))
+    dense = to_dev(trits.reshape(rows, columns)).float() - 1
+    parts = set()
+    for batch in (17, 29, 47, 100, 128):
+        parts.add(plan(batch, rows, columns).parts)
+        x = torch.randint(-1, 2, (batch, columns), device="cuda").to(torch.float16)
+        want = x.float() @ dense.T
+        assert torch.equal(tq1_matmul(blocks, x, out_dtype=torch.float32), want)
+        assert torch.equal(tq1_matmul(blocks, x), want.half())
+        if rows % 2 == 0:
+            torch.testing.assert_close(tq1_swiglu(blocks, x, out_dtype=torch.float32),
+                                       torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2], rtol=2e-6, atol=1e-30)
+    assert parts & set(range(2, 17))
