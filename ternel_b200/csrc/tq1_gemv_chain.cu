@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
             left -= seg;
             // One unit. BAD: some group of the chunk holds NaN/Inf activations (rare; in the forms with two loops kept out of
             // the common one so that it costs that neither branches nor registers).
-            auto unit = [&](auto bad_tag) {
+            auto unit = [&](auto bad_tag, bool more) {          // more: not the link's last unit
                 constexpr bool BAD = decltype(bad_tag)::value, AT_END = FORM == kChain;
                 const uint32_t bar = bar0 + 8u * cstage;
                 uint32_t arrived = mbar_test_wait(bar, cparity);
@@ -661,12 +661,6 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
                         acc2 = fmaf(scales2[sub], dot2, acc2);
                     }
                 }
-                // the stage consumed one iteration ago is free: refill it
-                ++consumed;
-                if (++cstage == kStages) { cstage = 0; cparity ^= 1u; }
-                __syncwarp();
-                if (issued - consumed < kStages - 1) issue_one();
-
                 // quad: lanes q=0 (groups 0,1) and q=2 (groups 2,3) -> chunk partial in lane q=0
                 acc1 += __shfl_down_sync(0xffffffffu, acc1, 2);
                 acc2 += __shfl_down_sync(0xffffffffu, acc2, 2);
@@ -675,12 +669,20 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
                     slot_publish(mine, acc1, tag);
                     slot_publish(mine + 8, acc2, tag);
                 }
+                // The stage consumed one iteration ago is free: refill it, after the sums have gone out. Behind the link's last unit the
+                // cursor's step to the next link takes some 600 clocks: that is left to the next link's beginning, where the wait for
+                // activations hides it. Eight layers of hidden 5120: 243.5 us with the refill before the sums, 238.7 after, 239.0 now;
+                // of hidden 2048: 135.5, 131.5 and 121.8. (With the activations asked for before the refill 240.0 and 119.7.)
+                ++consumed;
+                if (++cstage == kStages) { cstage = 0; cparity ^= 1u; }
+                __syncwarp();
+                if (more && issued - consumed < kStages - 1) issue_one();
                 mine += kTileRows;
             };
             if (FORM != kChain && chunk_bad)
-                for (int i = 0; i < seg; ++i) unit(std::true_type{});
+                for (int i = seg; i > 0; --i) unit(std::true_type{}, i > 1 || left > 0);
             else
-                for (int i = 0; i < seg; ++i) unit(std::false_type{});
+                for (int i = seg; i > 0; --i) unit(std::false_type{}, i > 1 || left > 0);
             t = 0;
             ++c;
         }
@@ -700,6 +702,7 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
             const float out_scale = L.out_scale;
             void *y = L.y;
             const int world = L.world;
+            unsigned long long *const out0 = world > 0 ? L.xout[0] : nullptr;
             // The tiles of chunk cc that this warp owns are those with t % chunks == cc: walk them directly.
             int cc = R.c_first, t0 = R.t_first, tm0 = R.t_first % chunks;
             for (int left = n_units; left > 0;) {
@@ -756,16 +759,16 @@ __global__ void __launch_bounds__(kThreads, 1) tq1_gemv_chain_kernel(const __gri
                     total *= out_scale;
                     if (writer && TQ1_IN_BOUNDS(row, swiglu ? N >> 1 : N, 12u)) {
                         const __half hv = __float2half_rn(total);
-                        if (y) {
-                            if (out_f32) static_cast<float *>(y)[row] = total;
-                            else static_cast<__half *>(y)[row] = hv;
-                        }
                         // hand-off: the rounded FP16 value and this link's tag in one word, to every rank
                         // (a partial sum over this rank's K shard travels as FP32: the reader adds the ranks' words)
                         const uint32_t payload = (flags & kFlagPartialOut) ? __float_as_uint(total)
                                                                            : (uint32_t)__half_as_ushort(hv);
-                        for (int pr = 0; pr < world; ++pr)
-                            word_publish(L.xout[pr] + row, payload, tag);
+                        if (out0) word_publish(out0 + row, payload, tag);
+                        for (int pr = 1; pr < world; ++pr) word_publish(L.xout[pr] + row, payload, tag);
+                        if (y) {
+                            if (out_f32) static_cast<float *>(y)[row] = total;
+                            else static_cast<__half *>(y)[row] = hv;
+                        }
                     }
                 }
                 t0 = 0;
