@@ -60,6 +60,8 @@ constexpr int kMaxStages = 24;
 
 // Warps that decode: 12 warps leave each 168 registers.
 constexpr int kMaxSlices = 11;
+constexpr int kMaxOwn = 96;                                     // row tiles that a CTA of a cluster adds up
+static_assert(8 * (2 * kMaxStages + kBufs * kMaxSlices + kMaxSlices + kMaxOwn) <= kBarBytes, "barrier area");
 __host__ __device__ constexpr int slice_halves(int nt) { return nt == 1 ? 2 : 1; }          // 64 registers of activations
 constexpr int kExtraWarps = 1;
 // Fewer warps than this would be long at filling the table (two of them: 1.1 us more than six; 8 tokens of 2048x512 6.5 us apart
@@ -238,6 +240,9 @@ slices_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     auto full_bar = [&](int s) { return base + kBarAddr + 8u * (uint32_t)s; };
     auto empty_bar = [&](int s) { return base + kBarAddr + 8u * (uint32_t)(kMaxStages + s); };
     auto sum_bar = [&](int s) { return base + kBarAddr + 8u * (uint32_t)(2 * kMaxStages + s); };
+    // clusters: one for each row tile that this CTA adds up, behind those of the slices' activations
+    auto tile_bar = [&](int s) { return base + kBarAddr + 8u * (uint32_t)(2 * kMaxStages + kBufs * prm.subsets + kMaxSlices + s); };
+    const int own_tiles = (n_tiles - rank + split - 1) >> split_log;
     auto x_bar = [&](int s) { return base + kBarAddr + 8u * (uint32_t)(2 * kMaxStages + kBufs * prm.subsets + s); };
 
     // ---- set-up that depends on no earlier kernel ---------------------------------------------------------------
@@ -250,9 +255,13 @@ slices_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             mbar_init(sum_bar(s), (uint32_t)n_slices);
         }
         for (int s = 0; s < n_slices; ++s) mbar_init(x_bar(s), 1);
+        if (split > 1)
+            for (int s = 0; s < own_tiles; ++s) mbar_init(tile_bar(s), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    if (tid == 0 && split > 1)                                  // the sums of all of the cluster's CTAs
+        for (int s = 0; s < own_tiles; ++s) mbar_expect_tx(tile_bar(s), (uint32_t)(split * NT * 8 * kTileRows * 4));
     const int word_x = chunk_lo * (kChunkBytes / 8);            // the map's elements are 8 bytes
     if (tid == 32) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&wmap) : "memory");
@@ -353,11 +362,13 @@ slices_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                             store_rows(prm, (tile_lo + i) * kTileRows + row, m, total);
                         } else {                                // to CTA i % split of the cluster, which adds the CTAs' sums
                             const int slot = (i >> split_log << split_log) + rank;
-                            uint32_t dst;
+                            uint32_t dst, bar;
                             asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst)
                                          : "r"(base + prm.sums_addr + 4u * (uint32_t)(slot * kPart + m * kTokenPitch + row)), "r"(i & (split - 1)));
-                            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
-                                         ::"r"(dst), "f"(total.x), "f"(total.y), "f"(total.z), "f"(total.w) : "memory");
+                            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(tile_bar(i >> split_log)), "r"(i & (split - 1)));
+                            asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+                                         ::"r"(dst), "r"(__float_as_uint(total.x)), "r"(__float_as_uint(total.y)),
+                                           "r"(__float_as_uint(total.z)), "r"(__float_as_uint(total.w)), "r"(bar) : "memory");
                         }
                     }
                     __syncwarp();
@@ -421,13 +432,13 @@ slices_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     if (dead)                                                   // a wait ran out: give the copies still in flight time to land
         for (int i = 0; i < 64; ++i) __nanosleep(20000);
     if (split > 1) {
-        // CTA r of the cluster has the CTAs' sums of every split-th tile; it adds them in the order of the columns
-        __syncwarp();
-        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        // CTA r of the cluster has the CTAs' sums of every split-th tile; it adds them in the order of the columns as they come in
+        // (with a cluster barrier before all of them 3 tokens of 264x17408 took 4.8 us, now 4.4; 8 of 640x8704 5.3 and 4.6; 12 of
+        // 1024x5120 5.6 and 5.3)
         const float *sums = reinterpret_cast<const float *>(smem + (prm.sums_addr - kWindow));
         for (int j = warp; rank + (j / (4 * NT) << split_log) < n_tiles; j += warps) {
             const int own = j / (4 * NT), p = j % (4 * NT), m = 8 * (p >> 2) + (p & 3) + (lane & 4), row = (lane & 3) * 4;
+            mbar_wait(tile_bar(own), 0, prm.status, dead);
             float4 total = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             for (int c = lane >> 3; c < split; c += 4)
                 total = add4(total, *reinterpret_cast<const float4 *>(sums + ((own << split_log) + c) * kPart + m * kTokenPitch + row));
@@ -493,6 +504,7 @@ SlicePlan slice_plan(int nt, int N, int K) {
         if (p.stages > kMaxStages) p.stages = kMaxStages;
         if (p.stages > per_cluster) p.stages = per_cluster;
         if (p.stages < (per_cluster < 2 * p.subsets ? per_cluster : p.subsets + 1)) continue;      // no room to fetch ahead
+        if (split > 1 && (per_cluster + split - 1) / split > kMaxOwn) continue;
         p.end = p.ring_addr + (uint32_t)p.stages * stage_bytes;
         p.ok = true;
         p.us = slice_us(split, p.slices, per_cluster);
