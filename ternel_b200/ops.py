@@ -261,7 +261,10 @@ def _upload(first: torch.Tensor, second: torch.Tensor, device: torch.device) -> 
         return tuple(array.to(device) for array in arrays)
     sizes = [array.numel() * array.element_size() for array in arrays]
     copies = [torch.empty(array.shape, dtype=array.dtype, device=device) for array in arrays]
-    staging = torch.empty(min(sum(sizes) + (1 << 20), _STAGING_BYTES), dtype=torch.uint8, pin_memory=True)
+    try:
+        staging = torch.empty(min(sum(sizes) + (1 << 20), _STAGING_BYTES), dtype=torch.uint8, pin_memory=True)
+    except RuntimeError:                # no pinned memory to be had: the driver's own way
+        return tuple(array.to(device) for array in arrays)
     check(_native.lib().tq1_upload_pair(copies[0].data_ptr(), arrays[0].data_ptr(), sizes[0],
                                         copies[1].data_ptr(), arrays[1].data_ptr(), sizes[1],
                                         staging.data_ptr(), staging.numel(), _stream_ptr(device)))
