@@ -236,6 +236,7 @@ static cudaError_t upload_parts(const UploadPart *parts, unsigned char *staging,
         if (t.joinable()) t.join();
     for (cudaEvent_t e : events)
         if (e) cudaEventDestroy(e);
+    if (err != cudaSuccess) cudaStreamSynchronize(stream);      // the caller may drop the staging: nothing reads it any more
     return err;
 }
 

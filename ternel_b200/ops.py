@@ -253,22 +253,25 @@ def validate_device_blocks(blocks: torch.Tensor) -> None:
 _STAGING_BYTES = 8 << 20            # pinned memory of an upload at most
 
 
-def _upload(first: torch.Tensor, second: torch.Tensor, device: torch.device) -> tuple[torch.Tensor, torch.Tensor]:
+def _upload(first: torch.Tensor, second: torch.Tensor, device: torch.device) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor | None]:
     """Contiguous copies of both on the current device, complete in the order of its current stream. Ordinary host memory goes
-    through pinned staging, filled by several threads while the transfer runs (``tq1_upload_pair``)."""
+    through pinned staging, filled by several threads while the transfer runs (``tq1_upload_pair``). The third result is that
+    staging: the transfers out of it are not known to torch's pool, so the caller holds it until the stream has been waited for."""
     arrays = [array.contiguous() for array in (first, second)]
-    if any(array.device.type != "cpu" or array.is_pinned() for array in arrays):
-        return tuple(array.to(device) for array in arrays)
+    plain = any(array.device.type != "cpu" or array.is_pinned() for array in arrays)
     sizes = [array.numel() * array.element_size() for array in arrays]
+    if not plain:
+        try:
+            staging = torch.empty(min(sum(sizes) + (1 << 20), _STAGING_BYTES), dtype=torch.uint8, pin_memory=True)
+        except RuntimeError:            # no pinned memory to be had: the driver's own way
+            plain = True
+    if plain:
+        return *(array.to(device) for array in arrays), None
     copies = [torch.empty(array.shape, dtype=array.dtype, device=device) for array in arrays]
-    try:
-        staging = torch.empty(min(sum(sizes) + (1 << 20), _STAGING_BYTES), dtype=torch.uint8, pin_memory=True)
-    except RuntimeError:                # no pinned memory to be had: the driver's own way
-        return tuple(array.to(device) for array in arrays)
     check(_native.lib().tq1_upload_pair(copies[0].data_ptr(), arrays[0].data_ptr(), sizes[0],
                                         copies[1].data_ptr(), arrays[1].data_ptr(), sizes[1],
                                         staging.data_ptr(), staging.numel(), _stream_ptr(device)))
-    return tuple(copies)
+    return *copies, staging
 
 
 def load_tiled_device(blocks: torch.Tensor, codes: torch.Tensor, scales: torch.Tensor, tile: int) -> None:
@@ -278,12 +281,17 @@ def load_tiled_device(blocks: torch.Tensor, codes: torch.Tensor, scales: torch.T
     returns, on whatever stream they are used next."""
     rows, groups = _check_blocks(blocks)
     with torch.cuda.device(blocks.device):
-        codes, scales = _upload(codes, scales, blocks.device)
-        counts = torch.empty(2, dtype=torch.int64, device=blocks.device)
-        # scanned and, where nothing was found, converted: one wait for both, by reading the counts
-        check(_native.lib().tq1_load_tiled_device(codes.data_ptr(), scales.data_ptr(), blocks.data_ptr(), rows, groups, tile,
-                                                  counts.data_ptr(), _stream_ptr(blocks.device)))
-        bad_full, bad_tail = counts.tolist()
+        codes, scales, staging = _upload(codes, scales, blocks.device)
+        try:
+            counts = torch.empty(2, dtype=torch.int64, device=blocks.device)
+            # scanned and, where nothing was found, converted: one wait for both, by reading the counts
+            check(_native.lib().tq1_load_tiled_device(codes.data_ptr(), scales.data_ptr(), blocks.data_ptr(), rows, groups, tile,
+                                                      counts.data_ptr(), _stream_ptr(blocks.device)))
+            bad_full, bad_tail = counts.tolist()
+        except BaseException:
+            torch.cuda.current_stream().synchronize()       # nothing is read from the staging any more
+            raise
+        del staging
     if bad_full or bad_tail:
         raise FormatError(out_of_range_message(bad_full, bad_tail))
 

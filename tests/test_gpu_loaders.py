@@ -138,3 +138,65 @@ def test_upload_through_staging_of_any_size(sizes, staging_bytes):
         got = device.cpu().numpy()
         assert np.array_equal(got[:host.size], host) and not got[host.size:].any()
     assert lib.tq1_upload_pair(devices[0].data_ptr(), hosts[0].ctypes.data, 1, None, None, 0, staging.data_ptr(), 1024, stream) != 0
+
+
+def _tiled_module(rows, columns, seed):
+    from ternel_b200.layout import PackedTensorLayout, pack_blocks
+    from ternel_b200.modules import PackedLinear
+    layout = PackedTensorLayout.for_tensor(rows, columns)
+    blocks, _ = random_blocks(rows, columns, seed=seed)
+    return PackedLinear(layout, device="cuda"), blocks, pack_blocks(blocks, layout=layout)
+
+
+def test_load_tiled_without_pinned_memory(monkeypatch):
+    """Where no staging can be pinned, the arrays are uploaded as they are."""
+    module, blocks, tiled = _tiled_module(768, 1408, 5)
+    empty, refused = torch.empty, []
+
+    def no_pinned(*args, **kwargs):
+        if kwargs.get("pin_memory"):
+            refused.append(args)
+            raise RuntimeError("out of pinned memory")
+        return empty(*args, **kwargs)
+    monkeypatch.setattr(torch, "empty", no_pinned)
+    module.load_tiled(*tiled)
+    assert refused and np.array_equal(module.blocks.cpu().numpy(), blocks)
+
+
+@pytest.mark.parametrize("fails", (False, True))
+def test_staging_is_held_until_its_transfers_are_done(monkeypatch, fails):
+    """The pool of pinned memory does not know of them: the staging goes back to it after the stream has been waited for."""
+    import weakref
+    from ternel_b200 import _native
+    module, blocks, tiled = _tiled_module(768, 1408, 6)
+    empty, held, seen, synchronize = torch.empty, [], [], torch.cuda.Stream.synchronize
+
+    def noted(*args, **kwargs):
+        tensor = empty(*args, **kwargs)
+        if kwargs.get("pin_memory"):
+            held.append(weakref.ref(tensor))
+        return tensor
+
+    class Library:
+        def __getattr__(self, name):
+            return getattr(real, name)
+
+        def tq1_load_tiled_device(self, *args):
+            seen.append(held[0]() is not None)
+            return -1 if fails else real.tq1_load_tiled_device(*args)
+
+    def waited(stream):
+        seen.append(held[0]() is not None)
+        synchronize(stream)
+    real = _native.lib()
+    monkeypatch.setattr(torch, "empty", noted)
+    monkeypatch.setattr(torch.cuda.Stream, "synchronize", waited)
+    monkeypatch.setattr(_native, "lib", Library)
+    if fails:
+        with pytest.raises(Exception):
+            module.load_tiled(*tiled)
+        assert seen == [True, True]
+    else:
+        module.load_tiled(*tiled)
+        assert seen == [True] and np.array_equal(module.blocks.cpu().numpy(), blocks)
+    assert len(held) == 1
