@@ -243,6 +243,24 @@ int tq1_debug_linear_as(int form, const uint8_t *blocks, const void *x, void *y,
     return fail(TQ1_ERR_INVALID, "tq1_debug_linear_as: form %d does not take %dx%dx%d", form, M, N, K);
 }
 
+// Tests only: the layout of a call by the kernel of `form` (TQ1_FORM_STREAM_GEMV: one or two activation rows as a call of their own),
+// whether or not the rules would send it there. layout: CTAs of a cluster, sets of warps, ring stages, row tiles of
+// a cluster. All zero: that kernel does not take it.
+int tq1_debug_call_layout(int form, int M, int N, int K, const int *rooms, int *layout) {
+    if (!layout || M <= 0 || N <= 0 || K <= 0 || K % kGroup) return fail(TQ1_ERR_INVALID, "tq1_debug_call_layout: bad call");
+    CallLayout l = {};
+    if (form == TQ1_FORM_STREAM_GEMV) {
+        if (!gemv_tiles_layout(M, N, K, rooms, &l)) l = {};
+    } else {
+        return fail(TQ1_ERR_INVALID, "tq1_debug_call_layout: form %d", form);
+    }
+    layout[0] = l.cluster;
+    layout[1] = l.sets;
+    layout[2] = l.stages;
+    layout[3] = l.tiles;
+    return TQ1_OK;
+}
+
 int tq1_debug_force_token_tile(int token_tile) {
     if (gemm_tc_force_tile(token_tile) != TQ1_OK)
         return fail(TQ1_ERR_INVALID, "tq1_debug_force_token_tile: %d is not 0, 16, 32, 64, 128 or 256", token_tile);

@@ -48,10 +48,12 @@ constexpr uint32_t kWindowEnd = 227 * 1024;
 constexpr int kMinWarps = 8;                                    // fewer would be long at the table
 constexpr int kLag = 2;                                         // a tile is added up while the second one after it is decoded
 constexpr int kBufs = 2 * kLag;
-constexpr int kMaxStages = 48;
 constexpr int kMaxOwn = 128;                                    // tiles that a CTA of a cluster adds up
 constexpr int kMaxTokens = 2;
-static_assert(8 * (kMaxStages + kMaxWarps * kBufs + kMaxOwn) <= 2048, "barrier area");
+// The barriers: sums; ring; where clusters split K, one for each tile that a CTA adds up.
+constexpr int kRingBars = kMaxWarps * kBufs, kTileBars = 256 - kMaxOwn;
+constexpr int kMaxStages = (kLag + 1) * kMaxWarps, kMaxStagesSplit = 48;
+static_assert(kRingBars + kMaxStages <= 256 && kRingBars + kMaxStagesSplit <= kTileBars, "barrier area of 2048 bytes");
 
 struct TileParams {
     const __half *x;                                            // [tokens][chunks * 512]
@@ -60,7 +62,7 @@ struct TileParams {
     int N, chunks;
     int tiles, clusters;                                        // row tiles, clusters of the grid
     int split_log, slices, subsets;                             // CTAs of a cluster; chunks of a CTA at most; sets of warps
-    int stages, early, pitch;                                   // ring stages; those that lie apart from the scratch; bytes from row to row
+    int stages, early, pitch;                                   // ring stages; those that are filled before the planes; bytes from row to row
     uint32_t plane_addr, xchg_addr, sums_addr, ring_addr;       // the scratch (planes, exchange) lies where the last stages are
     int y_f32, swiglu;
 };
@@ -150,11 +152,9 @@ tiles_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ T
     const int n_tiles = (int)((long long)(cluster + 1) * prm.tiles / prm.clusters) - tile_lo;
     const int set_warps = n_slices * TOKENS;                // of this CTA's sets
     const uint32_t stage_bytes = (uint32_t)(kTileRows * prm.pitch);
-    auto full_bar = [&](int s) { return base + kBarAddr + 8u * (uint32_t)s; };
-    auto sum_bar = [&](int s) { return base + kBarAddr + 8u * (uint32_t)(kMaxStages + s); };
-
-    // clusters: one for each tile that this CTA adds up
-    auto tile_bar = [&](int s) { return base + kBarAddr + 8u * (uint32_t)(kMaxStages + kMaxWarps * kBufs + s); };
+    auto sum_bar = [&](int s) { return base + kBarAddr + 8u * (uint32_t)s; };
+    auto full_bar = [&](int s) { return base + kBarAddr + 8u * (uint32_t)(kRingBars + s); };
+    auto tile_bar = [&](int s) { return base + kBarAddr + 8u * (uint32_t)(kTileBars + s); };
     const int own_tiles = (n_tiles - rank + split - 1) >> split_log;
 
     // ---- set-up that depends on no earlier kernel ---------------------------------------------------------------
@@ -170,7 +170,7 @@ tiles_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ T
     if (tid == 32) asm volatile("prefetch.tensormap [%0];" ::"l"(&wmap) : "memory");
     const int word_x = chunk_lo * (kChunkBytes / 8);            // the map's elements are 8 bytes
     if (warp == warps - 1 && elect_one())                       // the first tiles: into L2 (a hint, whatever they hold by now)
-        for (int i = 0; i < min(prm.stages, n_tiles); ++i)
+        for (int i = 0; i < min(prm.early, n_tiles); ++i)
             asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];"
                          ::"l"(&wmap), "r"(word_x), "r"((tile_lo + i) * kTileRows) : "memory");
     // what no activation is paired with (scales, half of the word that two lanes share) stays zero
@@ -253,7 +253,7 @@ tiles_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ T
         gpow[sub] = gc.pow;
         gbad[sub] = gc.bad;
     }
-    if (prm.early < min(prm.stages, n_tiles)) {                 // the other stages' place is free now
+    if (prm.early < min(prm.stages, n_tiles)) {                 // the other stages: their place may have been the scratch
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (warp == warps - 1 && elect_one())
@@ -366,7 +366,7 @@ float tile_us(int split_log, int set_warps, int subsets, int per_cluster) {
     return 3.0f + (split_log ? 1.2f : 0.0f) + (sm > chain ? sm : chain);
 }
 
-TilePlan tile_plan(int tokens, int N, int K) {
+TilePlan tile_plan(int tokens, int N, int K, const int *rooms = nullptr) {
     TilePlan best = {};
     const int chunks = K / kChunkCols, tiles = (N + kTileRows - 1) / kTileRows;
     for (int log = 0; log <= 3; ++log) {
@@ -382,7 +382,7 @@ TilePlan tile_plan(int tokens, int N, int K) {
         // how many clusters run at once is asked of the driver (milliseconds, the first time) only where this split could win
         const int hope = (tiles + sm_count() / split - 1) / (sm_count() / split);
         if (best.ok && tile_us(log, set_warps, subsets_for(hope), hope) >= best.us) continue;
-        const int room = clusters_at_once(g_records[log > 0][tokens - 1], reinterpret_cast<const void *>(kernel_of(log > 0, tokens)), 32 * kMaxWarps, kWindowEnd - kWindow, 1 << log);
+        const int room = rooms ? rooms[split] : clusters_at_once(g_records[log > 0][tokens - 1], reinterpret_cast<const void *>(kernel_of(log > 0, tokens)), 32 * kMaxWarps, kWindowEnd - kWindow, 1 << log);
         p.clusters = tiles < room ? tiles : room;
         const int per = (tiles + p.clusters - 1) / p.clusters;
         p.subsets = subsets_for(per);
@@ -395,17 +395,24 @@ TilePlan tile_plan(int tokens, int N, int K) {
         const uint32_t stage_bytes = (uint32_t)(kTileRows * p.pitch);
         const uint32_t plane_bytes = aligned((size_t)set_warps * kPlaneChunk), scratch = plane_bytes + kMaxWarps * 2 * kGroup * 4;
         if (p.ring_addr + scratch + stage_bytes > kWindowEnd) continue;
-        const auto stages_in = [&](uint32_t end) { const int n = (int)((end - p.ring_addr) / stage_bytes); return n > kMaxStages ? kMaxStages : n; };
+        const auto stages_in = [&](uint32_t end) { const int n = (int)((end - p.ring_addr) / stage_bytes), most = log ? kMaxStagesSplit : kMaxStages; return n > most ? most : n; };
         p.stages = stages_in(kWindowEnd) < per ? stages_in(kWindowEnd) : per;
-        // a stage is asked for again kLag turns of its set after it was read
-        while (p.subsets > 1 && p.stages < per && p.stages <= kLag * p.subsets) --p.subsets;
-        if (p.stages < per && p.stages <= kLag * p.subsets) continue;
+        if (p.stages < per) {
+            // A stage is asked for again kLag turns of its set after it was read. And it belongs to one set: a wait for a barrier's
+            // parity tells a phase from the one before it only, so who waits has to have seen that one.
+            while (p.subsets > 1 && p.stages <= kLag * p.subsets + p.stages % p.subsets) --p.subsets;
+            p.stages -= p.stages % p.subsets;
+            if (p.stages <= kLag) continue;
+        }
         // the scratch lies at the end, behind all stages where there is room for that
         p.end = p.ring_addr + aligned((size_t)p.stages * stage_bytes) + scratch;
         if (p.end > kWindowEnd) p.end = kWindowEnd;
         p.plane_addr = p.end - scratch;
         p.xchg_addr = p.plane_addr + plane_bytes;
+        // The first stages are asked for by one warp while the others prepare the planes and then wait for it: a box to each set and
+        // no more (151936x512, sixty stages: all before the planes 9.9 us, twenty 9.2).
         p.early = stages_in(p.plane_addr) < p.stages ? stages_in(p.plane_addr) : p.stages;
+        if (p.early > kMaxWarps) p.early = kMaxWarps;
         p.ok = true;
         p.us = tile_us(log, set_warps, p.subsets, per);
         if (!best.ok || p.us < best.us) best = p;
@@ -414,6 +421,14 @@ TilePlan tile_plan(int tokens, int N, int K) {
 }
 
 }  // namespace
+
+bool gemv_tiles_layout(int M, int N, int K, const int *rooms, CallLayout *layout) {
+    if (M < 1 || M > kMaxTokens || !gemv_chain_shape_ok(N, K)) return false;
+    const TilePlan p = tile_plan(M, N, K, rooms);
+    if (!p.ok) return false;
+    *layout = {1 << p.split_log, p.subsets, p.stages, ((N + kTileRows - 1) / kTileRows + p.clusters - 1) / p.clusters};
+    return true;
+}
 
 bool try_gemv_tiles(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, bool swiglu, void *workspace,
                     cudaStream_t stream, int *status) {

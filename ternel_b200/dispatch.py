@@ -57,6 +57,26 @@ def plan(batch: int, rows: int, columns: int, *, aligned: bool = True, workspace
     return LinearPlan(KERNELS[kernel.value], tile.value, ctas.value, parts.value, FORMS[form.value])
 
 
+@dataclass(frozen=True)
+class RingLayout:
+    cluster: int         # CTAs that share a row tile's columns
+    sets: int            # sets of warps that take turns on the row tiles
+    stages: int          # row tiles that a CTA holds at a time
+    tiles: int           # row tiles of a cluster
+
+
+def ring_layout(form: str, batch: int, rows: int, columns: int, *, rooms: "dict[int, int] | None" = None) -> "RingLayout | None":
+    """How the kernel that streams row tiles for 1 and 2 activation rows (``"stream_gemv"``) lays out a call, whether or not the rules
+    send it there; None where it does not take it (a batch-1 call then is a chain of one link). ``rooms`` replaces what the driver
+    says of how many clusters of a size run at once."""
+    ask = _native.lib().tq1_debug_call_layout
+    ask.restype, ask.argtypes = ctypes.c_int, [ctypes.c_int] * 4 + [ctypes.c_void_p] * 2
+    given = (ctypes.c_int * 17)(*(rooms.get(size, 0) for size in range(17))) if rooms is not None else None
+    out = (ctypes.c_int * 4)()
+    check(ask({name: number for number, name in FORMS.items()}[form], batch, rows, columns, given, out))
+    return RingLayout(*out) if out[0] else None
+
+
 def looped_tokens() -> int:
     """Largest batch the library runs as passes of the batch-1 kernel (found by probing the plan)."""
     tokens = 1

@@ -46,6 +46,27 @@ def test_equals_the_chain_kernel(rows, columns):
             assert torch.equal(tq1_swiglu(blocks, x[:batch], out_dtype=torch.float32), gated[:batch])
 
 
+# Rings that are gone round: two sets of warps on eight stages, three on twelve, five and two on twenty, twenty on sixty, and two
+# and one on six in a cluster of two
+ROUND = ((40961, 5120, 1), (34816, 3072, 1), (50001, 2048, 1), (50001, 2048, 2), (151934, 512, 1), (34815, 10240, 1), (34815, 10240, 2))
+
+
+@pytest.mark.parametrize(("rows", "columns", "batch"), ROUND)
+def test_stages_that_are_filled_again(rows, columns, batch):
+    from ternel_b200.dispatch import ring_layout
+    from ternel_b200.ops import tq1_matmul
+    from ternel_b200.stack import random_blocks_device
+    layout = ring_layout("stream_gemv", batch, rows, columns)
+    assert layout.tiles > layout.stages
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(rows + columns)
+    blocks = random_blocks_device(rows, columns, gen, "cuda")
+    x = torch.randn((batch, columns), generator=gen, device="cuda").to(torch.float16)
+    want = single_links(blocks, x, False)
+    for _ in range(3):
+        assert torch.equal(tq1_matmul(blocks, x, out_dtype=torch.float32), want)
+
+
 @pytest.mark.parametrize("value", (np.inf, -np.inf, np.nan))
 @pytest.mark.parametrize(("rows", "columns"), ((70, 1024), (40, 10240)))
 def test_non_finite_groups(rows, columns, value):

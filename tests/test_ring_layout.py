@@ -1,0 +1,28 @@
+"""Rings of row tiles that several sets of warps take turns on (host logic, no GPU needed)."""
+
+import pytest
+
+from ternel_b200.dispatch import ring_layout
+
+ROWS = (100, 5120, 9000, 17408, 20000, 34816, 50000, 100000, 151936, 262144)
+COLUMNS = (*range(512, 5121, 512), 7680, 9728, 10240, 15360, 17408, 19456, 20480, 32768, 40960, 65536)
+
+
+@pytest.mark.parametrize(("form", "batch"), (("stream_gemv", 1), ("stream_gemv", 2)))
+def test_a_barrier_of_the_ring_belongs_to_one_set(form, batch):
+    """A wait for a phase's parity returns at once while the phase before that is still open. So whoever waits for a tile has to have
+    waited for the tile before it on the same barrier: tiles on one barrier are whole turns of the sets apart. And a stage is not
+    filled again before its tile was read."""
+    around = 0
+    for columns in COLUMNS:
+        for rows in ROWS:
+            layout = ring_layout(form, batch, rows, columns) if rows * columns < 1.3e9 else None
+            if layout is None:
+                continue
+            assert 1 <= layout.sets <= 20 and 1 <= layout.stages
+            if layout.stages >= layout.tiles:
+                continue
+            around += 1
+            assert layout.stages % layout.sets == 0, (rows, columns, layout)
+            assert layout.stages > layout.sets, (rows, columns, layout)
+    assert around > 40
