@@ -243,14 +243,16 @@ int tq1_debug_linear_as(int form, const uint8_t *blocks, const void *x, void *y,
     return fail(TQ1_ERR_INVALID, "tq1_debug_linear_as: form %d does not take %dx%dx%d", form, M, N, K);
 }
 
-// Tests only: the layout of a call by the kernel of `form` (TQ1_FORM_STREAM_GEMV: one or two activation rows as a call of their own),
-// whether or not the rules would send it there. layout: CTAs of a cluster, sets of warps, ring stages, row tiles of
+// Tests only: the layout of a call by the kernel of `form` (TQ1_FORM_STREAM_GEMV: one or two activation rows as a call of their own;
+// TQ1_FORM_SLICES), whether or not the rules would send it there. layout: CTAs of a cluster, sets of warps, ring stages, row tiles of
 // a cluster. All zero: that kernel does not take it.
 int tq1_debug_call_layout(int form, int M, int N, int K, const int *rooms, int *layout) {
     if (!layout || M <= 0 || N <= 0 || K <= 0 || K % kGroup) return fail(TQ1_ERR_INVALID, "tq1_debug_call_layout: bad call");
     CallLayout l = {};
     if (form == TQ1_FORM_STREAM_GEMV) {
         if (!gemv_tiles_layout(M, N, K, rooms, &l)) l = {};
+    } else if (form == TQ1_FORM_SLICES) {
+        if (!gemm_slices_layout(M, N, K, rooms, &l)) l = {};
     } else {
         return fail(TQ1_ERR_INVALID, "tq1_debug_call_layout: form %d", form);
     }

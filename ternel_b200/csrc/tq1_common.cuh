@@ -171,9 +171,10 @@ bool try_gemv_tiles(const uint8_t *blocks, const __half *x, void *y, bool y_f32,
 // (rooms[size]), in place of what the driver says.
 struct CallLayout {
     int cluster;                        // CTAs of a cluster
-    int sets, stages, tiles;            // sets of warps, ring stages, row tiles of a cluster at most
+    int sets, stages, tiles;            // sets of warps, ring stages, row tiles of a cluster at most (batch-1 and slice kernel)
 };
 bool gemv_tiles_layout(int M, int N, int K, const int *rooms, CallLayout *layout);
+bool gemm_slices_layout(int M, int N, int K, const int *rooms, CallLayout *layout);
 int launch_shard_wait(const ShardDev &shard, unsigned *status, cudaStream_t stream);
 int launch_shard_push(const __half *local, int M, int n_local, const ShardDev &shard, cudaStream_t stream);
 int launch_epoch_advance(unsigned *epoch_base, unsigned delta, cudaStream_t stream);

@@ -473,7 +473,7 @@ float slice_us(int split, int slices, int per_cluster) {
 }
 
 // The K split with the smallest modelled time.
-SlicePlan slice_plan(int nt, int N, int K) {
+SlicePlan slice_plan(int nt, int N, int K, const int *rooms = nullptr) {
     SlicePlan best = {};
     const int per = slice_halves(nt), halves = K / 256 / per, tiles = (N + kTileRows - 1) / kTileRows;
     for (int log = 0; log <= 3; ++log) {
@@ -484,7 +484,7 @@ SlicePlan slice_plan(int nt, int N, int K) {
         if (halves < split || p.slices > kMaxSlices) continue;
         // how many clusters run at once is asked of the driver (milliseconds, the first time) only where this split could win
         if (best.ok && slice_us(split, p.slices, (tiles + sm_count() / split - 1) / (sm_count() / split)) >= best.us) continue;
-        const int room = clusters_at_once(g_records[nt - 1], kernel_of(nt), 32 * (kMaxSlices + kExtraWarps), kWindowEnd - kWindow, 1 << log);
+        const int room = rooms ? rooms[split] : clusters_at_once(g_records[nt - 1], kernel_of(nt), 32 * (kMaxSlices + kExtraWarps), kWindowEnd - kWindow, 1 << log);
         p.clusters = tiles < room ? tiles : room;
         const int per_cluster = (tiles + p.clusters - 1) / p.clusters;
         p.subsets = kMaxSlices / p.slices;
@@ -504,6 +504,12 @@ SlicePlan slice_plan(int nt, int N, int K) {
         if (p.stages > kMaxStages) p.stages = kMaxStages;
         if (p.stages > per_cluster) p.stages = per_cluster;
         if (p.stages < (per_cluster < 2 * p.subsets ? per_cluster : p.subsets + 1)) continue;      // no room to fetch ahead
+        if (p.stages < per_cluster) {
+            // A stage belongs to one set of warps: a wait for a barrier's parity tells a phase from the one before it only, so who
+            // waits has to have seen that one.
+            while (p.subsets > 1 && p.stages < 2 * p.subsets) --p.subsets;
+            p.stages -= p.stages % p.subsets;
+        }
         if (split > 1 && (per_cluster + split - 1) / split > kMaxOwn) continue;
         p.end = p.ring_addr + (uint32_t)p.stages * stage_bytes;
         p.ok = true;
@@ -560,6 +566,14 @@ static SlicePlan preferred_plan(int M, int N, int K) {
     SlicePlan p = slice_plan(nt, N, K);
     p.ok = p.ok && call_us(p, nt, (N + kTileRows - 1) / kTileRows) < (nt == 1 ? 1.0f : 1.04f) * gemm_tc_few_us(N, K);
     return p;
+}
+
+bool gemm_slices_layout(int M, int N, int K, const int *rooms, CallLayout *layout) {
+    if (M < 3 || M > 16 || K % 512) return false;
+    const SlicePlan p = slice_plan(M <= 8 ? 1 : 2, N, K, rooms);
+    if (!p.ok) return false;
+    *layout = {p.split, p.subsets, p.stages, ((N + kTileRows - 1) / kTileRows + p.clusters - 1) / p.clusters};
+    return true;
 }
 
 bool gemm_slices_preferred(int M, int N, int K) { return preferred_plan(M, N, K).ok; }

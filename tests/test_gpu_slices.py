@@ -36,6 +36,30 @@ def test_slices_against_float64(rows, columns, batch):
     assert np.array_equal(half, got.astype(np.float16).astype(np.float32))
 
 
+@pytest.mark.parametrize(("rows", "columns", "batch"), ((70001, 512, 4), (34810, 2560, 8), (50001, 2048, 3), (70001, 512, 12)))
+def test_stages_that_are_filled_again(rows, columns, batch):
+    """Several sets of warps whose ring is gone round, by the C ABI's name for this kernel. Whole numbers, so every sum is exact."""
+    from ternel_b200 import _native
+    from ternel_b200.dispatch import ring_layout
+    layout = ring_layout("slices", batch, rows, columns)
+    assert layout.sets > 1 and layout.tiles > layout.stages
+    rng = np.random.default_rng(rows)
+    groups = rows * columns // 128
+    trits = rng.integers(0, 3, size=(groups, 128), dtype=np.uint8)
+    scales = np.ones(groups, np.float16).view(np.uint8).reshape(-1, 2)
+    blocks = to_dev(o.encode_blocks(scales, trits).reshape(rows, columns // 128, 28))
+    x = torch.randint(-1, 2, (batch, columns), device="cuda").to(torch.float16)
+    want = x.float() @ (to_dev(trits.reshape(rows, columns)).float() - 1).T
+    y, ws = torch.empty((batch, rows), dtype=torch.float32, device="cuda"), torch.zeros(1 << 16, dtype=torch.uint8, device="cuda")
+    run = _native.lib().tq1_debug_linear_as
+    run.restype = ctypes.c_int
+    run.argtypes = [ctypes.c_int, *_native.SIGNATURES["tq1_linear_f16"][1][:8], ctypes.c_void_p]
+    for _ in range(3):
+        assert run(3, blocks.data_ptr(), x.data_ptr(), y.data_ptr(), 1, batch, rows, columns, ws.data_ptr(),
+                   torch.cuda.current_stream().cuda_stream) == 0
+        assert torch.equal(y, want) and int(ws[:4].view(torch.int32)) == 0
+
+
 @pytest.mark.parametrize("batch", (3, 16))
 @pytest.mark.parametrize("offset", (1, 2, 4))
 def test_results_off_the_wide_grid(batch, offset):

@@ -8,7 +8,7 @@ ROWS = (100, 5120, 9000, 17408, 20000, 34816, 50000, 100000, 151936, 262144)
 COLUMNS = (*range(512, 5121, 512), 7680, 9728, 10240, 15360, 17408, 19456, 20480, 32768, 40960, 65536)
 
 
-@pytest.mark.parametrize(("form", "batch"), (("stream_gemv", 1), ("stream_gemv", 2)))
+@pytest.mark.parametrize(("form", "batch"), (("stream_gemv", 1), ("stream_gemv", 2), ("slices", 3), ("slices", 9)))
 def test_a_barrier_of_the_ring_belongs_to_one_set(form, batch):
     """A wait for a phase's parity returns at once while the phase before that is still open. So whoever waits for a tile has to have
     waited for the tile before it on the same barrier: tiles on one barrier are whole turns of the sets apart. And a stage is not
