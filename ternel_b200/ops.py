@@ -262,7 +262,7 @@ def _upload(first: torch.Tensor, second: torch.Tensor, device: torch.device) -> 
     sizes = [array.numel() * array.element_size() for array in arrays]
     if not plain:
         try:
-            staging = torch.empty(min(sum(sizes) + (1 << 20), _STAGING_BYTES), dtype=torch.uint8, pin_memory=True)
+            staging = torch.empty(min(sum(sizes) + (1 << 20), _STAGING_BYTES), dtype=torch.uint8, device="cpu", pin_memory=True)
         except RuntimeError:            # no pinned memory to be had: the driver's own way
             plain = True
     if plain:

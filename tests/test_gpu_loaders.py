@@ -163,6 +163,23 @@ def test_load_tiled_without_pinned_memory(monkeypatch):
     assert refused and np.array_equal(module.blocks.cpu().numpy(), blocks)
 
 
+@pytest.mark.parametrize("device", ("cuda", "meta", "cpu"))
+def test_load_tiled_under_a_default_device(monkeypatch, device):
+    """The staging is pinned host memory whatever tensors are made on by default."""
+    module, blocks, tiled = _tiled_module(768, 1408, 7)
+    empty, staged = torch.empty, []
+
+    def noted(*args, **kwargs):
+        tensor = empty(*args, **kwargs)
+        if kwargs.get("pin_memory"):
+            staged.append(tensor.is_pinned() and tensor.data_ptr() != 0)
+        return tensor
+    monkeypatch.setattr(torch, "empty", noted)
+    with torch.device(device):
+        module.load_tiled(*tiled)
+    assert staged == [True] and np.array_equal(module.blocks.cpu().numpy(), blocks)
+
+
 @pytest.mark.parametrize("fails", (False, True))
 def test_staging_is_held_until_its_transfers_are_done(monkeypatch, fails):
     """The pool of pinned memory does not know of them: the staging goes back to it after the stream has been waited for."""
