@@ -167,11 +167,12 @@ int launch_gemv_single(const uint8_t *blocks, const __half *x, void *y, bool y_f
 // workspace's first word is the status word) and returns true where it takes the call.
 bool try_gemv_tiles(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, bool swiglu, void *workspace,
                     cudaStream_t stream, int *status);
-// How a call would be laid out (tests; launches nothing). rooms: null, or how many clusters of 1, 2, .. kMaxCluster CTAs run at once
+// How a call is laid out by the batch-1 or the slice kernel where that one takes it (tests; launches nothing). rooms: null, or how many clusters of 1, 2, .. kMaxCluster CTAs run at once
 // (rooms[size]), in place of what the driver says.
 struct CallLayout {
     int cluster;                        // CTAs of a cluster
-    int sets, stages, tiles;            // sets of warps, ring stages, row tiles of a cluster at most (batch-1 and slice kernel)
+    int sets, stages, tiles;            // sets of warps, ring stages, row tiles of a cluster at most
+    bool preferred;                     // over the kernel that takes the call otherwise
 };
 bool gemv_tiles_layout(int M, int N, int K, const int *rooms, CallLayout *layout);
 bool gemm_slices_layout(int M, int N, int K, const int *rooms, CallLayout *layout);

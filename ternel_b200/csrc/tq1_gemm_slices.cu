@@ -572,7 +572,7 @@ bool gemm_slices_layout(int M, int N, int K, const int *rooms, CallLayout *layou
     if (M < 3 || M > 16 || K % 512) return false;
     const SlicePlan p = slice_plan(M <= 8 ? 1 : 2, N, K, rooms);
     if (!p.ok) return false;
-    *layout = {p.split, p.subsets, p.stages, ((N + kTileRows - 1) / kTileRows + p.clusters - 1) / p.clusters};
+    *layout = {p.split, p.subsets, p.stages, ((N + kTileRows - 1) / kTileRows + p.clusters - 1) / p.clusters, gemm_slices_preferred(M, N, K)};
     return true;
 }
 

@@ -16,6 +16,8 @@
 //   cluster   2, 4 or 8 CTAs split K where one CTA has no warps for it; partial sums go to the CTA that adds a tile's through
 //             distributed shared memory
 //
+// Where even four CTAs would not do, or do no better, the chain kernel takes the call (not_behind_chain).
+//
 // The table (256 entries, 32 copies each) is worked out by the CTA's warps, four entries per instruction.
 //
 // What bounds it: many rows, the loop of the units, 105 clocks of an SM each (76 wavefronts of shared memory, about 330 instructions
@@ -27,6 +29,7 @@
 // 71.5 us, before them 50.3); loop bookkeeping left to kernel parameters and divisions (50.3, 45.8); a thread's barriers and a
 // cluster barrier around the sums of split K (5120x17408 12.2, 11.3 with st.async and a barrier per tile).
 #include <cuda.h>
+#include <math.h>
 
 #include <type_traits>
 
@@ -346,7 +349,7 @@ tiles_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ T
 
 // ---- host ---------------------------------------------------------------------------------------------------------
 struct TilePlan {
-    bool ok;
+    bool ok, faster;                                            // fits; and is not behind the chain kernel
     float us;
     int split_log, slices, subsets, clusters, stages, pitch;
     int early;
@@ -366,9 +369,24 @@ float tile_us(int split_log, int set_warps, int subsets, int per_cluster) {
     return 3.0f + (split_log ? 1.2f : 0.0f) + (sm > chain ? sm : chain);
 }
 
+// Columns that only four or eight CTAs have room for: their clusters leave SMs idle (132 and 120 work), and a CTA has ten to twenty
+// warps as the columns come out, while the chain kernel's units fall evenly on 148 times sixteen. One row, the chain kernel and this
+// one (us): 20000x20480 30.9, 28.5; 34816x18944 42.1, 43.6; 9000x25600 20.3, 22.1; 20000x25600 35.9, 41.0; 34816x32768 75.4, 100; two
+// rows: 5000x25600 25.1, 23.9; 20000x25600 66, 78. Times fitted to 283 such calls (within 6 and 4%, 2-norm): what they choose is 0.4%
+// above the better one on average; of 51 calls that this kernel lost 3 to 33% with three are left, of at most 5%, and ten are given up
+// that it was 3 to 13% faster with. Narrower matrices are its own: with none of 208 it was behind by more than 2.2%.
+bool not_behind_chain(const TilePlan &p, int tokens, int tiles, int chunks) {
+    const float per = (float)((tiles + p.clusters - 1) / p.clusters), units = (float)(tiles * (long long)chunks) / (float)sm_count();
+    const float turns = ceilf(per / (float)p.subsets), other = (float)(tokens - 1);
+    const float own = 4.35f + per * (float)(p.slices * tokens) * (0.054f - 0.005f * other) + 0.22f * turns;
+    const float chain = 5.4f + 2.4f * other + (float)tokens * (0.0707f * units + 0.0186f * (float)chunks);
+    return own <= chain;
+}
+
 TilePlan tile_plan(int tokens, int N, int K, const int *rooms = nullptr) {
     TilePlan best = {};
     const int chunks = K / kChunkCols, tiles = (N + kTileRows - 1) / kTileRows;
+    bool narrow = false;                                        // two CTAs have room for the columns
     for (int log = 0; log <= 3; ++log) {
         const int split = 1 << log;
         TilePlan p = {};
@@ -415,8 +433,10 @@ TilePlan tile_plan(int tokens, int N, int K, const int *rooms = nullptr) {
         if (p.early > kMaxWarps) p.early = kMaxWarps;
         p.ok = true;
         p.us = tile_us(log, set_warps, p.subsets, per);
+        narrow = narrow || log < 2;
         if (!best.ok || p.us < best.us) best = p;
     }
+    best.faster = best.ok && (narrow || not_behind_chain(best, tokens, tiles, chunks));
     return best;
 }
 
@@ -426,7 +446,7 @@ bool gemv_tiles_layout(int M, int N, int K, const int *rooms, CallLayout *layout
     if (M < 1 || M > kMaxTokens || !gemv_chain_shape_ok(N, K)) return false;
     const TilePlan p = tile_plan(M, N, K, rooms);
     if (!p.ok) return false;
-    *layout = {1 << p.split_log, p.subsets, p.stages, ((N + kTileRows - 1) / kTileRows + p.clusters - 1) / p.clusters};
+    *layout = {1 << p.split_log, p.subsets, p.stages, ((N + kTileRows - 1) / kTileRows + p.clusters - 1) / p.clusters, p.faster};
     return true;
 }
 
@@ -435,7 +455,7 @@ bool try_gemv_tiles(const uint8_t *blocks, const __half *x, void *y, bool y_f32,
     if (M < 1 || M > kMaxTokens || !gemv_chain_supported(blocks, N, K)) return false;
     const TilePlan p = tile_plan(M, N, K);
     const EncodeTiledFn encode = encode_tiled_fn();
-    if (!p.ok || !encode) return false;
+    if (!p.faster || !encode) return false;
     TileParams prm;
     prm.x = x;
     prm.y = y;

@@ -63,6 +63,7 @@ class RingLayout:
     sets: int            # sets of warps that take turns on the row tiles
     stages: int          # row tiles that a CTA holds at a time
     tiles: int           # row tiles of a cluster
+    preferred: bool      # what the rules say: of one row, this kernel or a chain of one link; of three to sixteen, this one or tcgen05
 
 
 def ring_layout(form: str, batch: int, rows: int, columns: int, *, rooms: "dict[int, int] | None" = None) -> "RingLayout | None":
@@ -72,9 +73,9 @@ def ring_layout(form: str, batch: int, rows: int, columns: int, *, rooms: "dict[
     ask = _native.lib().tq1_debug_call_layout
     ask.restype, ask.argtypes = ctypes.c_int, [ctypes.c_int] * 4 + [ctypes.c_void_p] * 2
     given = (ctypes.c_int * 17)(*(rooms.get(size, 0) for size in range(17))) if rooms is not None else None
-    out = (ctypes.c_int * 4)()
+    out = (ctypes.c_int * 5)()
     check(ask({name: number for number, name in FORMS.items()}[form], batch, rows, columns, given, out))
-    return RingLayout(*out) if out[0] else None
+    return RingLayout(*out[:4], bool(out[4])) if out[0] else None
 
 
 def looped_tokens() -> int:

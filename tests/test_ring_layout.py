@@ -26,3 +26,17 @@ def test_a_barrier_of_the_ring_belongs_to_one_set(form, batch):
             assert layout.stages % layout.sets == 0, (rows, columns, layout)
             assert layout.stages > layout.sets, (rows, columns, layout)
     assert around > 40
+
+
+@pytest.mark.parametrize(("batch", "rows", "columns"), (
+    (1, 60000, 18944), (1, 9000, 25600), (1, 20000, 25600), (1, 34816, 32768), (1, 9000, 49152), (2, 9000, 25600), (2, 20000, 25600)))
+def test_wide_matrices_that_the_chain_kernel_is_faster_for(batch, rows, columns):
+    """By 6% and more in recorded times: clusters of four and eight CTAs leave SMs idle, and these have work for all of them."""
+    assert not ring_layout("stream_gemv", batch, rows, columns).preferred
+
+
+@pytest.mark.parametrize(("batch", "rows", "columns"), (
+    (1, 1024, 5120), (1, 151936, 5120), (1, 34816, 17408), (1, 100000, 10240), (2, 17408, 5120), (2, 5120, 17408), (2, 20000, 10240),
+    (1, 1000, 25600), (1, 9000, 20480), (1, 5000, 40960), (2, 5000, 20480), (2, 1000, 40960)))
+def test_matrices_that_the_tile_kernel_is_faster_for(batch, rows, columns):
+    assert ring_layout("stream_gemv", batch, rows, columns).preferred
