@@ -146,9 +146,10 @@ int tq1_linear_f16(const uint8_t *blocks, const void *x, void *y, int y_is_f32,
     if (M == 1 && gemv_chain_fits(blocks, N, K))
         return launch_gemv_single(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, N, K, false, workspace,
                                   kWsSlotRegionBytes, s);
-    if (gemv_looped_fits(blocks, M, N, K) && need >= kWsScratchOffset)
-        return launch_gemv_looped(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, false, workspace, s);
     int status = TQ1_OK;
+    if (need >= kWsScratchOffset &&
+        try_gemv_looped(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, false, workspace, s, &status))
+        return status;
     if ((reinterpret_cast<uintptr_t>(blocks) & 15) == 0 &&
         try_gemm_slices(blocks, static_cast<const __half *>(x), y, y_is_f32 != 0, M, N, K, workspace, s, false, &status))
         return status;
@@ -182,9 +183,8 @@ int tq1_linear_swiglu_f16(const uint8_t *blocks, const void *x, void *y, int y_i
         return fail(TQ1_ERR_WORKSPACE, "tq1_linear_swiglu_f16: workspace of %zu bytes (256-byte aligned) required", need);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (gemv) return launch_gemv_single(blocks, xh, y, y_is_f32 != 0, rows, K, true, workspace, kWsSlotRegionBytes, s);
-    if (gemv_looped_fits(blocks, M, rows, K))
-        return launch_gemv_looped(blocks, xh, y, y_is_f32 != 0, M, rows, K, true, workspace, s);
     int status = TQ1_OK;
+    if (try_gemv_looped(blocks, xh, y, y_is_f32 != 0, M, rows, K, true, workspace, s, &status)) return status;
     if (try_gemm_slices(blocks, xh, y, y_is_f32 != 0, M, rows, K, workspace, s, true, &status)) return status;
     return launch_gemm_tc(blocks, xh, y, y_is_f32 != 0, M, rows, K, workspace, s, true);
 }
@@ -193,8 +193,8 @@ int tq1_linear_plan(int M, int N, int K, int aligned, int *kernel, int *token_ti
     if (!kernel || !token_tile || !ctas || !parts) return fail(TQ1_ERR_INVALID, "tq1_linear_plan: null pointer");
     if (M <= 0 || N <= 0 || K <= 0 || K % kGroup) return fail(TQ1_ERR_INVALID, "tq1_linear_plan: bad shape");
     *token_tile = *ctas = *parts = 0;
-    if ((M == 1 || gemv_loop_preferred(M)) && aligned && gemv_chain_shape_ok(N, K)) {
-        *kernel = TQ1_KERNEL_STREAM_GEMV;       // M > 1: one launch of M passes of the batch-1 kernel
+    if (aligned && (M == 1 ? gemv_chain_shape_ok(N, K) : gemv_looped_shape_ok(M, N, K))) {
+        *kernel = TQ1_KERNEL_STREAM_GEMV;       // the tile kernel or the chain kernel
     } else if (aligned && gemm_tc_shape_ok(M, N, K)) {
         *kernel = TQ1_KERNEL_TENSOR_CORE;
         gemm_tc_plan(M, N, K, token_tile, ctas, parts);

@@ -154,11 +154,11 @@ bool gemv_chain_supported(const uint8_t *blocks, int N, int K);
 bool gemv_chain_fits(const uint8_t *blocks, int N, int K);      // also checks the current device's SM count
 size_t gemv_chain_workspace_bytes(int N, int K);
 size_t gemv_chain_workspace_bound(int N, int K);                // for this matrix and every smaller one
-// a few activation rows as M links of one launch over the same weights
-bool gemv_looped_fits(const uint8_t *blocks, int M, int N, int K);
-int launch_gemv_looped(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, bool swiglu,
-                       void *workspace, cudaStream_t stream);
-bool gemv_loop_preferred(int M);
+// Two activation rows as exact sums too (more while a sweep is recorded): by the tile kernel, or as M links of one launch over the same
+// weights. Launches it (`status` is what came of that) and returns true where one of them takes the call.
+bool gemv_looped_shape_ok(int M, int N, int K);
+bool try_gemv_looped(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, bool swiglu, void *workspace,
+                     cudaStream_t stream, int *status);
 int gemv_set_loop_tokens(int tokens);       // sweep recording only; process-global
 // slot_bytes: room for partial-sum slots behind the workspace's control words
 int launch_gemv_single(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int N, int K, bool swiglu,

@@ -1096,14 +1096,11 @@ int launch_gemv_single(const uint8_t *blocks, const __half *x, void *y, bool y_f
 }
 
 
-// Two activation rows: the tile kernel, else (and for more rows, while a sweep is recorded) one launch of M independent links over
-// the same weights, of which the second and later passes read them from L2.
-int launch_gemv_looped(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, bool swiglu,
-                       void *workspace, cudaStream_t stream) {
-    int rc;
-    if (try_gemv_tiles(blocks, x, y, y_f32, M, N, K, swiglu, workspace, stream, &rc)) return rc;
+// One launch of M independent links over the same weights, of which the second and later passes read them from L2.
+static int launch_gemv_looped(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, bool swiglu,
+                              void *workspace, cudaStream_t stream) {
     int grid = 0;
-    rc = gemv_chain_grid(&grid);
+    int rc = gemv_chain_grid(&grid);
     if (rc != TQ1_OK) return rc;
     if (M < 1 || M > kInlineLinks) return fail(TQ1_ERR_INVALID, "tq1 chain: %d activation rows do not fit one launch", M);
     tq1_chain_link links[kInlineLinks];
@@ -1123,24 +1120,36 @@ int launch_gemv_looped(const uint8_t *blocks, const __half *x, void *y, bool y_f
                              kRegionSlotsTwo, 2, stream);
 }
 
-// Largest M that tq1_linear_f16 sends through launch_gemv_looped (0 or 1: none). Every matrix that the batch-1 kernel takes
-// goes this way, because its sums are exact integers per group: two tokens of 5120x5120 are 7e-8 from the FP64 result
+// Largest M that goes through try_gemv_looped (0 or 1: none): two rows by the tile kernel or as two links of the chain kernel, whichever
+// fits and is faster, because their sums are exact integers per group: two tokens of 5120x5120 are 7e-8 from the FP64 result
 // (2-norm) against 1.2e-6 of the batched kernel's FP32 accumulators. Two tokens, weights out of HBM, the tile kernel, two links of
 // the chain kernel and the batched kernel: 1024x5120 4.8, 8.9 and 9.7 us, 5120x5120 9.0, 11.6 and 10.8, 17408x5120 14.7, 19.0 and 17.9.
+// Where two links' slots do not fit, the tile and the batched kernel: 151936x5120 76.7 and 89.7, 60000x10240 61 and 75, 151936x6144
+// 108.7 and 106.7. The batched kernel takes what has neither: more than 1 Mi rows x chunks and a width of more than 10240 columns that
+// not_behind_chain (tq1_gemv_tiles.cu) is against.
 static int g_loop_tokens = 2;
-bool gemv_loop_preferred(int M) { return M >= 2 && M <= g_loop_tokens; }
+static bool gemv_loop_preferred(int M) { return M >= 2 && M <= g_loop_tokens; }
 int gemv_set_loop_tokens(int tokens) {
     if (tokens < 0 || tokens > kInlineLinks) return TQ1_ERR_INVALID;
     g_loop_tokens = tokens;
     return TQ1_OK;
 }
-// The looped path takes the shape when one link holds the whole matrix in one slot region of the two.
-bool gemv_looped_fits(const uint8_t *blocks, int M, int N, int K) {
+// Links of one launch take a matrix that fits one slot region of the two.
+static bool looped_links_fit(int N, int K) {
+    return rows_per_link(N, K, kRegionSlotsTwo) == N && span_ok((N + kTileRows - 1) / kTileRows, K / kChunkCols, sm_count());
+}
+bool gemv_looped_shape_ok(int M, int N, int K) {
+    if (!gemv_loop_preferred(M) || !gemv_chain_shape_ok(N, K)) return false;
+    CallLayout tiles;
+    return looped_links_fit(N, K) || (gemv_tiles_layout(M, N, K, nullptr, &tiles) && tiles.preferred);
+}
+bool try_gemv_looped(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, bool swiglu, void *workspace,
+                     cudaStream_t stream, int *status) {
     if (!gemv_loop_preferred(M) || !gemv_chain_supported(blocks, N, K)) return false;
-    int grid = 0;
-    if (gemv_chain_grid(&grid) != TQ1_OK) return false;
-    if (rows_per_link(N, K, kRegionSlotsTwo) != N) return false;
-    return span_ok((N + kTileRows - 1) / kTileRows, K / kChunkCols, grid);
+    if (try_gemv_tiles(blocks, x, y, y_f32, M, N, K, swiglu, workspace, stream, status)) return true;
+    if (!looped_links_fit(N, K)) return false;
+    *status = launch_gemv_looped(blocks, x, y, y_f32, M, N, K, swiglu, workspace, stream);
+    return true;
 }
 
 // Whether the chain kernel takes one product of this shape on the current device.

@@ -58,6 +58,13 @@ def test_two_rows_of_any_matrix_take_the_exact_kernel():
         assert plan(2, rows, columns).kernel == "stream_gemv"
 
 
+def test_two_rows_that_neither_exact_kernel_takes_are_planned_as_they_run():
+    """More rows than two links have slots for: the tile kernel, where it has room for the columns; else the batched one."""
+    assert plan(2, 151936, 5120).kernel == "stream_gemv"
+    assert plan(2, 9008, 65536).kernel == plan(2, 9008, 65536).form.replace("tcgen05", "tensor_core") == "tensor_core"
+    assert plan(2, 8192, 65536).kernel == plan(1, 9008, 65536).kernel == "stream_gemv"
+
+
 def test_rule_between_the_forms_of_the_group_sums():
     """The line is drawn by times behind another kernel, where the tcgen05 form begins 1 to 2 us later than it does in the recorded
     rows of calls: up to 20% of the shortest calls (383 rows), 10% of the others."""

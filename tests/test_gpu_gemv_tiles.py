@@ -67,6 +67,22 @@ def test_stages_that_are_filled_again(rows, columns, batch):
         assert torch.equal(tq1_matmul(blocks, x, out_dtype=torch.float32), want)
 
 
+@pytest.mark.parametrize(("rows", "columns"), ((151936, 5120), (60000, 10240)))
+def test_two_rows_of_more_than_two_links_have_slots_for(rows, columns):
+    from ternel_b200.dispatch import plan
+    from ternel_b200.ops import tq1_matmul, tq1_swiglu
+    from ternel_b200.stack import random_blocks_device
+    assert plan(2, rows, columns).kernel == "stream_gemv"
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(rows)
+    blocks = random_blocks_device(rows, columns, gen, "cuda")
+    x = torch.randn((2, columns), generator=gen, device="cuda").to(torch.float16)
+    for call in (tq1_matmul, tq1_swiglu):
+        both = call(blocks, x, out_dtype=torch.float32)
+        for m in range(2):
+            assert torch.equal(both[m:m + 1], call(blocks, x[m:m + 1], out_dtype=torch.float32))
+
+
 @pytest.mark.parametrize("value", (np.inf, -np.inf, np.nan))
 @pytest.mark.parametrize(("rows", "columns"), ((70, 1024), (40, 10240)))
 def test_non_finite_groups(rows, columns, value):
