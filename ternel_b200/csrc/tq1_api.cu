@@ -48,6 +48,13 @@ cudaError_t tq1::opt_in(KernelRecord &record, const void *kernel, size_t smem, b
     return err;
 }
 
+// What is made of the driver's answer: it says 0 of a size that this device cannot run, and nothing on a machine without one, where
+// calls are planned only.
+static int cluster_count(bool answered, int n, bool device, int size) {
+    static const int of_b200[kMaxCluster + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15, 14, 14, 8, 8, 8, 8, 8, 8};
+    return answered ? n : device ? 0 : of_b200[size];
+}
+
 int tq1::clusters_at_once(KernelRecord &record, const void *kernel, unsigned threads, size_t smem, int size) {
     if (size == 1) return sm_count();
     std::atomic<int> &known = record.clusters[device_slot()][size];
@@ -64,14 +71,17 @@ int tq1::clusters_at_once(KernelRecord &record, const void *kernel, unsigned thr
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         if (size > 8) cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (opt_in(record, kernel, smem) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
-            cudaGetLastError();                                 // no device, say: planning only
-            const int of_b200[kMaxCluster + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15, 14, 14, 8, 8, 8, 8, 8, 8};
-            n = of_b200[size];
+        const bool answered = opt_in(record, kernel, smem) == cudaSuccess && cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess;
+        int devices = 0;
+        if (!answered) {
+            cudaGetLastError();
+            if (cudaGetDeviceCount(&devices) != cudaSuccess) { cudaGetLastError(); devices = 0; }
         }
+        n = cluster_count(answered, n, devices > 0, size);
+        if (n < 1) n = -1;                                      // known to be none
         known.store(n, std::memory_order_relaxed);
     }
-    return n;
+    return n > 0 ? n : 0;
 }
 
 namespace {
@@ -244,7 +254,7 @@ int tq1_debug_linear_as(int form, const uint8_t *blocks, const void *x, void *y,
 }
 
 // Tests only: the layout of a call by the kernel of `form` (TQ1_FORM_STREAM_GEMV: one or two activation rows as a call of their own;
-// TQ1_FORM_SLICES), whether or not the rules would send it there. layout: CTAs of a cluster, sets of warps, ring stages, row tiles of
+// TQ1_FORM_SLICES; TQ1_FORM_TCGEN05, whose sets are the parts of a tile, and which has no ring stages here), whether or not the rules would send it there. layout: CTAs of a cluster, sets of warps, ring stages, row tiles of
 // a cluster, and whether the rules do. All zero: it does not fit that kernel.
 int tq1_debug_call_layout(int form, int M, int N, int K, const int *rooms, int *layout) {
     if (!layout || M <= 0 || N <= 0 || K <= 0 || K % kGroup) return fail(TQ1_ERR_INVALID, "tq1_debug_call_layout: bad call");
@@ -253,6 +263,8 @@ int tq1_debug_call_layout(int form, int M, int N, int K, const int *rooms, int *
         if (!gemv_tiles_layout(M, N, K, rooms, &l)) l = {};
     } else if (form == TQ1_FORM_SLICES) {
         if (!gemm_slices_layout(M, N, K, rooms, &l)) l = {};
+    } else if (form == TQ1_FORM_TCGEN05) {
+        if (!gemm_tc_layout(M, N, K, rooms, &l)) l = {};
     } else {
         return fail(TQ1_ERR_INVALID, "tq1_debug_call_layout: form %d", form);
     }
@@ -263,6 +275,9 @@ int tq1_debug_call_layout(int form, int M, int N, int K, const int *rooms, int *
     layout[4] = l.preferred;
     return TQ1_OK;
 }
+
+// Tests only.
+int tq1_debug_cluster_count(int answered, int n, int device, int size) { return cluster_count(answered != 0, n, device != 0, size); }
 
 int tq1_debug_force_token_tile(int token_tile) {
     if (gemm_tc_force_tile(token_tile) != TQ1_OK)

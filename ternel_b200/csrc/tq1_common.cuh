@@ -77,7 +77,7 @@ struct KernelRecord {
 // The kernel may have `smem` bytes of dynamic shared memory.
 cudaError_t opt_in(KernelRecord &record, const void *kernel, size_t smem, bool large_clusters = false);
 // Clusters of `size` CTAs of a kernel that run at the same time: fewer than SMs / CTAs where the SMs of a GPC are no
-// multiple of it (with one CTA per SM 74 of 2, 33 of 4 and 15 of 8 on this part).
+// multiple of it (with one CTA per SM 74 of 2, 33 of 4 and 15 of 8 on this part); 0 where none does.
 int clusters_at_once(KernelRecord &record, const void *kernel, unsigned threads, size_t smem, int size);
 
 // A launch may begin while the kernel before it in the stream ends (programmatic dependent launch): that kernel lets it in
@@ -167,7 +167,7 @@ int launch_gemv_single(const uint8_t *blocks, const __half *x, void *y, bool y_f
 // workspace's first word is the status word) and returns true where it takes the call.
 bool try_gemv_tiles(const uint8_t *blocks, const __half *x, void *y, bool y_f32, int M, int N, int K, bool swiglu, void *workspace,
                     cudaStream_t stream, int *status);
-// How a call is laid out by the batch-1 or the slice kernel where that one takes it (tests; launches nothing). rooms: null, or how many clusters of 1, 2, .. kMaxCluster CTAs run at once
+// How a call is laid out by a kernel that takes it (tests; launches nothing). rooms: null, or how many clusters of 1, 2, .. kMaxCluster CTAs run at once
 // (rooms[size]), in place of what the driver says.
 struct CallLayout {
     int cluster;                        // CTAs of a cluster
@@ -176,6 +176,7 @@ struct CallLayout {
 };
 bool gemv_tiles_layout(int M, int N, int K, const int *rooms, CallLayout *layout);
 bool gemm_slices_layout(int M, int N, int K, const int *rooms, CallLayout *layout);
+bool gemm_tc_layout(int M, int N, int K, const int *rooms, CallLayout *layout);      // parts of a tile as sets; 1: no cluster adds them up
 int launch_shard_wait(const ShardDev &shard, unsigned *status, cudaStream_t stream);
 int launch_shard_push(const __half *local, int M, int n_local, const ShardDev &shard, cudaStream_t stream);
 int launch_epoch_advance(unsigned *epoch_base, unsigned delta, cudaStream_t stream);

@@ -992,8 +992,8 @@ Tiling make_tiling(int tile, int M, int N, int K) {
 }
 
 // A tile's parts add up in a cluster.
-bool clustered(int tile, const WorkSplit &w) {
-    return tile <= 128 && w.splits > 1 && w.splits <= kMaxCluster && w.tiles_total <= cluster_room(tile, w.splits);
+bool clustered(int tile, const WorkSplit &w, const int *rooms = nullptr) {
+    return tile <= 128 && w.splits > 1 && w.splits <= kMaxCluster && w.tiles_total <= (rooms ? rooms[w.splits] : cluster_room(tile, w.splits));
 }
 
 // Activation rows per tile. Up to 16 rows always take the 16-row tile. Beyond that the tile with the smallest modelled
@@ -1103,6 +1103,13 @@ void gemm_tc_plan(int M, int N, int K, int *tile, int *ctas, int *parts) {
     *tile = t.tile;
     *ctas = t.ctas();
     *parts = t.work.splits;
+}
+
+bool gemm_tc_layout(int M, int N, int K, const int *rooms, CallLayout *layout) {
+    if (!gemm_tc_shape_ok(M, N, K)) return false;
+    const Tiling t = pick_tiling(M, N, K);
+    *layout = {clustered(t.tile, t.work, rooms) ? t.work.splits : 1, t.work.splits, 0, t.work.tiles_total, true};
+    return true;
 }
 
 bool gemm_tc_shape_ok(int M, int N, int K) { return M >= 2 && N >= 1 && K % (kChunkGroups * kGroup) == 0; }

@@ -401,6 +401,7 @@ TilePlan tile_plan(int tokens, int N, int K, const int *rooms = nullptr) {
         const int hope = (tiles + sm_count() / split - 1) / (sm_count() / split);
         if (best.ok && tile_us(log, set_warps, subsets_for(hope), hope) >= best.us) continue;
         const int room = rooms ? rooms[split] : clusters_at_once(g_records[log > 0][tokens - 1], reinterpret_cast<const void *>(kernel_of(log > 0, tokens)), 32 * kMaxWarps, kWindowEnd - kWindow, 1 << log);
+        if (room < 1) continue;
         p.clusters = tiles < room ? tiles : room;
         const int per = (tiles + p.clusters - 1) / p.clusters;
         p.subsets = subsets_for(per);

@@ -69,7 +69,8 @@ class RingLayout:
 def ring_layout(form: str, batch: int, rows: int, columns: int, *, rooms: "dict[int, int] | None" = None) -> "RingLayout | None":
     """How the kernel that streams row tiles for 1 and 2 activation rows (``"stream_gemv"``) or that for 3 to 16 (``"slices"``) lays out
     a call, whether or not the rules send it there; None where it does not take it (a batch-1 call then is a chain of one link).
-    ``rooms`` replaces what the driver says of how many clusters of a size run at once."""
+    ``"tcgen05"``: the parts of an output tile as ``sets``, and in ``cluster`` the CTAs that add them up, 1 where they meet in the
+    workspace. ``rooms`` replaces what the driver says of how many clusters of a size run at once."""
     ask = _native.lib().tq1_debug_call_layout
     ask.restype, ask.argtypes = ctypes.c_int, [ctypes.c_int] * 4 + [ctypes.c_void_p] * 2
     given = (ctypes.c_int * 17)(*(rooms.get(size, 0) for size in range(17))) if rooms is not None else None

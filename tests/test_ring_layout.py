@@ -40,3 +40,21 @@ def test_wide_matrices_that_the_chain_kernel_is_faster_for(batch, rows, columns)
     (1, 1000, 25600), (1, 9000, 20480), (1, 5000, 40960), (2, 5000, 20480), (2, 1000, 40960)))
 def test_matrices_that_the_tile_kernel_is_faster_for(batch, rows, columns):
     assert ring_layout("stream_gemv", batch, rows, columns).preferred
+
+
+def test_cluster_sizes_that_the_device_cannot_run_are_left_out():
+    """The driver answers 0 of them; only a machine without a device has no answer (calls are planned for a B200 there)."""
+    import ctypes
+    from ternel_b200 import _native
+    count = _native.lib().tq1_debug_cluster_count
+    count.restype, count.argtypes = ctypes.c_int, [ctypes.c_int] * 4
+    assert count(1, 33, 1, 4) == 33 and count(1, 0, 1, 16) == 0         # answered
+    assert count(0, 0, 1, 16) == 0 and count(0, 0, 0, 16) == 8          # an error, with a device and without one
+    none, pairs = {1: 148}, {1: 148, 2: 74}
+    for form, batch in (("stream_gemv", 1), ("slices", 8)):
+        assert ring_layout(form, batch, 1024, 2560, rooms=none).cluster == 1
+        assert ring_layout(form, batch, 5120, 17408).cluster > 1
+        assert ring_layout(form, batch, 5120, 17408, rooms=none) is None
+        assert ring_layout(form, batch, 1024, 10240, rooms=pairs).cluster == 2
+    assert ring_layout("tcgen05", 100, 130, 16384).cluster == 16
+    assert ring_layout("tcgen05", 100, 130, 16384, rooms=none).cluster == 1
