@@ -17,6 +17,11 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+// For a thread of a cluster one of whose waits ran out: until all others have ended or come here too. They may still be writing into
+// this CTA's shared memory, which is gone when its threads have ended (their own waits have a limit as well).
+__device__ __forceinline__ void stay_with_cluster() {
+    asm volatile("barrier.cluster.arrive.relaxed;\n\tbarrier.cluster.wait;" ::: "memory");
+}
 // One lane of a converged warp. Branching on it (and not on the lane number) tells the compiler that a single thread
 // runs the branch, so the operands of tcgen05.mma stay in uniform registers: 25 clocks per MMA issued instead of 134
 // (a loop over the lanes that might hold different operands), which had paced every token tile below 256.

@@ -446,6 +446,7 @@ slices_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             total = join4(total);
             if (lane < 8) store_rows(prm, (tile_lo + rank + (own << split_log)) * kTileRows + row, m, total);
         }
+        if (dead) stay_with_cluster();
     }
 }
 

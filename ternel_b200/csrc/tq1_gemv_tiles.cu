@@ -338,12 +338,13 @@ tiles_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ T
     }
     if (dead)                                                   // a wait ran out: give the copies still in flight time to land
         for (int i = 0; i < 64; ++i) __nanosleep(20000);
-    if (SPLIT) {                                                // the cluster's sums of this CTA's tiles; nobody writes here later
+    if (SPLIT) {                                                // the cluster's sums of this CTA's tiles; when they are there nobody writes here any more
         const float *sums = reinterpret_cast<const float *>(at(prm.sums_addr));
         for (int j = warp; j < own_tiles * TOKENS; j += warps) {
             mbar_wait(tile_bar(j / TOKENS), 0, prm.status, dead);
             finish_tile<TOKENS>(prm, sums + (size_t)j * prm.chunks * kTileRows, tile_lo + rank + (j / TOKENS << split_log), j % TOKENS, lane);
         }
+        if (dead) stay_with_cluster();
     }
 }
 
