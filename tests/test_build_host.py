@@ -1,6 +1,8 @@
 """When the eager call path is built again (host code only)."""
 
 import os
+import shutil
+import subprocess
 
 import pytest
 
@@ -33,3 +35,14 @@ def test_another_pytorch_or_a_newer_source_makes_it_stale(monkeypatch, tmp_path)
     assert build.binding_is_stale()
     with pytest.raises(_native.NativeLibraryMissing, match="torch 1.0"):
         _native.binding()
+
+
+def test_host_functions_begin_on_a_cache_line():
+    """What packs blocks loses a tenth and more where it does not."""
+    if not shutil.which("nm"):
+        pytest.skip("no nm")
+    listed = subprocess.run(["nm", str(build.LIB_PATH)], capture_output=True, text=True, check=True).stdout.splitlines()
+    codec = [line.split() for line in listed if "checked_parts" in line and "_M_run" in line or line.endswith(" T tq1_pack_blocks")]
+    assert len(codec) >= 2
+    for address, _, name in codec:
+        assert int(address, 16) % 64 == 0, (address, name)
