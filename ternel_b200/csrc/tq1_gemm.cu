@@ -376,6 +376,20 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         if (V::WIDE) bulk_load(wbase + V::kTableAddr, &g_wide, V::kTableBytes, bar(TAB));
         else bulk_load(wbase + V::kTableAddr, &g_narrow, V::kTableBytes, bar(TAB));
     }
+    if (warp == kMmaWarp) {
+        const uint32_t where = wbase + V::kBarAddr + 1008;
+        if (CG == 2) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(where), "r"((uint32_t)V::kTmemCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(where), "r"((uint32_t)V::kTmemCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
+        // The next kernel in the stream may start its own set-up from now on: not before this CTA has its tensor memory (a CTA of that
+        // kernel beside it could take it, and waits for this kernel), and no later: beside another stream's kernels a launch that
+        // comes after what is set up below finds no SM for longer (48 tokens of 5120x17408 beside elementwise kernels 99 us, now 81).
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     // The segments, and for a decode warp the packed bytes that it requests ahead of its decoding: the walks are set up and the
     // first bytes brought to L2 (a hint, whatever they hold by now) while earlier kernels run. Behind the wait below this
     // took 4700 clocks up to the first decoded byte, now 2800.
@@ -435,16 +449,6 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         __syncwarp();
     }
     if (warp == kXWarp && elect_one()) asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");
-    if (warp == kMmaWarp) {
-        const uint32_t where = wbase + V::kBarAddr + 1008;
-        if (CG == 2) {
-            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(where), "r"((uint32_t)V::kTmemCols) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-        } else {
-            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(where), "r"((uint32_t)V::kTmemCols) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        }
-    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     if (CG == 2) {
         asm volatile("barrier.cluster.arrive.release;" ::: "memory");
@@ -454,9 +458,7 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
     }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
-    // The next kernel in the stream may start its own set-up; everything below touches memory that earlier kernels
-    // may have written or may still read.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // everything below touches memory that earlier kernels may have written or may still read
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     bool dead = false;
