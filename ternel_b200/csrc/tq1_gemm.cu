@@ -443,7 +443,7 @@ tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         }
     };
     if (warp < kDecode) {
-        if (seek() && elect_one())
+        if (seek() && packed_row() < prm.N && elect_one())          // rows past the end are filled in, not fetched
             asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];"
                          ::"l"(&wmap), "r"((p_c0 + p_unit) * kChunkBytes), "r"(packed_row()) : "memory");
         __syncwarp();
