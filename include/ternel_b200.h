@@ -174,7 +174,7 @@ int tq1_linear_swiglu_f16(const uint8_t *blocks, const void *x, void *y, int y_i
 #define TQ1_KERNEL_TENSOR_CORE 2
 #define TQ1_KERNEL_GROUP_SUMS 3
 #define TQ1_FORM_ROWS 0
-#define TQ1_FORM_STREAM_GEMV 1
+#define TQ1_FORM_STREAM_GEMV 1          /* exact sums: a call of its own, or (wide matrices) links of the chain kernel */
 #define TQ1_FORM_TCGEN05 2              /* of TQ1_KERNEL_TENSOR_CORE */
 #define TQ1_FORM_SLICES 3               /* of TQ1_KERNEL_TENSOR_CORE: mma.sync out of registers, 3 to 16 rows */
 #define TQ1_FORM_GROUPS_FEW 4           /* of TQ1_KERNEL_GROUP_SUMS: mma.sync, 16 weight rows a CTA */

@@ -44,7 +44,8 @@ class LinearPlan:
     ctas: int
     parts: int           # equal K parts per tile, 0 = stream-K ranges
     form: str            # the kernel that runs, one of FORMS: "slices" takes some of "tensor_core"'s calls of up to 16 rows
-                         # (the tile, CTAs and parts are the tcgen05 kernel's), and "group_sums" has three
+                         # (the tile, CTAs and parts are the tcgen05 kernel's), and "group_sums" has three. ring_layout() tells the
+                         # two kernels of "stream_gemv" apart, and how the tcgen05 kernel's parts are added up
 
 
 def plan(batch: int, rows: int, columns: int, *, aligned: bool = True, workspace: bool = True) -> LinearPlan:

@@ -185,6 +185,7 @@ SMALL_CASE_MODULES = [
     "tests/test_gpu_chain.py", "tests/test_gpu_linear.py", "tests/test_gpu_swiglu.py", "tests/test_gpu_embedding.py",
     "tests/test_gpu_gemv_stream.py", "tests/test_gpu_gemm.py", "tests/test_gpu_sharded.py", "tests/test_gpu_loaders.py",
     "tests/test_gpu_slices.py", "tests/test_gpu_groups_tcgen05.py", "tests/test_gpu_dependent_launches.py",
+    "tests/test_gpu_gemv_tiles.py",
 ]
 
 

@@ -253,19 +253,21 @@ def test_segments_that_follow_one_another(columns):
                                    rtol=2e-6, atol=1e-30)
 
 
-@pytest.mark.parametrize(("rows", "columns"), ((50, 2048), (130, 4608), (1001, 5120), (2046, 17408), (5120, 8704)))
+@pytest.mark.parametrize(("rows", "columns"), ((50, 2048), (130, 4608), (1001, 5120), (2046, 17408), (5120, 8704),
+                                               (130, 9728), (130, 12288), (130, 16384)))
 def test_parts_that_a_cluster_adds(rows, columns):
-    """Tiles cut into two to nine equal parts, with rows past the last whole quad, and columns that the CTAs of a cluster do not
-    share evenly. Whole numbers, so every sum is exact."""
-    from ternel_b200.dispatch import plan
+    """Tiles cut into two to sixteen equal parts (more than eight CTAs a cluster have to be asked for), with rows past the last whole
+    quad, and columns that the CTAs of a cluster do not share evenly. Whole numbers, so every sum is exact. Many parts of sixteen
+    tiles are more clusters than run at once: these meet in the workspace."""
+    from ternel_b200.dispatch import ring_layout
     from ternel_b200.ops import tq1_matmul, tq1_swiglu
     rng = np.random.default_rng(rows)
     trits = rng.integers(0, 3, size=(rows * columns // 128, 128), dtype=np.uint8)
     blocks = to_dev(o.encode_blocks(ones_scale(rows * columns // 128), trits).reshape(rows, columns // 128, 28))
     dense = to_dev(trits.reshape(rows, columns)).float() - 1
-    parts = set()
     for batch in (17, 29, 47, 100, 128):
-        parts.add(plan(batch, rows, columns).parts)
+        layout = ring_layout("tcgen05", batch, rows, columns)
+        assert layout.sets > 1 and layout.cluster in ((1, layout.sets) if columns == 17408 else (layout.sets,))
         x = torch.randint(-1, 2, (batch, columns), device="cuda").to(torch.float16)
         want = x.float() @ dense.T
         assert torch.equal(tq1_matmul(blocks, x, out_dtype=torch.float32), want)
@@ -273,4 +275,3 @@ def test_parts_that_a_cluster_adds(rows, columns):
         if rows % 2 == 0:
             torch.testing.assert_close(tq1_swiglu(blocks, x, out_dtype=torch.float32),
                                        torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2], rtol=2e-6, atol=1e-30)
-    assert parts & set(range(2, 17))

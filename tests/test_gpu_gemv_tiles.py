@@ -10,10 +10,10 @@ from tests.gpu_util import random_blocks, to_dev
 pytestmark = pytest.mark.gpu
 
 # (rows, columns): one row, tile remainders, twenty sets of one chunk and fewer; the widest K range of one CTA (18 chunks), and
-# clusters of two (19 chunks: uneven halves, 34), four (two activation rows of 34) and eight (128 chunks: the most); several tiles
-# per set, more tiles than ring stages
+# clusters of four (19 and 34 chunks: parts of unequal length) and eight (80 chunks, the most for two activation rows, and 128,
+# where two rows are links of the chain kernel); several tiles per set
 SHAPES = ((1, 512), (15, 512), (2375, 512), (50002, 512), (33, 1536), (4100, 4096), (12018, 5120), (2400, 9216), (2390, 9728),
-          (1202, 17408), (49, 65536))
+          (1202, 17408), (49, 40960), (49, 65536))
 
 
 def single_links(blocks, x, swiglu):
@@ -28,7 +28,11 @@ def single_links(blocks, x, swiglu):
 
 @pytest.mark.parametrize(("rows", "columns"), SHAPES)
 def test_equals_the_chain_kernel(rows, columns):
+    from ternel_b200.dispatch import ring_layout
     from ternel_b200.ops import tq1_matmul, tq1_swiglu
+    for batch in (1, 2):
+        layout = ring_layout("stream_gemv", batch, rows, columns)
+        assert layout is None if (batch, columns) == (2, 65536) else layout.preferred
     host, rng = random_blocks(rows, columns, seed=rows + columns, dist="tests")
     blocks = to_dev(host)
     x = to_dev(rng.standard_normal((2, columns)).astype(np.float16))
