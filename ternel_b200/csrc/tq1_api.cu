@@ -254,8 +254,9 @@ int tq1_debug_linear_as(int form, const uint8_t *blocks, const void *x, void *y,
 }
 
 // Tests only: the layout of a call by the kernel of `form` (TQ1_FORM_STREAM_GEMV: one or two activation rows as a call of their own;
-// TQ1_FORM_SLICES; TQ1_FORM_TCGEN05, whose sets are the parts of a tile, and which has no ring stages here), whether or not the rules would send it there. layout: CTAs of a cluster, sets of warps, ring stages, row tiles of
-// a cluster, and whether the rules do. All zero: it does not fit that kernel.
+// TQ1_FORM_SLICES; TQ1_FORM_TCGEN05, whose sets are the parts of a tile, and which has no ring stages here), whether or not the rules
+// would send it there. layout: CTAs of a cluster, sets of warps, ring stages, row tiles of a cluster, and whether the rules do. All
+// zero: it does not fit that kernel.
 int tq1_debug_call_layout(int form, int M, int N, int K, const int *rooms, int *layout) {
     if (!layout || M <= 0 || N <= 0 || K <= 0 || K % kGroup) return fail(TQ1_ERR_INVALID, "tq1_debug_call_layout: bad call");
     CallLayout l = {};

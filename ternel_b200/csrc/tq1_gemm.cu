@@ -329,9 +329,12 @@ struct GemmParams {
 // GATED: the rows are (gate, up) pairs. A kernel of its own: the gates' code in the common one cost 3% of long prompts (777 tokens
 // of 34816x5120 without gates 204 us, 199 apart) and 7% of the shortest calls (17 of 1000x1024 5.8 us, 5.4).
 // CLUSTERED: every tile is cut into equal parts, and the CTAs of a cluster, one for each, add them through distributed shared
-// memory. Through the workspace a part's way out, the count and the sum by the last CTA took 4 us of the 8.4 that 20 tokens of
-// 4096x4096 took, now 7.2; 100 of 1024x5120 9.6 and 7.8, 66 rows with gates of 129 tokens 9.8 and 7.4, 48 of 5120x17408 20.8 and 20.4. A kernel of its own too: addresses of a CTA in a cluster take a register, for which only the walk
-// over several segments makes room (64 tokens of 17408x5120 as one kernel 21.3 -> 23.4 us).
+// memory. Through the workspace a part's way out, the count and the sum by the last CTA took 4 us of a call. The same build with the
+// parts in the workspace and in a cluster, calls in a row (us): 20 tokens of 4096x4096 8.4 and 7.4, 100 of 1024x5120 9.4 and 7.9, 129 of
+// 66x5120 8.7 and 6.9, 100 of 130x12288 12.0 and 8.0, 48 of 5120x17408 19.8 and 19.9. Beside another stream's kernels a cluster waits
+// until a GPC has room for all of it: with 4096^3 products of bf16 there the five calls take 38 and 55, 26 and 40, 10 and 11, 18 and 39,
+// 68 and 70 us. A kernel of its own too: addresses of a CTA in a cluster take a register, for which only the walk over several
+// segments makes room (64 tokens of 17408x5120 as one kernel 21.3 -> 23.4 us).
 template <class V, bool GATED, bool CLUSTERED>
 __global__ void __launch_bounds__(V::kThreads, V::kMinCtas)
 tq1_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
@@ -998,12 +1001,12 @@ bool clustered(int tile, const WorkSplit &w, const int *rooms = nullptr) {
     return tile <= 128 && w.splits > 1 && w.splits <= kMaxCluster && w.tiles_total <= (rooms ? rooms[w.splits] : cluster_room(tile, w.splits));
 }
 
-// Activation rows per tile. Up to 16 rows always take the 16-row tile. Beyond that the tile with the smallest modelled
-// time wins: launch and pipeline fill, chunks a slot works through (decode, plus products per token), segments it stores,
-// and the sums of shared tiles. The constants (us) are fitted to the recorded sweep in
-// ternel_b200/dispatch_sweep_b200.json; tests replay the file (the choice is within 10% of the best recorded tile for every
-// case), which was made when the parts of a tile met in the workspace. The choice has been kept since: it also says how many columns an
-// accumulator covers, and with them the error. g_forced_tile overrides the rule while a sweep is being recorded.
+// Activation rows per tile. Up to 16 rows always take the 16-row tile. Beyond that the choice is one of error as much as of time: it
+// says how many columns an accumulator covers. It was made for time, when the parts of a tile met in the workspace: the smallest modelled
+// time of launch and pipeline fill, chunks a slot works through (decode, plus products per token), segments it stores, and the sums of
+// shared tiles, with constants (us) fitted to the sweep of that form in ternel_b200/dispatch_sweep_b200.json, which tests replay (within
+// 10% of the best recorded tile for every case). The times have changed since and the choice has not: the tiles that would be the
+// fastest now, by up to 1.7 times, have longer accumulators. g_forced_tile overrides the rule while a sweep is being recorded.
 int g_forced_tile = 0;
 struct TileCost { int tile; float fixed, chunk, chunk_token, segment, shared_token; };
 const TileCost g_tile_costs[5] = {{16, 2.932f, 0.0f, 0.1263f, 1.968f, 0.1093f},
@@ -1087,9 +1090,9 @@ int gemm_tc_force_tile(int nt) {
 
 bool gemm_tc_forced() { return g_forced_tile != 0; }
 
-// What draws the line between this kernel and the slice kernel, whose sums have a third to a tenth of the error: fitted to 1022 calls
-// behind another kernel when parts still met in the workspace, and kept. (Since a cluster adds them this kernel would be the faster
-// one for 39 of 380 calls of nine to sixteen tokens that the line leaves to the other, by 11% on average.)
+// What draws the line between this kernel and the slice kernel, whose sums have a third to a tenth of the error: times fitted to 1022
+// calls behind another kernel when parts still met in the workspace. The line is kept for the error: since a cluster adds the parts this
+// kernel would be the faster one for 39 of 380 calls of nine to sixteen tokens that are left to the other, by 11% on average.
 float gemm_tc_few_us(int N, int K) {
     const Tiling t = make_tiling(16, 16, N, K);
     const WorkSplit &w = t.work;

@@ -485,7 +485,8 @@ SlicePlan slice_plan(int nt, int N, int K, const int *rooms = nullptr) {
         if (halves < split || p.slices > kMaxSlices) continue;
         // how many clusters run at once is asked of the driver (milliseconds, the first time) only where this split could win
         if (best.ok && slice_us(split, p.slices, (tiles + sm_count() / split - 1) / (sm_count() / split)) >= best.us) continue;
-        const int room = rooms ? rooms[split] : clusters_at_once(g_records[nt - 1], kernel_of(nt), 32 * (kMaxSlices + kExtraWarps), kWindowEnd - kWindow, 1 << log);
+        const int room = rooms ? rooms[split] : clusters_at_once(g_records[nt - 1], kernel_of(nt), 32 * (kMaxSlices + kExtraWarps),
+                                                                 kWindowEnd - kWindow, split);
         if (room < 1) continue;
         p.clusters = tiles < room ? tiles : room;
         const int per_cluster = (tiles + p.clusters - 1) / p.clusters;
