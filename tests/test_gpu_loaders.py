@@ -180,6 +180,16 @@ def test_load_tiled_under_a_default_device(monkeypatch, device):
     assert staged == [True] and np.array_equal(module.blocks.cpu().numpy(), blocks)
 
 
+@pytest.mark.parametrize(("rows", "columns", "staged"), ((48, 512, 0), (192, 1280, 0), (496, 640, 1)))
+def test_small_arrays_are_not_staged(monkeypatch, rows, columns, staged):
+    """Below 64 KiB the driver's own way is the faster one."""
+    module, blocks, tiled = _tiled_module(rows, columns, 8)
+    empty, pinned = torch.empty, []
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: (pinned.append(a) if k.get("pin_memory") else None, empty(*a, **k))[1])
+    module.load_tiled(*tiled)
+    assert len(pinned) == staged and np.array_equal(module.blocks.cpu().numpy(), blocks)
+
+
 @pytest.mark.parametrize("fails", (False, True))
 def test_staging_is_held_until_its_transfers_are_done(monkeypatch, fails):
     """The pool of pinned memory does not know of them: the staging goes back to it after the stream has been waited for."""
